@@ -540,13 +540,20 @@ class BatchEngine {
     // Merge vertices of both trees, ascending id (the job's CP-block scratch
     // is free once the analysis is done).
     const int N = J.dim.N;
-    int* cand = static_cast<int*>(scratch((size_t)2 * N * sizeof(int) + 256));
+    // The two lists, then the component table and the membership words.
+    const size_t cand_bytes = ((size_t)2 * N * sizeof(int) + 255) & ~size_t(255);
+    const size_t member_words = (size_t)2 * jh.nb * (kCpBlock / 32);
+    int* cand = static_cast<int*>(scratch(cand_bytes + (kMergeWords + member_words) * 4));
     if (!cand) return EXTREMZ_OOM;
+    unsigned* table = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(cand) + cand_bytes);
+    unsigned* member = table + kMergeWords;
     int* ctot = J.ctr + C_CAND;  // two free counter slots of the finished job
-    launch(K_OTHER, k_pp_cand_count<T>, jh.nb, kCpBlock, J.f, J.dim, jh.bcount);
+    launch(K_OTHER, k_pp_merge_table, kMergeWords * 32 / 256, 256, table);
+    launch(K_OTHER, k_pp_cand_count<T>, jh.nb, kCpBlock, J.f, J.dim, (const unsigned*)table, member,
+           jh.bcount);
     launch(K_OTHER, k_scan_lists, 1, 1024, jh.bcount, jh.nb, 2, ctot);
-    launch(K_OTHER, k_pp_cand_write<T>, jh.nb, kCpBlock, J.f, J.dim, (const int*)jh.bcount, cand,
-           cand + N);
+    launch(K_OTHER, k_pp_cand_write, dim3((jh.nb + 7) / 8, 2), 256, (const unsigned*)member, jh.nb,
+           (const int*)jh.bcount, cand, cand + N);
     int ns[2];
     EZ_CHECK(cudaMemcpyAsync(ns, ctot, sizeof(ns), cudaMemcpyDeviceToHost, st_));
     EZ_CHECK(cudaStreamSynchronize(st_));

@@ -61,12 +61,25 @@ __device__ __forceinline__ int link_comps(int nodes) {
   return comps;
 }
 
+// Which of the 2^14 sets of link vertices fall into two or more components, one
+// bit per set (kMergeWords words, 2 KB).  Flooding the link at every voxel took
+// 17 ms per pass of a 160x144x128 field; the sets are few, so each call floods
+// each set once (a few microseconds) and a voxel's test is a bit in shared
+// memory.
+constexpr int kMergeWords = (1 << kNumDirs) / 32;
+__global__ void __launch_bounds__(256) k_pp_merge_table(unsigned* __restrict__ table) {
+  const int set = blockIdx.x * 256 + threadIdx.x;
+  const unsigned m = __ballot_sync(0xffffffffu, link_comps(set) >= 2);
+  if (lane_id() == 0) table[set >> 5] = m;
+}
+
 // Merge vertices of the two trees, from the link itself rather than the
 // lookup table (which has no entries for grids thinner than 3 voxels): bit 0
 // when the upper link (split tree) has two or more components, bit 1 when the
 // lower link (join tree) has.
 template <class T>
-__device__ __forceinline__ int merge_bits(const T* __restrict__ a, const Dims& g, int v) {
+__device__ __forceinline__ int merge_bits(const T* __restrict__ a, const Dims& g, int v,
+                                          const unsigned* table) {
   int x, y, z;
   coords(v, g, x, y, z);
   const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
@@ -78,58 +91,54 @@ __device__ __forceinline__ int merge_bits(const T* __restrict__ a, const Dims& g
     const int u = v + dir_x(d) + dir_y(d) * g.W + dir_z(d) * g.W * g.H;
     if (above(a[u], u, c, v)) up |= 1 << d;
   }
-  return (link_comps(up) >= 2 ? 1 : 0) | (link_comps(valid & ~up) >= 2 ? 2 : 0);
+  const int lo = valid & ~up;
+  return (int)(table[up >> 5] >> (up & 31) & 1u) | (int)(table[lo >> 5] >> (lo & 31) & 1u) << 1;
 }
 
 // Ordered compaction of the merge vertices (split list 0, join list 1): block
-// counts, then (after k_scan_lists) the writes in ascending id.
+// counts with each warp's membership words (list l's word of ids 32w .. 32w+31
+// at member[l * kCpBlock / 32 * blocks + w]), then (after k_scan_lists) the
+// writes in ascending id from those words: the field is read once.
 template <class T>
 __global__ void __launch_bounds__(kCpBlock) k_pp_cand_count(const T* __restrict__ a, Dims g,
+                                                            const unsigned* __restrict__ table,
+                                                            unsigned* __restrict__ member,
                                                             int* __restrict__ bcount) {
+  __shared__ unsigned tab[kMergeWords];
   __shared__ int cnt[2];
+  if (threadIdx.x < kMergeWords) tab[threadIdx.x] = table[threadIdx.x];
   if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
   __syncthreads();
   const int v = blockIdx.x * kCpBlock + threadIdx.x;
-  const int b = v < g.N ? merge_bits(a, g, v) : 0;
+  const int b = v < g.N ? merge_bits(a, g, v, tab) : 0;
   for (int l = 0; l < 2; ++l) {
     const unsigned m = __ballot_sync(0xffffffffu, (b >> l) & 1);
-    if (lane_id() == 0 && m) atomicAdd(&cnt[l], __popc(m));
+    if (lane_id() == 0) {
+      member[(l * gridDim.x + blockIdx.x) * (kCpBlock / 32) + threadIdx.x / 32] = m;
+      if (m) atomicAdd(&cnt[l], __popc(m));
+    }
   }
   __syncthreads();
   if (threadIdx.x < 2) bcount[threadIdx.x * gridDim.x + blockIdx.x] = cnt[threadIdx.x];
 }
 
-template <class T>
-__global__ void __launch_bounds__(kCpBlock) k_pp_cand_write(const T* __restrict__ a, Dims g,
-                                                            const int* __restrict__ boff,
-                                                            int* __restrict__ split,
-                                                            int* __restrict__ join) {
-  __shared__ int wcnt[2][32];
-  const int v = blockIdx.x * kCpBlock + threadIdx.x;
-  const int b = v < g.N ? merge_bits(a, g, v) : 0;
-  const unsigned lt = (1u << lane_id()) - 1u;
-  unsigned m[2];
-  for (int l = 0; l < 2; ++l) {
-    m[l] = __ballot_sync(0xffffffffu, (b >> l) & 1);
-    if (lane_id() == 0) wcnt[l][threadIdx.x / 32] = __popc(m[l]);
+// One warp per 1024-id block and list (blockIdx.y): a lane per membership word.
+__global__ void __launch_bounds__(256) k_pp_cand_write(const unsigned* __restrict__ member, int nb,
+                                                       const int* __restrict__ boff,
+                                                       int* __restrict__ split,
+                                                       int* __restrict__ join) {
+  const int b = blockIdx.x * 8 + (int)(threadIdx.x >> 5), l = blockIdx.y;
+  if (b >= nb) return;  // whole warps leave together
+  unsigned m = member[(l * nb + b) * (kCpBlock / 32) + (int)lane_id()];
+  const int c = __popc(m);
+  int incl = c;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane_id() >= (unsigned)o) incl += y;
   }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    for (int l = 0; l < 2; ++l) {
-      const int w = wcnt[l][threadIdx.x];
-      int wi = w;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, wi, o);
-        if (lane_id() >= (unsigned)o) wi += y;
-      }
-      wcnt[l][threadIdx.x] = wi - w;
-    }
-  }
-  __syncthreads();
-  int* outs[2] = {split, join};
-  for (int l = 0; l < 2; ++l)
-    if ((b >> l) & 1)
-      outs[l][boff[l * gridDim.x + blockIdx.x] + wcnt[l][threadIdx.x / 32] + __popc(m[l] & lt)] = v;
+  int pos = boff[l * nb + b] + incl - c;
+  int* out = l ? join : split;
+  for (; m; m &= m - 1) out[pos++] = b * kCpBlock + (int)lane_id() * 32 + __ffs(m) - 1;
 }
 
 // Sort keys: 64-bit order-preserving value key, complemented for a
