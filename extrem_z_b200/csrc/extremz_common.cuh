@@ -113,6 +113,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, long l
   }
   return false;
 }
+// Makes a tensor map that a copy engine or kernel wrote to global memory visible
+// to the tensor-map proxy: an SM may still hold the map that was at the same
+// address before (a slot's maps are rewritten for every job), and a graph
+// launch right behind the copy was seen to load the previous job's field.
+// Needed once per block before its first use of the map.
+__device__ __forceinline__ void tma_map_acquire(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
 // 3-D tiled bulk copy global -> shared.  x must be a multiple of 16 bytes
 // (callers start boxes 4 elements left of a 32-aligned tile origin).
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,

@@ -205,6 +205,7 @@ __device__ __forceinline__ bool load_tile(Tile<T>& s, uint64_t* bar, const CUten
                                           int by, int bz, unsigned parity = 0, bool init = true) {
   if (tma) {
     if (threadIdx.x == 0) {
+      tma_map_acquire(map);
       if (init) mbar_init(bar, 1);
       mbar_expect_tx(bar, (unsigned)sizeof(Tile<T>));
       tma_load_3d(&s.v[0][0][0], map, bx - kXOff, by - 1, bz - 1, bar);
