@@ -104,7 +104,11 @@ constexpr int kFlagTrackEdits = 1 << 28;
 // with the wrong-neighbour arbitration, and the wrong-extremum / wrong-saddle
 // detection of both trees), no edit.
 constexpr int kFlagCensus = 1 << 27;
-constexpr int kInternalFlags = kFlagKeepInput | kFlagAnalysis | kFlagTrackEdits | kFlagCensus;
+// Internal job flag, with kFlagAnalysis: the analysis ends with the types and
+// labels (no critical-point lists).
+constexpr int kFlagLabels = 1 << 26;
+constexpr int kInternalFlags =
+    kFlagKeepInput | kFlagAnalysis | kFlagTrackEdits | kFlagCensus | kFlagLabels;
 
 constexpr long long job_bytes_voxels(long long n, long long ksz) {
   return arr_bytes(n, 1) + arr_bytes(n, 2)                          // otype, olm
@@ -138,6 +142,17 @@ constexpr long long job_bytes_cps(long long ns2, long long ns1, long long nmax, 
          + arr_bytes(nmin + 1, 4) + arr_bytes(e1, 4) + arr_bytes(nmin, 4)
          + 2 * arr_bytes(nmax > nmin ? nmax : nmin, 4)
          + arr_bytes((nmax > nmin ? nmax : nmin) / 1024 + 2, 4) + 4096;
+}
+
+// An analysis job (kFlagAnalysis) takes the original field's types, masks and
+// labels, the extremum index and the CP block counts; then the CP lists.
+constexpr long long job_bytes_analysis(long long n) {
+  return arr_bytes(n, 1) + arr_bytes(n, 2) + 3 * arr_bytes(n, 4)
+         + arr_bytes(6 * ((n + kCpBlock - 1) / kCpBlock), 4)
+         + arr_bytes(6 * ((n + kCpBlock - 1) / kCpBlock / 1024 + 1), 4) + 4096;
+}
+constexpr long long job_bytes_lists(long long ns2, long long ns1, long long nmax, long long nmin) {
+  return arr_bytes(ns2, 4) + arr_bytes(ns1, 4) + arr_bytes(nmax, 4) + arr_bytes(nmin, 4) + 4096;
 }
 
 // Per tile: change mark.
@@ -192,6 +207,14 @@ struct JobHost {
     trace[trace_len++] = b;
     trace[trace_len++] = c3;
   }
+};
+
+// Where an analysis job writes its types and labels when the caller's buffers
+// can be written in place (null: into the workspace).
+struct LabelOut {
+  int8_t* type = nullptr;
+  int* ds = nullptr;
+  int* as = nullptr;
 };
 
 template <class T>
@@ -281,7 +304,8 @@ class BatchEngine {
 
   // Admits a job.  storage: borrowed workspace (nullptr = allocate).
   int admit(const T* f, T* g, int W, int H, int D, const extremz_params& p, int32_t* trace,
-            int trace_cap, Arena* storage, long long tag, int* slot_out) {
+            int trace_cap, Arena* storage, long long tag, int* slot_out,
+            const LabelOut& out = LabelOut()) {
     int slot = -1;
     for (int i = 0; i < kMaxSel; ++i)
       if (!slots_[i].used) {
@@ -318,9 +342,11 @@ class BatchEngine {
     // copy of the incoming field when an edit stream will be encoded).
     const bool keep_input = (p.flags & kFlagKeepInput) != 0;
     const bool track_edits = (p.flags & kFlagTrackEdits) != 0;
+    const bool analysis = (p.flags & kFlagAnalysis) != 0;
     const long long ntiles = (long long)((W + TX - 1) / TX) * ((H + TY - 1) / TY) * ((D + TZ - 1) / TZ);
-    const long long need = (storage ? job_bytes<T>(N)
-                                    : job_bytes_voxels(N, sizeof(K)) + job_bytes_tiles(ntiles)) +
+    const long long need = (storage    ? job_bytes<T>(N)
+                            : analysis ? job_bytes_analysis(N)
+                                       : job_bytes_voxels(N, sizeof(K)) + job_bytes_tiles(ntiles)) +
                            (keep_input ? arr_bytes(N, sizeof(T)) : 0) +
                            (track_edits ? arr_bytes((N + 31) / 32, 4) : 0);
     if (storage) {
@@ -345,51 +371,57 @@ class BatchEngine {
       jh.own_arena = true;
     }
     Arena& A = jh.arena;
-    J.otype = A.take<int8_t>(N);
+    J.otype = out.type ? out.type : A.take<int8_t>(N);
     J.olm = A.take<uint16_t>(N);
-    J.ds = A.take<int>(N);
-    J.as = A.take<int>(N);
-    J.dds = A.take<int>(N);
-    J.das = A.take<int>(N);
+    J.ds = out.ds ? out.ds : A.take<int>(N);
+    J.as = out.as ? out.as : A.take<int>(N);
     J.ext = A.take<int>(N);
-    J.delta = A.take<K>(N);
-    J.counter = A.take<int>(N);
-    J.touched = A.take<int>(N);
-    J.mm = A.take<int>(N);
-    J.mm_next = A.take<int>(N);
-    J.mstat = A.take<uint8_t>(N);
-    J.dirty = A.take<int>(N);
-    J.dstamp = A.take<int>(N);
-    J.rstamp = A.take<int>(N);
-    J.claim = A.take<unsigned long long>(N);
-    J.taken = A.take<int>(N);
-    J.taken1 = A.take<int>(N);
-    J.cand = A.take<int>(N);
-    J.cand_next = A.take<int>(N);
-    J.flagged = A.take<int>(N);
-    J.flagged1 = A.take<int>(N);
-    J.cand_j = A.take<int>(N);
-    J.mis = A.take<uint8_t>(N);
-    J.pdd = A.take<int>(N);
-    J.pda = A.take<int>(N);
-    J.vchg = A.take<unsigned>((N + 31) / 32);
-    J.rtouch2 = A.take<unsigned>((N + 31) / 32);
-    J.rtouch1 = A.take<unsigned>((N + 31) / 32);
-    J.wchg2 = A.take<unsigned>((N + 31) / 32);
-    J.wchg1 = A.take<unsigned>((N + 31) / 32);
-    J.dirtyv = A.take<uint8_t>(N);
     jh.nb = (N + kCpBlock - 1) / kCpBlock;
-    J.bdirty = A.take<int>(jh.nb);
-    J.hcnt = A.take<int>(jh.nb);
     jh.bcount = A.take<int>(6ll * jh.nb);
     jh.chunk = A.take<int>(6ll * ((jh.nb + 1023) / 1024));
     J.cpoff = jh.bcount;
     jh.ntiles = ((W + TX - 1) / TX) * ((H + TY - 1) / TY) * ((D + TZ - 1) / TZ);
-    J.tdirty = A.take<uint8_t>(jh.ntiles);
-
-    J.g0 = keep_input ? A.take<T>(N) : nullptr;
-    J.edited = track_edits ? A.take<unsigned>((N + 31) / 32) : nullptr;
-    if (!J.tdirty || (keep_input && !J.g0) || (track_edits && !J.edited)) {
+    if (!jh.chunk) {
+      free_job(jh);
+      return EXTREMZ_OOM;
+    }
+    // An analysis reads and writes nothing else.
+    if (!analysis) {
+      J.dds = A.take<int>(N);
+      J.das = A.take<int>(N);
+      J.delta = A.take<K>(N);
+      J.counter = A.take<int>(N);
+      J.touched = A.take<int>(N);
+      J.mm = A.take<int>(N);
+      J.mm_next = A.take<int>(N);
+      J.mstat = A.take<uint8_t>(N);
+      J.dirty = A.take<int>(N);
+      J.dstamp = A.take<int>(N);
+      J.rstamp = A.take<int>(N);
+      J.claim = A.take<unsigned long long>(N);
+      J.taken = A.take<int>(N);
+      J.taken1 = A.take<int>(N);
+      J.cand = A.take<int>(N);
+      J.cand_next = A.take<int>(N);
+      J.flagged = A.take<int>(N);
+      J.flagged1 = A.take<int>(N);
+      J.cand_j = A.take<int>(N);
+      J.mis = A.take<uint8_t>(N);
+      J.pdd = A.take<int>(N);
+      J.pda = A.take<int>(N);
+      J.vchg = A.take<unsigned>((N + 31) / 32);
+      J.rtouch2 = A.take<unsigned>((N + 31) / 32);
+      J.rtouch1 = A.take<unsigned>((N + 31) / 32);
+      J.wchg2 = A.take<unsigned>((N + 31) / 32);
+      J.wchg1 = A.take<unsigned>((N + 31) / 32);
+      J.dirtyv = A.take<uint8_t>(N);
+      J.bdirty = A.take<int>(jh.nb);
+      J.hcnt = A.take<int>(jh.nb);
+      J.tdirty = A.take<uint8_t>(jh.ntiles);
+      J.g0 = keep_input ? A.take<T>(N) : nullptr;
+      J.edited = track_edits ? A.take<unsigned>((N + 31) / 32) : nullptr;
+    }
+    if ((!analysis && !J.tdirty) || (keep_input && !J.g0) || (track_edits && !J.edited)) {
       free_job(jh);
       return EXTREMZ_OOM;
     }
@@ -1044,7 +1076,9 @@ class BatchEngine {
   // counts, or the rest of borrowed storage.
   int take_cp_storage(JobHost<T>& jh, int ns2, int ns1, int nmax, int nmin, int e2, int e1) {
     if (!jh.own_arena) return EXTREMZ_OK;  // borrowed: carve from the same arena
-    const long long need = job_bytes_cps(ns2, ns1, nmax, nmin, e2, e1, sizeof(K));
+    const long long need = (jh.p.flags & kFlagAnalysis)
+                               ? job_bytes_lists(ns2, ns1, nmax, nmin)
+                               : job_bytes_cps(ns2, ns1, nmax, nmin, e2, e1, sizeof(K));
     void* base = nullptr;
     const cudaError_t e = pool_mem_ ? cudaMallocFromPoolAsync(&base, (size_t)need, pool_mem_, st_)
                                     : cudaMallocAsync(&base, (size_t)need, st_);
@@ -1093,10 +1127,11 @@ class BatchEngine {
         launch(K_SETUP, k_jump2<T, false>, grid_, 256, jobs, s);
         for (int i : sel) {
           JobHost<T>& j = slots_[i];
+          j.waiting = true;
+          if (j.p.flags & kFlagLabels) continue;
           launch(K_OTHER, k_cp_count, (j.nb + kCpWarps - 1) / kCpWarps, 32 * kCpWarps,
                  (const int8_t*)j.J.otype, (const uint16_t*)j.J.olm, j.J.dim, j.nb, j.bcount);
           EZ_RUN(scan_counts(j.bcount, j.nb, 6, j.J.ctr + C_NS2, j.chunk));
-          j.waiting = true;
         }
         return EXTREMZ_OK;
       case PC_SETUP_B:
@@ -1349,6 +1384,13 @@ class BatchEngine {
     J.sad1 = A.take<int>(ns1);
     J.maxima = A.take<int>(nmax);
     J.minima = A.take<int>(nmin);
+    if (!J.minima) return EXTREMZ_OOM;
+    launch(K_OTHER, k_cp_write, (jh.nb + kCpWarps - 1) / kCpWarps, 32 * kCpWarps,
+           (const int8_t*)J.otype, N, jh.nb, (const int*)jh.bcount,
+           J.sad2, J.sad1, J.maxima, J.minima);
+    launch(K_OTHER, k_ext_index<T>, grid_, 256, J);
+    // The lists and the extremum index are all that an analysis needs.
+    if (jh.p.flags & kFlagAnalysis) return EXTREMZ_OK;
     J.orow2 = A.take<int>((long long)ns2 * kRowStride);
     J.orm2 = A.take<int4>(ns2);
     J.oend2 = A.take<int4>(ns2);
@@ -1383,10 +1425,6 @@ class BatchEngine {
     J.wlong = A.take<int>(ne);
     int* chunk = A.take<int>(ne / 1024 + 2);
     if (!jh.checksum || !J.ext_id || !J.ocnt1 || !J.first_sj || !chunk) return EXTREMZ_OOM;
-    launch(K_OTHER, k_cp_write, (jh.nb + kCpWarps - 1) / kCpWarps, 32 * kCpWarps,
-           (const int8_t*)J.otype, N, jh.nb, (const int*)jh.bcount,
-           J.sad2, J.sad1, J.maxima, J.minima);
-    launch(K_OTHER, k_ext_index<T>, grid_, 256, J);
     // Per side: the rows (with their compact copies, each named extremum's
     // extreme saddle key and entry count), the entry lists' offsets, then the
     // extreme saddle ids and the entries.  The sides share the selection
@@ -1532,7 +1570,8 @@ class BatchEngine {
     JobHost<T>& j = slots_[slot];
     switch (j.pc) {
       case PC_SETUP_A:
-        j.pc = PC_SETUP_B;
+        if (j.p.flags & kFlagLabels) finish(slot, EXTREMZ_OK);
+        else j.pc = PC_SETUP_B;
         return EXTREMZ_OK;
       case PC_CL_DETECT:
       case PC_CL_ROUND:
