@@ -130,6 +130,7 @@ constexpr long long job_bytes_voxels(long long n, long long ksz) {
 constexpr long long job_bytes_cps(long long ns2, long long ns1, long long nmax, long long nmin,
                                   long long e2, long long e1, long long ksz) {
   return arr_bytes(ns2, 4) + arr_bytes(ns1, 4) + arr_bytes(nmax, 4) + arr_bytes(nmin, 4)
+         + arr_bytes(ns2, 2)                                        // smask2
          + arr_bytes(ns2 * kRowStride, 4) + arr_bytes(ns2 * 2, 4) + arr_bytes(ns2, 1)
          + arr_bytes(ns1 * kRowStride, 4) + arr_bytes(ns1 * 2, 4) + arr_bytes(ns1, 1)
          + 2 * arr_bytes(ns2, 16) + 2 * arr_bytes(ns1, 16)  // compact rows (orm, oend)
@@ -334,6 +335,7 @@ class BatchEngine {
     J.iter_cap = p.device_iter_cap > 0 ? p.device_iter_cap : J.dim.N + 1;
     J.pass_chunk = p.tune_pass_chunk > 0 ? p.tune_pass_chunk : 4;
     J.wn_lockstep = (p.flags & EXTREMZ_FLAG_WN_ASCENDING) == 0;
+    J.join_rows = p.preserve_join || (p.flags & kFlagCensus);
     jh.blocks_per_sm = p.tune_blocks_per_sm > 0 ? p.tune_blocks_per_sm : 8;
     J.tb = tb_;
     J.ctr = ctr_dev_ + (size_t)slot * C_COUNT;
@@ -1270,11 +1272,22 @@ class BatchEngine {
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
       case PC_SADDLE_J:
-      case PC_FINAL_JOIN:
+      case PC_FINAL_JOIN: {
         ctl(s, OP_SADDLE_JOIN_BEGIN);
-        launch(K_OTHER, k_wis_mark<T, false>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wis_update<T, false>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wis_long<T, false>, 2 * sms_, 256, jobs, s);
+        std::vector<int> lists, once;
+        for (int i : sel) (slots_[i].J.join_rows ? lists : once).push_back(i);
+        if (!lists.empty()) {
+          const Sel ls = make_sel(lists, false);
+          launch(K_OTHER, k_wis_mark<T, false>, grid_, 256, jobs, ls);
+          launch(K_OTHER, k_wis_update<T, false>, grid_, 256, jobs, ls);
+          launch(K_OTHER, k_wis_long<T, false>, 2 * sms_, 256, jobs, ls);
+        }
+        if (!once.empty()) {
+          const Sel os = make_sel(once, false);
+          launch(K_OTHER, k_join_keys<T>, grid_, 256, jobs, os);
+          launch(K_OTHER, k_join_ids<T>, grid_, 256, jobs, os);
+          launch(K_OTHER, k_join_scan<T>, grid_, 256, jobs, os);
+        }
         launch(K_OTHER, k_wis_collect<T, false>, grid_, 256, jobs, s, 1);
         launch(K_APPLY, k_apply<T>, grid_, 256, jobs, s);
         for (int i : sel) {
@@ -1283,6 +1296,7 @@ class BatchEngine {
           else slots_[i].waiting = true;
         }
         return EXTREMZ_OK;
+      }
       case PC_PRE_END:
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
@@ -1391,6 +1405,7 @@ class BatchEngine {
     launch(K_OTHER, k_ext_index<T>, grid_, 256, J);
     // The lists and the extremum index are all that an analysis needs.
     if (jh.p.flags & kFlagAnalysis) return EXTREMZ_OK;
+    J.smask2 = A.take<uint16_t>(ns2);
     J.orow2 = A.take<int>((long long)ns2 * kRowStride);
     J.orm2 = A.take<int4>(ns2);
     J.oend2 = A.take<int4>(ns2);
@@ -1429,14 +1444,15 @@ class BatchEngine {
     // extreme saddle key and entry count), the entry lists' offsets, then the
     // extreme saddle ids and the entries.  The sides share the selection
     // scratch (ext_key, ext_id), so they go one after the other.  Rows name
-    // only extrema, so a side with rows has extrema.
+    // only extrema, so a side with rows has extrema.  Without join_rows the
+    // minima's side waits for the final join pass (k_join_*), which wants its
+    // scratch filled.
     if (nmax) {
       launch(K_OTHER, k_fill<K>, grid_, 256, J.ext_key, K(0), (long long)nmax);
       launch(K_OTHER, k_fill<int>, grid_, 256, J.ext_id, -1, (long long)nmax);
       EZ_CHECK(cudaMemsetAsync(J.moff2, 0, (size_t)(nmax + 1) * 4, st_));
     }
-    launch(K_SETUP, k_rows<T, true>, grid_, 256, J, J.f, (const int*)J.ds, (const int*)J.sad2,
-           (int)C_NS2, J.orow2, J.ocnt2, J.orm2, J.oend2);
+    launch(K_SETUP, k_rows<T, true>, grid_, 256, J);
     if (nmax) {
       EZ_RUN(entry_lists(J.moff2, J.wstamp2, nmax, chunk));
       launch(K_OTHER, k_extreme_saddle<T, true>, grid_, 256, J);
@@ -1446,27 +1462,30 @@ class BatchEngine {
       launch(K_OTHER, k_fill<int>, grid_, 256, J.first_s, kInf, (long long)nmax);
       EZ_CHECK(cudaMemsetAsync(J.flag2, 0, nmax * 4, st_));
     }
-    if (nmin) {
+    if (nmin && (J.join_rows || jh.p.final_join)) {
       launch(K_OTHER, k_fill<K>, grid_, 256, J.ext_key, ~K(0), (long long)nmin);
       launch(K_OTHER, k_fill<int>, grid_, 256, J.ext_id, kInf, (long long)nmin);
-      EZ_CHECK(cudaMemsetAsync(J.moff1, 0, (size_t)(nmin + 1) * 4, st_));
-    }
-    launch(K_SETUP, k_rows<T, false>, grid_, 256, J, J.f, (const int*)J.as, (const int*)J.sad1,
-           (int)C_NS1, J.orow1, J.ocnt1, J.orm1, J.oend1);
-    if (nmin) {
-      EZ_RUN(entry_lists(J.moff1, J.wstamp1, nmin, chunk));
-      launch(K_OTHER, k_extreme_saddle<T, false>, grid_, 256, J);
-      EZ_CHECK(cudaMemsetAsync(J.wstamp1, 0, (size_t)nmin * 4, st_));
-      EZ_CHECK(cudaMemcpyAsync(J.smallest, J.ext_id, nmin * 4, cudaMemcpyDeviceToDevice, st_));
-      launch(K_OTHER, k_fill<int>, grid_, 256, J.ext_id, kInf, (long long)nmin);
-      launch(K_OTHER, k_fill<int>, grid_, 256, J.first_min1, kInf, (long long)nmin);
       launch(K_OTHER, k_fill<int>, grid_, 256, J.first_sj, kInf, (long long)nmin);
-      EZ_CHECK(cudaMemsetAsync(J.flag_min2, 0, nmin * 4, st_));
+    }
+    if (!J.join_rows) {
+      J.smallest = J.ext_id;  // as k_join_ids leaves it
+    } else {
+      if (nmin) EZ_CHECK(cudaMemsetAsync(J.moff1, 0, (size_t)(nmin + 1) * 4, st_));
+      launch(K_SETUP, k_rows<T, false>, grid_, 256, J);
+      if (nmin) {
+        EZ_RUN(entry_lists(J.moff1, J.wstamp1, nmin, chunk));
+        launch(K_OTHER, k_extreme_saddle<T, false>, grid_, 256, J);
+        EZ_CHECK(cudaMemsetAsync(J.wstamp1, 0, (size_t)nmin * 4, st_));
+        EZ_CHECK(cudaMemcpyAsync(J.smallest, J.ext_id, nmin * 4, cudaMemcpyDeviceToDevice, st_));
+        launch(K_OTHER, k_fill<int>, grid_, 256, J.ext_id, kInf, (long long)nmin);
+        launch(K_OTHER, k_fill<int>, grid_, 256, J.first_min1, kInf, (long long)nmin);
+        EZ_CHECK(cudaMemsetAsync(J.flag_min2, 0, nmin * 4, st_));
+      }
     }
     // Decompressed row slots start at zero: the reference's rows are fresh
     // cudaMalloc memory read before first written (:5338-5341, :3128-3130).
     if (ns2) EZ_CHECK(cudaMemsetAsync(J.drow2, 0, (size_t)ns2 * 2 * 4, st_));
-    if (ns1) EZ_CHECK(cudaMemsetAsync(J.drow1, 0, (size_t)ns1 * 2 * 4, st_));
+    if (ns1 && J.join_rows) EZ_CHECK(cudaMemsetAsync(J.drow1, 0, (size_t)ns1 * 2 * 4, st_));
     // Every tile's pointers are computed in the first manifold round.
     EZ_CHECK(cudaMemsetAsync(J.tdirty, 1, (size_t)jh.ntiles, st_));
     // Block stamps start below the first round's; no root is touched.

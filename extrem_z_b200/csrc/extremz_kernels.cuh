@@ -26,6 +26,8 @@ struct Job {
 
   int8_t* otype;      // original vertex type (-1, 0..5)
   uint16_t* olm;      // original lower-star direction mask
+  uint16_t* smask2;   // per 2-saddle row: its upper-neighbour directions in the original field
+                      // (a 1-saddle's lower ones are olm)
   uint8_t* ocnt2; uint8_t* ocnt1;  // original row counts (compact copy of row[14])
   int* ds; int* as;   // original steepest ascent / descent roots
   int* dds; int* das; // decompressed roots
@@ -90,6 +92,8 @@ struct Job {
   const CUtensorMap* map_g;
   int tma_f, tma_g;
   int iter_cap;  // device-side limit of pointer jumping and path walks
+  int join_rows;  // the 1-saddles' rows are read during the correction (preserve_join, or a
+                  // census); else only the final join pass looks at them (k_join_*)
   int pass_chunk; // 1024-id blocks per saddle-pass work item (a tuning knob)
   int wn_lockstep; // wrong neighbours by the lockstep resolution (k_wn_step, the
                    // default), else in ascending saddle order (k_wn_vote / commit / resolve)
@@ -1130,44 +1134,49 @@ __global__ void k_ext_index(Job<T> J) {
 // and the count are written, so entries past a shorter row keep their last
 // value, as in the reference.
 // ---------------------------------------------------------------------------
+// Vertex-id offsets of the 14 directions, for loops over the set bits of a
+// direction mask (threads 0..13 fill it; the caller synchronises).
+__device__ __forceinline__ void fill_offsets(int* off, const Dims& g) {
+  if (threadIdx.x < kNumDirs) {
+    const int d = threadIdx.x;
+    off[d] = ddx(d) + ddy(d) * g.W + ddz(d) * g.W * g.H;
+  }
+}
+
+// The rows of one side of the original field.  A saddle's neighbours on the
+// side are the set bits of the direction mask that the classification left
+// (upper neighbours of a 2-saddle, lower ones of a 1-saddle): 4.3 of 14 on
+// average and 8.2 in the fullest lane of a warp, so the passes below go over
+// set bits in groups of four, up to the warp's fullest lane, and no neighbour
+// value is read or compared.  Bound by the label and value gathers and by the
+// issue of the per-entry work: 1.58 ms for the 22 M 2-saddles of the 512^3
+// benchmark field, 2.38 ms when it went over all 14 directions and compared
+// their values.
 template <class T, bool kAsc>
-__global__ void __launch_bounds__(256, 4) k_rows(Job<T> J, const T* __restrict__ a,
-                                              const int* __restrict__ lab, const int* __restrict__ sad,
-                                              int ns_slot, int* __restrict__ rows,
-                                              uint8_t* __restrict__ ocnt, int4* __restrict__ orm,
-                                              int4* __restrict__ oend) {
-  const int ns = J.ctr[ns_slot];
+__global__ void __launch_bounds__(256, 4) k_rows(Job<T> J) {
+  __shared__ int off[kNumDirs];
+  fill_offsets(off, J.dim);
+  __syncthreads();
+  const T* __restrict__ a = J.f;
+  const int* __restrict__ lab = kAsc ? J.ds : J.as;
+  const int* __restrict__ sad = kAsc ? J.sad2 : J.sad1;
+  const int ns = J.ctr[kAsc ? C_NS2 : C_NS1];
+  int* __restrict__ rows = kAsc ? J.orow2 : J.orow1;
   const int stride = gridDim.x * blockDim.x;
   const Dims g = J.dim;
-  const int WH = g.W * g.H;
   for (int base = blockIdx.x * blockDim.x; base < ns; base += stride) {  // uniform per warp
     const int i = base + threadIdx.x;
     const bool act = i < ns;
     const int s = act ? sad[i] : 0;
-    int x, y, z;
-    coords(s, g, x, y, z);
-    const int valid = act ? valid_mask(boundary_code(x, y, z, g.W, g.H, g.D)) : 0;
     const T sv = a[s];
-    // Neighbour values, then the side's labels, then their values: three
-    // batches of independent loads; the sort below compares cached values.
-    T val[kNumDirs];
-#pragma unroll
-    for (int d = 0; d < kNumDirs; ++d)
-      val[d] = (valid >> d & 1) ? a[s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH] : T(0);
-    int lb[kNumDirs];
-#pragma unroll
-    for (int d = 0; d < kNumDirs; ++d) {
-      const int r = s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
-      const bool side = (valid >> d & 1) && (kAsc ? above(val[d], r, sv, s) : below(val[d], r, sv, s));
-      lb[d] = side ? lab[r] : -1;
+    unsigned side = act ? J.olm[s] : 0u;
+    if (kAsc && act) {
+      int x, y, z;
+      coords(s, g, x, y, z);
+      side = (unsigned)valid_mask(boundary_code(x, y, z, g.W, g.H, g.D)) & ~side;
+      J.smask2[i] = (uint16_t)side;
     }
-#pragma unroll
-    for (int d = 0; d < kNumDirs; ++d) val[d] = lb[d] >= 0 ? a[lb[d]] : T(0);
-    unsigned keep = 0;
-#pragma unroll
-    for (int d = 0; d < kNumDirs; ++d)
-      if (lb[d] >= 0 && (!kAsc || tabs(T(val[d] - sv)) >= J.thr)) keep |= 1u << d;
-    const int cnt = __popc(keep);
+    const int pmax = (int)__reduce_max_sync(0xffffffffu, __popc(side));
     // The reference sorts each row (insertionSort :1795-1811, descending, for
     // ascending rows; reversed_insertionSort :1813-1829, ascending, for
     // descending rows) by (value, label).  What is read back from an original
@@ -1178,28 +1187,51 @@ __global__ void __launch_bounds__(256, 4) k_rows(Job<T> J, const T* __restrict__
     // sorted: the first and last entry come from one pass, and the entries
     // are kept in direction order as extremum indices, a repeated label's
     // entry as -1.
+    int lb[16], mp[16];
+    unsigned keep = 0u, dup = 0u;  // by position among the side's neighbours
     int fl = -1, ll = -1;
     T fv = T(0), lv = T(0);
+    unsigned rest = side;
 #pragma unroll
-    for (int d = 0; d < kNumDirs; ++d) {
-      if (!(keep >> d & 1u)) continue;
-      // Strict comparisons: among equal entries (one label) the first kept
-      // direction stays, so first and last are never a repeat.
-      const bool first = fl < 0 || (kAsc ? above(val[d], lb[d], fv, fl) : below(val[d], lb[d], fv, fl));
-      const bool last = ll < 0 || (kAsc ? below(val[d], lb[d], lv, ll) : above(val[d], lb[d], lv, ll));
-      if (first) { fv = val[d]; fl = lb[d]; }
-      if (last) { lv = val[d]; ll = lb[d]; }
+    for (int h = 0; h < 16; h += 4) {
+#pragma unroll
+      for (int q = h; q < h + 4; ++q) lb[q] = mp[q] = -1;
+      if (h >= pmax) continue;  // uniform per warp
+#pragma unroll
+      for (int q = h; q < h + 4; ++q) {
+        if (rest) lb[q] = lab[s + off[__ffs((int)rest) - 1]];
+        rest &= rest - 1u;
+      }
+      T val[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) val[q] = lb[h + q] >= 0 ? a[lb[h + q]] : T(0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (lb[h + q] >= 0) mp[h + q] = J.ext[lb[h + q]];
+#pragma unroll
+      for (int q = h; q < h + 4; ++q) {
+        const T v = val[q - h];
+        if (lb[q] < 0 || (kAsc && !(tabs(T(v - sv)) >= J.thr))) continue;
+        bool again = false;  // an earlier kept entry has the label
+#pragma unroll
+        for (int e = 0; e < q; ++e) again |= lb[e] == lb[q] && (keep >> e & 1u);
+        keep |= 1u << q;
+        if (again) {
+          dup |= 1u << q;
+          continue;
+        }
+        const bool first = fl < 0 || (kAsc ? above(v, lb[q], fv, fl) : below(v, lb[q], fv, fl));
+        const bool last = ll < 0 || (kAsc ? below(v, lb[q], lv, ll) : above(v, lb[q], lv, ll));
+        if (first) { fv = v; fl = lb[q]; }
+        if (last) { lv = v; ll = lb[q]; }
+      }
     }
-    unsigned dup = 0u;  // kept entries whose label an earlier kept entry has
-#pragma unroll
-    for (int d = 1; d < kNumDirs; ++d)
-#pragma unroll
-      for (int e = 0; e < d; ++e)
-        if ((keep >> e & keep >> d & 1u) && lb[e] == lb[d]) dup |= 1u << d;
+    const int cnt = __popc(keep);
     int* out = rows + (long long)i * kRowStride;
     if (act) {
-      ocnt[i] = (uint8_t)cnt;
-      oend[i] = make_int4(fl, ll, fl >= 0 ? J.ext[fl] : -1, ll >= 0 ? J.ext[ll] : -1);
+      (kAsc ? J.ocnt2 : J.ocnt1)[i] = (uint8_t)cnt;
+      (kAsc ? J.oend2 : J.oend1)[i] =
+          make_int4(fl, ll, fl >= 0 ? J.ext[fl] : -1, ll >= 0 ? J.ext[ll] : -1);
     }
     // Per kept entry, at its position among the kept ones: the first four in
     // the compact copy, the rest in the row.  And the first pass of
@@ -1212,40 +1244,46 @@ __global__ void __launch_bounds__(256, 4) k_rows(Job<T> J, const T* __restrict__
     using KK = typename KeyOf<T>::K;
     const KK key = KeyOf<T>::enc(sv + T(0));  // -0 and +0 compare equal
     int* mcount = kAsc ? J.moff2 : J.moff1;
-    // The extremum indices of the fresh entries first, all gathers in flight
-    // together (loads after an atomic would wait for it).
-    int mp[kNumDirs];
+    // Entries that count: kept and not a repeat.
 #pragma unroll
-    for (int d = 0; d < kNumDirs; ++d)
-      mp[d] = (keep >> d & ~dup >> d & 1u) ? J.ext[lb[d]] : -1;
+    for (int q = 0; q < kNumDirs; ++q)
+      if (!(keep & ~dup & 1u << q)) mp[q] = -1;
     int m0 = -1, m1 = -1, m2 = -1, m3 = -1;
     int pos = 0;
 #pragma unroll
-    for (int d = 0; d < kNumDirs; ++d) {
-      const bool kd = keep >> d & 1u;
-      const unsigned grp = __match_any_sync(0xffffffffu, mp[d]);
-      if (mp[d] >= 0 && (grp & ((1u << lane_id()) - 1u)) == 0u) atomicAdd(mcount + mp[d], __popc(grp));
-      if (kd) {
-        m0 = pos == 0 ? mp[d] : m0;
-        m1 = pos == 1 ? mp[d] : m1;
-        m2 = pos == 2 ? mp[d] : m2;
-        m3 = pos == 3 ? mp[d] : m3;
-        if (pos >= 4) out[pos] = mp[d];
-        ++pos;
+    for (int h = 0; h < 16; h += 4) {
+      if (h >= pmax) continue;
+#pragma unroll
+      for (int q = h; q < h + 4; ++q) {
+        if (q >= kNumDirs) continue;
+        const unsigned grp = __match_any_sync(0xffffffffu, mp[q]);
+        if (mp[q] >= 0 && (grp & ((1u << lane_id()) - 1u)) == 0u) atomicAdd(mcount + mp[q], __popc(grp));
+        if (keep >> q & 1u) {
+          if (q < 4 || pos < 4) {  // pos <= q
+            m0 = pos == 0 ? mp[q] : m0;
+            m1 = pos == 1 ? mp[q] : m1;
+            m2 = pos == 2 ? mp[q] : m2;
+            m3 = pos == 3 ? mp[q] : m3;
+          } else {
+            out[pos] = mp[q];
+          }
+          ++pos;
+        }
       }
     }
-    if (act) orm[i] = make_int4(m0, m1, m2, m3);
-    // Then the key reads, seven at a time, and the atomics they call for.
+    if (act) (kAsc ? J.orm2 : J.orm1)[i] = make_int4(m0, m1, m2, m3);
+    // Then the key reads, four at a time, and the atomics they call for.
 #pragma unroll
-    for (int h = 0; h < kNumDirs; h += 7) {
-      KK cur[7];
+    for (int h = 0; h < 16; h += 4) {
+      if (h >= pmax) continue;
+      KK cur[4];
 #pragma unroll
-      for (int d = 0; d < 7; ++d) cur[d] = mp[h + d] >= 0 ? J.ext_key[mp[h + d]] : KK(0);
+      for (int q = 0; q < 4; ++q) cur[q] = mp[h + q] >= 0 ? J.ext_key[mp[h + q]] : KK(0);
 #pragma unroll
-      for (int d = 0; d < 7; ++d) {
-        if (mp[h + d] < 0 || !(kAsc ? key > cur[d] : key < cur[d])) continue;
-        if (kAsc) atomicMax(J.ext_key + mp[h + d], key);
-        else atomicMin(J.ext_key + mp[h + d], key);
+      for (int q = 0; q < 4; ++q) {
+        if (mp[h + q] < 0 || !(kAsc ? key > cur[q] : key < cur[q])) continue;
+        if (kAsc) atomicMax(J.ext_key + mp[h + q], key);
+        else atomicMin(J.ext_key + mp[h + q], key);
       }
     }
   }
@@ -1545,58 +1583,84 @@ __device__ __noinline__ int row_entry_k(const Job<T>& J, int s, int k) {
 
 // One saddle of one side: its decompressed row summary (count, first and
 // last entry in row order) into the row slots, and whether some neighbour on
-// the side has a wrong label.  The loads go out in three batches of
-// independent gathers (neighbour values; labels and mismatch bits of the
-// neighbours on the side; the labels' values), not one dependent chain per
-// neighbour.
+// the side has a wrong label.
+//
+// known: no value changed since a detection that found no mismatch, so the
+// saddle's neighbours on the side are the original field's (its type and
+// lower star matched): the direction mask is read instead of 14 neighbour
+// values.  Two thirds of the rounds, the first one (every saddle) among them,
+// run right after such a detection (with the 1-saddles' shortcut below: 7.0 ->
+// 5.7 ms per 512^3 correction).  The loop goes over the set bits four at a
+// time, so that a group's gathers (labels and mismatch bits; the labels'
+// values) are in flight together.
+//
+// A 1-saddle's slots are read only with join_rows; else only its seed bit is
+// needed: the mismatch bytes of its neighbours.
 template <class T, bool kSplit>
-__device__ __forceinline__ bool saddle_row(const Job<T>& J, int i, int s) {
-  const Dims g = J.dim;
-  const int WH = g.W * g.H;
-  int x, y, z;
-  coords(s, g, x, y, z);
-  const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
+__device__ __forceinline__ bool saddle_row(const Job<T>& J, const int* __restrict__ off, int i,
+                                           int s, bool known) {
   const T* __restrict__ gv = J.g;
   const int* __restrict__ lab = kSplit ? J.dds : J.das;
+  const uint8_t* __restrict__ mis = J.mis;
   const T sv = __ldg(gv + s);
-  // Neighbour values, then the side's labels and mismatch bytes, then the
-  // labels' values: batches of independent gathers, values seven at a time
-  // (fourteen live values spill at 64 registers).
-  unsigned side = 0;
+  unsigned side = 0u;
+  if (known) {
+    side = kSplit ? J.smask2[i] : J.olm[s];
+  } else {
+    const Dims g = J.dim;
+    const int WH = g.W * g.H;
+    int x, y, z;
+    coords(s, g, x, y, z);
+    const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
+    // Values seven at a time (fourteen live values spill at 64 registers).
 #pragma unroll
-  for (int h = 0; h < kNumDirs; h += 7) {
-    T val[7];
+    for (int h = 0; h < kNumDirs; h += 7) {
+      T val[7];
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
-      const int d = h + q;
-      val[q] = (valid >> d & 1) ? __ldg(gv + s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH) : T(0);
-    }
+      for (int q = 0; q < 7; ++q) {
+        const int d = h + q;
+        val[q] = (valid >> d & 1) ? __ldg(gv + s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH) : T(0);
+      }
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
-      const int d = h + q;
-      const int r = s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
-      if ((valid >> d & 1) && (kSplit ? above(val[q], r, sv, s) : below(val[q], r, sv, s)))
-        side |= 1u << d;
+      for (int q = 0; q < 7; ++q) {
+        const int d = h + q;
+        const int r = s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
+        if ((valid >> d & 1) && (kSplit ? above(val[q], r, sv, s) : below(val[q], r, sv, s)))
+          side |= 1u << d;
+      }
     }
   }
-  int ml[kNumDirs];
   int mb = 0;
+  if (!kSplit && !J.join_rows) {
+    while (side) {
 #pragma unroll
-  for (int d = 0; d < kNumDirs; ++d) {
-    const int r = s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
-    ml[d] = (side >> d & 1) ? __ldg(lab + r) : -1;
-    mb |= (side >> d & 1) ? __ldg(J.mis + r) : 0;
+      for (int q = 0; q < 4; ++q) {
+        if (side) mb |= __ldg(mis + s + off[__ffs((int)side) - 1]);
+        side &= side - 1u;
+      }
+    }
+    return (mb >> 1) & 1;
   }
   T fv = T(0), lv = T(0);
   int cnt = 0, fm = -1, lm = -1;
+  while (side) {
+    int ml[4];
+    T val[4];
 #pragma unroll
-  for (int h = 0; h < kNumDirs; h += 7) {
-    T val[7];
+    for (int q = 0; q < 4; ++q) {
+      ml[q] = -1;
+      if (side) {
+        const int r = s + off[__ffs((int)side) - 1];
+        ml[q] = __ldg(lab + r);
+        mb |= __ldg(mis + r);
+      }
+      side &= side - 1u;
+    }
 #pragma unroll
-    for (int q = 0; q < 7; ++q) val[q] = ml[h + q] >= 0 ? __ldg(gv + ml[h + q]) : T(0);
+    for (int q = 0; q < 4; ++q) val[q] = ml[q] >= 0 ? __ldg(gv + ml[q]) : T(0);
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
-      const int m = ml[h + q];
+    for (int q = 0; q < 4; ++q) {
+      const int m = ml[q];
       const T v = val[q];
       if (m >= 0 && (!kSplit || tabs(T(v - sv)) >= J.thr)) {
         if (cnt == 0 || row_first<T, kSplit>(v, m, fv, fm)) { fv = v; fm = m; }
@@ -1676,9 +1740,15 @@ __device__ __forceinline__ bool saddle_inputs_changed(const Job<T>& J, int s) {
 template <class T>
 __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict__ jobs,
                                                         const __grid_constant__ Sel sel) {
+  __shared__ int off[kNumDirs];
   for (int jk = 0; jk < sel.n; ++jk) {
     const Job<T>& J = jobs[sel.idx[jk]];
     if (J.ctr[C_MFSKIP]) continue;
+    __syncthreads();  // every thread is done with the last job's offsets
+    fill_offsets(off, J.dim);
+    __syncthreads();
+    // No mismatch at the last detection and no value changed since.
+    const bool known = J.ctr[C_MM] == 0 && J.ctr[C_DIRTY] == 0;
     const int ns2 = J.ctr[C_NS2], ns1 = J.ctr[C_NS1];
     const int nb = (J.dim.N + kCpBlock - 1) / kCpBlock;
     const int chunk = J.pass_chunk;
@@ -1741,7 +1811,8 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
           s = split ? J.sad2[i] : J.sad1[i];
           const uint8_t kept = hb[i];  // loaded with the id: no round trip of its own
           if (all_new || saddle_inputs_changed(J, s)) {
-            has = split ? saddle_row<T, true>(J, i, s) : saddle_row<T, false>(J, i, s);
+            has = split ? saddle_row<T, true>(J, off, i, s, known)
+                        : saddle_row<T, false>(J, off, i, s, known);
             hb[i] = (uint8_t)has;
           } else {  // rows and seed bit as computed in an earlier round
             has = kept != 0;
@@ -2346,6 +2417,143 @@ __global__ void __launch_bounds__(256) k_wis_collect(const Job<T>* __restrict__ 
     const unsigned b = __ballot_sync(0xffffffffu, hit);
     if (lane_id() == 0 && b) atomicAdd(cnt, __popc(b));
   }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The final saddle_loops_join (:5997) of a job whose 1-saddle rows nothing
+// else reads (join_rows == 0): get_wrong_index_saddles_join looks at them
+// once, so no entry lists are built and nothing is kept between scans.  Three
+// passes over the 1-saddles of the original field: the extreme value key per
+// minimum (k_join_keys, which also leaves each row's distinct minima in orm1 /
+// orow1 / ocnt1), the smallest id at that key (k_join_ids: together
+// findSmallestSaddlePerMin :4915-4940), and the first row per minimum whose
+// saddle comes before that smallest saddle in the decompressed field
+// (k_join_scan, into first_sj for k_wis_collect).  Scratch ext_key, ext_id
+// (= smallest) and first_sj were filled at setup.  1.9 ms for the 22 M
+// 1-saddles of the 512^3 benchmark field, where their rows, entry lists and
+// first full scan took 4.2 ms; a job that ends early does not run them.
+// ---------------------------------------------------------------------------
+template <class T>
+__global__ void __launch_bounds__(256, 4) k_join_keys(const Job<T>* __restrict__ jobs,
+                                                      const __grid_constant__ Sel sel) {
+  __shared__ int off[kNumDirs];
+  for (int jk = 0; jk < sel.n; ++jk) {
+    const Job<T>& J = jobs[sel.idx[jk]];
+    __syncthreads();  // every thread is done with the last job's offsets
+    fill_offsets(off, J.dim);
+    __syncthreads();
+    using KK = typename KeyOf<T>::K;
+    const int ns = J.ctr[C_NS1];
+    const int* __restrict__ lab = J.as;
+    const int* __restrict__ ext = J.ext;
+    const int stride = gridDim.x * blockDim.x;
+    for (int base = blockIdx.x * blockDim.x; base < ns; base += stride) {  // uniform per warp
+      const int i = base + threadIdx.x;
+      const bool act = i < ns;
+      const int s = act ? J.sad1[i] : 0;
+      unsigned rest = act ? J.olm[s] : 0u;
+      const int pmax = (int)__reduce_max_sync(0xffffffffu, __popc(rest));
+      const KK key = KeyOf<T>::enc(J.f[s] + T(0));  // -0 and +0 compare equal
+      // Distinct labels in direction order, kept as extremum indices.
+      int lb[16], mp[16];
+      int cnt = 0, m0 = -1, m1 = -1, m2 = -1, m3 = -1;
+#pragma unroll
+      for (int h = 0; h < 16; h += 4) {
+#pragma unroll
+        for (int q = h; q < h + 4; ++q) lb[q] = mp[q] = -1;
+        if (h >= pmax) continue;  // uniform per warp
+#pragma unroll
+        for (int q = h; q < h + 4; ++q) {
+          if (rest) lb[q] = lab[s + off[__ffs((int)rest) - 1]];
+          rest &= rest - 1u;
+        }
+#pragma unroll
+        for (int q = h; q < h + 4; ++q) {
+          bool fresh = lb[q] >= 0;
+#pragma unroll
+          for (int e = 0; e < q; ++e) fresh &= lb[e] != lb[q];
+          if (fresh) mp[q] = ext[lb[q]];
+        }
+#pragma unroll
+        for (int q = h; q < h + 4; ++q) {
+          if (mp[q] < 0) continue;
+          m0 = cnt == 0 ? mp[q] : m0;
+          m1 = cnt == 1 ? mp[q] : m1;
+          m2 = cnt == 2 ? mp[q] : m2;
+          m3 = cnt == 3 ? mp[q] : m3;
+          if (cnt >= 4) J.orow1[(long long)i * kRowStride + cnt] = mp[q];
+          ++cnt;
+        }
+        KK cur[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cur[q] = mp[h + q] >= 0 ? J.ext_key[mp[h + q]] : KK(0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (mp[h + q] >= 0 && key < cur[q]) atomicMin(J.ext_key + mp[h + q], key);
+      }
+      if (act) {
+        J.ocnt1[i] = (uint8_t)cnt;
+        J.orm1[i] = make_int4(m0, m1, m2, m3);
+      }
+    }
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) k_join_ids(const Job<T>* __restrict__ jobs,
+                                                  const __grid_constant__ Sel sel) {
+  for (int jk = 0; jk < sel.n; ++jk) {
+    const Job<T>& J = jobs[sel.idx[jk]];
+    using KK = typename KeyOf<T>::K;
+    const int ns = J.ctr[C_NS1];
+    const int stride = gridDim.x * blockDim.x;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
+      const int s = J.sad1[i], cnt = J.ocnt1[i];
+      const int4 m4 = J.orm1[i];
+      const KK key = KeyOf<T>::enc(J.f[s] + T(0));
+      const int m[4] = {m4.x, m4.y, m4.z, m4.w};
+      KK cur[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) cur[q] = m[q] >= 0 ? J.ext_key[m[q]] : KK(0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (m[q] >= 0 && cur[q] == key) atomicMin(J.ext_id + m[q], s);
+      for (int p = 4; p < cnt; ++p) {
+        const int mm = J.orow1[(long long)i * kRowStride + p];
+        if (J.ext_key[mm] == key) atomicMin(J.ext_id + mm, s);
+      }
+    }
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) k_join_scan(const Job<T>* __restrict__ jobs,
+                                                   const __grid_constant__ Sel sel) {
+  for (int jk = 0; jk < sel.n; ++jk) {
+    const Job<T>& J = jobs[sel.idx[jk]];
+    const T* __restrict__ g = J.g;
+    const int ns = J.ctr[C_NS1];
+    const int stride = gridDim.x * blockDim.x;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
+      const int s = J.sad1[i], cnt = J.ocnt1[i];
+      const int4 m4 = J.orm1[i];
+      const T gs = g[s];
+      const int m[4] = {m4.x, m4.y, m4.z, m4.w};
+      int t[4];
+      T gt[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) t[q] = m[q] >= 0 ? J.ext_id[m[q]] : s;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) gt[q] = t[q] != s ? g[t[q]] : T(0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (t[q] != s && below(gs, s, gt[q], t[q])) atomicMin(J.first_sj + m[q], i * kRowStride);
+      for (int p = 4; p < cnt; ++p) {
+        const int mm = J.orow1[(long long)i * kRowStride + p], tt = J.ext_id[mm];
+        if (tt != s && below(gs, s, g[tt], tt)) atomicMin(J.first_sj + mm, i * kRowStride);
+      }
+    }
   }
 }
 
