@@ -114,13 +114,13 @@ constexpr long long job_bytes_voxels(long long n, long long ksz) {
   return arr_bytes(n, 1) + arr_bytes(n, 2)                          // otype, olm
          + 5 * arr_bytes(n, 4)                                      // ds, as, dds, das, ext
          + arr_bytes(n, ksz) + 3 * arr_bytes(n, 4)                  // delta, counter, touched, mm
-         + arr_bytes(n, 4) + arr_bytes(n, 1) + 3 * arr_bytes(n, 4)  // mm_next, mstat, dirty, stamps
-         + arr_bytes(n, 8) + 2 * arr_bytes(n, 4)                    // claim, taken, taken1
+         + arr_bytes(n, 4) + arr_bytes(n, 1) + 2 * arr_bytes(n, 4)  // mm_next, mstat, dirty lists
+         + arr_bytes(n, 8)                                          // claim
          + 4 * arr_bytes(n, 4)                                      // cand(_next), flagged(1)
          + arr_bytes(n, 4) + arr_bytes(n, 1)                        // cand_j, mis
          + 2 * arr_bytes(n, 4)                                      // pdd, pda
          + arr_bytes((n + 31) / 32, 4) + arr_bytes(n, 1)            // change bitset, dirtyv
-         + 4 * arr_bytes((n + 31) / 32, 4)  // wrong-saddle change bitsets, touched roots
+         + 8 * arr_bytes((n + 31) / 32, 4)  // wrong-saddle change, touched roots, dirty, taken
          + 2 * arr_bytes((n + kCpBlock - 1) / kCpBlock, 4)  // dirtyv stamp, seed count per block
          + arr_bytes(6 * ((n + kCpBlock - 1) / kCpBlock), 4)        // CP block counts
          + arr_bytes(6 * ((n + kCpBlock - 1) / kCpBlock / 1024 + 1), 4)  // and their chunk sums
@@ -157,7 +157,7 @@ constexpr long long job_bytes_lists(long long ns2, long long ns1, long long nmax
 }
 
 // Per tile: change mark.
-constexpr long long job_bytes_tiles(long long nt) { return arr_bytes(nt, 1); }
+constexpr long long job_bytes_tiles(long long nt) { return arr_bytes(nt, 4); }
 
 // Worst case (every voxel a critical point of every kind; a voxel's upper and
 // lower neighbours, at most 14, give the row entries of both sides; at most
@@ -182,6 +182,7 @@ struct JobHost {
   bool waiting = false;   // stopped at a branch that needs this tick's counters
   cudaEvent_t input_ready = nullptr;  // the decompressed field is still arriving until this event
   int outer = 0, rounds = 0, cloop_total = 0, manifold_rounds = 0;
+  int reused = 0;         // manifold rounds that launched nothing: no value had changed
   int nfc = 0, nfc1 = 0;
   int c[11] = {0};        // loop-test counters (:5603-5605)
   bool dense_done = false;
@@ -398,11 +399,8 @@ class BatchEngine {
       J.mm_next = A.take<int>(N);
       J.mstat = A.take<uint8_t>(N);
       J.dirty = A.take<int>(N);
-      J.dstamp = A.take<int>(N);
-      J.rstamp = A.take<int>(N);
+      J.dirty1 = A.take<int>(N);
       J.claim = A.take<unsigned long long>(N);
-      J.taken = A.take<int>(N);
-      J.taken1 = A.take<int>(N);
       J.cand = A.take<int>(N);
       J.cand_next = A.take<int>(N);
       J.flagged = A.take<int>(N);
@@ -416,10 +414,14 @@ class BatchEngine {
       J.rtouch1 = A.take<unsigned>((N + 31) / 32);
       J.wchg2 = A.take<unsigned>((N + 31) / 32);
       J.wchg1 = A.take<unsigned>((N + 31) / 32);
+      J.dbits = A.take<unsigned>((N + 31) / 32);
+      J.dbits1 = A.take<unsigned>((N + 31) / 32);
+      J.taken = A.take<unsigned>((N + 31) / 32);
+      J.taken1 = A.take<unsigned>((N + 31) / 32);
       J.dirtyv = A.take<uint8_t>(N);
       J.bdirty = A.take<int>(jh.nb);
       J.hcnt = A.take<int>(jh.nb);
-      J.tdirty = A.take<uint8_t>(jh.ntiles);
+      J.tdirty = A.take<int>(jh.ntiles);
       J.g0 = keep_input ? A.take<T>(N) : nullptr;
       J.edited = track_edits ? A.take<unsigned>((N + 31) / 32) : nullptr;
     }
@@ -458,7 +460,7 @@ class BatchEngine {
     r->manifold_rounds = j.manifold_rounds;
     std::memcpy(r->counters, j.c, sizeof(j.c));
     r->error_bits = ctr_host_ ? ctr_host_[(size_t)slot * C_COUNT + C_ERROR] : 0;
-    r->manifold_reused = ctr_host_ ? ctr_host_[(size_t)slot * C_COUNT + C_MFREUSED] : 0;
+    r->manifold_reused = j.reused + (ctr_host_ ? ctr_host_[(size_t)slot * C_COUNT + C_MFREUSED] : 0);
     for (int k = 0; k < 4; ++k)
       r->cp_counts[k] = ctr_host_ ? ctr_host_[(size_t)slot * C_COUNT + C_NS2 + k] : 0;
   }
@@ -719,6 +721,7 @@ class BatchEngine {
   int tick_issue() {
     issued_ = false;
     ++tick_id_;
+    const long long launches0 = launches_;
     // A tick whose launches repeat an earlier tick's exactly (kernels, launch
     // shapes and arguments; per-job state is read from device memory) runs as
     // one CUDA graph: recorded, captured the third time its signature is
@@ -755,7 +758,10 @@ class BatchEngine {
     recording_ = false;
     if (rc != EXTREMZ_OK) return rc;
     if (graph && !pending_.empty()) EZ_RUN(run_recorded());
-    if (!issued_) return EXTREMZ_OK;
+    // A tick that launched nothing (a manifold round over an unchanged field, a
+    // re-read of the counters) leaves the host's copy as it is.
+    launched_ = launches_ != launches0;
+    if (!launched_) return EXTREMZ_OK;
     EZ_CHECK(cudaGetLastError());
     // The counter blocks up to the last slot in use (the host reads no other).
     int hi = 0;
@@ -770,8 +776,10 @@ class BatchEngine {
   int tick_complete() {
     if (!issued_) return EXTREMZ_OK;
     issued_ = false;
-    EZ_CHECK(cudaStreamSynchronize(st_));
-    fold_timings();
+    if (launched_) {
+      EZ_CHECK(cudaStreamSynchronize(st_));
+      fold_timings();
+    }
     for (int i = 0; i < kMaxSel; ++i) {
       JobHost<T>& j = slots_[i];
       if (!j.used || j.pc == PC_DONE) continue;
@@ -839,7 +847,7 @@ class BatchEngine {
   static constexpr int kCaptureAt = 3;
   cudaStream_t cap_ = nullptr;  // capture stream
   cudaMemPool_t pool_mem_ = nullptr;
-  bool ready_ = false, borrowed_ = false, issued_ = false;
+  bool ready_ = false, borrowed_ = false, issued_ = false, launched_ = false;
   long long tick_id_ = 0;
   int grid_ = 1184;  // grid of the grid-stride kernels for the phase being issued
   int sms_ = 148;
@@ -1110,7 +1118,27 @@ class BatchEngine {
     return s;
   }
 
-  void ctl(const Sel& s, int op) { launch(K_OTHER, k_ctl<T>, 1, 64, jobs_dev_, s, op); }
+  // Block spans for the grid-stride kernels: a block per 1024 voxels of each
+  // job, scaled down to the grid of the phase (the SMs times the blocks-per-SM
+  // knob; twice that when several jobs share it), at least one block each.
+  Sel make_span(const std::vector<int>& slots) const {
+    Sel s;
+    std::memset(&s, 0, sizeof(s));
+    s.n = (int)slots.size();
+    const long long budget = s.n > 1 ? 2ll * grid_ : grid_;
+    long long want = 0;
+    for (int i : slots) want += slots_[i].nb;
+    int off = 0;
+    for (int k = 0; k < s.n; ++k) {
+      const long long nb = slots_[slots[k]].nb;
+      s.idx[k] = slots[k];
+      s.off[k] = off;
+      off += (int)std::max(1ll, want <= budget ? nb : nb * budget / want);
+    }
+    s.off[s.n] = off;
+    return s;
+  }
+  static int blocks(const Sel& s) { return s.off[s.n]; }
 
   // ------------------------------------------------------------- phases --
   int run_phase(int ph, const std::vector<int>& sel) {
@@ -1120,13 +1148,14 @@ class BatchEngine {
     if (ph == PC_CL_ROUND || ph == PC_RLOOPS || ph == PC_SLOOPS || ph == PC_SADDLE ||
         ph == PC_SLOOPS_J || ph == PC_SADDLE_J || ph == PC_FINAL_JOIN)
       for (int i : sel) slots_[i].applied_tick = tick_id_;  // phases that apply edits
-    const Sel s = make_sel(sel, false);
-    const Sel st = make_sel(sel, true);
+    const Sel s = make_span(sel);
+    const int nb = blocks(s);
     const Job<T>* jobs = jobs_dev_;
     switch (ph) {
-      case PC_SETUP_A:
+      case PC_SETUP_A: {
+        const Sel st = make_sel(sel, true);
         launch(K_SETUP, k_direction<T, false>, st.off[st.n], 256, jobs, st);
-        launch(K_SETUP, k_jump2<T, false>, grid_, 256, jobs, s);
+        launch(K_SETUP, k_jump2<T, false>, nb, 256, jobs, s);
         for (int i : sel) {
           JobHost<T>& j = slots_[i];
           j.waiting = true;
@@ -1136,6 +1165,7 @@ class BatchEngine {
           EZ_RUN(scan_counts(j.bcount, j.nb, 6, j.J.ctr + C_NS2, j.chunk));
         }
         return EXTREMZ_OK;
+      }
       case PC_SETUP_B:
         for (int i : sel) {
           const int rc = setup_b(i);
@@ -1153,40 +1183,36 @@ class BatchEngine {
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
       case PC_CL_ROUND:
-        ctl(s, OP_ZERO_TOUCHED);
-        launch(K_PROPOSE, k_propose_cp<T>, grid_, 256, jobs, s);
-        launch(K_APPLY, k_apply<T>, grid_, 256, jobs, s);
+        launch(K_PROPOSE, k_propose_cp<T>, nb, 256, jobs, s);
+        launch(K_APPLY, k_apply<T>, nb, 256, jobs, s);
         detect(sel);
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
       case PC_RLOOPS:
-        ctl(s, OP_ZERO_TOUCHED);
-        launch(K_FIXPATH, k_fixpath<T, true>, grid_, 256, jobs, s);
-        launch(K_FIXPATH, k_fixpath<T, false>, grid_, 256, jobs, s);
-        launch(K_APPLY, k_apply<T>, grid_, 256, jobs, s);
+        launch(K_FIXPATH, k_fixpath<T>, nb, 256, jobs, s);
+        launch(K_APPLY, k_apply<T>, nb, 256, jobs, s);
         for (int i : sel) slots_[i].pc = PC_MANIFOLD;
         return EXTREMZ_OK;
       case PC_MANIFOLD: {
         // Jobs known on the host to have no value change since their last
         // manifold round began (no edit in the counters of the last tick, none
-        // issued in this one) get only the round's bookkeeping; their kernels
-        // would return at once.  The others run the round (whose kernels
-        // check again on the device).
-        std::vector<int> quiet, busy;
+        // issued in this one) launch nothing; their kernels would return at
+        // once.  The others run the round (whose kernels check again on the
+        // device).
+        std::vector<int> busy;
         for (int i : sel) {
-          const JobHost<T>& j = slots_[i];
+          JobHost<T>& j = slots_[i];
           const bool known_clean =
               j.manifold_rounds > 0 && j.applied_tick != tick_id_ && h(i, C_CHANGED) == 0;
-          (known_clean ? quiet : busy).push_back(i);
+          if (known_clean) j.reused += 1;
+          else busy.push_back(i);
         }
-        if (!quiet.empty()) ctl(make_sel(quiet, false), OP_MF_BEGIN);
         if (!busy.empty()) {
-          const Sel bs = make_sel(busy, false), bt = make_sel(busy, true);
-          ctl(bs, OP_MF_BEGIN);
+          const Sel bs = make_span(busy);
           // Steepest pointers: every tile in a job's first round, one block
-          // per tile; in later rounds the tiles that changed, listed first,
-          // then taken by a fixed grid (a launch of one block per tile of
-          // the field costs more than the few changed tiles).
+          // per tile; in later rounds the tiles that changed, as k_apply
+          // listed them, taken by a fixed grid (a launch of one block per tile
+          // of the field costs more than the few changed tiles).
           std::vector<int> fresh, later;
           for (int i : busy) (slots_[i].manifold_rounds == 0 ? fresh : later).push_back(i);
           if (!fresh.empty()) {
@@ -1194,47 +1220,45 @@ class BatchEngine {
             launch(K_DIRECTION_FIRST, k_direction<T, true>, ft.off[ft.n], 256, jobs, ft);
           }
           if (!later.empty()) {
-            const Sel ls = make_sel(later, false), lt = make_sel(later, true);
-            const int ntiles = lt.off[lt.n];
-            launch(K_DIRECTION, k_tile_list<T>,
-                   std::max(1, std::min((ntiles + 255) / 256, 2 * sms_)), 256, jobs, ls);
-            launch(K_DIRECTION, k_direction_list<T>, std::max(1, std::min(ntiles, 4 * sms_)),
-                   256, jobs, ls);
+            const Sel lt = tile_span(later);
+            launch(K_DIRECTION, k_direction_list<T>, blocks(lt), 256, jobs, lt);
           }
-          if (!fresh.empty())
-            launch(K_JUMP_FIRST, k_jump2<T, true, false>, grid_, 256, jobs, make_sel(fresh, false));
-          if (!later.empty())
-            launch(K_JUMP, k_jump2<T, true, true>, grid_, 256, jobs, make_sel(later, false));
-          launch(K_OTHER, k_clear_changed<T>, grid_, 256, jobs, bs);
-          launch(K_ROWS, k_saddle_pass<T>, grid_, 256, jobs, bs);
-          bool vote = false;
+          if (!fresh.empty()) {
+            const Sel fs = make_span(fresh);
+            launch(K_JUMP_FIRST, k_jump2<T, true, false>, blocks(fs), 256, jobs, fs);
+          }
+          if (!later.empty()) {
+            const Sel ls = make_span(later);
+            launch(K_JUMP, k_jump2<T, true, true>, blocks(ls), 256, jobs, ls);
+          }
+          launch(K_ROWS, k_saddle_pass<T>, blocks(bs), 256, jobs, bs);
           // Lockstep jobs: the fourteen steps in one block per job when the
           // job's previous round had short candidate lists (the counts of
           // that round are still in the host copy of its counters), else one
           // grid launch per step.  Either is exact for any list length.
-          std::vector<int> lock_small, lock_large;
+          std::vector<int> vote, lock_small, lock_large;
           for (int i : busy) {
             if (!slots_[i].J.wn_lockstep) {
-              vote = true;
+              vote.push_back(i);
               continue;
             }
             const bool small = slots_[i].manifold_rounds > 0 &&
                                h(i, C_CAND) + h(i, C_CANDJ) <= kWnBlockMax;
             (small ? lock_small : lock_large).push_back(i);
           }
-          if (vote) {
-            wn_rounds<true>(bs);  // its completion brings in the join side's list
-            wn_rounds<false>(bs);
+          if (!vote.empty()) {
+            const Sel vs = make_span(vote);
+            wn_rounds<true>(vs);  // its completion brings in the join side's list
+            wn_rounds<false>(vs);
           }
           if (!lock_small.empty()) {
             const Sel ss = make_sel(lock_small, false);
             launch(K_WRONG_NBR, k_wn_steps_block<T>, ss.n, 1024, jobs, ss);
           }
           if (!lock_large.empty()) {
-            const Sel sl = make_sel(lock_large, false);
-            const int grid = std::min(grid_, 2 * sms_);
+            const Sel sl = make_span(lock_large);
             for (int d = 0; d < kNumDirs; ++d)
-              launch(K_WRONG_NBR, k_wn_step<T>, grid, 256, jobs, sl, d);
+              launch(K_WRONG_NBR, k_wn_step<T>, blocks(sl), 256, jobs, sl, d);
           }
         }
         for (int i : sel) {
@@ -1244,52 +1268,40 @@ class BatchEngine {
         return EXTREMZ_OK;
       }
       case PC_SLOOPS:
-        ctl(s, OP_SLOOPS_BEGIN);
-        launch(K_OTHER, k_wim_scan<T, true>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wim_collect<T, true>, grid_, 256, jobs, s, 1);
-        launch(K_APPLY, k_apply<T>, grid_, 256, jobs, s);
+        launch(K_OTHER, k_wim_scan<T, true>, nb, 256, jobs, s);
+        launch(K_OTHER, k_wim_collect<T, true>, nb, 256, jobs, s, 1);
+        launch(K_APPLY, k_apply<T>, nb, 256, jobs, s);
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
       case PC_SADDLE:
-        ctl(s, OP_SADDLE_BEGIN);
-        launch(K_OTHER, k_wis_mark<T, true>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wis_update<T, true>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wis_long<T, true>, 2 * sms_, 256, jobs, s);
-        launch(K_OTHER, k_wis_collect<T, true>, grid_, 256, jobs, s, 1);
-        launch(K_APPLY, k_apply<T>, grid_, 256, jobs, s);
+        wis_scan<true>(s, 1);
+        launch(K_APPLY, k_apply<T>, nb, 256, jobs, s);
         for (int i : sel) {
           slots_[i].pending.push_back(PH_SADDLE);
           slots_[i].pc = joinb(slots_[i]);
         }
         return EXTREMZ_OK;
       case PC_SLOOPS_J:
-        ctl(s, OP_SLOOPS_JOIN_BEGIN);
-        launch(K_OTHER, k_wim_scan<T, false>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wim_collect<T, false>, grid_, 256, jobs, s, 1);
-        launch(K_OTHER, k_wim_min2_scan<T>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wim_min2_collect<T>, grid_, 256, jobs, s);
-        launch(K_APPLY, k_apply<T>, grid_, 256, jobs, s);
+        launch(K_OTHER, k_wim_scan<T, false>, nb, 256, jobs, s);
+        launch(K_OTHER, k_wim_collect<T, false>, nb, 256, jobs, s, 1);
+        launch(K_OTHER, k_wim_min2_scan<T>, nb, 256, jobs, s);
+        launch(K_OTHER, k_wim_min2_collect<T>, nb, 256, jobs, s);
+        launch(K_APPLY, k_apply<T>, nb, 256, jobs, s);
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
       case PC_SADDLE_J:
       case PC_FINAL_JOIN: {
-        ctl(s, OP_SADDLE_JOIN_BEGIN);
         std::vector<int> lists, once;
         for (int i : sel) (slots_[i].J.join_rows ? lists : once).push_back(i);
-        if (!lists.empty()) {
-          const Sel ls = make_sel(lists, false);
-          launch(K_OTHER, k_wis_mark<T, false>, grid_, 256, jobs, ls);
-          launch(K_OTHER, k_wis_update<T, false>, grid_, 256, jobs, ls);
-          launch(K_OTHER, k_wis_long<T, false>, 2 * sms_, 256, jobs, ls);
-        }
+        if (!lists.empty()) wis_scan<false>(make_span(lists), 1);
         if (!once.empty()) {
-          const Sel os = make_sel(once, false);
-          launch(K_OTHER, k_join_keys<T>, grid_, 256, jobs, os);
-          launch(K_OTHER, k_join_ids<T>, grid_, 256, jobs, os);
-          launch(K_OTHER, k_join_scan<T>, grid_, 256, jobs, os);
+          const Sel os = make_span(once);
+          launch(K_OTHER, k_join_keys<T>, blocks(os), 256, jobs, os);
+          launch(K_OTHER, k_join_ids<T>, blocks(os), 256, jobs, os);
+          launch(K_OTHER, k_join_scan<T>, blocks(os), 256, jobs, os);
+          launch(K_OTHER, k_wis_collect<T, false>, blocks(os), 256, jobs, os, 1);
         }
-        launch(K_OTHER, k_wis_collect<T, false>, grid_, 256, jobs, s, 1);
-        launch(K_APPLY, k_apply<T>, grid_, 256, jobs, s);
+        launch(K_APPLY, k_apply<T>, nb, 256, jobs, s);
         for (int i : sel) {
           slots_[i].pending.push_back(PH_SADDLE_JOIN);
           if (ph == PC_SADDLE_J) slots_[i].pc = endb(slots_[i]);
@@ -1301,26 +1313,18 @@ class BatchEngine {
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
       case PC_DET3:
-        ctl(s, OP_DETECT3_BEGIN);
-        launch(K_OTHER, k_wim_scan<T, true>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wim_collect<T, true>, grid_, 256, jobs, s, 0);
-        launch(K_OTHER, k_wis_mark<T, true>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wis_update<T, true>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wis_long<T, true>, 2 * sms_, 256, jobs, s);
-        launch(K_OTHER, k_wis_collect<T, true>, grid_, 256, jobs, s, 0);
+        launch(K_OTHER, k_wim_scan<T, true>, nb, 256, jobs, s);
+        launch(K_OTHER, k_wim_collect<T, true>, nb, 256, jobs, s, 0);
+        wis_scan<true>(s, 0);
         for (int i : sel) {
           slots_[i].pending.push_back(PH_DETECT3);
           slots_[i].pc = (slots_[i].p.flags & kFlagCensus) ? PC_DET3J : join3(slots_[i]);
         }
         return EXTREMZ_OK;
       case PC_DET3J:
-        ctl(s, OP_DETECT3_JOIN_BEGIN);
-        launch(K_OTHER, k_wim_scan<T, false>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wim_collect<T, false>, grid_, 256, jobs, s, 0);
-        launch(K_OTHER, k_wis_mark<T, false>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wis_update<T, false>, grid_, 256, jobs, s);
-        launch(K_OTHER, k_wis_long<T, false>, 2 * sms_, 256, jobs, s);
-        launch(K_OTHER, k_wis_collect<T, false>, grid_, 256, jobs, s, 0);
+        launch(K_OTHER, k_wim_scan<T, false>, nb, 256, jobs, s);
+        launch(K_OTHER, k_wim_collect<T, false>, nb, 256, jobs, s, 0);
+        wis_scan<false>(s, 0);
         for (int i : sel) slots_[i].pc = PC_FINAL_DETECT;
         return EXTREMZ_OK;
       case PC_FINAL_DETECT:
@@ -1332,24 +1336,44 @@ class BatchEngine {
     }
   }
 
+  // Blocks over a selection's listed tiles: a job's share of four per SM goes
+  // by its tiles.
+  Sel tile_span(const std::vector<int>& slots) const {
+    Sel s = make_sel(slots, true);
+    const long long total = s.off[s.n], budget = 4ll * sms_;
+    int off = 0;
+    for (int k = 0; k < s.n; ++k) {
+      const long long nt = slots_[s.idx[k]].ntiles;
+      s.off[k] = off;
+      off += (int)std::max(1ll, total <= budget ? nt : nt * budget / total);
+    }
+    s.off[s.n] = off;
+    return s;
+  }
+
+  // The incremental wrong-saddle scan of one side; fix: with its proposals.
+  template <bool kMax>
+  void wis_scan(const Sel& s, int fix) {
+    const Job<T>* jobs = jobs_dev_;
+    launch(K_OTHER, k_wis_mark<T, kMax>, blocks(s), 256, jobs, s);
+    launch(K_OTHER, k_wis_update<T, kMax>, blocks(s), 256, jobs, s);
+    launch(K_OTHER, k_wis_long<T, kMax>, blocks(s), 256, jobs, s);
+    launch(K_OTHER, k_wis_collect<T, kMax>, blocks(s), 256, jobs, s, fix);
+  }
+
   // Mismatch detection: dense the first time a job detects, then incremental
   // over the neighbourhoods of the vertices changed since.
   void detect(const std::vector<int>& sel) {
     std::vector<int> dense, incr;
     for (int i : sel) (slots_[i].dense_done ? incr : dense).push_back(i);
     if (!dense.empty()) {
-      const Sel s = make_sel(dense, false), st = make_sel(dense, true);
-      ctl(s, OP_DETECT_DENSE_BEGIN);
-      launch(K_DETECT, k_classify<T, true>, st.off[st.n], 256, (const Job<T>*)jobs_dev_, st);
-      ctl(s, OP_DETECT_END_DENSE);
+      const Sel st = make_sel(dense, true);
+      launch(K_DETECT, k_classify<T>, st.off[st.n], 256, (const Job<T>*)jobs_dev_, st);
       for (int i : dense) slots_[i].dense_done = true;
     }
     if (!incr.empty()) {
-      const Sel s = make_sel(incr, false);
-      ctl(s, OP_DETECT_BEGIN);
-      launch(K_DETECT, k_redetect<T>, grid_, 256, (const Job<T>*)jobs_dev_, s);
-      launch(K_DETECT, k_keep<T>, grid_, 256, (const Job<T>*)jobs_dev_, s);
-      ctl(s, OP_DETECT_END);
+      const Sel s = make_span(incr);
+      launch(K_DETECT, k_redetect<T>, blocks(s), 256, jobs_dev_, s);
     }
   }
 
@@ -1358,12 +1382,9 @@ class BatchEngine {
   template <bool kSplit>
   void wn_rounds(const Sel& s) {
     const Job<T>* jobs = jobs_dev_;
-    // Candidate lists are short next to the field (a few per cent of the
-    // saddles at most), so two blocks per SM cover them.
-    const int grid = std::min(grid_, 2 * sms_);
     for (int r = 0; r < kWnGridRounds; ++r) {
-      launch(K_WRONG_NBR, k_wn_vote<T, kSplit>, grid, 256, jobs, s, r);
-      launch(K_WRONG_NBR, k_wn_commit<T, kSplit>, grid, 256, jobs, s, r);
+      launch(K_WRONG_NBR, k_wn_vote<T, kSplit>, blocks(s), 256, jobs, s, r);
+      launch(K_WRONG_NBR, k_wn_commit<T, kSplit>, blocks(s), 256, jobs, s, r);
     }
     launch(K_WRONG_NBR, k_wn_resolve<T, kSplit>, s.n, 1024, jobs_dev_, s);
   }
@@ -1487,19 +1508,19 @@ class BatchEngine {
     if (ns2) EZ_CHECK(cudaMemsetAsync(J.drow2, 0, (size_t)ns2 * 2 * 4, st_));
     if (ns1 && J.join_rows) EZ_CHECK(cudaMemsetAsync(J.drow1, 0, (size_t)ns1 * 2 * 4, st_));
     // Every tile's pointers are computed in the first manifold round.
-    EZ_CHECK(cudaMemsetAsync(J.tdirty, 1, (size_t)jh.ntiles, st_));
+    EZ_CHECK(cudaMemsetAsync(J.tdirty, 1, (size_t)jh.ntiles * 4, st_));
     // Block stamps start below the first round's; no root is touched.
     EZ_CHECK(cudaMemsetAsync(J.bdirty, 0, (size_t)jh.nb * 4, st_));
     EZ_CHECK(cudaMemsetAsync(J.rtouch2, 0, (size_t)((N + 31) / 32) * 4, st_));
     EZ_CHECK(cudaMemsetAsync(J.rtouch1, 0, (size_t)((N + 31) / 32) * 4, st_));
-    // Proposal buffer at the sentinel, edit counters at -1 (:5082), stamps 0.
+    // Proposal buffer at the sentinel; edit counters, which only edit_type 0
+    // reads, at -1 (:5082); no changed vertex; arbitration votes, which only the
+    // ascending order reads, at 0.
     launch(K_OTHER, k_fill<K>, grid_, 256, J.delta, J.sentinel_key, (long long)N);
-    launch(K_OTHER, k_fill<int>, grid_, 256, J.counter, -1, (long long)N);
-    EZ_CHECK(cudaMemsetAsync(J.claim, 0, (size_t)N * 8, st_));
-    EZ_CHECK(cudaMemsetAsync(J.taken, 0, (size_t)N * 4, st_));
-    EZ_CHECK(cudaMemsetAsync(J.taken1, 0, (size_t)N * 4, st_));
-    EZ_CHECK(cudaMemsetAsync(J.dstamp, 0, (size_t)N * 4, st_));
-    EZ_CHECK(cudaMemsetAsync(J.rstamp, 0, (size_t)N * 4, st_));
+    if (J.edit_type == 0) launch(K_OTHER, k_fill<int>, grid_, 256, J.counter, -1, (long long)N);
+    if (!J.wn_lockstep) EZ_CHECK(cudaMemsetAsync(J.claim, 0, (size_t)N * 8, st_));
+    EZ_CHECK(cudaMemsetAsync(J.dbits, 0, (size_t)((N + 31) / 32) * 4, st_));
+    EZ_CHECK(cudaMemsetAsync(J.dbits1, 0, (size_t)((N + 31) / 32) * 4, st_));
     EZ_CHECK(cudaMemsetAsync(J.vchg, 0xff, (size_t)((N + 31) / 32) * 4, st_));
     EZ_CHECK(cudaMemsetAsync(J.wchg2, 0, (size_t)((N + 31) / 32) * 4, st_));
     EZ_CHECK(cudaMemsetAsync(J.wchg1, 0, (size_t)((N + 31) / 32) * 4, st_));

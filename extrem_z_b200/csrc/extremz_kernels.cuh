@@ -39,12 +39,12 @@ struct Job {
   int* mm;            // mismatch list: v | cat << 29
   int* mm_next;       // the list being rebuilt by the incremental detection
   uint8_t* mstat;     // current mismatch categories of every vertex
-  int* dirty;         // vertices whose value changed since the last detection
-  int* dstamp;        // dirty-list membership stamps (== dirty epoch)
-  int* rstamp;        // re-evaluation stamps (== detection epoch)
-  unsigned long long* claim;  // wrong-neighbour arbitration, (round << 32) | ~saddle
-  int* taken;         // wrong-neighbour flag stamps (== call id when flagged)
-  int* taken1;
+  int* dirty; int* dirty1;  // vertices whose value changed since the last detection, and since
+                            // the one before it (they change roles at each detection)
+  unsigned* dbits; unsigned* dbits1;  // their membership bitsets
+  unsigned long long* claim;  // wrong-neighbour arbitration in ascending saddle order,
+                              // (round << 32) | ~saddle
+  unsigned* taken; unsigned* taken1;  // bitsets: neighbours flagged in this manifold round
   int* cand; int* cand_next;  // wrong-neighbour candidate saddles (side being resolved)
   int* cand_j;        // join-side candidates, produced with the split side's
   int* flagged; int* flagged1;  // flagged neighbours (split / join)
@@ -60,8 +60,8 @@ struct Job {
   int* cpoff;         // per list (2-saddles, 1-saddles, maxima, minima) and
                       // 1024-id block: offset of the block's first entry
   int* pdd; int* pda; // decompressed steepest pointers, tile-compressed (k_direction)
-  uint8_t* tdirty;    // per tile: a value in the tile or its halo changed since
-                      // the tile's pointers were computed
+  int* tdirty;        // per tile: a value in the tile or its halo changed since the tile's
+                      // pointers were computed (k_apply lists the tile in cand_next then)
   unsigned* rtouch2; unsigned* rtouch1;  // bitsets: labels (of dds / das) of the vertices of
                                          // the tiles whose pointers this round recomputes
 
@@ -100,10 +100,12 @@ struct Job {
 };
 
 // Jobs served by one launch.  Every per-round kernel takes the device array of
-// job descriptors and a selection: indices into that array and, for tile
-// kernels, the exclusive prefix of the selected jobs' tile counts (a block's
-// flat index picks its job by binary search).  A plain correction is a
-// selection of one job.
+// job descriptors and a selection: indices into that array and the exclusive
+// prefix of the selected jobs' block counts (for tile kernels their tile
+// counts); a block's flat index picks its job by binary search.  A block works
+// on one job, so the jobs of a launch run side by side: when every block went
+// through all jobs in turn, a launch over 32 small jobs took 32 times the
+// latency of one.  A plain correction is a selection of one job.
 constexpr int kMaxSel = 64;
 struct Sel {
   int n;
@@ -111,31 +113,87 @@ struct Sel {
   int off[kMaxSel + 1];
 };
 
+// Job of a grid-stride kernel's block, the block's index among the job's blocks
+// and their number.
+template <class J>
+__device__ __forceinline__ J& span_job(J* __restrict__ jobs, const Sel& sel, int& blk, int& nblk) {
+  int lo = 0, hi = sel.n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (sel.off[mid] <= (int)blockIdx.x) lo = mid;
+    else hi = mid - 1;
+  }
+  blk = (int)blockIdx.x - sel.off[lo];
+  nblk = sel.off[lo + 1] - sel.off[lo];
+  return jobs[sel.idx[lo]];
+}
+
 // Indices into the device counter block.
 enum Ctr : int {
   C_MM = 0, C_CMAX, C_CMIN, C_CSAD, C_TOUCHED, C_NFC, C_NFC1, C_CAND, C_CAND_NEXT,
   C_WMC, C_WMC2, C_WSC, C_WMIN, C_WMIN2, C_WSCJ, C_NS2, C_NS1, C_NMAX, C_NMIN,
   C_E2, C_E1,  // row entries of the 2-saddles' / 1-saddles' original rows (upper bound)
   C_ERROR,
-  C_CHANGED,   // some value changed since the last manifold round began
+  C_CHANGED,   // some value changed since the last computed manifold round began
   C_DIRTY, C_MM_NEXT, C_CANDJ,
-  C_MFSKIP,    // this manifold round repeats the last one's inputs: kernels skip it
   C_MFDONE,    // a manifold round has run
-  C_MFREUSED,  // manifold rounds skipped so far
-  // Per-job epochs and stamps, advanced by k_ctl so that one launch can serve
-  // jobs at different points of their correction.
-  C_DEPOCH,    // dirty-list epoch (k_apply)
-  C_REPOCH,    // re-evaluation epoch (k_redetect / k_keep)
-  C_WNSTAMP,   // wrong-neighbour flag stamp, one per manifold round
+  C_MFREUSED,  // manifold rounds whose kernels found nothing changed
+  // Per-job epochs and stamps, so that one launch can serve jobs at different
+  // points of their correction.  There are no launches for bookkeeping: a
+  // counter is reset by a kernel that does not use it, or by the last block of
+  // one that does (last_block).
+  C_DEPOCH,    // detections so far; its parity picks dirty / dirty1
+  C_DIRTYP,    // entries of the dirty list of the detection before
+  C_AMAX, C_AMIN, C_ASAD,  // mismatch counts of the detection under way
+  C_WNSTAMP,   // computed manifold rounds so far; a round's stamp is this + 1
   C_WNROUND,   // wrong-neighbour arbitration round (vote high word)
   C_WNSMALL,   // this side's candidate list is small: the block completion does it all
-  C_MFFIRST,   // the manifold round being computed is the job's first: every input is new
-  C_TLIST,     // tiles listed for this manifold round's steepest pointers (k_tile_list)
-  C_WEP2, C_WEP1,  // wrong-saddle scan epochs (maxima, minima); epoch 1 computes every extremum
+  C_TLIST,     // tiles listed for the next manifold round's steepest pointers (k_apply)
+  C_WEP2, C_WEP1,  // wrong-saddle scans so far (maxima, minima); the first computes every extremum
   C_AFF,       // extrema queued for the current wrong-saddle update
   C_WLONG,     // of those, the ones with long entry lists (wlong)
+  C_DONE,      // blocks that have finished the current kernel (last_block)
   C_COUNT
 };
+
+// True, for the whole block, in the last of a job's nblk blocks to get here:
+// every write of the others is visible to it.  Leaves the ticket at zero.
+__device__ __forceinline__ bool last_block(int* ctr, int nblk) {
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ctr + C_DONE, 1) == nblk - 1;
+    if (last) ctr[C_DONE] = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return last != 0;
+}
+
+// A manifold round's outputs (labels, row slots, flagged neighbours and their
+// counts) are functions of the decompressed field alone, so when no value
+// changed since the last computed round began they are still in place and the
+// round's kernels return at once.
+__device__ __forceinline__ bool mf_skip(const int* ctr) {
+  return ctr[C_MFDONE] && !ctr[C_CHANGED];
+}
+__device__ __forceinline__ int mf_stamp(const int* ctr) { return ctr[C_WNSTAMP] + 1; }
+// Start of a computed round, in its first kernel (which uses none of these).
+__device__ __forceinline__ void mf_begin(int* ctr) {
+  ctr[C_NFC] = ctr[C_NFC1] = 0;
+  ctr[C_CAND] = ctr[C_CANDJ] = ctr[C_CAND_NEXT] = 0;
+}
+// End of a round, by one thread when everything else in it is done.
+__device__ __forceinline__ void mf_end(int* ctr) {
+  if (mf_skip(ctr)) {
+    ctr[C_MFREUSED] += 1;
+    return;
+  }
+  ctr[C_CHANGED] = 0;
+  ctr[C_MFDONE] = 1;
+  ctr[C_WNSTAMP] += 1;
+}
 // Error bits in ctr[C_ERROR].
 constexpr int kErrJump = 1, kErrPath = 2, kErrTile = 4, kErrResolve = 8;
 // Ids per changed-input flag of the jump (the CP-list block size, kCpBlock).
@@ -144,14 +202,25 @@ constexpr int kCpBlockJ = 1024;
 template <class T>
 __device__ __forceinline__ T tabs(T v) { return v < T(0) ? -v : v; }
 
+// Direction components packed two bits per direction (component + 1), so a
+// runtime direction index decodes with a shift and a mask.
+__host__ __device__ constexpr unsigned pack_dir(int axis) {
+  unsigned p = 0;
+  for (int d = 0; d < kNumDirs; ++d)
+    p |= (unsigned)((axis == 0 ? dir_x(d) : axis == 1 ? dir_y(d) : dir_z(d)) + 1) << (2 * d);
+  return p;
+}
+__device__ __forceinline__ int ddx(int d) { return (int)((pack_dir(0) >> (2 * d)) & 3u) - 1; }
+__device__ __forceinline__ int ddy(int d) { return (int)((pack_dir(1) >> (2 * d)) & 3u) - 1; }
+__device__ __forceinline__ int ddz(int d) { return (int)((pack_dir(2) >> (2 * d)) & 3u) - 1; }
+
 // ---------------------------------------------------------------------------
 // Classification over a shared-memory halo tile.
 //
-// Replaces classifyVertex_CUDA (:3720-3911).  kDetect = false writes the
-// original type and lower-star mask (type=0 call, :5289); kDetect = true is the
-// fused mismatch detection of the type=1 call (:3856-3910), appending each
-// mismatching vertex once with its categories (max, min, saddle) through
-// warp ballots.
+// Replaces classifyVertex_CUDA (:3720-3911): the original field's types and
+// lower-star masks (type=0 call, :5289) come from the direction pass over it;
+// k_classify is the fused mismatch detection of the type=1 call (:3856-3910),
+// appending each mismatching vertex once with its categories (max, min, saddle).
 // ---------------------------------------------------------------------------
 constexpr int TX = 32, TY = 8, TZ = 4;
 // Tile kernels run 256 threads, one per (x, y) column of the tile.
@@ -186,16 +255,21 @@ __device__ __forceinline__ const Job<T>& tile_job(const Job<T>* __restrict__ job
   return J;
 }
 
-// Marks the tiles whose halo tile contains vertex (x, y, z): those holding
-// one of its 26 neighbours or itself.
-__device__ __forceinline__ void mark_tiles(uint8_t* tdirty, const Dims& g, int x, int y, int z) {
+// Lists the tiles whose halo tile contains vertex (x, y, z), those holding one
+// of its 26 neighbours or itself, unless they are listed already (or not yet
+// computed: every mark is set before a job's first round).
+__device__ __forceinline__ void mark_tiles(int* tdirty, int* list, int* count, const Dims& g, int x,
+                                           int y, int z) {
   const int ntx = (g.W + TX - 1) / TX, nty = (g.H + TY - 1) / TY;
   const int x0 = max(x - 1, 0) / TX, x1 = min(x + 1, g.W - 1) / TX;
   const int y0 = max(y - 1, 0) / TY, y1 = min(y + 1, g.H - 1) / TY;
   const int z0 = max(z - 1, 0) / TZ, z1 = min(z + 1, g.D - 1) / TZ;
   for (int c = z0; c <= z1; ++c)
     for (int b = y0; b <= y1; ++b)
-      for (int a = x0; a <= x1; ++a) tdirty[(c * nty + b) * ntx + a] = 1;
+      for (int a = x0; a <= x1; ++a) {
+        const int t = (c * nty + b) * ntx + a;
+        if (tdirty[t] == 0 && atomicExch(tdirty + t, 1) == 0) list[atomicAdd(count, 1)] = t;
+      }
 }
 
 // Halo tile: TMA box (one bulk tensor copy, zero fill outside the grid) when
@@ -300,14 +374,14 @@ __device__ __forceinline__ void count_cats(int* ctr, int cat) {
   const unsigned bn = __ballot_sync(0xffffffffu, cat & kCatMin);
   const unsigned bs = __ballot_sync(0xffffffffu, cat & kCatSaddle);
   if (lane_id() == 0) {
-    if (bm) atomicAdd(ctr + C_CMAX, __popc(bm));
-    if (bn) atomicAdd(ctr + C_CMIN, __popc(bn));
-    if (bs) atomicAdd(ctr + C_CSAD, __popc(bs));
+    if (bm) atomicAdd(ctr + C_AMAX, __popc(bm));
+    if (bn) atomicAdd(ctr + C_AMIN, __popc(bn));
+    if (bs) atomicAdd(ctr + C_ASAD, __popc(bs));
   }
 }
 
-// kDetect = false classifies f (setup), true classifies g (detection).
-template <class T, bool kDetect>
+// The first detection of a job: the whole decompressed field.
+template <class T>
 __global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ jobs,
                                                   const __grid_constant__ Sel sel) {
   __shared__ Tile<T> s;
@@ -315,23 +389,21 @@ __global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ job
   int bx, by, bz;
   const Job<T>& J = tile_job(jobs, sel, bx, by, bz);
   const Dims g = J.dim;
-  const T* a = kDetect ? J.g : J.f;
   // The block decides together: its threads meet at barriers further on.
-  if (!__syncthreads_and(load_tile<T>(s, &bar, kDetect ? J.map_g : J.map_f,
-                                      kDetect ? J.tma_g : J.tma_f, a, g, bx, by, bz))) {
+  if (!__syncthreads_and(load_tile<T>(s, &bar, J.map_g, J.tma_g, J.g, g, bx, by, bz))) {
     if (threadIdx.x == 0) atomicOr(J.ctr + C_ERROR, kErrTile);
     return;
   }
   // Detection: the tile's mismatching vertices are gathered in shared memory
   // and appended with one global atomic per block (per warp, the appends of a
   // dense pass all queue on the same counter).
-  __shared__ int s_list[kDetect ? TZ * TY * TX : 1];
+  __shared__ int s_list[TZ * TY * TX];
   __shared__ int s_n, s_base, s_cat[3];
-  if (kDetect && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     s_n = 0;
     s_cat[0] = s_cat[1] = s_cat[2] = 0;
   }
-  if (kDetect) __syncthreads();
+  __syncthreads();
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   // A tile off the field's faces has every direction valid at every voxel.
   const bool interior = bx > 0 && by > 0 && bz > 0 && bx + TX < g.W && by + TY < g.H &&
@@ -346,32 +418,25 @@ __global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ job
       int lm, um;
       tile_masks(s, tx, ty, tz, valid, lm, um);
       const int t = type_from_masks(lm, um, valid, bc, J.tb);
-      if (!kDetect) {
-        J.otype[v] = (int8_t)t;
-        J.olm[v] = (uint16_t)lm;
-      } else {
-        const int cat = mismatch_cats(t, J.otype[v], lm, J.olm[v]);
-        J.mstat[v] = (uint8_t)cat;
-        if (cat) {
-          s_list[atomicAdd(&s_n, 1)] = v | (cat << kCatShift);
-          if (cat & kCatMax) atomicAdd(&s_cat[0], 1);
-          if (cat & kCatMin) atomicAdd(&s_cat[1], 1);
-          if (cat & kCatSaddle) atomicAdd(&s_cat[2], 1);
-        }
+      const int cat = mismatch_cats(t, J.otype[v], lm, J.olm[v]);
+      J.mstat[v] = (uint8_t)cat;
+      if (cat) {
+        s_list[atomicAdd(&s_n, 1)] = v | (cat << kCatShift);
+        if (cat & kCatMax) atomicAdd(&s_cat[0], 1);
+        if (cat & kCatMin) atomicAdd(&s_cat[1], 1);
+        if (cat & kCatSaddle) atomicAdd(&s_cat[2], 1);
       }
     }
   }
-  if (kDetect) {
-    __syncthreads();
-    if (threadIdx.x == 0 && s_n) {
-      s_base = atomicAdd(J.ctr + C_MM, s_n);
-      if (s_cat[0]) atomicAdd(J.ctr + C_CMAX, s_cat[0]);
-      if (s_cat[1]) atomicAdd(J.ctr + C_CMIN, s_cat[1]);
-      if (s_cat[2]) atomicAdd(J.ctr + C_CSAD, s_cat[2]);
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < s_n; k += blockDim.x) J.mm[s_base + k] = s_list[k];
+  __syncthreads();
+  if (threadIdx.x == 0 && s_n) {
+    s_base = atomicAdd(J.ctr + C_MM, s_n);
+    if (s_cat[0]) atomicAdd(J.ctr + C_CMAX, s_cat[0]);
+    if (s_cat[1]) atomicAdd(J.ctr + C_CMIN, s_cat[1]);
+    if (s_cat[2]) atomicAdd(J.ctr + C_CSAD, s_cat[2]);
   }
+  __syncthreads();
+  for (int k = threadIdx.x; k < s_n; k += blockDim.x) J.mm[s_base + k] = s_list[k];
 }
 
 // ---------------------------------------------------------------------------
@@ -379,11 +444,15 @@ __global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ job
 //
 // The type of v depends only on the values of v and its 14 neighbours, so after
 // the first dense detection only the closed neighbourhoods of vertices whose
-// value changed can change status.  k_redetect re-evaluates them (once each,
-// by stamp) and appends the mismatching ones to the next list; k_keep carries
-// over the entries of the previous list that were not re-evaluated.  The
-// resulting set equals a dense re-detection (the lists are unordered; every
-// consumer merges by atomic max).
+// value changed can change status.  k_redetect re-evaluates them, once each: a
+// vertex belongs to the first changed vertex of its closed neighbourhood, in
+// direction order with itself first, found from the membership bitset of the
+// changed vertices.  Beside that it carries over the entries of the previous
+// list that have no changed vertex in their neighbourhood.  The resulting set
+// equals a dense re-detection (the lists are unordered; every consumer merges by
+// atomic max).  Its last block publishes the counts and swaps the lists, so a
+// detection is one launch (four with a stamp per vertex, a second kernel for the
+// carried entries and two for the bookkeeping).
 // ---------------------------------------------------------------------------
 template <class T>
 __device__ __forceinline__ int global_type(const Job<T>& J, int v, int& lmask) {
@@ -415,64 +484,90 @@ __device__ __forceinline__ int global_type(const Job<T>& J, int v, int& lmask) {
   return __ldg(J.tb.lut + off + up);
 }
 
+__device__ __forceinline__ bool bit_of(const unsigned* bits, int v) {
+  return bits[v >> 5] >> (v & 31) & 1u;
+}
+
 template <class T>
-__global__ void __launch_bounds__(256) k_redetect(const Job<T>* __restrict__ jobs,
+__global__ void __launch_bounds__(256) k_redetect(Job<T>* __restrict__ jobs,
                                                   const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
-  const int n = J.ctr[C_DIRTY];
-  const int epoch = J.ctr[C_REPOCH];
-  const long long total = (long long)n * (kNumDirs + 1);
-  const long long stride = (long long)gridDim.x * blockDim.x;
+  int blk, nblk;
+  Job<T>& J = span_job(jobs, sel, blk, nblk);
   const Dims g = J.dim;
-  for (long long base = blockIdx.x * (long long)blockDim.x; base < total; base += stride) {
+  const bool odd = J.ctr[C_DEPOCH] & 1;
+  const int* __restrict__ dirty = odd ? J.dirty1 : J.dirty;
+  const unsigned* __restrict__ bits = odd ? J.dbits1 : J.dbits;
+  const int n = J.ctr[C_DIRTY], nmm = J.ctr[C_MM];
+  const long long nd = (long long)n * (kNumDirs + 1), total = nd + nmm;
+  const long long stride = (long long)nblk * blockDim.x;
+  for (long long base = blk * (long long)blockDim.x; base < total; base += stride) {
     const long long e = base + threadIdx.x;
     int cat = 0, v = -1;
-    if (e < total) {
-      const int c = J.dirty[e / (kNumDirs + 1)];
+    if (e < nd) {
+      const int c = dirty[e / (kNumDirs + 1)];
       const int d = (int)(e % (kNumDirs + 1)) - 1;  // -1: the vertex itself
       v = c;
       if (d >= 0) {
         int x, y, z;
         coords(c, g, x, y, z);
-        v = dir_valid(d, boundary_code(x, y, z, g.W, g.H, g.D))
-                ? c + dir_x(d) + dir_y(d) * g.W + dir_z(d) * g.W * g.H
-                : -1;
+        v = -1;
+        const int dx = ddx(d), dy = ddy(d), dz = ddz(d);
+        if ((unsigned)(x + dx) < (unsigned)g.W && (unsigned)(y + dy) < (unsigned)g.H &&
+            (unsigned)(z + dz) < (unsigned)g.D) {
+          v = c + dx + dy * g.W + dz * g.W * g.H;
+          // From v, c lies in direction d ^ 1: v is c's unless v itself or a
+          // neighbour in an earlier direction changed too.
+          const int valid = valid_mask(boundary_code(x + dx, y + dy, z + dz, g.W, g.H, g.D));
+          bool earlier = bit_of(bits, v);
+#pragma unroll
+          for (int k = 0; k < kNumDirs; ++k)
+            if (k < (d ^ 1) && (valid >> k & 1))
+              earlier |= bit_of(bits, v + dir_x(k) + dir_y(k) * g.W + dir_z(k) * g.W * g.H);
+          if (earlier) v = -1;
+        }
       }
-      if (v >= 0 && atomicExch(J.rstamp + v, epoch) != epoch) {
+      if (v >= 0) {
         int lm;
         const int t = global_type(J, v, lm);
         cat = mismatch_cats(t, J.otype[v], lm, J.olm[v]);
         J.mstat[v] = (uint8_t)cat;
       }
+    } else if (e < total) {
+      const int ent = J.mm[e - nd];
+      v = ent & ((1 << kCatShift) - 1);
+      int x, y, z;
+      coords(v, g, x, y, z);
+      const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
+      bool near = bit_of(bits, v);
+#pragma unroll
+      for (int k = 0; k < kNumDirs; ++k)
+        if (valid >> k & 1)
+          near |= bit_of(bits, v + dir_x(k) + dir_y(k) * g.W + dir_z(k) * g.W * g.H);
+      if (!near) cat = (unsigned)ent >> kCatShift;
     }
     const int slot = warp_append(J.ctr + C_MM_NEXT, cat != 0, 0xffffffffu);
     if (slot >= 0) J.mm_next[slot] = v | (cat << kCatShift);
     count_cats(J.ctr, cat);
   }
-  }
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) k_keep(const Job<T>* __restrict__ jobs,
-                                              const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
-  const int n = J.ctr[C_MM];
-  const int epoch = J.ctr[C_REPOCH];
-  const int stride = gridDim.x * blockDim.x;
-  for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
-    const int e = base + threadIdx.x;
-    int ent = 0, cat = 0;
-    if (e < n) {
-      ent = J.mm[e];
-      const int v = ent & ((1 << kCatShift) - 1);
-      if (J.rstamp[v] != epoch) cat = (unsigned)ent >> kCatShift;
-    }
-    const int slot = warp_append(J.ctr + C_MM_NEXT, cat != 0, 0xffffffffu);
-    if (slot >= 0) J.mm_next[slot] = ent;
-    count_cats(J.ctr, cat);
-  }
+  // The bits of the detection before this one, for the next edits.
+  const int np = J.ctr[C_DIRTYP];
+  const int* prev = odd ? J.dirty : J.dirty1;
+  unsigned* pbits = odd ? J.dbits : J.dbits1;
+  for (int e = blk * blockDim.x + threadIdx.x; e < np; e += (int)stride) pbits[prev[e] >> 5] = 0u;
+  if (last_block(J.ctr, nblk) && threadIdx.x == 0) {
+    volatile int* c = J.ctr;  // counted by other blocks
+    int* t = J.mm;
+    J.mm = J.mm_next;
+    J.mm_next = t;
+    c[C_MM] = c[C_MM_NEXT];
+    c[C_MM_NEXT] = 0;
+    c[C_CMAX] = c[C_AMAX];
+    c[C_CMIN] = c[C_AMIN];
+    c[C_CSAD] = c[C_ASAD];
+    c[C_AMAX] = c[C_AMIN] = c[C_ASAD] = 0;
+    c[C_DIRTYP] = n;
+    c[C_DIRTY] = 0;
+    c[C_DEPOCH] += 1;
   }
 }
 
@@ -488,18 +583,6 @@ __global__ void __launch_bounds__(256) k_keep(const Job<T>* __restrict__ jobs,
 // only tiles marked dirty (a value in the tile or its halo changed) are
 // recomputed; the others keep their pointers, which depend on nothing else.
 // ---------------------------------------------------------------------------
-// Direction components packed two bits per direction (component + 1), so a
-// runtime direction index decodes with a shift and a mask.
-__host__ __device__ constexpr unsigned pack_dir(int axis) {
-  unsigned p = 0;
-  for (int d = 0; d < kNumDirs; ++d)
-    p |= (unsigned)((axis == 0 ? dir_x(d) : axis == 1 ? dir_y(d) : dir_z(d)) + 1) << (2 * d);
-  return p;
-}
-__device__ __forceinline__ int ddx(int d) { return (int)((pack_dir(0) >> (2 * d)) & 3u) - 1; }
-__device__ __forceinline__ int ddy(int d) { return (int)((pack_dir(1) >> (2 * d)) & 3u) - 1; }
-__device__ __forceinline__ int ddz(int d) { return (int)((pack_dir(2) >> (2 * d)) & 3u) - 1; }
-
 // Steepest-ascent and steepest-descent directions of one tile voxel: the
 // maximum (minimum) of (value, id) over the voxel and its valid neighbours.
 // Ids are scanned in ascending order so that ">=" keeps the larger id on a tie;
@@ -638,33 +721,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 6) k_direction(const
   __shared__ int hexit[TZ * TY * TX], lexit[TZ * TY * TX];
   int bx, by, bz, tile;
   const Job<T>& J = tile_job(jobs, sel, bx, by, bz, &tile);
-  if (kDec && J.ctr[C_MFSKIP]) return;  // same inputs as the last manifold round
-  if (kDec && !J.tdirty[tile]) return;  // tile and halo unchanged: pointers stand
+  if (kDec) {
+    if (mf_skip(J.ctr)) return;  // same inputs as the last manifold round
+    if (tile == 0 && threadIdx.x == 0) mf_begin(J.ctr);
+    if (!J.tdirty[tile]) return;  // tile and halo unchanged: pointers stand
+  }
   if (!direction_tile<T, kDec>(J, s, &bar, hnext, lnext, hexit, lexit, bx, by, bz, 0, true))
     return;
   if (kDec && threadIdx.x == 0) J.tdirty[tile] = 0;
-}
-
-// The tiles of each selected job whose tile or halo changed since their
-// pointers were computed (every tile in a job's first round), into the
-// job's tile list (cand_next, free at this point of a manifold round;
-// count C_TLIST, zeroed when the round begins).
-template <class T>
-__global__ void __launch_bounds__(256) k_tile_list(const Job<T>* __restrict__ jobs,
-                                                   const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    if (J.ctr[C_MFSKIP]) continue;
-    const int nt = ((J.dim.W + TX - 1) / TX) * ((J.dim.H + TY - 1) / TY) *
-                   ((J.dim.D + TZ - 1) / TZ);
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x; base < nt; base += stride) {  // uniform per warp
-      const int t = base + threadIdx.x;
-      const bool dirty = t < nt && J.tdirty[t];
-      const int slot = warp_append(J.ctr + C_TLIST, dirty, 0xffffffffu);
-      if (slot >= 0) J.cand_next[slot] = t;
-    }
-  }
 }
 
 // A manifold round's steepest pointers of the decompressed field: a fixed
@@ -682,30 +746,30 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
   __shared__ int16_t hnext[TZ * TY * TX], lnext[TZ * TY * TX];
   __shared__ int hexit[TZ * TY * TX], lexit[TZ * TY * TX];
   unsigned loads = 0;  // TMA loads issued by this block: the barrier's phase
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    if (J.ctr[C_MFSKIP]) continue;
-    const int n = J.ctr[C_TLIST];
-    const int ntx = (J.dim.W + TX - 1) / TX, nty = (J.dim.H + TY - 1) / TY;
-    for (int k = blockIdx.x; k < n; k += gridDim.x) {
-      const int t = J.cand_next[k];
-      const int bx = (t % ntx) * TX, by = ((t / ntx) % nty) * TY, bz = (t / (ntx * nty)) * TZ;
-      __syncthreads();  // every thread is done with the shared tile of the last one
-      const bool tma = J.tma_g != 0;
-      if (!direction_tile<T, true>(J, s, &bar, hnext, lnext, hexit, lexit, bx, by, bz,
-                                   loads & 1u, loads == 0))
-        return;
-      loads += tma;
-      if (threadIdx.x == 0) J.tdirty[t] = 0;
-      const int x = bx + (int)threadIdx.x % TX, y = by + (int)threadIdx.x / TX;
-      if (x < J.dim.W && y < J.dim.H) {
-        for (int tz = 0; tz < TZ && bz + tz < J.dim.D; ++tz) {
-          const int v = x + y * J.dim.W + (bz + tz) * J.dim.W * J.dim.H;
-          const int r2 = J.dds[v], r1 = J.das[v];
-          // Read first: most roots are marked by many vertices.
-          if (!(J.rtouch2[r2 >> 5] >> (r2 & 31) & 1u)) atomicOr(J.rtouch2 + (r2 >> 5), 1u << (r2 & 31));
-          if (!(J.rtouch1[r1 >> 5] >> (r1 & 31) & 1u)) atomicOr(J.rtouch1 + (r1 >> 5), 1u << (r1 & 31));
-        }
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (mf_skip(J.ctr)) return;
+  if (blk == 0 && threadIdx.x == 0) mf_begin(J.ctr);
+  const int n = J.ctr[C_TLIST];
+  const int ntx = (J.dim.W + TX - 1) / TX, nty = (J.dim.H + TY - 1) / TY;
+  for (int k = blk; k < n; k += nblk) {
+    const int t = J.cand_next[k];
+    const int bx = (t % ntx) * TX, by = ((t / ntx) % nty) * TY, bz = (t / (ntx * nty)) * TZ;
+    __syncthreads();  // every thread is done with the shared tile of the last one
+    const bool tma = J.tma_g != 0;
+    if (!direction_tile<T, true>(J, s, &bar, hnext, lnext, hexit, lexit, bx, by, bz, loads & 1u,
+                                 loads == 0))
+      return;
+    loads += tma;
+    if (threadIdx.x == 0) J.tdirty[t] = 0;
+    const int x = bx + (int)threadIdx.x % TX, y = by + (int)threadIdx.x / TX;
+    if (x < J.dim.W && y < J.dim.H) {
+      for (int tz = 0; tz < TZ && bz + tz < J.dim.D; ++tz) {
+        const int v = x + y * J.dim.W + (bz + tz) * J.dim.W * J.dim.H;
+        const int r2 = J.dds[v], r1 = J.das[v];
+        // Read first: most roots are marked by many vertices.
+        if (!(J.rtouch2[r2 >> 5] >> (r2 & 31) & 1u)) atomicOr(J.rtouch2 + (r2 >> 5), 1u << (r2 & 31));
+        if (!(J.rtouch1[r1 >> 5] >> (r1 & 31) & 1u)) atomicOr(J.rtouch1 + (r1 >> 5), 1u << (r1 & 31));
       }
     }
   }
@@ -726,9 +790,12 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
 template <class T, bool kDec, bool kLater = false>
 __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ jobs,
                                                const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
-  if (kDec && J.ctr[C_MFSKIP]) continue;
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (kDec) {
+    if (mf_skip(J.ctr)) return;
+    if (blk == 0 && threadIdx.x == 0) J.ctr[C_TLIST] = 0;  // the listed tiles are done
+  }
   // Original field: in place on ds / as.  Decompressed field: from the
   // tile-compressed pointers pdd / pda (kept for the next round) into dds / das.
   const int* a = kDec ? J.pdd : J.ds;
@@ -778,7 +845,7 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       // value, either label, or the value of either label's root).  The
       // change bitset starts full, so the first round marks every vertex.
       const unsigned c1 = vchg[u1 >> 5] >> (u1 & 31), c2 = vchg[u2 >> 5] >> (u2 & 31);
-      dirtyv[v] = ((o1 != u1) | (o2 != u2) | ((c0 | c1 | c2) & 1u)) ? (uint8_t)J.ctr[C_WNSTAMP]
+      dirtyv[v] = ((o1 != u1) | (o2 != u2) | ((c0 | c1 | c2) & 1u)) ? (uint8_t)mf_stamp(J.ctr)
                                                                     : (uint8_t)0;
       mis[v] = (uint8_t)((u1 != r1) | (u2 != r2) << 1);
     }
@@ -803,7 +870,7 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       // old labels of the recomputed tiles' vertices) keeps its labels and
       // mismatch bits and has no changed input (a changed value, own or of a
       // root, lies in a recomputed tile too).
-      const int stamp = J.ctr[C_WNSTAMP];
+      const int stamp = mf_stamp(J.ctr);
       const unsigned st8 = (unsigned)stamp & 0xffu;
       // Returns the quad's labels through u1 / u2 (the old ones when it is
       // not followed) and the old ones through o1 / o2 (-1 in a first round).
@@ -891,17 +958,16 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
         if (dv) J.bdirty[v0 >> 10] = stamp;
       };
       const int nq = N >> 2;
-      const int qstride = gridDim.x * blockDim.x;
-      for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += qstride) {
+      const int qstride = nblk * blockDim.x;
+      for (int q = blk * blockDim.x + threadIdx.x; q < nq; q += qstride) {
         int u1[4], u2[4], o1[4], o2[4];
         quad(q << 2, u1, u2, o1, o2);
       }
-      continue;
+      return;
     }
   }
-  const int stride = gridDim.x * blockDim.x;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < N; v += stride) jump_one(v);
-  }
+  const int stride = nblk * blockDim.x;
+  for (int v = blk * blockDim.x + threadIdx.x; v < N; v += stride) jump_one(v);
 }
 
 // ---------------------------------------------------------------------------
@@ -1386,13 +1452,13 @@ __device__ __forceinline__ void propose(const Job<T>& J, int i, T d) {
 // c_loop(0..2) (:2887-3055) over the mismatch list.
 template <class T>
 __global__ void __launch_bounds__(256) k_propose_cp(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
   const int n = J.ctr[C_MM];
-  const int stride = gridDim.x * blockDim.x;
+  const int stride = nblk * blockDim.x;
   const Dims g = J.dim;
   const int WH = g.W * g.H;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+  for (int e = blk * blockDim.x + threadIdx.x; e < n; e += stride) {
     const int ent = J.mm[e];
     const int v = ent & ((1 << kCatShift) - 1);
     const int cat = (unsigned)ent >> kCatShift;
@@ -1459,54 +1525,63 @@ __global__ void __launch_bounds__(256) k_propose_cp(const Job<T>* __restrict__ j
       }
     }
   }
-  }
 }
 
 // applyDeltaBuffer (:3061-3111) over the vertices that received a proposal;
 // the proposal buffer is reset to the sentinel on the way (init_delta).
 template <class T>
 __global__ void __launch_bounds__(256) k_apply(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
-  const int dirty_epoch = J.ctr[C_DEPOCH];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  const bool odd = J.ctr[C_DEPOCH] & 1;
+  int* dirty = odd ? J.dirty1 : J.dirty;
+  unsigned* bits = odd ? J.dbits1 : J.dbits;
   const int n = J.ctr[C_TOUCHED];
-  const int stride = gridDim.x * blockDim.x;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    const int v = J.touched[e];
-    const T d = KeyOf<T>::dec(J.delta[v]);
-    J.delta[v] = J.sentinel_key;
-    if (d == J.sentinel) continue;
-    const T fv = J.f[v];
-    const T g0 = J.g[v];
-    T gv = g0;
-    if (J.edit_type == 0) {
-      const int c = J.counter[v];
-      if (c < J.q - 1 && tabs(T(fv - (gv + d))) <= J.bound) {
-        gv += d;
-        J.counter[v] = c + 1;
+  const int stride = nblk * blockDim.x;
+  for (int base = blk * blockDim.x; base < n; base += stride) {  // uniform per warp
+    const int e = base + threadIdx.x;
+    int v = 0;
+    bool fresh = false;  // changed, and not in the dirty list yet
+    if (e < n) {
+      v = J.touched[e];
+      const T d = KeyOf<T>::dec(J.delta[v]);
+      J.delta[v] = J.sentinel_key;
+      const T fv = J.f[v];
+      const T g0 = J.g[v];
+      T gv = g0;
+      if (d == J.sentinel) {
+      } else if (J.edit_type == 0) {
+        const int c = J.counter[v];
+        if (c < J.q - 1 && tabs(T(fv - (gv + d))) <= J.bound) {
+          gv += d;
+          J.counter[v] = c + 1;
+        } else {
+          J.counter[v] = J.q;
+          gv = fv - J.bound;
+        }
       } else {
-        J.counter[v] = J.q;
-        gv = fv - J.bound;
+        if (tabs(T(fv - (gv + d))) <= J.bound) gv += d;
+        else gv = fv - J.bound;
       }
-    } else {
-      if (tabs(T(fv - (gv + d))) <= J.bound) gv += d;
-      else gv = fv - J.bound;
+      if (KeyOf<T>::enc(gv) != KeyOf<T>::enc(g0)) {
+        J.g[v] = gv;
+        J.ctr[C_CHANGED] = 1;
+        const int w = v >> 5;
+        const unsigned bit = 1u << (v & 31);
+        fresh = !(atomicOr(bits + w, bit) & bit);
+        atomicOr(J.vchg + w, bit);
+        atomicOr(J.wchg2 + w, bit);
+        if (J.join_rows) atomicOr(J.wchg1 + w, bit);
+        if (J.edited) atomicOr(J.edited + w, bit);
+        int x, y, z;
+        coords(v, J.dim, x, y, z);
+        mark_tiles(J.tdirty, J.cand_next, J.ctr + C_TLIST, J.dim, x, y, z);
+      }
     }
-    J.g[v] = gv;
-    if (KeyOf<T>::enc(gv) != KeyOf<T>::enc(g0)) {
-      J.ctr[C_CHANGED] = 1;
-      atomicOr(J.vchg + (v >> 5), 1u << (v & 31));
-      atomicOr(J.wchg2 + (v >> 5), 1u << (v & 31));
-      atomicOr(J.wchg1 + (v >> 5), 1u << (v & 31));
-      if (J.edited) atomicOr(J.edited + (v >> 5), 1u << (v & 31));
-      int x, y, z;
-      coords(v, J.dim, x, y, z);
-      mark_tiles(J.tdirty, J.dim, x, y, z);
-      if (atomicExch(J.dstamp + v, dirty_epoch) != dirty_epoch)
-        J.dirty[atomicAdd(J.ctr + C_DIRTY, 1)] = v;
-    }
+    const int slot = warp_append(J.ctr + C_DIRTY, fresh, 0xffffffffu);
+    if (slot >= 0) dirty[slot] = v;
   }
-  }
+  if (last_block(J.ctr, nblk) && threadIdx.x == 0) J.ctr[C_TOUCHED] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1685,23 +1760,6 @@ __device__ __forceinline__ bool saddle_row(const Job<T>& J, const int* __restric
   return (mb >> (kSplit ? 0 : 1)) & 1;
 }
 
-// Clears the value-change bitset after a computed round's jump has read it.
-template <class T>
-__global__ void k_clear_changed(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    if (J.ctr[C_MFSKIP]) continue;
-    const int nw = (J.dim.N + 31) >> 5;
-    const int stride = gridDim.x * blockDim.x;
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += stride) {
-      J.vchg[w] = 0u;
-      J.rtouch2[w] = 0u;
-      J.rtouch1[w] = 0u;
-    }
-
-  }
-}
-
 // Whether any input of saddle s's rows changed since the previous computed
 // round: the changed-input byte of s or of a neighbour (see k_jump2).
 template <class T>
@@ -1711,7 +1769,7 @@ __device__ __forceinline__ bool saddle_inputs_changed(const Job<T>& J, int s) {
   coords(s, g, x, y, z);
   const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
   // Changed-input bytes hold the low byte of the round stamp that set them.
-  const uint8_t st8 = (uint8_t)J.ctr[C_WNSTAMP];
+  const uint8_t st8 = (uint8_t)mf_stamp(J.ctr);
   bool d = J.dirtyv[s] == st8;
 #pragma unroll
   for (int k = 0; k < kNumDirs; ++k)
@@ -1741,161 +1799,165 @@ template <class T>
 __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict__ jobs,
                                                         const __grid_constant__ Sel sel) {
   __shared__ int off[kNumDirs];
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    if (J.ctr[C_MFSKIP]) continue;
-    __syncthreads();  // every thread is done with the last job's offsets
-    fill_offsets(off, J.dim);
-    __syncthreads();
-    // No mismatch at the last detection and no value changed since.
-    const bool known = J.ctr[C_MM] == 0 && J.ctr[C_DIRTY] == 0;
-    const int ns2 = J.ctr[C_NS2], ns1 = J.ctr[C_NS1];
-    const int nb = (J.dim.N + kCpBlock - 1) / kCpBlock;
-    const int chunk = J.pass_chunk;
-    const int nchunk = (nb + chunk - 1) / chunk;
-    // In the first round every changed-input byte is set (the change bitset
-    // starts full), so the check is skipped.
-    const bool all_new = J.ctr[C_MFFIRST] != 0;
-    // Later rounds first ask the jump's per-block flags (written when N is a
-    // multiple of 4) whether any changed-input byte is set where the chunk's
-    // saddles could see one: the 3 x 3 row windows of the planes and rows
-    // next to the chunk, one id wider on each side.
-    const bool by_block = !all_new && (J.dim.N & 3) == 0;
-    const long long W = J.dim.W, WH = W * J.dim.H, N = J.dim.N;
-    for (int c = blockIdx.x; c < nchunk; c += gridDim.x) {
-      const int b0 = c * chunk, b1 = min(b0 + chunk, nb);
-      const int a2 = J.cpoff[b0], e2 = b1 < nb ? J.cpoff[b1] : ns2;
-      const int a1 = J.cpoff[nb + b0], e1 = b1 < nb ? J.cpoff[nb + b1] : ns1;
-      const int n2 = e2 - a2, n = n2 + (e1 - a1);
-      if (by_block) {
-        int seen = 0;
-        if (threadIdx.x < 9) {
-          const int t = (int)threadIdx.x;  // signed: the offsets below go negative
-          const long long off = (long long)(t / 3 - 1) * WH + (long long)(t % 3 - 1) * W;
-          const long long lo = max(0ll, (long long)b0 * kCpBlock + off - 1);
-          const long long hi = min(N - 1, (long long)b1 * kCpBlock - 1 + off + 1);
-          const int stamp = J.ctr[C_WNSTAMP];
-          for (long long b = lo >> 10; b <= (hi >> 10) && lo <= hi; ++b)
-            seen |= J.bdirty[b] == stamp;
-        }
-        if (!__syncthreads_or(seen)) {  // no saddle here has a changed input
-          // Seed bits as computed in an earlier round; none set: nothing to list.
-          if (J.hcnt[c] == 0) continue;
-          for (int base = 0; base < n; base += blockDim.x) {
-            const int k = base + threadIdx.x;
-            const bool split = k < n2;
-            bool has = false;
-            int s = 0;
-            if (k < n) {
-              const int i = split ? a2 + k : a1 + k - n2;
-              s = split ? J.sad2[i] : J.sad1[i];
-              has = (split ? J.has2 : J.has1)[i] != 0;
-            }
-            const int slot2 = warp_append(J.ctr + C_CAND, has && split, 0xffffffffu);
-            if (slot2 >= 0) J.cand[slot2] = s;
-            const int slot1 = warp_append(J.ctr + C_CANDJ, has && !split, 0xffffffffu);
-            if (slot1 >= 0) J.cand_j[slot1] = s;
-          }
-          continue;
-        }
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (mf_skip(J.ctr)) return;
+  fill_offsets(off, J.dim);
+  // The bitsets that the round's jump has read, and the flags of the last
+  // round's wrong neighbours, start empty again.
+  const int nw = (J.dim.N + 31) >> 5;
+  for (int w = blk * blockDim.x + threadIdx.x; w < nw; w += nblk * blockDim.x) {
+    J.vchg[w] = 0u;
+    J.rtouch2[w] = 0u;
+    J.rtouch1[w] = 0u;
+    J.taken[w] = 0u;
+    J.taken1[w] = 0u;
+  }
+  __syncthreads();
+  // No mismatch at the last detection and no value changed since.
+  const bool known = J.ctr[C_MM] == 0 && J.ctr[C_DIRTY] == 0;
+  const int ns2 = J.ctr[C_NS2], ns1 = J.ctr[C_NS1];
+  const int nb = (J.dim.N + kCpBlock - 1) / kCpBlock;
+  const int chunk = J.pass_chunk;
+  const int nchunk = (nb + chunk - 1) / chunk;
+  // In the first round every changed-input byte is set (the change bitset
+  // starts full), so the check is skipped.
+  const bool all_new = J.ctr[C_MFDONE] == 0;
+  // Later rounds first ask the jump's per-block flags (written when N is a
+  // multiple of 4) whether any changed-input byte is set where the chunk's
+  // saddles could see one: the 3 x 3 row windows of the planes and rows
+  // next to the chunk, one id wider on each side.
+  const bool by_block = !all_new && (J.dim.N & 3) == 0;
+  const long long W = J.dim.W, WH = W * J.dim.H, N = J.dim.N;
+  for (int c = blk; c < nchunk; c += nblk) {
+    const int b0 = c * chunk, b1 = min(b0 + chunk, nb);
+    const int a2 = J.cpoff[b0], e2 = b1 < nb ? J.cpoff[b1] : ns2;
+    const int a1 = J.cpoff[nb + b0], e1 = b1 < nb ? J.cpoff[nb + b1] : ns1;
+    const int n2 = e2 - a2, n = n2 + (e1 - a1);
+    if (by_block) {
+      int seen = 0;
+      if (threadIdx.x < 9) {
+        const int t = (int)threadIdx.x;  // signed: the offsets below go negative
+        const long long off = (long long)(t / 3 - 1) * WH + (long long)(t % 3 - 1) * W;
+        const long long lo = max(0ll, (long long)b0 * kCpBlock + off - 1);
+        const long long hi = min(N - 1, (long long)b1 * kCpBlock - 1 + off + 1);
+        const int stamp = mf_stamp(J.ctr);
+        for (long long b = lo >> 10; b <= (hi >> 10) && lo <= hi; ++b)
+          seen |= J.bdirty[b] == stamp;
       }
-      int nhas = 0;  // seed bits set in the chunk
-      for (int base = 0; base < n; base += blockDim.x) {  // uniform in the block
-        const int k = base + threadIdx.x;
-        const bool split = k < n2;
-        bool has = false;
-        int s = 0;
-        if (k < n) {
-          const int i = split ? a2 + k : a1 + k - n2;
-          uint8_t* hb = split ? J.has2 : J.has1;
-          s = split ? J.sad2[i] : J.sad1[i];
-          const uint8_t kept = hb[i];  // loaded with the id: no round trip of its own
-          if (all_new || saddle_inputs_changed(J, s)) {
-            has = split ? saddle_row<T, true>(J, off, i, s, known)
-                        : saddle_row<T, false>(J, off, i, s, known);
-            hb[i] = (uint8_t)has;
-          } else {  // rows and seed bit as computed in an earlier round
-            has = kept != 0;
+      if (!__syncthreads_or(seen)) {  // no saddle here has a changed input
+        // Seed bits as computed in an earlier round; none set: nothing to list.
+        if (J.hcnt[c] == 0) continue;
+        for (int base = 0; base < n; base += blockDim.x) {
+          const int k = base + threadIdx.x;
+          const bool split = k < n2;
+          bool has = false;
+          int s = 0;
+          if (k < n) {
+            const int i = split ? a2 + k : a1 + k - n2;
+            s = split ? J.sad2[i] : J.sad1[i];
+            has = (split ? J.has2 : J.has1)[i] != 0;
           }
+          const int slot2 = warp_append(J.ctr + C_CAND, has && split, 0xffffffffu);
+          if (slot2 >= 0) J.cand[slot2] = s;
+          const int slot1 = warp_append(J.ctr + C_CANDJ, has && !split, 0xffffffffu);
+          if (slot1 >= 0) J.cand_j[slot1] = s;
         }
-        const int slot2 = warp_append(J.ctr + C_CAND, has && split, 0xffffffffu);
-        if (slot2 >= 0) J.cand[slot2] = s;
-        const int slot1 = warp_append(J.ctr + C_CANDJ, has && !split, 0xffffffffu);
-        if (slot1 >= 0) J.cand_j[slot1] = s;
-        nhas += __syncthreads_count(has);
+        continue;
       }
-      if (threadIdx.x == 0) J.hcnt[c] = nhas;
     }
+    int nhas = 0;  // seed bits set in the chunk
+    for (int base = 0; base < n; base += blockDim.x) {  // uniform in the block
+      const int k = base + threadIdx.x;
+      const bool split = k < n2;
+      bool has = false;
+      int s = 0;
+      if (k < n) {
+        const int i = split ? a2 + k : a1 + k - n2;
+        uint8_t* hb = split ? J.has2 : J.has1;
+        s = split ? J.sad2[i] : J.sad1[i];
+        const uint8_t kept = hb[i];  // loaded with the id: no round trip of its own
+        if (all_new || saddle_inputs_changed(J, s)) {
+          has = split ? saddle_row<T, true>(J, off, i, s, known)
+                      : saddle_row<T, false>(J, off, i, s, known);
+          hb[i] = (uint8_t)has;
+        } else {  // rows and seed bit as computed in an earlier round
+          has = kept != 0;
+        }
+      }
+      const int slot2 = warp_append(J.ctr + C_CAND, has && split, 0xffffffffu);
+      if (slot2 >= 0) J.cand[slot2] = s;
+      const int slot1 = warp_append(J.ctr + C_CANDJ, has && !split, 0xffffffffu);
+      if (slot1 >= 0) J.cand_j[slot1] = s;
+      nhas += __syncthreads_count(has);
+    }
+    if (threadIdx.x == 0) J.hcnt[c] = nhas;
   }
 }
 
 template <class T, bool kSplit>
 __global__ void __launch_bounds__(256) k_wn_vote(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel,
                                                  int r) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
-  if (J.ctr[C_MFSKIP] || J.wn_lockstep) continue;
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (mf_skip(J.ctr) || J.wn_lockstep) return;
   if (r == 0) {
     // A short list (every round after the first few of a correction) goes to
     // the block completion whole: the grid rounds would be launches with
     // nothing to do.
     const bool small = J.ctr[C_CAND] <= kWnBlockMax;
-    if (blockIdx.x == 0 && threadIdx.x == 0) J.ctr[C_WNSMALL] = small;
-    if (small) continue;
+    if (blk == 0 && threadIdx.x == 0) J.ctr[C_WNSMALL] = small;
+    if (small) return;
   } else if (J.ctr[C_WNSMALL]) {
-    continue;
+    return;
   }
   const unsigned long long round = (unsigned)(J.ctr[C_WNROUND] + r + 1);
-  const int stamp = J.ctr[C_WNSTAMP];
   const int n = J.ctr[C_CAND + (r & 1)];
   const int* cur = (r & 1) ? J.cand_next : J.cand;
   // The list this round's commit fills (the one read two rounds ago).
-  if (blockIdx.x == 0 && threadIdx.x == 0) J.ctr[C_CAND + ((r + 1) & 1)] = 0;
-  const int* taken = kSplit ? J.taken : J.taken1;
-  const int stride = gridDim.x * blockDim.x;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+  if (blk == 0 && threadIdx.x == 0) J.ctr[C_CAND + ((r + 1) & 1)] = 0;
+  const unsigned* taken = kSplit ? J.taken : J.taken1;
+  const int stride = nblk * blockDim.x;
+  for (int e = blk * blockDim.x + threadIdx.x; e < n; e += stride) {
     const int s = cur[e];
     int ids[kNumDirs];
     const int k = wn_candidates<T, kSplit>(J, s, ids);
     const unsigned long long vote = (round << 32) | (unsigned)(~s);
     for (int j = 0; j < k; ++j)
-      if (taken[ids[j]] != stamp) atomicMax(J.claim + ids[j], vote);
-  }
+      if (!bit_of(taken, ids[j])) atomicMax(J.claim + ids[j], vote);
   }
 }
 
 template <class T, bool kSplit>
 __global__ void __launch_bounds__(256) k_wn_commit(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel,
                                                    int r) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
-  if (J.ctr[C_MFSKIP] || J.ctr[C_WNSMALL] || J.wn_lockstep) continue;
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (mf_skip(J.ctr) || J.ctr[C_WNSMALL] || J.wn_lockstep) return;
   const unsigned long long round = (unsigned)(J.ctr[C_WNROUND] + r + 1);
-  const int stamp = J.ctr[C_WNSTAMP];
   const int n = J.ctr[C_CAND + (r & 1)];
   const int* cur = (r & 1) ? J.cand_next : J.cand;
   int* nxt = (r & 1) ? J.cand : J.cand_next;
   int* nnext = J.ctr + C_CAND + ((r + 1) & 1);
-  int* taken = kSplit ? J.taken : J.taken1;
+  unsigned* taken = kSplit ? J.taken : J.taken1;
   int* flagged = kSplit ? J.flagged : J.flagged1;
   int* nflag = J.ctr + (kSplit ? C_NFC : C_NFC1);
-  const int stride = gridDim.x * blockDim.x;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+  const int stride = nblk * blockDim.x;
+  for (int e = blk * blockDim.x + threadIdx.x; e < n; e += stride) {
     const int s = cur[e];
     int ids[kNumDirs];
     const int k = wn_candidates<T, kSplit>(J, s, ids);
     int first = -1;
     for (int j = 0; j < k; ++j)
-      if (taken[ids[j]] != stamp) { first = ids[j]; break; }
+      if (!bit_of(taken, ids[j])) { first = ids[j]; break; }
     if (first < 0) continue;  // every candidate already flagged: resolved
     const unsigned long long vote = (round << 32) | (unsigned)(~s);
     if (J.claim[first] == vote) {
-      taken[first] = stamp;
+      atomicOr(taken + (first >> 5), 1u << (first & 31));
       flagged[atomicAdd(nflag, 1)] = first;
     } else {
       nxt[atomicAdd(nnext, 1)] = s;
     }
-  }
   }
 }
 
@@ -1912,14 +1974,22 @@ constexpr int kWnGridRounds = 3;
 // device iteration limit bounds them as well.  claim and taken are read
 // through L2 (__ldcg): other threads of the block update them with atomics
 // and stores between the barriers.
+// A flag bit as the last barrier left it: other threads set bits of the same
+// word by atomics in L2.
+__device__ __forceinline__ bool taken_now(const unsigned* bits, int v) {
+  return __ldcg(bits + (v >> 5)) >> (v & 31) & 1u;
+}
+
 template <class T, bool kSplit>
 __global__ void __launch_bounds__(1024) k_wn_resolve(Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
   if (blockIdx.x >= sel.n) return;
   Job<T>& J = jobs[sel.idx[blockIdx.x]];
-  if (J.ctr[C_MFSKIP] || J.wn_lockstep) return;
+  if (mf_skip(J.ctr)) {
+    if (!kSplit && threadIdx.x == 0) mf_end(J.ctr);
+    return;
+  }
   __shared__ int s_next;
-  const int stamp = J.ctr[C_WNSTAMP];
-  int* taken = kSplit ? J.taken : J.taken1;
+  unsigned* taken = kSplit ? J.taken : J.taken1;
   int* flagged = kSplit ? J.flagged : J.flagged1;
   int* nflag = J.ctr + (kSplit ? C_NFC : C_NFC1);
   // The grid-wide rounds left their list in parity kWnGridRounds & 1; a short
@@ -1944,7 +2014,7 @@ __global__ void __launch_bounds__(1024) k_wn_resolve(Job<T>* __restrict__ jobs, 
       const int k = wn_candidates<T, kSplit>(J, s, ids);
       const unsigned long long vote = hi | (unsigned)(~s);
       for (int j = 0; j < k; ++j)
-        if (__ldcg(taken + ids[j]) != stamp) atomicMax(J.claim + ids[j], vote);
+        if (!taken_now(taken, ids[j])) atomicMax(J.claim + ids[j], vote);
     }
     if (threadIdx.x == 0) s_next = 0;
     __syncthreads();
@@ -1954,14 +2024,14 @@ __global__ void __launch_bounds__(1024) k_wn_resolve(Job<T>* __restrict__ jobs, 
       const int k = wn_candidates<T, kSplit>(J, s, ids);
       int first = -1;
       for (int j = 0; j < k; ++j)
-        if (__ldcg(taken + ids[j]) != stamp) {
+        if (!taken_now(taken, ids[j])) {
           first = ids[j];
           break;
         }
       if (first < 0) continue;  // every candidate already flagged: resolved
       const unsigned long long vote = hi | (unsigned)(~s);
       if (__ldcg(J.claim + first) == vote) {
-        taken[first] = stamp;
+        atomicOr(taken + (first >> 5), 1u << (first & 31));
         flagged[atomicAdd(nflag, 1)] = first;
       } else {
         nxt[atomicAdd(&s_next, 1)] = s;
@@ -1985,6 +2055,7 @@ __global__ void __launch_bounds__(1024) k_wn_resolve(Job<T>* __restrict__ jobs, 
       J.ctr[C_CAND] = 0;
     }
     J.ctr[C_CAND_NEXT] = 0;
+    if (!kSplit) mf_end(J.ctr);
   }
 }
 
@@ -1999,45 +2070,41 @@ __global__ void __launch_bounds__(1024) k_wn_resolve(Job<T>* __restrict__ jobs, 
 // (get_wrong_split_neighbors / _join_, src/ExtreM_cuda.cu:2400-2513): a shared
 // candidate goes to the saddle that meets it at the earlier neighbour index.
 // The two sides flag into separate arrays, as the reference's two kernels do,
-// so one step serves both.  A saddle's resolution is marked in claim[]
-// (unused by this mode) with the round's stamp: the low 32-bit half for the
-// split side, the high half for the join side, so that a saddle on both lists
-// (type 3) keeps one mark per side.
+// so one step serves both.  A resolved saddle is complemented in its list (a
+// saddle on both lists, type 3, is resolved on each side by itself).
 template <class T>
-__device__ __forceinline__ void wn_step_entry(const Job<T>& J, int e, int n2, int d, int stamp) {
+__device__ __forceinline__ void wn_step_entry(const Job<T>& J, int e, int n2, int d) {
   const bool split = e < n2;
-  const int s = split ? J.cand[e] : J.cand_j[e - n2];
+  int* const at = split ? J.cand + e : J.cand_j + (e - n2);
+  const int s = *at;
+  if (s < 0) return;
   const Dims g = J.dim;
   int x, y, z;
   coords(s, g, x, y, z);
   if (!dir_valid(d, boundary_code(x, y, z, g.W, g.H, g.D))) return;
-  unsigned* mark = reinterpret_cast<unsigned*>(J.claim + s) + (split ? 0 : 1);
-  const unsigned done = (unsigned)stamp | 0x80000000u;  // never the zeroed initial value
-  if (*mark == done) return;
   const int r = s + ddx(d) + ddy(d) * g.W + ddz(d) * g.W * g.H;
   const T sv = J.g[s], rv = J.g[r];
   if (!(split ? above(rv, r, sv, s) : below(rv, r, sv, s))) return;
-  int* taken = split ? J.taken : J.taken1;
-  if ((split ? J.dds[r] == J.ds[r] : J.das[r] == J.as[r]) || taken[r] == stamp) return;
-  taken[r] = stamp;
+  unsigned* taken = split ? J.taken : J.taken1;
+  if ((split ? J.dds[r] == J.ds[r] : J.das[r] == J.as[r]) || taken_now(taken, r)) return;
+  atomicOr(taken + (r >> 5), 1u << (r & 31));
   (split ? J.flagged : J.flagged1)[atomicAdd(J.ctr + (split ? C_NFC : C_NFC1), 1)] = r;
-  *mark = done;
+  *at = ~s;
 }
 
 // One step over every selected job's two candidate lists (a large list: one
-// launch per direction).
+// launch per direction).  The last step ends the round.
 template <class T>
 __global__ void __launch_bounds__(256) k_wn_step(const Job<T>* __restrict__ jobs,
                                                  const __grid_constant__ Sel sel, int d) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    if (J.ctr[C_MFSKIP] || !J.wn_lockstep) continue;
-    const int stamp = J.ctr[C_WNSTAMP];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (!mf_skip(J.ctr)) {
     const int n2 = J.ctr[C_CAND], n = n2 + J.ctr[C_CANDJ];
-    const int stride = gridDim.x * blockDim.x;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride)
-      wn_step_entry(J, e, n2, d, stamp);
+    const int stride = nblk * blockDim.x;
+    for (int e = blk * blockDim.x + threadIdx.x; e < n; e += stride) wn_step_entry(J, e, n2, d);
   }
+  if (d == kNumDirs - 1 && last_block(J.ctr, nblk) && threadIdx.x == 0) mf_end(J.ctr);
 }
 
 // All fourteen steps in one block per job, with a barrier between steps (a
@@ -2048,61 +2115,66 @@ __global__ void __launch_bounds__(1024) k_wn_steps_block(const Job<T>* __restric
                                                          const __grid_constant__ Sel sel) {
   if (blockIdx.x >= sel.n) return;
   const Job<T>& J = jobs[sel.idx[blockIdx.x]];
-  if (J.ctr[C_MFSKIP] || !J.wn_lockstep) return;
-  const int stamp = J.ctr[C_WNSTAMP];
-  const int n2 = J.ctr[C_CAND], n = n2 + J.ctr[C_CANDJ];
-  for (int d = 0; d < kNumDirs; ++d) {
-    for (int e = threadIdx.x; e < n; e += blockDim.x) wn_step_entry(J, e, n2, d, stamp);
-    __syncthreads();
+  if (!mf_skip(J.ctr)) {
+    const int n2 = J.ctr[C_CAND], n = n2 + J.ctr[C_CANDJ];
+    for (int d = 0; d < kNumDirs; ++d) {
+      for (int e = threadIdx.x; e < n; e += blockDim.x) wn_step_entry(J, e, n2, d);
+      __syncthreads();
+    }
   }
+  if (threadIdx.x == 0) mf_end(J.ctr);
 }
 
 // ---------------------------------------------------------------------------
 // fixpath (:4046-4206): walk the steepest ascent (descent) of both fields from a
 // flagged vertex until they diverge; lower the decompressed choice (split) or
-// the original choice (join).
+// the original choice (join).  Both sides' lists in one launch: their proposals
+// merge by atomic max.
 // ---------------------------------------------------------------------------
 template <class T, bool kSplit>
-__global__ void __launch_bounds__(256) k_fixpath(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
-  const int cap = J.iter_cap;
-  const int n = J.ctr[kSplit ? C_NFC : C_NFC1];
-  const int* list = kSplit ? J.flagged : J.flagged1;
-  const int stride = gridDim.x * blockDim.x;
+__device__ __forceinline__ void fixpath_from(const Job<T>& J, int cur) {
   const Dims g = J.dim;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    int cur = list[e];
-    int t = -1, fl = -1;
-    int steps = 0;
-    for (; steps < cap; ++steps) {
-      int ids[kNumDirs];
-      const int nn = neighbours(cur, g, ids, nullptr);
-      int ni = cur, nd = cur;
-      T fi = J.f[cur], gd = J.g[cur];
-      for (int j = 0; j < nn; ++j) {
-        const int r = ids[j];
-        const T fr = J.f[r], gr = J.g[r];
-        if (kSplit) {
-          if (fi < fr || (fi == fr && ni < r)) { ni = r; fi = fr; }
-          if (gd < gr || (gd == gr && nd < r)) { nd = r; gd = gr; }
-        } else {
-          if (fi > fr || (fi == fr && ni > r)) { ni = r; fi = fr; }
-          if (gd > gr || (gd == gr && nd > r)) { nd = r; gd = gr; }
-        }
+  const int cap = J.iter_cap;
+  int t = -1, fl = -1;
+  int steps = 0;
+  for (; steps < cap; ++steps) {
+    int ids[kNumDirs];
+    const int nn = neighbours(cur, g, ids, nullptr);
+    int ni = cur, nd = cur;
+    T fi = J.f[cur], gd = J.g[cur];
+    for (int j = 0; j < nn; ++j) {
+      const int r = ids[j];
+      const T fr = J.f[r], gr = J.g[r];
+      if (kSplit) {
+        if (fi < fr || (fi == fr && ni < r)) { ni = r; fi = fr; }
+        if (gd < gr || (gd == gr && nd < r)) { nd = r; gd = gr; }
+      } else {
+        if (fi > fr || (fi == fr && ni > r)) { ni = r; fi = fr; }
+        if (gd > gr || (gd == gr && nd > r)) { nd = r; gd = gr; }
       }
-      if (ni != nd) { t = ni; fl = nd; break; }
-      if (ni == cur) break;
-      cur = ni;
     }
-    if (steps == cap) {
-      atomicOr(J.ctr + C_ERROR, kErrPath);
-      continue;
-    }
-    if (fl == t) continue;
-    const int target = kSplit ? fl : t;
-    propose(J, target, step_delta(J, target));
+    if (ni != nd) { t = ni; fl = nd; break; }
+    if (ni == cur) break;
+    cur = ni;
   }
+  if (steps == cap) {
+    atomicOr(J.ctr + C_ERROR, kErrPath);
+    return;
+  }
+  if (fl == t) return;
+  const int target = kSplit ? fl : t;
+  propose(J, target, step_delta(J, target));
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) k_fixpath(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  const int n2 = J.ctr[C_NFC], n = n2 + J.ctr[C_NFC1];
+  const int stride = nblk * blockDim.x;
+  for (int e = blk * blockDim.x + threadIdx.x; e < n; e += stride) {
+    if (e < n2) fixpath_from<T, true>(J, J.flagged[e]);
+    else fixpath_from<T, false>(J, J.flagged1[e - n2]);
   }
 }
 
@@ -2113,15 +2185,19 @@ __global__ void __launch_bounds__(256) k_fixpath(const Job<T>* __restrict__ jobs
 // ---------------------------------------------------------------------------
 template <class T, bool kMax>
 __global__ void __launch_bounds__(256) k_wim_scan(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (blk == 0 && threadIdx.x == 0) {  // counted by k_wim_collect
+    J.ctr[kMax ? C_WMC : C_WMIN] = 0;
+    J.ctr[kMax ? C_WMC2 : C_WMIN2] = 0;
+  }
   const int ns = J.ctr[kMax ? C_NS2 : C_NS1];
   const int4* oend = kMax ? J.oend2 : J.oend1;
   const int* drow = kMax ? J.drow2 : J.drow1;
   int* first = kMax ? J.first1 : J.first_min1;
   int* flag = kMax ? J.flag2 : J.flag_min2;
-  const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
+  const int stride = nblk * blockDim.x;
+  for (int i = blk * blockDim.x + threadIdx.x; i < ns; i += stride) {
     const int cnt = (kMax ? J.ocnt2 : J.ocnt1)[i];
     if (cnt == 0) continue;
     // Original entries 0 and count - 1 (labels, extremum indices) against the
@@ -2131,15 +2207,14 @@ __global__ void __launch_bounds__(256) k_wim_scan(const Job<T>* __restrict__ job
     if (o.x != d.x) atomicMin(first + o.z, i);
     if (o.y != d.y) flag[o.w] = 1;
   }
-  }
 }
 
 // Collect per extremum, count, propose the fix and reset the arbitration slots.
 // fix = false: detection only (the third block of the outer loop, :5932-5951).
 template <class T, bool kMax>
 __global__ void __launch_bounds__(256) k_wim_collect(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel, int fix) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
   const int next = J.ctr[kMax ? C_NMAX : C_NMIN];
   const int* ext_list = kMax ? J.maxima : J.minima;
   const int* drow = kMax ? J.drow2 : J.drow1;
@@ -2147,8 +2222,8 @@ __global__ void __launch_bounds__(256) k_wim_collect(const Job<T>* __restrict__ 
   int* flag = kMax ? J.flag2 : J.flag_min2;
   int* c1 = J.ctr + (kMax ? C_WMC : C_WMIN);
   int* c2 = J.ctr + (kMax ? C_WMC2 : C_WMIN2);
-  const int stride = gridDim.x * blockDim.x;
-  for (int base = blockIdx.x * blockDim.x; base < next; base += stride) {
+  const int stride = nblk * blockDim.x;
+  for (int base = blk * blockDim.x; base < next; base += stride) {
     const int m = base + threadIdx.x;
     bool h1 = false, h2 = false;
     if (m < next) {
@@ -2182,7 +2257,6 @@ __global__ void __launch_bounds__(256) k_wim_collect(const Job<T>* __restrict__ 
       if (b2) atomicAdd(c2, __popc(b2));
     }
   }
-  }
 }
 
 // get_wrong_index_min direction 1 (:3157-3168, fix :3393-3410) keeps the pair of
@@ -2192,31 +2266,29 @@ __global__ void __launch_bounds__(256) k_wim_collect(const Job<T>* __restrict__ 
 // scans).
 template <class T>
 __global__ void __launch_bounds__(256) k_wim_min2_scan(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
   const int ns = J.ctr[C_NS1];
-  const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
+  const int stride = nblk * blockDim.x;
+  for (int i = blk * blockDim.x + threadIdx.x; i < ns; i += stride) {
     const int cnt = J.ocnt1[i];
     if (cnt == 0) continue;
     const int4 o = J.oend1[i];
     if (o.y != J.drow1[2ll * i + 1]) atomicMin(J.ext_id + o.w, i);
   }
-  }
 }
 template <class T>
 __global__ void __launch_bounds__(256) k_wim_min2_collect(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
   const int next = J.ctr[C_NMIN];
-  const int stride = gridDim.x * blockDim.x;
-  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < next; m += stride) {
+  const int stride = nblk * blockDim.x;
+  for (int m = blk * blockDim.x + threadIdx.x; m < next; m += stride) {
     const int row = J.ext_id[m];
     if (row == kInf) continue;
     J.ext_id[m] = kInf;
     const int target = J.drow1[2ll * row + 1];
     propose(J, target, step_delta(J, target));
-  }
   }
 }
 
@@ -2261,32 +2333,32 @@ __device__ __forceinline__ int side_row(const Job<T>& J, int v) {
 template <class T, bool kMax>
 __global__ void __launch_bounds__(256) k_wis_mark(const Job<T>* __restrict__ jobs,
                                                   const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    const int epoch = J.ctr[kMax ? C_WEP2 : C_WEP1];
-    unsigned* chg = kMax ? J.wchg2 : J.wchg1;
-    const uint8_t* ocnt = kMax ? J.ocnt2 : J.ocnt1;
-    const int4* orm = kMax ? J.orm2 : J.orm1;
-    const int* rows = kMax ? J.orow2 : J.orow1;
-    int* stamp = kMax ? J.wstamp2 : J.wstamp1;
-    const int nw = (J.dim.N + 31) >> 5;
-    const int stride = gridDim.x * blockDim.x;
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += stride) {
-      unsigned bits = chg[w];
-      if (!bits) continue;
-      chg[w] = 0u;
-      if (epoch == 1) continue;
-      for (; bits; bits &= bits - 1) {
-        const int i = side_row<T, kMax>(J, (w << 5) + __ffs(bits) - 1);
-        if (i < 0) continue;
-        const int cnt = ocnt[i];
-        const int4 m4 = orm[i];
-        for (int p = 0; p < cnt; ++p) {
-          const int m = p == 0 ? m4.x : p == 1 ? m4.y : p == 2 ? m4.z : p == 3 ? m4.w
-                                                               : rows[(long long)i * kRowStride + p];
-          if (m < 0) continue;  // a repeated label
-          if (atomicExch(stamp + m, epoch) != epoch) J.aff[atomicAdd(J.ctr + C_AFF, 1)] = m;
-        }
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (blk == 0 && threadIdx.x == 0) J.ctr[kMax ? C_WSC : C_WSCJ] = 0;  // counted by k_wis_collect
+  const int epoch = J.ctr[kMax ? C_WEP2 : C_WEP1] + 1;
+  unsigned* chg = kMax ? J.wchg2 : J.wchg1;
+  const uint8_t* ocnt = kMax ? J.ocnt2 : J.ocnt1;
+  const int4* orm = kMax ? J.orm2 : J.orm1;
+  const int* rows = kMax ? J.orow2 : J.orow1;
+  int* stamp = kMax ? J.wstamp2 : J.wstamp1;
+  const int nw = (J.dim.N + 31) >> 5;
+  const int stride = nblk * blockDim.x;
+  for (int w = blk * blockDim.x + threadIdx.x; w < nw; w += stride) {
+    unsigned bits = chg[w];
+    if (!bits) continue;
+    chg[w] = 0u;
+    if (epoch == 1) continue;
+    for (; bits; bits &= bits - 1) {
+      const int i = side_row<T, kMax>(J, (w << 5) + __ffs(bits) - 1);
+      if (i < 0) continue;
+      const int cnt = ocnt[i];
+      const int4 m4 = orm[i];
+      for (int p = 0; p < cnt; ++p) {
+        const int m = p == 0 ? m4.x : p == 1 ? m4.y : p == 2 ? m4.z : p == 3 ? m4.w
+                                                             : rows[(long long)i * kRowStride + p];
+        if (m < 0) continue;  // a repeated label
+        if (atomicExch(stamp + m, epoch) != epoch) J.aff[atomicAdd(J.ctr + C_AFF, 1)] = m;
       }
     }
   }
@@ -2326,34 +2398,33 @@ constexpr int kWisShort = 48;
 template <class T, bool kMax>
 __global__ void __launch_bounds__(256) k_wis_update(const Job<T>* __restrict__ jobs,
                                                     const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    const bool all = J.ctr[kMax ? C_WEP2 : C_WEP1] == 1;
-    const int n = all ? J.ctr[kMax ? C_NMAX : C_NMIN] : J.ctr[C_AFF];
-    const int* sad = kMax ? J.sad2 : J.sad1;
-    const int* best = kMax ? J.largest : J.smallest;
-    const int* off = kMax ? J.moff2 : J.moff1;
-    const int* ent = kMax ? J.ment2 : J.ment1;
-    int* first = kMax ? J.first_s : J.first_sj;
-    const int N = J.dim.N;
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {  // uniform per warp
-      const int e = base + threadIdx.x;
-      bool lng = false;
-      int m = 0;
-      if (e < n) {
-        m = all ? e : J.aff[e];
-        const int tb = best[m];
-        const int k0 = off[m], k1 = off[m + 1];
-        lng = k1 - k0 > kWisShort;
-        // An extremum named by no row has no saddle.
-        if (!lng)
-          first[m] = (tb >= 0 && tb < N) ? wis_first<T, kMax>(J, sad, ent, k0, k1, 1, tb, J.g[tb])
-                                         : kInf;
-      }
-      const int slot = warp_append(J.ctr + C_WLONG, lng, 0xffffffffu);
-      if (slot >= 0) J.wlong[slot] = m;
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  const bool all = J.ctr[kMax ? C_WEP2 : C_WEP1] == 0;
+  const int n = all ? J.ctr[kMax ? C_NMAX : C_NMIN] : J.ctr[C_AFF];
+  const int* sad = kMax ? J.sad2 : J.sad1;
+  const int* best = kMax ? J.largest : J.smallest;
+  const int* off = kMax ? J.moff2 : J.moff1;
+  const int* ent = kMax ? J.ment2 : J.ment1;
+  int* first = kMax ? J.first_s : J.first_sj;
+  const int N = J.dim.N;
+  const int stride = nblk * blockDim.x;
+  for (int base = blk * blockDim.x; base < n; base += stride) {  // uniform per warp
+    const int e = base + threadIdx.x;
+    bool lng = false;
+    int m = 0;
+    if (e < n) {
+      m = all ? e : J.aff[e];
+      const int tb = best[m];
+      const int k0 = off[m], k1 = off[m + 1];
+      lng = k1 - k0 > kWisShort;
+      // An extremum named by no row has no saddle.
+      if (!lng)
+        first[m] = (tb >= 0 && tb < N) ? wis_first<T, kMax>(J, sad, ent, k0, k1, 1, tb, J.g[tb])
+                                       : kInf;
     }
+    const int slot = warp_append(J.ctr + C_WLONG, lng, 0xffffffffu);
+    if (slot >= 0) J.wlong[slot] = m;
   }
 }
 
@@ -2362,40 +2433,43 @@ template <class T, bool kMax>
 __global__ void __launch_bounds__(256) k_wis_long(const Job<T>* __restrict__ jobs,
                                                   const __grid_constant__ Sel sel) {
   __shared__ int part[8];
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    const int n = J.ctr[C_WLONG];
-    const int* sad = kMax ? J.sad2 : J.sad1;
-    const int* ent = kMax ? J.ment2 : J.ment1;
-    const int* off = kMax ? J.moff2 : J.moff1;
-    for (int e = blockIdx.x; e < n; e += gridDim.x) {  // uniform per block
-      const int m = J.wlong[e];
-      const int tb = (kMax ? J.largest : J.smallest)[m];  // valid: the lists are non-empty
-      int hit = wis_first<T, kMax>(J, sad, ent, off[m] + (int)threadIdx.x, off[m + 1], 256, tb,
-                                   J.g[tb]);
-      for (int o = 16; o > 0; o >>= 1) hit = min(hit, __shfl_xor_sync(0xffffffffu, hit, o));
-      if (lane_id() == 0) part[threadIdx.x >> 5] = hit;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) hit = min(hit, part[w]);
-        (kMax ? J.first_s : J.first_sj)[m] = hit;
-      }
-      __syncthreads();
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  const int n = J.ctr[C_WLONG];
+  const int* sad = kMax ? J.sad2 : J.sad1;
+  const int* ent = kMax ? J.ment2 : J.ment1;
+  const int* off = kMax ? J.moff2 : J.moff1;
+  for (int e = blk; e < n; e += nblk) {  // uniform per block
+    const int m = J.wlong[e];
+    const int tb = (kMax ? J.largest : J.smallest)[m];  // valid: the lists are non-empty
+    int hit = wis_first<T, kMax>(J, sad, ent, off[m] + (int)threadIdx.x, off[m + 1], 256, tb,
+                                 J.g[tb]);
+    for (int o = 16; o > 0; o >>= 1) hit = min(hit, __shfl_xor_sync(0xffffffffu, hit, o));
+    if (lane_id() == 0) part[threadIdx.x >> 5] = hit;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) hit = min(hit, part[w]);
+      (kMax ? J.first_s : J.first_sj)[m] = hit;
     }
+    __syncthreads();
   }
 }
 
 template <class T, bool kMax>
 __global__ void __launch_bounds__(256) k_wis_collect(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel, int fix) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-  const Job<T>& J = jobs[sel.idx[jk]];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (blk == 0 && threadIdx.x == 0) {  // the scan is over: next epoch, empty queues
+    J.ctr[kMax ? C_WEP2 : C_WEP1] += 1;
+    J.ctr[C_AFF] = J.ctr[C_WLONG] = 0;
+  }
   const int next = J.ctr[kMax ? C_NMAX : C_NMIN];
   const int* sad = kMax ? J.sad2 : J.sad1;
   const int* best = kMax ? J.largest : J.smallest;
   int* first = kMax ? J.first_s : J.first_sj;
   int* cnt = J.ctr + (kMax ? C_WSC : C_WSCJ);
-  const int stride = gridDim.x * blockDim.x;
-  for (int base = blockIdx.x * blockDim.x; base < next; base += stride) {
+  const int stride = nblk * blockDim.x;
+  for (int base = blk * blockDim.x; base < next; base += stride) {
     const int m = base + threadIdx.x;
     bool hit = false;
     if (m < next && first[m] != kInf) {  // kept: the scan is incremental
@@ -2417,7 +2491,6 @@ __global__ void __launch_bounds__(256) k_wis_collect(const Job<T>* __restrict__ 
     const unsigned b = __ballot_sync(0xffffffffu, hit);
     if (lane_id() == 0 && b) atomicAdd(cnt, __popc(b));
   }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2438,64 +2511,63 @@ template <class T>
 __global__ void __launch_bounds__(256, 4) k_join_keys(const Job<T>* __restrict__ jobs,
                                                       const __grid_constant__ Sel sel) {
   __shared__ int off[kNumDirs];
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    __syncthreads();  // every thread is done with the last job's offsets
-    fill_offsets(off, J.dim);
-    __syncthreads();
-    using KK = typename KeyOf<T>::K;
-    const int ns = J.ctr[C_NS1];
-    const int* __restrict__ lab = J.as;
-    const int* __restrict__ ext = J.ext;
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x; base < ns; base += stride) {  // uniform per warp
-      const int i = base + threadIdx.x;
-      const bool act = i < ns;
-      const int s = act ? J.sad1[i] : 0;
-      unsigned rest = act ? J.olm[s] : 0u;
-      const int pmax = (int)__reduce_max_sync(0xffffffffu, __popc(rest));
-      const KK key = KeyOf<T>::enc(J.f[s] + T(0));  // -0 and +0 compare equal
-      // Distinct labels in direction order, kept as extremum indices.
-      int lb[16], mp[16];
-      int cnt = 0, m0 = -1, m1 = -1, m2 = -1, m3 = -1;
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (blk == 0 && threadIdx.x == 0) J.ctr[C_WSCJ] = 0;  // counted by k_wis_collect
+  fill_offsets(off, J.dim);
+  __syncthreads();
+  using KK = typename KeyOf<T>::K;
+  const int ns = J.ctr[C_NS1];
+  const int* __restrict__ lab = J.as;
+  const int* __restrict__ ext = J.ext;
+  const int stride = nblk * blockDim.x;
+  for (int base = blk * blockDim.x; base < ns; base += stride) {  // uniform per warp
+    const int i = base + threadIdx.x;
+    const bool act = i < ns;
+    const int s = act ? J.sad1[i] : 0;
+    unsigned rest = act ? J.olm[s] : 0u;
+    const int pmax = (int)__reduce_max_sync(0xffffffffu, __popc(rest));
+    const KK key = KeyOf<T>::enc(J.f[s] + T(0));  // -0 and +0 compare equal
+    // Distinct labels in direction order, kept as extremum indices.
+    int lb[16], mp[16];
+    int cnt = 0, m0 = -1, m1 = -1, m2 = -1, m3 = -1;
 #pragma unroll
-      for (int h = 0; h < 16; h += 4) {
+    for (int h = 0; h < 16; h += 4) {
 #pragma unroll
-        for (int q = h; q < h + 4; ++q) lb[q] = mp[q] = -1;
-        if (h >= pmax) continue;  // uniform per warp
+      for (int q = h; q < h + 4; ++q) lb[q] = mp[q] = -1;
+      if (h >= pmax) continue;  // uniform per warp
 #pragma unroll
-        for (int q = h; q < h + 4; ++q) {
-          if (rest) lb[q] = lab[s + off[__ffs((int)rest) - 1]];
-          rest &= rest - 1u;
-        }
-#pragma unroll
-        for (int q = h; q < h + 4; ++q) {
-          bool fresh = lb[q] >= 0;
-#pragma unroll
-          for (int e = 0; e < q; ++e) fresh &= lb[e] != lb[q];
-          if (fresh) mp[q] = ext[lb[q]];
-        }
-#pragma unroll
-        for (int q = h; q < h + 4; ++q) {
-          if (mp[q] < 0) continue;
-          m0 = cnt == 0 ? mp[q] : m0;
-          m1 = cnt == 1 ? mp[q] : m1;
-          m2 = cnt == 2 ? mp[q] : m2;
-          m3 = cnt == 3 ? mp[q] : m3;
-          if (cnt >= 4) J.orow1[(long long)i * kRowStride + cnt] = mp[q];
-          ++cnt;
-        }
-        KK cur[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) cur[q] = mp[h + q] >= 0 ? J.ext_key[mp[h + q]] : KK(0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (mp[h + q] >= 0 && key < cur[q]) atomicMin(J.ext_key + mp[h + q], key);
+      for (int q = h; q < h + 4; ++q) {
+        if (rest) lb[q] = lab[s + off[__ffs((int)rest) - 1]];
+        rest &= rest - 1u;
       }
-      if (act) {
-        J.ocnt1[i] = (uint8_t)cnt;
-        J.orm1[i] = make_int4(m0, m1, m2, m3);
+#pragma unroll
+      for (int q = h; q < h + 4; ++q) {
+        bool fresh = lb[q] >= 0;
+#pragma unroll
+        for (int e = 0; e < q; ++e) fresh &= lb[e] != lb[q];
+        if (fresh) mp[q] = ext[lb[q]];
       }
+#pragma unroll
+      for (int q = h; q < h + 4; ++q) {
+        if (mp[q] < 0) continue;
+        m0 = cnt == 0 ? mp[q] : m0;
+        m1 = cnt == 1 ? mp[q] : m1;
+        m2 = cnt == 2 ? mp[q] : m2;
+        m3 = cnt == 3 ? mp[q] : m3;
+        if (cnt >= 4) J.orow1[(long long)i * kRowStride + cnt] = mp[q];
+        ++cnt;
+      }
+      KK cur[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) cur[q] = mp[h + q] >= 0 ? J.ext_key[mp[h + q]] : KK(0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (mp[h + q] >= 0 && key < cur[q]) atomicMin(J.ext_key + mp[h + q], key);
+    }
+    if (act) {
+      J.ocnt1[i] = (uint8_t)cnt;
+      J.orm1[i] = make_int4(m0, m1, m2, m3);
     }
   }
 }
@@ -2503,26 +2575,25 @@ __global__ void __launch_bounds__(256, 4) k_join_keys(const Job<T>* __restrict__
 template <class T>
 __global__ void __launch_bounds__(256) k_join_ids(const Job<T>* __restrict__ jobs,
                                                   const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    using KK = typename KeyOf<T>::K;
-    const int ns = J.ctr[C_NS1];
-    const int stride = gridDim.x * blockDim.x;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
-      const int s = J.sad1[i], cnt = J.ocnt1[i];
-      const int4 m4 = J.orm1[i];
-      const KK key = KeyOf<T>::enc(J.f[s] + T(0));
-      const int m[4] = {m4.x, m4.y, m4.z, m4.w};
-      KK cur[4];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  using KK = typename KeyOf<T>::K;
+  const int ns = J.ctr[C_NS1];
+  const int stride = nblk * blockDim.x;
+  for (int i = blk * blockDim.x + threadIdx.x; i < ns; i += stride) {
+    const int s = J.sad1[i], cnt = J.ocnt1[i];
+    const int4 m4 = J.orm1[i];
+    const KK key = KeyOf<T>::enc(J.f[s] + T(0));
+    const int m[4] = {m4.x, m4.y, m4.z, m4.w};
+    KK cur[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) cur[q] = m[q] >= 0 ? J.ext_key[m[q]] : KK(0);
+    for (int q = 0; q < 4; ++q) cur[q] = m[q] >= 0 ? J.ext_key[m[q]] : KK(0);
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (m[q] >= 0 && cur[q] == key) atomicMin(J.ext_id + m[q], s);
-      for (int p = 4; p < cnt; ++p) {
-        const int mm = J.orow1[(long long)i * kRowStride + p];
-        if (J.ext_key[mm] == key) atomicMin(J.ext_id + mm, s);
-      }
+    for (int q = 0; q < 4; ++q)
+      if (m[q] >= 0 && cur[q] == key) atomicMin(J.ext_id + m[q], s);
+    for (int p = 4; p < cnt; ++p) {
+      const int mm = J.orow1[(long long)i * kRowStride + p];
+      if (J.ext_key[mm] == key) atomicMin(J.ext_id + mm, s);
     }
   }
 }
@@ -2530,124 +2601,29 @@ __global__ void __launch_bounds__(256) k_join_ids(const Job<T>* __restrict__ job
 template <class T>
 __global__ void __launch_bounds__(256) k_join_scan(const Job<T>* __restrict__ jobs,
                                                    const __grid_constant__ Sel sel) {
-  for (int jk = 0; jk < sel.n; ++jk) {
-    const Job<T>& J = jobs[sel.idx[jk]];
-    const T* __restrict__ g = J.g;
-    const int ns = J.ctr[C_NS1];
-    const int stride = gridDim.x * blockDim.x;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
-      const int s = J.sad1[i], cnt = J.ocnt1[i];
-      const int4 m4 = J.orm1[i];
-      const T gs = g[s];
-      const int m[4] = {m4.x, m4.y, m4.z, m4.w};
-      int t[4];
-      T gt[4];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  const T* __restrict__ g = J.g;
+  const int ns = J.ctr[C_NS1];
+  const int stride = nblk * blockDim.x;
+  for (int i = blk * blockDim.x + threadIdx.x; i < ns; i += stride) {
+    const int s = J.sad1[i], cnt = J.ocnt1[i];
+    const int4 m4 = J.orm1[i];
+    const T gs = g[s];
+    const int m[4] = {m4.x, m4.y, m4.z, m4.w};
+    int t[4];
+    T gt[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) t[q] = m[q] >= 0 ? J.ext_id[m[q]] : s;
+    for (int q = 0; q < 4; ++q) t[q] = m[q] >= 0 ? J.ext_id[m[q]] : s;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) gt[q] = t[q] != s ? g[t[q]] : T(0);
+    for (int q = 0; q < 4; ++q) gt[q] = t[q] != s ? g[t[q]] : T(0);
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (t[q] != s && below(gs, s, gt[q], t[q])) atomicMin(J.first_sj + m[q], i * kRowStride);
-      for (int p = 4; p < cnt; ++p) {
-        const int mm = J.orow1[(long long)i * kRowStride + p], tt = J.ext_id[mm];
-        if (tt != s && below(gs, s, g[tt], tt)) atomicMin(J.first_sj + mm, i * kRowStride);
-      }
+    for (int q = 0; q < 4; ++q)
+      if (t[q] != s && below(gs, s, gt[q], t[q])) atomicMin(J.first_sj + m[q], i * kRowStride);
+    for (int p = 4; p < cnt; ++p) {
+      const int mm = J.orow1[(long long)i * kRowStride + p], tt = J.ext_id[mm];
+      if (tt != s && below(gs, s, g[tt], tt)) atomicMin(J.first_sj + mm, i * kRowStride);
     }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Small helpers.
-// ---------------------------------------------------------------------------
-// Per-job control operations between kernels, one thread per selected job
-// (counter resets, epoch advances and list swaps; the job descriptors live in
-// device memory, so list swaps happen here too).
-enum CtlOp : int {
-  OP_DETECT_DENSE_BEGIN = 0,  // mismatch list and category counts to zero
-  OP_DETECT_BEGIN,            // next re-evaluation epoch, next list and counts to zero
-  OP_DETECT_END_DENSE,        // dirty list to zero, next dirty epoch
-  OP_DETECT_END,              // swap mismatch lists, then as OP_DETECT_END_DENSE
-  OP_MF_BEGIN,                // start of a manifold round: skip it if nothing changed,
-                              // else next flag stamp, flagged / candidate counts to zero
-  OP_ZERO_TOUCHED,
-  OP_SLOOPS_BEGIN,            // wrong_max counters and touched to zero
-  OP_SADDLE_BEGIN,            // wrong_saddle counter and touched to zero
-  OP_SLOOPS_JOIN_BEGIN,
-  OP_SADDLE_JOIN_BEGIN,
-  OP_DETECT3_BEGIN,           // wrong_max / wrong_saddle counters to zero
-  OP_DETECT3_JOIN_BEGIN
-};
-
-template <class T>
-__global__ void k_ctl(Job<T>* jobs, const __grid_constant__ Sel sel, int op) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= sel.n) return;
-  Job<T>& J = jobs[sel.idx[k]];
-  int* c = J.ctr;
-  switch (op) {
-    case OP_DETECT_DENSE_BEGIN:
-      c[C_MM] = c[C_CMAX] = c[C_CMIN] = c[C_CSAD] = 0;
-      break;
-    case OP_DETECT_BEGIN:
-      c[C_REPOCH] += 1;
-      c[C_MM_NEXT] = c[C_CMAX] = c[C_CMIN] = c[C_CSAD] = 0;
-      break;
-    case OP_DETECT_END: {
-      int* t = J.mm;
-      J.mm = J.mm_next;
-      J.mm_next = t;
-      c[C_MM] = c[C_MM_NEXT];
-    }  // fall through
-    case OP_DETECT_END_DENSE:
-      c[C_DIRTY] = 0;
-      c[C_DEPOCH] += 1;
-      break;
-    case OP_MF_BEGIN:
-      // The round's outputs (labels, row slots, flagged neighbours and their
-      // counts) are functions of the decompressed field alone, so when no
-      // value changed since the last round began they are still in place.
-      c[C_MFSKIP] = c[C_MFDONE] && !c[C_CHANGED];
-      c[C_MFREUSED] += c[C_MFSKIP];
-      c[C_MFFIRST] = !c[C_MFDONE];
-      c[C_CHANGED] = 0;
-      c[C_MFDONE] = 1;
-      if (c[C_MFSKIP]) break;
-      c[C_WNSTAMP] += 1;  // next flag stamp; flagged and candidate counts to zero
-      c[C_NFC] = c[C_NFC1] = 0;
-      c[C_CAND] = c[C_CANDJ] = c[C_CAND_NEXT] = c[C_TLIST] = 0;
-      break;
-    case OP_ZERO_TOUCHED:
-      c[C_TOUCHED] = 0;
-      break;
-    case OP_SLOOPS_BEGIN:
-      c[C_WMC] = c[C_WMC2] = c[C_TOUCHED] = 0;
-      break;
-    case OP_SADDLE_BEGIN:
-      c[C_WSC] = c[C_TOUCHED] = 0;
-      c[C_WEP2] += 1;  // next wrong-saddle epoch, empty queue
-      c[C_AFF] = c[C_WLONG] = 0;
-      break;
-    case OP_SLOOPS_JOIN_BEGIN:
-      c[C_WMIN] = c[C_WMIN2] = c[C_TOUCHED] = 0;
-      break;
-    case OP_SADDLE_JOIN_BEGIN:
-      c[C_WSCJ] = c[C_TOUCHED] = 0;
-      c[C_WEP1] += 1;
-      c[C_AFF] = c[C_WLONG] = 0;
-      break;
-    case OP_DETECT3_BEGIN:
-      c[C_WMC] = c[C_WMC2] = c[C_WSC] = 0;
-      c[C_WEP2] += 1;
-      c[C_AFF] = c[C_WLONG] = 0;
-      break;
-    case OP_DETECT3_JOIN_BEGIN:
-      c[C_WMIN] = c[C_WMIN2] = c[C_WSCJ] = 0;
-      c[C_WEP1] += 1;
-      c[C_AFF] = c[C_WLONG] = 0;
-      break;
-    default:
-      break;
   }
 }
 
