@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -182,6 +183,8 @@ struct JobHost {
   bool waiting = false;   // stopped at a branch that needs this tick's counters
   cudaEvent_t input_ready = nullptr;  // the decompressed field is still arriving until this event
   int outer = 0, rounds = 0, cloop_total = 0, manifold_rounds = 0;
+  bool wim_seen = false, wis_seen = false;  // the split side's scans ran since the last
+                                            // computed manifold round
   int reused = 0;         // manifold rounds that launched nothing: no value had changed
   int nfc = 0, nfc1 = 0;
   int c[11] = {0};        // loop-test counters (:5603-5605)
@@ -238,23 +241,24 @@ class BatchEngine {
     if (preset_tables) tb_ = *preset_tables;
     else if (int rc = device_tables(&tb_)) return rc;
     const size_t desc_bytes = sizeof(Job<T>) * kMaxSel;
-    const size_t map_bytes = sizeof(CUtensorMap) * 2 * kMaxSel;
     const size_t ctr_bytes = sizeof(int) * C_COUNT * kMaxSel;
     if (fixed_storage) {  // borrowed: carve the engine's arrays from it
       jobs_dev_ = fixed_storage->template take<Job<T>>(kMaxSel);
-      maps_dev_ = fixed_storage->template take<CUtensorMap>(2 * kMaxSel);
       ctr_dev_ = fixed_storage->template take<int>(C_COUNT * kMaxSel);
-      if (!jobs_dev_ || !maps_dev_ || !ctr_dev_) return EXTREMZ_OOM;
+      if (!jobs_dev_ || !ctr_dev_) return EXTREMZ_OOM;
       borrowed_ = true;
       ctr_host_ = static_ctr_host_;
     } else {
       if (cudaMalloc(&jobs_dev_, desc_bytes) != cudaSuccess ||
-          cudaMalloc(&maps_dev_, map_bytes) != cudaSuccess ||
-          cudaMalloc(&ctr_dev_, ctr_bytes) != cudaSuccess ||
-          cudaMallocHost(&ctr_host_, ctr_bytes) != cudaSuccess) {
+          cudaMalloc(&ctr_dev_, ctr_bytes + sizeof(unsigned)) != cudaSuccess ||
+          cudaMemset(ctr_dev_, 0, ctr_bytes + sizeof(unsigned)) != cudaSuccess ||
+          cudaMallocHost(&ctr_host_, ctr_bytes + sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
         return EXTREMZ_OOM;
       }
+      std::memset(ctr_host_, 0, ctr_bytes + sizeof(unsigned));
+      seq_dev_ = reinterpret_cast<unsigned*>(ctr_dev_ + C_COUNT * kMaxSel);
+      seq_host_ = reinterpret_cast<volatile unsigned*>(ctr_host_ + C_COUNT * kMaxSel);
     }
     slots_.assign(kMaxSel, JobHost<T>());
     ready_ = true;
@@ -266,12 +270,10 @@ class BatchEngine {
     for (auto& j : slots_) free_job(j);
     if (!borrowed_) {
       if (jobs_dev_) cudaFree(jobs_dev_);
-      if (maps_dev_) cudaFree(maps_dev_);
       if (ctr_dev_) cudaFree(ctr_dev_);
       if (ctr_host_) cudaFreeHost(ctr_host_);
     }
     jobs_dev_ = nullptr;
-    maps_dev_ = nullptr;
     ctr_dev_ = nullptr;
     ctr_host_ = nullptr;
     ready_ = false;
@@ -434,14 +436,9 @@ class BatchEngine {
     if (keep_input)
       EZ_CHECK(cudaMemcpyAsync(J.g0, g, (size_t)N * sizeof(T), cudaMemcpyDeviceToDevice, st_));
     // Tile maps of both fields (TMA when the stride allows).
-    CUtensorMap mf, mg;
     const bool tma_ok = (p.flags & EXTREMZ_FLAG_NO_TMA) == 0;
-    J.tma_f = tma_ok && make_tile_map(&mf, f, J.dim);
-    J.tma_g = tma_ok && make_tile_map(&mg, (const T*)g, J.dim);
-    EZ_CHECK(cudaMemcpyAsync(maps_dev_ + 2 * slot, &mf, sizeof(mf), cudaMemcpyHostToDevice, st_));
-    EZ_CHECK(cudaMemcpyAsync(maps_dev_ + 2 * slot + 1, &mg, sizeof(mg), cudaMemcpyHostToDevice, st_));
-    J.map_f = maps_dev_ + 2 * slot;
-    J.map_g = maps_dev_ + 2 * slot + 1;
+    J.tma_f = tma_ok && make_tile_map(&J.map_f, f, J.dim);
+    J.tma_g = tma_ok && make_tile_map(&J.map_g, (const T*)g, J.dim);
     EZ_CHECK(cudaMemsetAsync(J.ctr, 0, C_COUNT * sizeof(int), st_));
     EZ_CHECK(cudaMemcpyAsync(jobs_dev_ + slot, &J, sizeof(J), cudaMemcpyHostToDevice, st_));
     jh.pc = PC_SETUP_A;
@@ -482,7 +479,7 @@ class BatchEngine {
     int* bc = jh.bcount;  // 4 x nb ints, free once the correction is over
     launch(K_OTHER, k_enc_count<T>, nb, kCpBlock, (const T*)J.g0, (const T*)J.g,
            (const int*)J.counter, N, q, et, bc);
-    launch(K_OTHER, k_scan_lists, 1, 1024, bc, nb, 2, reinterpret_cast<int*>(acc + 4));
+    launch(K_OTHER, k_scan_lists, 2, 1024, bc, nb, reinterpret_cast<int*>(acc + 4), (int*)nullptr);
     launch(K_OTHER, k_enc_stats<T>, grid_, 256, J.f, (const T*)J.g0, (const T*)J.g, N, acc);
     unsigned long long h[8];
     EZ_CHECK(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, st_));
@@ -537,7 +534,7 @@ class BatchEngine {
     const int N = J.dim.N, nb = jh.nb;
     int* tot = reinterpret_cast<int*>(jh.checksum);
     launch(K_OTHER, k_edit_count, nb, 32, (const unsigned*)J.edited, N, jh.bcount);
-    launch(K_OTHER, k_scan_lists, 1, 1024, jh.bcount, nb, 1, tot);
+    launch(K_OTHER, k_scan_lists, 1, 1024, jh.bcount, nb, tot, (int*)nullptr);
     launch(K_OTHER, k_edit_write<T>, nb, 32, (const unsigned*)J.edited, (const T*)J.g, N,
            (const int*)jh.bcount, J.touched, reinterpret_cast<T*>(J.delta));
     EZ_CHECK(cudaMemcpyAsync(count, tot, sizeof(int), cudaMemcpyDeviceToHost, st_));
@@ -587,7 +584,7 @@ class BatchEngine {
     launch(K_OTHER, k_pp_merge_table, kMergeWords * 32 / 256, 256, table);
     launch(K_OTHER, k_pp_cand_count<T>, jh.nb, kCpBlock, J.f, J.dim, (const unsigned*)table, member,
            jh.bcount);
-    launch(K_OTHER, k_scan_lists, 1, 1024, jh.bcount, jh.nb, 2, ctot);
+    launch(K_OTHER, k_scan_lists, 2, 1024, jh.bcount, jh.nb, ctot, (int*)nullptr);
     launch(K_OTHER, k_pp_cand_write, dim3((jh.nb + 7) / 8, 2), 256, (const unsigned*)member, jh.nb,
            (const int*)jh.bcount, cand, cand + N);
     int ns[2];
@@ -722,6 +719,11 @@ class BatchEngine {
     issued_ = false;
     ++tick_id_;
     const long long launches0 = launches_;
+    if (!seq_known_) {  // an earlier tick ended in an error: take up its number
+      EZ_CHECK(cudaStreamSynchronize(st_));
+      seq_next_ = *seq_host_;
+      seq_known_ = true;
+    }
     // A tick whose launches repeat an earlier tick's exactly (kernels, launch
     // shapes and arguments; per-job state is read from device memory) runs as
     // one CUDA graph: recorded, captured the third time its signature is
@@ -755,20 +757,27 @@ class BatchEngine {
           }
       rc = run_phase(ph, sel);
     }
+    // A tick that launched nothing (a manifold round over an unchanged field, a
+    // re-read of the counters) leaves the host's copy as it is.
+    launched_ = rc == EXTREMZ_OK && launches_ != launches0;
+    int hi = 0;  // the counter blocks up to the last slot in use (the host reads no other)
+    for (int i = 0; i < kMaxSel; ++i)
+      if (slots_[i].used) hi = i + 1;
+    published_ = launched_ && seq_host_ && !profile_ && !capturing_stream();
+    if (published_) {
+      launch(K_OTHER, k_publish, 1, 256, (const int*)ctr_dev_, C_COUNT * hi, ctr_host_, seq_dev_,
+             seq_host_);
+      ++seq_next_;
+      seq_known_ = false;
+    }
     recording_ = false;
     if (rc != EXTREMZ_OK) return rc;
     if (graph && !pending_.empty()) EZ_RUN(run_recorded());
-    // A tick that launched nothing (a manifold round over an unchanged field, a
-    // re-read of the counters) leaves the host's copy as it is.
-    launched_ = launches_ != launches0;
     if (!launched_) return EXTREMZ_OK;
     EZ_CHECK(cudaGetLastError());
-    // The counter blocks up to the last slot in use (the host reads no other).
-    int hi = 0;
-    for (int i = 0; i < kMaxSel; ++i)
-      if (slots_[i].used) hi = i + 1;
-    EZ_CHECK(cudaMemcpyAsync(ctr_host_, ctr_dev_, sizeof(int) * C_COUNT * (size_t)hi,
-                             cudaMemcpyDeviceToHost, st_));
+    if (!published_)
+      EZ_CHECK(cudaMemcpyAsync(ctr_host_, ctr_dev_, sizeof(int) * C_COUNT * (size_t)hi,
+                               cudaMemcpyDeviceToHost, st_));
     return EXTREMZ_OK;
   }
 
@@ -777,7 +786,8 @@ class BatchEngine {
     if (!issued_) return EXTREMZ_OK;
     issued_ = false;
     if (launched_) {
-      EZ_CHECK(cudaStreamSynchronize(st_));
+      if (published_) EZ_RUN(await_published());
+      else EZ_CHECK(cudaStreamSynchronize(st_));
       fold_timings();
     }
     for (int i = 0; i < kMaxSel; ++i) {
@@ -794,6 +804,39 @@ class BatchEngine {
       }
     }
     return EXTREMZ_OK;
+  }
+
+  bool capturing_stream() const {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st_, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone)
+      return false;
+    cudaGetLastError();
+    return true;
+  }
+
+  // Waits for the tick's number.  The stream is asked now and then: an error
+  // ends the wait, and once all its work is done the number is there.
+  int await_published() {
+    for (;;) {
+      for (int k = 0; k < 2000; ++k) {
+        if (*seq_host_ == seq_next_) {
+          std::atomic_thread_fence(std::memory_order_acquire);
+          seq_known_ = true;
+          return EXTREMZ_OK;
+        }
+#if defined(__x86_64__)
+        __builtin_ia32_pause();
+#endif
+      }
+      const cudaError_t e = cudaStreamQuery(st_);
+      if (e == cudaErrorNotReady) continue;
+      EZ_CHECK(e);
+      if (*seq_host_ == seq_next_) continue;
+      EZ_CHECK(cudaStreamSynchronize(st_));
+      if (*seq_host_ == seq_next_) continue;
+      last_cuda_error() = cudaErrorUnknown;
+      return EXTREMZ_CUDA_ERR;
+    }
   }
 
   // Per-class timing of the launches since set_profile(true, ...).
@@ -853,9 +896,15 @@ class BatchEngine {
   int sms_ = 148;
   DeviceTables tb_{};
   Job<T>* jobs_dev_ = nullptr;
-  CUtensorMap* maps_dev_ = nullptr;
   int* ctr_dev_ = nullptr;
   int* ctr_host_ = nullptr;
+  // Number of the last published tick (k_publish), on the device and as the
+  // host sees it; the borrowed engine, whose host copy is not mapped, has none.
+  unsigned* seq_dev_ = nullptr;
+  volatile unsigned* seq_host_ = nullptr;
+  unsigned seq_next_ = 0;
+  bool seq_known_ = true;
+  bool published_ = false;  // this tick's counters come through k_publish
   int static_ctr_host_[C_COUNT * kMaxSel];
   std::vector<JobHost<T>> slots_;
   long long launches_ = 0;
@@ -1145,9 +1194,9 @@ class BatchEngine {
     int bps = 1;  // jobs share launches: the largest knob of the selection
     for (int i : sel) bps = std::max(bps, slots_[i].blocks_per_sm);
     grid_ = sms_ * bps;
-    if (ph == PC_CL_ROUND || ph == PC_RLOOPS || ph == PC_SLOOPS || ph == PC_SADDLE ||
-        ph == PC_SLOOPS_J || ph == PC_SADDLE_J || ph == PC_FINAL_JOIN)
-      for (int i : sel) slots_[i].applied_tick = tick_id_;  // phases that apply edits
+    if (ph == PC_CL_ROUND || ph == PC_RLOOPS || ph == PC_SLOOPS_J || ph == PC_SADDLE_J ||
+        ph == PC_FINAL_JOIN)
+      for (int i : sel) edits(i);  // phases that apply edits
     const Sel s = make_span(sel);
     const int nb = blocks(s);
     const Job<T>* jobs = jobs_dev_;
@@ -1179,9 +1228,17 @@ class BatchEngine {
         }
         return EXTREMZ_OK;
       case PC_CL_DETECT:
-        detect(sel);
+      case PC_FINAL_DETECT: {
+        // No value changed since the last detection: its list and counts stand.
+        std::vector<int> busy;
+        for (int i : sel) {
+          const JobHost<T>& j = slots_[i];
+          if (!j.dense_done || j.applied_tick == tick_id_ || h(i, C_DIRTY) > 0) busy.push_back(i);
+        }
+        detect(busy);
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
+      }
       case PC_CL_ROUND:
         launch(K_PROPOSE, k_propose_cp<T>, nb, 256, jobs, s);
         launch(K_APPLY, k_apply<T>, nb, 256, jobs, s);
@@ -1204,8 +1261,12 @@ class BatchEngine {
           JobHost<T>& j = slots_[i];
           const bool known_clean =
               j.manifold_rounds > 0 && j.applied_tick != tick_id_ && h(i, C_CHANGED) == 0;
-          if (known_clean) j.reused += 1;
-          else busy.push_back(i);
+          if (known_clean) {
+            j.reused += 1;
+          } else {
+            busy.push_back(i);
+            j.wim_seen = j.wis_seen = false;
+          }
         }
         if (!busy.empty()) {
           const Sel bs = make_span(busy);
@@ -1267,20 +1328,38 @@ class BatchEngine {
         }
         return EXTREMZ_OK;
       }
-      case PC_SLOOPS:
-        launch(K_OTHER, k_wim_scan<T, true>, nb, 256, jobs, s);
-        launch(K_OTHER, k_wim_collect<T, true>, nb, 256, jobs, s, 1);
-        launch(K_APPLY, k_apply<T>, nb, 256, jobs, s);
+      case PC_SLOOPS: {
+        // A scan of this very state that found nothing proposes nothing again.
+        std::vector<int> busy;
+        for (int i : sel)
+          if (!(still(i, slots_[i].wim_seen) && h(i, C_WMC) == 0 && h(i, C_WMC2) == 0))
+            busy.push_back(i);
+        if (!busy.empty()) {
+          const Sel bs = make_span(busy);
+          launch(K_OTHER, k_wim_scan<T, true>, blocks(bs), 256, jobs, bs);
+          launch(K_OTHER, k_wim_collect<T, true>, blocks(bs), 256, jobs, bs, 1);
+          launch(K_APPLY, k_apply<T>, blocks(bs), 256, jobs, bs);
+        }
+        for (int i : busy) edits(i).wim_seen = true;
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
-      case PC_SADDLE:
-        wis_scan<true>(s, 1);
-        launch(K_APPLY, k_apply<T>, nb, 256, jobs, s);
+      }
+      case PC_SADDLE: {
+        std::vector<int> busy;
+        for (int i : sel)
+          if (!(still(i, slots_[i].wis_seen) && h(i, C_WSC) == 0)) busy.push_back(i);
+        if (!busy.empty()) {
+          const Sel bs = make_span(busy);
+          wis_scan<true>(bs, 1);
+          launch(K_APPLY, k_apply<T>, blocks(bs), 256, jobs, bs);
+        }
+        for (int i : busy) edits(i).wis_seen = true;
         for (int i : sel) {
           slots_[i].pending.push_back(PH_SADDLE);
           slots_[i].pc = joinb(slots_[i]);
         }
         return EXTREMZ_OK;
+      }
       case PC_SLOOPS_J:
         launch(K_OTHER, k_wim_scan<T, false>, nb, 256, jobs, s);
         launch(K_OTHER, k_wim_collect<T, false>, nb, 256, jobs, s, 1);
@@ -1312,28 +1391,43 @@ class BatchEngine {
       case PC_PRE_END:
         for (int i : sel) slots_[i].waiting = true;
         return EXTREMZ_OK;
-      case PC_DET3:
-        launch(K_OTHER, k_wim_scan<T, true>, nb, 256, jobs, s);
-        launch(K_OTHER, k_wim_collect<T, true>, nb, 256, jobs, s, 0);
-        wis_scan<true>(s, 0);
+      case PC_DET3: {
+        std::vector<int> busy;
+        for (int i : sel)
+          if (!still(i, slots_[i].wim_seen && slots_[i].wis_seen)) busy.push_back(i);
+        if (!busy.empty()) {
+          const Sel bs = make_span(busy);
+          launch(K_OTHER, k_wim_scan<T, true>, blocks(bs), 256, jobs, bs);
+          launch(K_OTHER, k_wim_collect<T, true>, blocks(bs), 256, jobs, bs, 0);
+          wis_scan<true>(bs, 0);
+        }
+        for (int i : busy) slots_[i].wim_seen = slots_[i].wis_seen = true;
         for (int i : sel) {
           slots_[i].pending.push_back(PH_DETECT3);
           slots_[i].pc = (slots_[i].p.flags & kFlagCensus) ? PC_DET3J : join3(slots_[i]);
         }
         return EXTREMZ_OK;
+      }
       case PC_DET3J:
         launch(K_OTHER, k_wim_scan<T, false>, nb, 256, jobs, s);
         launch(K_OTHER, k_wim_collect<T, false>, nb, 256, jobs, s, 0);
         wis_scan<false>(s, 0);
         for (int i : sel) slots_[i].pc = PC_FINAL_DETECT;
         return EXTREMZ_OK;
-      case PC_FINAL_DETECT:
-        detect(sel);
-        for (int i : sel) slots_[i].waiting = true;
-        return EXTREMZ_OK;
       default:
         return EXTREMZ_OK;
     }
+  }
+
+  JobHost<T>& edits(int i) {
+    slots_[i].applied_tick = tick_id_;
+    return slots_[i];
+  }
+  // seen: a scan ran since job i's last computed manifold round.  True when no
+  // value has changed since that round, so that the scan's counts, which are in
+  // the host's copy, are those of the present field.
+  bool still(int i, bool seen) const {
+    return seen && slots_[i].applied_tick != tick_id_ && h(i, C_CHANGED) == 0;
   }
 
   // Blocks over a selection's listed tiles: a job's share of four per SM goes
@@ -1364,6 +1458,7 @@ class BatchEngine {
   // Mismatch detection: dense the first time a job detects, then incremental
   // over the neighbourhoods of the vertices changed since.
   void detect(const std::vector<int>& sel) {
+    if (sel.empty()) return;
     std::vector<int> dense, incr;
     for (int i : sel) (slots_[i].dense_done ? incr : dense).push_back(i);
     if (!dense.empty()) {
@@ -1390,21 +1485,44 @@ class BatchEngine {
   }
 
   // Exclusive scan of nl lists of n counts each (list l at c + l * n), the
-  // list totals into totals[0 .. nl); chunk holds nl * ceil(n / 1024) sums.
-  int scan_counts(int* c, int n, int nl, int* totals, int* chunk) {
+  // list totals into totals[0 .. nl), a second copy of the (one) scanned list
+  // into cursor; chunk holds nl * ceil(n / 1024) sums.  Up to one pass of a
+  // block (32 Ki counts) a block per list does it all.
+  int scan_counts(int* c, int n, int nl, int* totals, int* chunk, int* cursor = nullptr) {
+    if (n <= 32 * 1024) {
+      launch(K_OTHER, k_scan_lists, nl, 1024, c, n, totals, cursor);
+      return EXTREMZ_OK;
+    }
     const int nc = (n + 1023) / 1024;
     launch(K_OTHER, k_chunk_sums, dim3(nc, nl), 1024, (const int*)c, n, chunk);
-    launch(K_OTHER, k_scan_lists, 1, 1024, chunk, nc, nl, totals);
-    launch(K_OTHER, k_chunk_scan, dim3(nc, nl), 1024, c, n, (const int*)chunk);
+    launch(K_OTHER, k_scan_lists, nl, 1024, chunk, nc, totals, (int*)nullptr);
+    launch(K_OTHER, k_chunk_scan, dim3(nc, nl), 1024, c, n, (const int*)chunk, cursor);
     return EXTREMZ_OK;
   }
 
-  // Per-extremum entry counts cnt[0 .. n) into offsets (the total into cnt[n])
-  // and a copy of the offsets into cur, the fill cursors.
-  int entry_lists(int* cnt, int* cur, int n, int* chunk) {
-    EZ_RUN(scan_counts(cnt, n, 1, cnt + n, chunk));
-    EZ_CHECK(cudaMemcpyAsync(cur, cnt, (size_t)n * 4, cudaMemcpyDeviceToDevice, st_));
-    return EXTREMZ_OK;
+  // Arrays to fill before a job's first round, in one launch (k_fill_many).
+  struct Fills {
+    FillList f{};
+    template <class P>
+    void add(P* at, long long count, unsigned long long value) {
+      if (count <= 0) return;
+      const long long pieces = (count * (long long)sizeof(P) + 15) / 16;
+      f.at[f.n] = reinterpret_cast<ulonglong2*>(at);
+      f.end[f.n] = (f.n ? f.end[f.n - 1] : 0) + pieces;
+      f.value[f.n++] = value;
+    }
+  };
+  void fill(const Fills& fl) {
+    if (fl.f.n == 0) return;
+    const long long pieces = fl.f.end[fl.f.n - 1];
+    launch(K_OTHER, k_fill_many, (int)std::min<long long>(grid_, (pieces + 255) / 256), 256, fl.f);
+  }
+  // A 4-byte value in both halves of the pattern.
+  static constexpr unsigned long long twice(unsigned v) {
+    return (unsigned long long)v << 32 | v;
+  }
+  static constexpr unsigned long long key_pattern(K k) {
+    return sizeof(K) == 8 ? (unsigned long long)k : twice((unsigned)k);
   }
 
   int setup_b(int slot) {
@@ -1461,69 +1579,78 @@ class BatchEngine {
     J.wlong = A.take<int>(ne);
     int* chunk = A.take<int>(ne / 1024 + 2);
     if (!jh.checksum || !J.ext_id || !J.ocnt1 || !J.first_sj || !chunk) return EXTREMZ_OOM;
-    // Per side: the rows (with their compact copies, each named extremum's
-    // extreme saddle key and entry count), the entry lists' offsets, then the
-    // extreme saddle ids and the entries.  The sides share the selection
-    // scratch (ext_key, ext_id), so they go one after the other.  Rows name
-    // only extrema, so a side with rows has extrema.  Without join_rows the
-    // minima's side waits for the final join pass (k_join_*), which wants its
-    // scratch filled.
-    if (nmax) {
-      launch(K_OTHER, k_fill<K>, grid_, 256, J.ext_key, K(0), (long long)nmax);
-      launch(K_OTHER, k_fill<int>, grid_, 256, J.ext_id, -1, (long long)nmax);
-      EZ_CHECK(cudaMemsetAsync(J.moff2, 0, (size_t)(nmax + 1) * 4, st_));
+    const long long words = (N + 31) / 32;
+    const bool join_side = J.join_rows || jh.p.final_join;
+    Fills fl;
+    // The maxima's selection scratch, entry counts, arbitration slots and
+    // wrong-saddle results.
+    fl.add(J.ext_key, nmax, 0);
+    fl.add(J.largest, nmax, ~0ull);
+    fl.add(J.moff2, nmax + 1, 0);
+    fl.add(J.wstamp2, nmax, 0);
+    fl.add(J.first1, nmax, twice(kInf));
+    fl.add(J.first_s, nmax, twice(kInf));
+    fl.add(J.flag2, nmax, 0);
+    // The minima's; without join_rows only what the final join pass uses.
+    if (join_side) {
+      fl.add(J.smallest, nmin, twice(kInf));
+      fl.add(J.first_sj, nmin, twice(kInf));
     }
-    launch(K_SETUP, k_rows<T, true>, grid_, 256, J);
-    if (nmax) {
-      EZ_RUN(entry_lists(J.moff2, J.wstamp2, nmax, chunk));
-      launch(K_OTHER, k_extreme_saddle<T, true>, grid_, 256, J);
-      EZ_CHECK(cudaMemsetAsync(J.wstamp2, 0, (size_t)nmax * 4, st_));
-      EZ_CHECK(cudaMemcpyAsync(J.largest, J.ext_id, nmax * 4, cudaMemcpyDeviceToDevice, st_));
-      launch(K_OTHER, k_fill<int>, grid_, 256, J.first1, kInf, (long long)nmax);
-      launch(K_OTHER, k_fill<int>, grid_, 256, J.first_s, kInf, (long long)nmax);
-      EZ_CHECK(cudaMemsetAsync(J.flag2, 0, nmax * 4, st_));
-    }
-    if (nmin && (J.join_rows || jh.p.final_join)) {
-      launch(K_OTHER, k_fill<K>, grid_, 256, J.ext_key, ~K(0), (long long)nmin);
-      launch(K_OTHER, k_fill<int>, grid_, 256, J.ext_id, kInf, (long long)nmin);
-      launch(K_OTHER, k_fill<int>, grid_, 256, J.first_sj, kInf, (long long)nmin);
-    }
-    if (!J.join_rows) {
-      J.smallest = J.ext_id;  // as k_join_ids leaves it
-    } else {
-      if (nmin) EZ_CHECK(cudaMemsetAsync(J.moff1, 0, (size_t)(nmin + 1) * 4, st_));
-      launch(K_SETUP, k_rows<T, false>, grid_, 256, J);
-      if (nmin) {
-        EZ_RUN(entry_lists(J.moff1, J.wstamp1, nmin, chunk));
-        launch(K_OTHER, k_extreme_saddle<T, false>, grid_, 256, J);
-        EZ_CHECK(cudaMemsetAsync(J.wstamp1, 0, (size_t)nmin * 4, st_));
-        EZ_CHECK(cudaMemcpyAsync(J.smallest, J.ext_id, nmin * 4, cudaMemcpyDeviceToDevice, st_));
-        launch(K_OTHER, k_fill<int>, grid_, 256, J.ext_id, kInf, (long long)nmin);
-        launch(K_OTHER, k_fill<int>, grid_, 256, J.first_min1, kInf, (long long)nmin);
-        EZ_CHECK(cudaMemsetAsync(J.flag_min2, 0, nmin * 4, st_));
-      }
+    if (J.join_rows) {
+      fl.add(J.moff1, nmin + 1, 0);
+      fl.add(J.wstamp1, nmin, 0);
+      fl.add(J.first_min1, nmin, twice(kInf));
+      fl.add(J.flag_min2, nmin, 0);
+      fl.add(J.ext_id, nmin, twice(kInf));
+      fl.add(J.drow1, ns1 * 2ll, 0);
     }
     // Decompressed row slots start at zero: the reference's rows are fresh
     // cudaMalloc memory read before first written (:5338-5341, :3128-3130).
-    if (ns2) EZ_CHECK(cudaMemsetAsync(J.drow2, 0, (size_t)ns2 * 2 * 4, st_));
-    if (ns1 && J.join_rows) EZ_CHECK(cudaMemsetAsync(J.drow1, 0, (size_t)ns1 * 2 * 4, st_));
-    // Every tile's pointers are computed in the first manifold round.
-    EZ_CHECK(cudaMemsetAsync(J.tdirty, 1, (size_t)jh.ntiles * 4, st_));
-    // Block stamps start below the first round's; no root is touched.
-    EZ_CHECK(cudaMemsetAsync(J.bdirty, 0, (size_t)jh.nb * 4, st_));
-    EZ_CHECK(cudaMemsetAsync(J.rtouch2, 0, (size_t)((N + 31) / 32) * 4, st_));
-    EZ_CHECK(cudaMemsetAsync(J.rtouch1, 0, (size_t)((N + 31) / 32) * 4, st_));
+    fl.add(J.drow2, ns2 * 2ll, 0);
+    // Every tile's pointers are computed in the first manifold round, block
+    // stamps start below its stamp, no root is touched, every value counts as
+    // changed for it and none for the wrong-saddle scans and detections.
+    fl.add(J.tdirty, jh.ntiles, ~0ull);
+    fl.add(J.bdirty, jh.nb, 0);
+    fl.add(J.rtouch2, words, 0);
+    fl.add(J.rtouch1, words, 0);
+    fl.add(J.vchg, words, ~0ull);
+    fl.add(J.wchg2, words, 0);
+    if (J.join_rows) fl.add(J.wchg1, words, 0);
+    fl.add(J.dbits, words, 0);
+    fl.add(J.dbits1, words, 0);
+    fill(fl);
     // Proposal buffer at the sentinel; edit counters, which only edit_type 0
-    // reads, at -1 (:5082); no changed vertex; arbitration votes, which only the
-    // ascending order reads, at 0.
-    launch(K_OTHER, k_fill<K>, grid_, 256, J.delta, J.sentinel_key, (long long)N);
-    if (J.edit_type == 0) launch(K_OTHER, k_fill<int>, grid_, 256, J.counter, -1, (long long)N);
-    if (!J.wn_lockstep) EZ_CHECK(cudaMemsetAsync(J.claim, 0, (size_t)N * 8, st_));
-    EZ_CHECK(cudaMemsetAsync(J.dbits, 0, (size_t)((N + 31) / 32) * 4, st_));
-    EZ_CHECK(cudaMemsetAsync(J.dbits1, 0, (size_t)((N + 31) / 32) * 4, st_));
-    EZ_CHECK(cudaMemsetAsync(J.vchg, 0xff, (size_t)((N + 31) / 32) * 4, st_));
-    EZ_CHECK(cudaMemsetAsync(J.wchg2, 0, (size_t)((N + 31) / 32) * 4, st_));
-    EZ_CHECK(cudaMemsetAsync(J.wchg1, 0, (size_t)((N + 31) / 32) * 4, st_));
+    // reads, at -1 (:5082); arbitration votes, which only the ascending order
+    // reads, at 0.
+    Fills fv;
+    fv.add(J.delta, N, key_pattern(J.sentinel_key));
+    if (J.edit_type == 0) fv.add(J.counter, N, ~0ull);
+    if (!J.wn_lockstep) fv.add(J.claim, N, 0);
+    fill(fv);
+    // Per side: the rows (with their compact copies, each named extremum's
+    // extreme saddle key and entry count), the entry lists' offsets, then the
+    // extreme saddle ids and the entries.  The sides share the selection
+    // scratch (ext_key) and the fill cursors (aff), so they go one after the
+    // other.  Rows name only extrema, so a side with rows has extrema.  Without
+    // join_rows the minima's side waits for the final join pass (k_join_*).
+    launch(K_SETUP, k_rows<T, true>, grid_, 256, J);
+    if (nmax) {
+      EZ_RUN(scan_counts(J.moff2, nmax, 1, J.moff2 + nmax, chunk, J.aff));
+      launch(K_OTHER, k_extreme_saddle<T, true>, grid_, 256, J);
+    }
+    if (join_side) {
+      Fills fk;
+      fk.add(J.ext_key, nmin, ~0ull);
+      fill(fk);
+    }
+    if (J.join_rows) {
+      launch(K_SETUP, k_rows<T, false>, grid_, 256, J);
+      if (nmin) {
+        EZ_RUN(scan_counts(J.moff1, nmin, 1, J.moff1 + nmin, chunk, J.aff));
+        launch(K_OTHER, k_extreme_saddle<T, false>, grid_, 256, J);
+      }
+    }
     EZ_CHECK(cudaMemcpyAsync(jobs_dev_ + slot, &J, sizeof(J), cudaMemcpyHostToDevice, st_));
     return EXTREMZ_OK;
   }

@@ -484,7 +484,7 @@ constexpr size_t kNoAllocScratchBytes = kNoAllocEngineBytes + (size_t)kNoAllocMa
 // Both engines (float and double) carve their descriptor, tile-map and
 // counter arrays from the first part.
 constexpr size_t kEngineArrayBytes(size_t job) {
-  return ((job * kMaxSel + 255) & ~size_t(255)) + ((sizeof(CUtensorMap) * 2 * kMaxSel + 255) & ~size_t(255)) +
+  return ((job * kMaxSel + 255) & ~size_t(255)) +
          ((sizeof(int) * C_COUNT * kMaxSel + 255) & ~size_t(255));
 }
 static_assert(kEngineArrayBytes(sizeof(Job<float>)) + kEngineArrayBytes(sizeof(Job<double>)) <=

@@ -83,13 +83,13 @@ struct Job {
   int* aff;                     // extrema queued for the wrong-saddle update
   int* wlong;                   // of those, the ones with long entry lists
   unsigned* wchg2; unsigned* wchg1;  // bitsets: values changed since the last wrong-saddle scan
-  K* ext_key; int* ext_id;      // largest / smallest saddle selection scratch; ext_id then
-                                // the lowest-row arbitration of get_wrong_index_min (kInf)
+  K* ext_key;                   // largest / smallest saddle selection scratch
+  int* ext_id;                  // lowest-row arbitration of get_wrong_index_min (kInf)
 
   int* ctr;  // device counters, see Ctr
   DeviceTables tb;
-  const CUtensorMap* map_f;  // tile maps of f and g in device memory (when tma_f / tma_g)
-  const CUtensorMap* map_g;
+  CUtensorMap map_f, map_g;  // tile maps of f and g (when tma_f / tma_g); the kernels that load
+                             // tiles read the descriptor in device memory
   int tma_f, tma_g;
   int iter_cap;  // device-side limit of pointer jumping and path walks
   int join_rows;  // the 1-saddles' rows are read during the correction (preserve_join, or a
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ job
   const Job<T>& J = tile_job(jobs, sel, bx, by, bz);
   const Dims g = J.dim;
   // The block decides together: its threads meet at barriers further on.
-  if (!__syncthreads_and(load_tile<T>(s, &bar, J.map_g, J.tma_g, J.g, g, bx, by, bz))) {
+  if (!__syncthreads_and(load_tile<T>(s, &bar, &J.map_g, J.tma_g, J.g, g, bx, by, bz))) {
     if (threadIdx.x == 0) atomicOr(J.ctr + C_ERROR, kErrTile);
     return;
   }
@@ -651,7 +651,7 @@ __device__ __noinline__ bool direction_tile(const Job<T>& J, Tile<T>& s, uint64_
   int* ds = kDec ? J.pdd : J.ds;
   int* as = kDec ? J.pda : J.as;
   // The block decides together: its threads meet at a barrier further on.
-  if (!__syncthreads_and(load_tile<T>(s, bar, kDec ? J.map_g : J.map_f, kDec ? J.tma_g : J.tma_f,
+  if (!__syncthreads_and(load_tile<T>(s, bar, kDec ? &J.map_g : &J.map_f, kDec ? J.tma_g : J.tma_f,
                                       a, g, bx, by, bz, parity, init))) {
     if (threadIdx.x == 0) atomicOr(J.ctr + C_ERROR, kErrTile);
     return false;
@@ -1053,63 +1053,65 @@ __global__ void __launch_bounds__(32 * kCpWarps) k_cp_count(const int8_t* __rest
   }
 }
 
-// Single block: exclusive scan of nlists x nb block counts in place, list
-// totals to totals[0 .. nlists).  The CP lists use totals = ctr + C_NS2.  Each
-// thread takes 32 consecutive counts per pass.
-__global__ void __launch_bounds__(1024) k_scan_lists(int* __restrict__ bcount, int nb, int nlists,
-                                                     int* totals) {
+// Exclusive scan of gridDim.x lists of nb counts in place (a block per list),
+// list totals to totals[0 .. gridDim.x).  The CP lists use totals = ctr + C_NS2.
+// Each thread takes 32 consecutive counts per pass.  cursor (optional, one
+// list): a second copy of the scanned counts.
+__global__ void __launch_bounds__(1024) k_scan_lists(int* __restrict__ bcount, int nb, int* totals,
+                                                     int* __restrict__ cursor) {
   constexpr int kPer = 32;
   __shared__ int carry;
   __shared__ int warp_sums[32];
-  for (int l = 0; l < nlists; ++l) {
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    int* c = bcount + (long long)l * nb;
-    for (int base = 0; base < nb; base += 1024 * kPer) {
-      const int i0 = base + (int)threadIdx.x * kPer;
-      int x[kPer];
-      int sum = 0;
+  const int l = blockIdx.x;
+  if (threadIdx.x == 0) carry = 0;
+  __syncthreads();
+  int* c = bcount + (long long)l * nb;
+  for (int base = 0; base < nb; base += 1024 * kPer) {
+    const int i0 = base + (int)threadIdx.x * kPer;
+    int x[kPer];
+    int sum = 0;
 #pragma unroll
-      for (int k = 0; k < kPer; ++k) {
-        x[k] = i0 + k < nb ? c[i0 + k] : 0;
-        sum += x[k];
-      }
-      int incl = sum;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane_id() >= (unsigned)o) incl += y;
-      }
-      if (lane_id() == 31) warp_sums[threadIdx.x / 32] = incl;
-      __syncthreads();
-      if (threadIdx.x < 32) {
-        int w = warp_sums[threadIdx.x], wi = w;
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, wi, o);
-          if (lane_id() >= (unsigned)o) wi += y;
-        }
-        warp_sums[threadIdx.x] = wi - w;
-      }
-      __syncthreads();
-      int run = carry + warp_sums[threadIdx.x / 32] + incl - sum;
-#pragma unroll
-      for (int k = 0; k < kPer; ++k) {
-        if (i0 + k < nb) c[i0 + k] = run;
-        run += x[k];
-      }
-      __syncthreads();
-      if (threadIdx.x == 1023) carry = run;
-      __syncthreads();
+    for (int k = 0; k < kPer; ++k) {
+      x[k] = i0 + k < nb ? c[i0 + k] : 0;
+      sum += x[k];
     }
-    if (threadIdx.x == 0) totals[l] = carry;
+    int incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane_id() >= (unsigned)o) incl += y;
+    }
+    if (lane_id() == 31) warp_sums[threadIdx.x / 32] = incl;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      int w = warp_sums[threadIdx.x], wi = w;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, wi, o);
+        if (lane_id() >= (unsigned)o) wi += y;
+      }
+      warp_sums[threadIdx.x] = wi - w;
+    }
+    __syncthreads();
+    int run = carry + warp_sums[threadIdx.x / 32] + incl - sum;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      if (i0 + k < nb) {
+        c[i0 + k] = run;
+        if (cursor) cursor[i0 + k] = run;
+      }
+      run += x[k];
+    }
+    __syncthreads();
+    if (threadIdx.x == 1023) carry = run;
     __syncthreads();
   }
+  if (threadIdx.x == 0) totals[l] = carry;
 }
 
 // Exclusive scan in place of lists of n counts (list l at c + l * n, one per
 // blockIdx.y) for lists too long for one block: the sum of every 1024-count
 // chunk (k_chunk_sums, into sums + l * gridDim.x), a scan of the sums with the
-// list totals (k_scan_lists, one block), then each chunk scanned from its
-// offset (k_chunk_scan).
+// list totals (k_scan_lists), then each chunk scanned from its offset
+// (k_chunk_scan).
 __global__ void __launch_bounds__(1024) k_chunk_sums(const int* __restrict__ c, int n,
                                                      int* __restrict__ sums) {
   __shared__ int ws[32];
@@ -1128,7 +1130,8 @@ __global__ void __launch_bounds__(1024) k_chunk_sums(const int* __restrict__ c, 
 }
 
 __global__ void __launch_bounds__(1024) k_chunk_scan(int* __restrict__ c, int n,
-                                                     const int* __restrict__ offs) {
+                                                     const int* __restrict__ offs,
+                                                     int* __restrict__ cursor) {
   __shared__ int ws[32];
   c += (long long)blockIdx.y * n;
   offs += (long long)blockIdx.y * gridDim.x;
@@ -1151,7 +1154,11 @@ __global__ void __launch_bounds__(1024) k_chunk_scan(int* __restrict__ c, int n,
     ws[threadIdx.x] = wi - w;
   }
   __syncthreads();
-  if (i < n) c[i] = offs[blockIdx.x] + ws[threadIdx.x >> 5] + incl - x;
+  if (i < n) {
+    const int at = offs[blockIdx.x] + ws[threadIdx.x >> 5] + incl - x;
+    c[i] = at;
+    if (cursor) cursor[i] = at;
+  }
 }
 
 __global__ void __launch_bounds__(32 * kCpWarps) k_cp_write(const int8_t* __restrict__ otype,
@@ -1370,7 +1377,7 @@ __global__ void __launch_bounds__(256) k_extreme_saddle(Job<T> J) {
   const int* sad = kMax ? J.sad2 : J.sad1;
   const int* rows = kMax ? J.orow2 : J.orow1;
   const uint8_t* ocnt = kMax ? J.ocnt2 : J.ocnt1;
-  int* cur = kMax ? J.wstamp2 : J.wstamp1;
+  int* cur = J.aff;  // scratch until the first wrong-saddle scan
   int* ent = kMax ? J.ment2 : J.ment1;
   const int stride = gridDim.x * blockDim.x;
   // Uniform per warp: lanes naming the same extremum (neighbouring saddles
@@ -1414,8 +1421,8 @@ __global__ void __launch_bounds__(256) k_extreme_saddle(Job<T> J) {
         const int pos = __shfl_sync(0xffffffffu, at[q], __ffs(grp[q]) - 1) + __popc(below);
         if (m[q] < 0) continue;
         if (ek[q] == key) {
-          if (kMax) atomicMax(J.ext_id + m[q], s);
-          else atomicMin(J.ext_id + m[q], s);
+          if (kMax) atomicMax(J.largest + m[q], s);
+          else atomicMin(J.smallest + m[q], s);
         }
         ent[pos] = i * kRowStride + h + q;
       }
@@ -2262,7 +2269,7 @@ __global__ void __launch_bounds__(256) k_wim_collect(const Job<T>* __restrict__ 
 // get_wrong_index_min direction 1 (:3157-3168, fix :3393-3410) keeps the pair of
 // the lowest row per minimum and lowers the row's FALSE last entry, so it needs
 // the winning row: one more scan, arbitrating through ext_id (the setup's
-// scratch, left at kInf; first_sj keeps the wrong-saddle results between
+// array, left at kInf; first_sj keeps the wrong-saddle results between
 // scans).
 template <class T>
 __global__ void __launch_bounds__(256) k_wim_min2_scan(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
@@ -2502,8 +2509,8 @@ __global__ void __launch_bounds__(256) k_wis_collect(const Job<T>* __restrict__ 
 // orow1 / ocnt1), the smallest id at that key (k_join_ids: together
 // findSmallestSaddlePerMin :4915-4940), and the first row per minimum whose
 // saddle comes before that smallest saddle in the decompressed field
-// (k_join_scan, into first_sj for k_wis_collect).  Scratch ext_key, ext_id
-// (= smallest) and first_sj were filled at setup.  1.9 ms for the 22 M
+// (k_join_scan, into first_sj for k_wis_collect).  ext_key, smallest and first_sj
+// were filled at setup.  1.9 ms for the 22 M
 // 1-saddles of the 512^3 benchmark field, where their rows, entry lists and
 // first full scan took 4.2 ms; a job that ends early does not run them.
 // ---------------------------------------------------------------------------
@@ -2590,10 +2597,10 @@ __global__ void __launch_bounds__(256) k_join_ids(const Job<T>* __restrict__ job
     for (int q = 0; q < 4; ++q) cur[q] = m[q] >= 0 ? J.ext_key[m[q]] : KK(0);
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      if (m[q] >= 0 && cur[q] == key) atomicMin(J.ext_id + m[q], s);
+      if (m[q] >= 0 && cur[q] == key) atomicMin(J.smallest + m[q], s);
     for (int p = 4; p < cnt; ++p) {
       const int mm = J.orow1[(long long)i * kRowStride + p];
-      if (J.ext_key[mm] == key) atomicMin(J.ext_id + mm, s);
+      if (J.ext_key[mm] == key) atomicMin(J.smallest + mm, s);
     }
   }
 }
@@ -2614,14 +2621,14 @@ __global__ void __launch_bounds__(256) k_join_scan(const Job<T>* __restrict__ jo
     int t[4];
     T gt[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) t[q] = m[q] >= 0 ? J.ext_id[m[q]] : s;
+    for (int q = 0; q < 4; ++q) t[q] = m[q] >= 0 ? J.smallest[m[q]] : s;
 #pragma unroll
     for (int q = 0; q < 4; ++q) gt[q] = t[q] != s ? g[t[q]] : T(0);
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if (t[q] != s && below(gs, s, gt[q], t[q])) atomicMin(J.first_sj + m[q], i * kRowStride);
     for (int p = 4; p < cnt; ++p) {
-      const int mm = J.orow1[(long long)i * kRowStride + p], tt = J.ext_id[mm];
+      const int mm = J.orow1[(long long)i * kRowStride + p], tt = J.smallest[mm];
       if (tt != s && below(gs, s, g[tt], tt)) atomicMin(J.first_sj + mm, i * kRowStride);
     }
   }
@@ -2630,6 +2637,43 @@ __global__ void __launch_bounds__(256) k_join_scan(const Job<T>* __restrict__ jo
 // ---------------------------------------------------------------------------
 // Small helpers.
 // ---------------------------------------------------------------------------
+// Initial contents of a job's arrays in one launch: segment k is `chunks`
+// 16-byte pieces (arrays are padded to 256 bytes) of the 8-byte pattern `value`.
+// One launch in place of some twenty fills and clears, whose issue took the host
+// longer than a small field's setup takes the device.
+constexpr int kMaxFills = 28;
+struct FillList {
+  int n;
+  ulonglong2* at[kMaxFills];
+  long long end[kMaxFills];  // inclusive prefix of the segments' pieces
+  unsigned long long value[kMaxFills];
+};
+__global__ void __launch_bounds__(256) k_fill_many(const __grid_constant__ FillList f) {
+  const long long total = f.end[f.n - 1], stride = (long long)gridDim.x * blockDim.x;
+  int k = 0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += stride) {
+    while (i >= f.end[k]) ++k;
+    const unsigned long long v = f.value[k];
+    f.at[k][i - (k ? f.end[k - 1] : 0)] = make_ulonglong2(v, v);
+  }
+}
+
+// The counter blocks to the host's (mapped) copy at the end of a tick, then the
+// tick's number, which the host waits for: a copy and a stream synchronisation
+// behind the kernels took about 8 us longer.
+__global__ void __launch_bounds__(256) k_publish(const int* __restrict__ ctr, int n, int* host,
+                                                 unsigned* seq, volatile unsigned* host_seq) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) host[i] = ctr[i];
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned s = *seq + 1u;
+    *seq = s;
+    __threadfence_system();
+    *host_seq = s;
+  }
+}
+
 template <class K>
 __global__ void k_fill(K* p, K v, long long n) {
   const long long stride = (long long)gridDim.x * blockDim.x;
