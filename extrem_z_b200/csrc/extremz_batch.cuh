@@ -252,13 +252,14 @@ class BatchEngine {
       if (cudaMalloc(&jobs_dev_, desc_bytes) != cudaSuccess ||
           cudaMalloc(&ctr_dev_, ctr_bytes + sizeof(unsigned)) != cudaSuccess ||
           cudaMemset(ctr_dev_, 0, ctr_bytes + sizeof(unsigned)) != cudaSuccess ||
-          cudaMallocHost(&ctr_host_, ctr_bytes + sizeof(unsigned)) != cudaSuccess) {
+          cudaMallocHost(&ctr_host_, 3 * ctr_bytes) != cudaSuccess) {
         cudaGetLastError();
         return EXTREMZ_OOM;
       }
-      std::memset(ctr_host_, 0, ctr_bytes + sizeof(unsigned));
+      std::memset(ctr_host_, 0, 3 * ctr_bytes);
       seq_dev_ = reinterpret_cast<unsigned*>(ctr_dev_ + C_COUNT * kMaxSel);
-      seq_host_ = reinterpret_cast<volatile unsigned*>(ctr_host_ + C_COUNT * kMaxSel);
+      static_assert(C_COUNT * kMaxSel % 2 == 0, "the published counters are 8-byte aligned");
+      pub_host_ = reinterpret_cast<volatile unsigned long long*>(ctr_host_ + C_COUNT * kMaxSel);
     }
     slots_.assign(kMaxSel, JobHost<T>());
     ready_ = true;
@@ -721,7 +722,7 @@ class BatchEngine {
     const long long launches0 = launches_;
     if (!seq_known_) {  // an earlier tick ended in an error: take up its number
       EZ_CHECK(cudaStreamSynchronize(st_));
-      seq_next_ = *seq_host_;
+      EZ_CHECK(cudaMemcpy(&seq_next_, seq_dev_, sizeof(unsigned), cudaMemcpyDeviceToHost));
       seq_known_ = true;
     }
     // A tick whose launches repeat an earlier tick's exactly (kernels, launch
@@ -763,10 +764,11 @@ class BatchEngine {
     int hi = 0;  // the counter blocks up to the last slot in use (the host reads no other)
     for (int i = 0; i < kMaxSel; ++i)
       if (slots_[i].used) hi = i + 1;
-    published_ = launched_ && seq_host_ && !profile_ && !capturing_stream();
-    if (published_) {
-      launch(K_OTHER, k_publish, 1, 256, (const int*)ctr_dev_, C_COUNT * hi, ctr_host_, seq_dev_,
-             seq_host_);
+    pub_n_ = launched_ && pub_host_ && !profile_ && !capturing_stream() ? C_COUNT * hi : 0;
+    if (launched_)
+      launch(K_OTHER, k_tick_end<T>, 1, 256, jobs_dev_, ctr_dev_, hi, seq_dev_,
+             pub_n_ ? pub_host_ : (volatile unsigned long long*)nullptr);
+    if (pub_n_) {
       ++seq_next_;
       seq_known_ = false;
     }
@@ -775,7 +777,7 @@ class BatchEngine {
     if (graph && !pending_.empty()) EZ_RUN(run_recorded());
     if (!launched_) return EXTREMZ_OK;
     EZ_CHECK(cudaGetLastError());
-    if (!published_)
+    if (!pub_n_)
       EZ_CHECK(cudaMemcpyAsync(ctr_host_, ctr_dev_, sizeof(int) * C_COUNT * (size_t)hi,
                                cudaMemcpyDeviceToHost, st_));
     return EXTREMZ_OK;
@@ -786,7 +788,7 @@ class BatchEngine {
     if (!issued_) return EXTREMZ_OK;
     issued_ = false;
     if (launched_) {
-      if (published_) EZ_RUN(await_published());
+      if (pub_n_) EZ_RUN(await_published());
       else EZ_CHECK(cudaStreamSynchronize(st_));
       fold_timings();
     }
@@ -814,29 +816,35 @@ class BatchEngine {
     return true;
   }
 
-  // Waits for the tick's number.  The stream is asked now and then: an error
-  // ends the wait, and once all its work is done the number is there.
+  // Takes over the published counters as they arrive.  The stream is asked now
+  // and then: an error ends the wait, and once all its work is done they are
+  // there.
   int await_published() {
-    for (;;) {
-      for (int k = 0; k < 2000; ++k) {
-        if (*seq_host_ == seq_next_) {
-          std::atomic_thread_fence(std::memory_order_acquire);
-          seq_known_ = true;
-          return EXTREMZ_OK;
-        }
+    bool all_done = false;
+    for (int i = 0, spins = 0; i < pub_n_;) {
+      const unsigned long long p = pub_host_[i];
+      if ((unsigned)(p >> 32) == seq_next_) {
+        ctr_host_[i++] = (int)(unsigned)p;
+        continue;
+      }
 #if defined(__x86_64__)
-        __builtin_ia32_pause();
+      __builtin_ia32_pause();
 #endif
+      if (++spins < 4000) continue;
+      spins = 0;
+      if (all_done) {
+        last_cuda_error() = cudaErrorUnknown;
+        return EXTREMZ_CUDA_ERR;
       }
       const cudaError_t e = cudaStreamQuery(st_);
       if (e == cudaErrorNotReady) continue;
       EZ_CHECK(e);
-      if (*seq_host_ == seq_next_) continue;
       EZ_CHECK(cudaStreamSynchronize(st_));
-      if (*seq_host_ == seq_next_) continue;
-      last_cuda_error() = cudaErrorUnknown;
-      return EXTREMZ_CUDA_ERR;
+      all_done = true;
     }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    seq_known_ = true;
+    return EXTREMZ_OK;
   }
 
   // Per-class timing of the launches since set_profile(true, ...).
@@ -884,6 +892,7 @@ class BatchEngine {
   unsigned long long graph_clock_ = 0;
   long long graph_replays_ = 0, graph_captures_ = 0;
   static constexpr size_t kMaxGraphs = 256;
+  static constexpr unsigned long long kGraphRest = 8192;  // ticks
   // A signature is captured at its third sighting: ticks of a single
   // correction repeat many times, while a batch's changing selections often
   // repeat once or twice, where a capture would not pay for itself.
@@ -898,13 +907,15 @@ class BatchEngine {
   Job<T>* jobs_dev_ = nullptr;
   int* ctr_dev_ = nullptr;
   int* ctr_host_ = nullptr;
-  // Number of the last published tick (k_publish), on the device and as the
-  // host sees it; the borrowed engine, whose host copy is not mapped, has none.
+  // Published counters (k_tick_end): the mapped host copy, a counter in the low
+  // half and its tick's number in the high half of each entry; the number of the
+  // last tick on the device, and of the one the host waits for.  The borrowed
+  // engine, whose host copy is not mapped, copies instead.
+  volatile unsigned long long* pub_host_ = nullptr;
   unsigned* seq_dev_ = nullptr;
-  volatile unsigned* seq_host_ = nullptr;
   unsigned seq_next_ = 0;
   bool seq_known_ = true;
-  bool published_ = false;  // this tick's counters come through k_publish
+  int pub_n_ = 0;           // counters published by this tick; 0: copied
   int static_ctr_host_[C_COUNT * kMaxSel];
   std::vector<JobHost<T>> slots_;
   long long launches_ = 0;
@@ -1070,10 +1081,18 @@ class BatchEngine {
       run_direct();
       return EXTREMZ_OK;
     }
-    if (graphs_.size() >= kMaxGraphs) {  // evict the least recently used
+    if (graphs_.size() >= kMaxGraphs) {
+      // The least recently used one makes room only once it has rested for a
+      // while: a batch of many fields has more distinct ticks than the cache
+      // holds, and a pass over them would capture each in place of one that the
+      // next pass wants.
       auto old = graphs_.begin();
       for (auto g = graphs_.begin(); g != graphs_.end(); ++g)
         if (g->second.last < old->second.last) old = g;
+      if (graph_clock_ - old->second.last < kGraphRest) {
+        run_direct();
+        return EXTREMZ_OK;
+      }
       cudaGraphExecDestroy(old->second.exec);
       release_graph_events(old->second);
       graphs_.erase(old);
@@ -1314,7 +1333,7 @@ class BatchEngine {
           }
           if (!lock_small.empty()) {
             const Sel ss = make_sel(lock_small, false);
-            launch(K_WRONG_NBR, k_wn_steps_block<T>, ss.n, 1024, jobs, ss);
+            launch(K_WRONG_NBR, k_wn_steps_block<T>, ss.n * kWnCluster, 1024, jobs, ss);
           }
           if (!lock_large.empty()) {
             const Sel sl = make_span(lock_large);
@@ -1468,7 +1487,7 @@ class BatchEngine {
     }
     if (!incr.empty()) {
       const Sel s = make_span(incr);
-      launch(K_DETECT, k_redetect<T>, blocks(s), 256, jobs_dev_, s);
+      launch(K_DETECT, k_redetect<T>, blocks(s), 256, (const Job<T>*)jobs_dev_, s);
     }
   }
 

@@ -140,8 +140,8 @@ enum Ctr : int {
   C_MFREUSED,  // manifold rounds whose kernels found nothing changed
   // Per-job epochs and stamps, so that one launch can serve jobs at different
   // points of their correction.  There are no launches for bookkeeping: a
-  // counter is reset by a kernel that does not use it, or by the last block of
-  // one that does (last_block).
+  // counter is reset by a kernel that does not use it, or at the end of the tick
+  // (k_tick_end).
   C_DEPOCH,    // detections so far; its parity picks dirty / dirty1
   C_DIRTYP,    // entries of the dirty list of the detection before
   C_AMAX, C_AMIN, C_ASAD,  // mismatch counts of the detection under way
@@ -152,24 +152,9 @@ enum Ctr : int {
   C_WEP2, C_WEP1,  // wrong-saddle scans so far (maxima, minima); the first computes every extremum
   C_AFF,       // extrema queued for the current wrong-saddle update
   C_WLONG,     // of those, the ones with long entry lists (wlong)
-  C_DONE,      // blocks that have finished the current kernel (last_block)
+  C_DETECTED, C_MFRUN,  // a detection, a manifold round ran in this tick
   C_COUNT
 };
-
-// True, for the whole block, in the last of a job's nblk blocks to get here:
-// every write of the others is visible to it.  Leaves the ticket at zero.
-__device__ __forceinline__ bool last_block(int* ctr, int nblk) {
-  __shared__ int last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(ctr + C_DONE, 1) == nblk - 1;
-    if (last) ctr[C_DONE] = 0;
-    __threadfence();
-  }
-  __syncthreads();
-  return last != 0;
-}
 
 // A manifold round's outputs (labels, row slots, flagged neighbours and their
 // counts) are functions of the decompressed field alone, so when no value
@@ -179,12 +164,14 @@ __device__ __forceinline__ bool mf_skip(const int* ctr) {
   return ctr[C_MFDONE] && !ctr[C_CHANGED];
 }
 __device__ __forceinline__ int mf_stamp(const int* ctr) { return ctr[C_WNSTAMP] + 1; }
-// Start of a computed round, in its first kernel (which uses none of these).
+// Start of a round, in its first kernel (which uses none of these).
 __device__ __forceinline__ void mf_begin(int* ctr) {
+  ctr[C_MFRUN] = 1;
+  if (mf_skip(ctr)) return;
   ctr[C_NFC] = ctr[C_NFC1] = 0;
   ctr[C_CAND] = ctr[C_CANDJ] = ctr[C_CAND_NEXT] = 0;
 }
-// End of a round, by one thread when everything else in it is done.
+// End of a round.
 __device__ __forceinline__ void mf_end(int* ctr) {
   if (mf_skip(ctr)) {
     ctr[C_MFREUSED] += 1;
@@ -257,19 +244,25 @@ __device__ __forceinline__ const Job<T>& tile_job(const Job<T>* __restrict__ job
 
 // Lists the tiles whose halo tile contains vertex (x, y, z), those holding one
 // of its 26 neighbours or itself, unless they are listed already (or not yet
-// computed: every mark is set before a job's first round).
+// computed: every mark is set before a job's first round).  The marks of the (at
+// most eight) tiles are read together.
 __device__ __forceinline__ void mark_tiles(int* tdirty, int* list, int* count, const Dims& g, int x,
                                            int y, int z) {
   const int ntx = (g.W + TX - 1) / TX, nty = (g.H + TY - 1) / TY;
   const int x0 = max(x - 1, 0) / TX, x1 = min(x + 1, g.W - 1) / TX;
   const int y0 = max(y - 1, 0) / TY, y1 = min(y + 1, g.H - 1) / TY;
   const int z0 = max(z - 1, 0) / TZ, z1 = min(z + 1, g.D - 1) / TZ;
-  for (int c = z0; c <= z1; ++c)
-    for (int b = y0; b <= y1; ++b)
-      for (int a = x0; a <= x1; ++a) {
-        const int t = (c * nty + b) * ntx + a;
-        if (tdirty[t] == 0 && atomicExch(tdirty + t, 1) == 0) list[atomicAdd(count, 1)] = t;
-      }
+  int t[8];
+  unsigned need = 0u;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const bool own = (!(k & 1) || x1 != x0) && (!(k & 2) || y1 != y0) && (!(k & 4) || z1 != z0);
+    t[k] = ((k & 4 ? z1 : z0) * nty + (k & 2 ? y1 : y0)) * ntx + (k & 1 ? x1 : x0);
+    if (own && tdirty[t[k]] == 0) need |= 1u << k;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if ((need >> k & 1u) && atomicExch(tdirty + t[k], 1) == 0) list[atomicAdd(count, 1)] = t[k];
 }
 
 // Halo tile: TMA box (one bulk tensor copy, zero fill outside the grid) when
@@ -450,9 +443,9 @@ __global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ job
 // changed vertices.  Beside that it carries over the entries of the previous
 // list that have no changed vertex in their neighbourhood.  The resulting set
 // equals a dense re-detection (the lists are unordered; every consumer merges by
-// atomic max).  Its last block publishes the counts and swaps the lists, so a
-// detection is one launch (four with a stamp per vertex, a second kernel for the
-// carried entries and two for the bookkeeping).
+// atomic max).  The end of the tick publishes the counts and swaps the lists
+// (detect_end), so a detection is one launch (four with a stamp per vertex, a
+// second kernel for the carried entries and two for the bookkeeping).
 // ---------------------------------------------------------------------------
 template <class T>
 __device__ __forceinline__ int global_type(const Job<T>& J, int v, int& lmask) {
@@ -489,10 +482,27 @@ __device__ __forceinline__ bool bit_of(const unsigned* bits, int v) {
 }
 
 template <class T>
-__global__ void __launch_bounds__(256) k_redetect(Job<T>* __restrict__ jobs,
+__device__ __forceinline__ void detect_end(Job<T>& J) {
+  int* c = J.ctr;
+  int* t = J.mm;
+  J.mm = J.mm_next;
+  J.mm_next = t;
+  c[C_MM] = c[C_MM_NEXT];
+  c[C_MM_NEXT] = 0;
+  c[C_CMAX] = c[C_AMAX];
+  c[C_CMIN] = c[C_AMIN];
+  c[C_CSAD] = c[C_ASAD];
+  c[C_AMAX] = c[C_AMIN] = c[C_ASAD] = 0;
+  c[C_DIRTYP] = c[C_DIRTY];
+  c[C_DIRTY] = 0;
+  c[C_DEPOCH] += 1;
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) k_redetect(const Job<T>* __restrict__ jobs,
                                                   const __grid_constant__ Sel sel) {
   int blk, nblk;
-  Job<T>& J = span_job(jobs, sel, blk, nblk);
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
   const Dims g = J.dim;
   const bool odd = J.ctr[C_DEPOCH] & 1;
   const int* __restrict__ dirty = odd ? J.dirty1 : J.dirty;
@@ -554,21 +564,7 @@ __global__ void __launch_bounds__(256) k_redetect(Job<T>* __restrict__ jobs,
   const int* prev = odd ? J.dirty : J.dirty1;
   unsigned* pbits = odd ? J.dbits : J.dbits1;
   for (int e = blk * blockDim.x + threadIdx.x; e < np; e += (int)stride) pbits[prev[e] >> 5] = 0u;
-  if (last_block(J.ctr, nblk) && threadIdx.x == 0) {
-    volatile int* c = J.ctr;  // counted by other blocks
-    int* t = J.mm;
-    J.mm = J.mm_next;
-    J.mm_next = t;
-    c[C_MM] = c[C_MM_NEXT];
-    c[C_MM_NEXT] = 0;
-    c[C_CMAX] = c[C_AMAX];
-    c[C_CMIN] = c[C_AMIN];
-    c[C_CSAD] = c[C_ASAD];
-    c[C_AMAX] = c[C_AMIN] = c[C_ASAD] = 0;
-    c[C_DIRTYP] = n;
-    c[C_DIRTY] = 0;
-    c[C_DEPOCH] += 1;
-  }
+  if (blk == 0 && threadIdx.x == 0) J.ctr[C_DETECTED] = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -722,8 +718,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 6) k_direction(const
   int bx, by, bz, tile;
   const Job<T>& J = tile_job(jobs, sel, bx, by, bz, &tile);
   if (kDec) {
-    if (mf_skip(J.ctr)) return;  // same inputs as the last manifold round
     if (tile == 0 && threadIdx.x == 0) mf_begin(J.ctr);
+    if (mf_skip(J.ctr)) return;  // same inputs as the last manifold round
     if (!J.tdirty[tile]) return;  // tile and halo unchanged: pointers stand
   }
   if (!direction_tile<T, kDec>(J, s, &bar, hnext, lnext, hexit, lexit, bx, by, bz, 0, true))
@@ -748,8 +744,8 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
   unsigned loads = 0;  // TMA loads issued by this block: the barrier's phase
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
-  if (mf_skip(J.ctr)) return;
   if (blk == 0 && threadIdx.x == 0) mf_begin(J.ctr);
+  if (mf_skip(J.ctr)) return;
   const int n = J.ctr[C_TLIST];
   const int ntx = (J.dim.W + TX - 1) / TX, nty = (J.dim.H + TY - 1) / TY;
   for (int k = blk; k < n; k += nblk) {
@@ -1456,6 +1452,27 @@ __device__ __forceinline__ void propose(const Job<T>& J, int i, T d) {
   }
 }
 
+// Several proposals of one thread: the atomics go out together, then the
+// vertices that left the sentinel are listed.  (One after the other, each waits
+// for the last one's round trip to L2.)
+template <class T, int kN>
+__device__ __forceinline__ void propose_all(const Job<T>& J, const int* at, const T* d, unsigned which) {
+  using K = typename KeyOf<T>::K;
+  K old[kN];
+#pragma unroll
+  for (int k = 0; k < kN; ++k)
+    old[k] = (which >> k & 1u) ? atomicMax(J.delta + at[k], KeyOf<T>::enc(d[k])) : K(0);
+  unsigned fresh = 0u;
+#pragma unroll
+  for (int k = 0; k < kN; ++k)
+    if ((which >> k & 1u) && old[k] == J.sentinel_key && KeyOf<T>::enc(d[k]) > old[k]) fresh |= 1u << k;
+  if (!fresh) return;
+  int slot = atomicAdd(J.ctr + C_TOUCHED, __popc(fresh));
+#pragma unroll
+  for (int k = 0; k < kN; ++k)
+    if (fresh >> k & 1u) J.touched[slot++] = at[k];
+}
+
 // c_loop(0..2) (:2887-3055) over the mismatch list.
 template <class T>
 __global__ void __launch_bounds__(256) k_propose_cp(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
@@ -1510,12 +1527,27 @@ __global__ void __launch_bounds__(256) k_propose_cp(const Job<T>* __restrict__ j
         if ((valid >> d & 1) && (gn[d] < gv || (gn[d] == gv && r < v))) dm |= 1 << d;
       }
       const int om = J.olm[v];
+      // The original's lower neighbours that are not lower now, four at a time,
+      // and the vertex itself when it has lower neighbours it should not have.
+      unsigned rest = (unsigned)(valid & om & ~dm) | ((dm & ~om) ? 1u << kNumDirs : 0u);
+      while (rest) {
+        int at[4];
+        T dl[4];
+        unsigned which = 0u;
 #pragma unroll
-      for (int d = 0; d < kNumDirs; ++d) {
-        const int r = v + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
-        if ((valid >> d & 1) && (om >> d & 1) && !(dm >> d & 1)) propose(J, r, step_delta(J, r));
+        for (int q = 0; q < 4; ++q) {
+          at[q] = v;
+          if (rest) {
+            const int d = __ffs((int)rest) - 1;
+            if (d < kNumDirs) at[q] = v + ddx(d) + ddy(d) * g.W + ddz(d) * WH;
+            which |= 1u << q;
+          }
+          rest &= rest - 1u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dl[q] = (which >> q & 1u) ? step_delta(J, at[q]) : T(0);
+        propose_all<T, 4>(J, at, dl, which);
       }
-      if (dm & ~om) propose(J, v, step_delta(J, v));
     }
     if (cat & kCatMax) {  // c_loop(0) (:2890-2963)
       if (ot != 4) {
@@ -1588,7 +1620,6 @@ __global__ void __launch_bounds__(256) k_apply(const Job<T>* __restrict__ jobs, 
     const int slot = warp_append(J.ctr + C_DIRTY, fresh, 0xffffffffu);
     if (slot >= 0) dirty[slot] = v;
   }
-  if (last_block(J.ctr, nblk) && threadIdx.x == 0) J.ctr[C_TOUCHED] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1991,10 +2022,7 @@ template <class T, bool kSplit>
 __global__ void __launch_bounds__(1024) k_wn_resolve(Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
   if (blockIdx.x >= sel.n) return;
   Job<T>& J = jobs[sel.idx[blockIdx.x]];
-  if (mf_skip(J.ctr)) {
-    if (!kSplit && threadIdx.x == 0) mf_end(J.ctr);
-    return;
-  }
+  if (mf_skip(J.ctr)) return;
   __shared__ int s_next;
   unsigned* taken = kSplit ? J.taken : J.taken1;
   int* flagged = kSplit ? J.flagged : J.flagged1;
@@ -2062,7 +2090,6 @@ __global__ void __launch_bounds__(1024) k_wn_resolve(Job<T>* __restrict__ jobs, 
       J.ctr[C_CAND] = 0;
     }
     J.ctr[C_CAND_NEXT] = 0;
-    if (!kSplit) mf_end(J.ctr);
   }
 }
 
@@ -2100,36 +2127,106 @@ __device__ __forceinline__ void wn_step_entry(const Job<T>& J, int e, int n2, in
 }
 
 // One step over every selected job's two candidate lists (a large list: one
-// launch per direction).  The last step ends the round.
+// launch per direction).
 template <class T>
 __global__ void __launch_bounds__(256) k_wn_step(const Job<T>* __restrict__ jobs,
                                                  const __grid_constant__ Sel sel, int d) {
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
-  if (!mf_skip(J.ctr)) {
-    const int n2 = J.ctr[C_CAND], n = n2 + J.ctr[C_CANDJ];
-    const int stride = nblk * blockDim.x;
-    for (int e = blk * blockDim.x + threadIdx.x; e < n; e += stride) wn_step_entry(J, e, n2, d);
-  }
-  if (d == kNumDirs - 1 && last_block(J.ctr, nblk) && threadIdx.x == 0) mf_end(J.ctr);
+  if (mf_skip(J.ctr)) return;
+  const int n2 = J.ctr[C_CAND], n = n2 + J.ctr[C_CANDJ];
+  const int stride = nblk * blockDim.x;
+  for (int e = blk * blockDim.x + threadIdx.x; e < n; e += stride) wn_step_entry(J, e, n2, d);
 }
 
-// All fourteen steps in one block per job, with a barrier between steps (a
-// short list: fourteen grid launches would cost more than the work).  The
-// barrier makes one step's flags and marks visible to the next.
+// Candidate directions of entry e: the neighbours on its side whose label
+// differs from the original's.  All gathers of the fourteen go out together.
 template <class T>
-__global__ void __launch_bounds__(1024) k_wn_steps_block(const Job<T>* __restrict__ jobs,
-                                                         const __grid_constant__ Sel sel) {
-  if (blockIdx.x >= sel.n) return;
-  const Job<T>& J = jobs[sel.idx[blockIdx.x]];
-  if (!mf_skip(J.ctr)) {
-    const int n2 = J.ctr[C_CAND], n = n2 + J.ctr[C_CANDJ];
-    for (int d = 0; d < kNumDirs; ++d) {
-      for (int e = threadIdx.x; e < n; e += blockDim.x) wn_step_entry(J, e, n2, d);
+__device__ __forceinline__ unsigned wn_mask(const Job<T>& J, bool split, int s) {
+  const Dims g = J.dim;
+  const int WH = g.W * g.H;
+  int x, y, z;
+  coords(s, g, x, y, z);
+  const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
+  const T sv = J.g[s];
+  const uint8_t bit = split ? 1 : 2;
+  unsigned m = 0u;
+#pragma unroll
+  for (int d = 0; d < kNumDirs; ++d) {
+    if (!(valid >> d & 1)) continue;
+    const int r = s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
+    const T rv = J.g[r];
+    if ((J.mis[r] & bit) && (split ? above(rv, r, sv, s) : below(rv, r, sv, s))) m |= 1u << d;
+  }
+  return m;
+}
+
+// All fourteen steps in one launch for a short list (fourteen grid launches
+// would cost more than the work): a cluster of eight blocks per job, with a
+// cluster barrier between steps, or its first block alone with a block barrier
+// when each of its threads then has at most two entries.  A thread first finds
+// its entries' candidate directions (wn_mask; the first kWnHeld entries' in
+// registers, the others' in cand_next), so that a step is one look at the flag
+// of one neighbour: 4-6 us for a few hundred saddles, where a chain of five
+// dependent loads per step took 14-20 us, and a list that outgrew the block
+// (several thousand saddles) 500 us.
+constexpr int kWnCluster = 8, kWnHeld = 2;
+template <class T>
+__global__ void __cluster_dims__(kWnCluster, 1, 1) __launch_bounds__(1024)
+    k_wn_steps_block(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
+  const int job = blockIdx.x / kWnCluster, rank = blockIdx.x % kWnCluster;
+  const Job<T>& J = jobs[sel.idx[job]];
+  __shared__ int off[kNumDirs];
+  fill_offsets(off, J.dim);
+  __syncthreads();
+  if (mf_skip(J.ctr)) return;  // the whole cluster
+  const int n2 = J.ctr[C_CAND], n = n2 + J.ctr[C_CANDJ];
+  const bool alone = n <= kWnHeld * 1024;  // the same in every block of the cluster
+  if (alone && rank) return;
+  const int t0 = alone ? (int)threadIdx.x : rank * 1024 + (int)threadIdx.x;
+  const int stride = alone ? 1024 : kWnCluster * 1024;
+  auto entry = [&](int e) { return e < n2 ? J.cand[e] : J.cand_j[e - n2]; };
+  int hs[kWnHeld];
+  unsigned hm[kWnHeld];
+#pragma unroll
+  for (int k = 0; k < kWnHeld; ++k) {
+    const int e = t0 + k * stride;
+    hs[k] = e < n ? entry(e) : 0;
+    hm[k] = e < n ? wn_mask(J, e < n2, hs[k]) : 0u;
+  }
+  // cand_next holds N entries; the two lists together may have more only when
+  // over half of all vertices are candidates of both sides.
+  const int cap = J.dim.N;
+  for (int e = t0 + kWnHeld * stride; e < n && e < cap; e += stride)
+    J.cand_next[e] = (int)wn_mask(J, e < n2, entry(e));
+  // Flags the direction-d candidate of saddle s; true when it was free.
+  auto take = [&](bool split, int s, int d) {
+    const int r = s + off[d];
+    unsigned* taken = split ? J.taken : J.taken1;
+    if (taken_now(taken, r)) return false;
+    atomicOr(taken + (r >> 5), 1u << (r & 31));
+    (split ? J.flagged : J.flagged1)[atomicAdd(J.ctr + (split ? C_NFC : C_NFC1), 1)] = r;
+    return true;
+  };
+  for (int d = 0; d < kNumDirs; ++d) {
+#pragma unroll
+    for (int k = 0; k < kWnHeld; ++k)
+      if ((hm[k] >> d & 1u) && take(t0 + k * stride < n2, hs[k], d)) hm[k] = 0u;
+    for (int e = t0 + kWnHeld * stride; e < n; e += stride) {
+      if (e < cap) {
+        if ((J.cand_next[e] >> d & 1) && take(e < n2, entry(e), d)) J.cand_next[e] = 0;
+      } else {
+        wn_step_entry(J, e, n2, d);
+      }
+    }
+    if (d + 1 == kNumDirs) break;
+    if (alone) {
       __syncthreads();
+    } else {
+      asm volatile("barrier.cluster.arrive.release;\n"
+                   "barrier.cluster.wait.acquire;" ::: "memory");
     }
   }
-  if (threadIdx.x == 0) mf_end(J.ctr);
 }
 
 // ---------------------------------------------------------------------------
@@ -2144,21 +2241,28 @@ __device__ __forceinline__ void fixpath_from(const Job<T>& J, int cur) {
   const int cap = J.iter_cap;
   int t = -1, fl = -1;
   int steps = 0;
+  const int WH = g.W * g.H;
   for (; steps < cap; ++steps) {
-    int ids[kNumDirs];
-    const int nn = neighbours(cur, g, ids, nullptr);
+    int x, y, z;
+    coords(cur, g, x, y, z);
+    const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
     int ni = cur, nd = cur;
     T fi = J.f[cur], gd = J.g[cur];
-    for (int j = 0; j < nn; ++j) {
-      const int r = ids[j];
-      const T fr = J.f[r], gr = J.g[r];
-      if (kSplit) {
-        if (fi < fr || (fi == fr && ni < r)) { ni = r; fi = fr; }
-        if (gd < gr || (gd == gr && nd < r)) { nd = r; gd = gr; }
-      } else {
-        if (fi > fr || (fi == fr && ni > r)) { ni = r; fi = fr; }
-        if (gd > gr || (gd == gr && nd > r)) { nd = r; gd = gr; }
-      }
+    // Both fields' neighbours through static indices, so that a step's loads are
+    // in flight together.
+    T fr[kNumDirs], gr[kNumDirs];
+#pragma unroll
+    for (int d = 0; d < kNumDirs; ++d) {
+      const int r = cur + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
+      fr[d] = (valid >> d & 1) ? J.f[r] : T(0);
+      gr[d] = (valid >> d & 1) ? J.g[r] : T(0);
+    }
+#pragma unroll
+    for (int d = 0; d < kNumDirs; ++d) {
+      const int r = cur + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
+      if (!(valid >> d & 1)) continue;
+      if (kSplit ? above(fr[d], r, fi, ni) : below(fr[d], r, fi, ni)) { ni = r; fi = fr[d]; }
+      if (kSplit ? above(gr[d], r, gd, nd) : below(gr[d], r, gd, nd)) { nd = r; gd = gr[d]; }
     }
     if (ni != nd) { t = ni; fl = nd; break; }
     if (ni == cur) break;
@@ -2197,6 +2301,7 @@ __global__ void __launch_bounds__(256) k_wim_scan(const Job<T>* __restrict__ job
   if (blk == 0 && threadIdx.x == 0) {  // counted by k_wim_collect
     J.ctr[kMax ? C_WMC : C_WMIN] = 0;
     J.ctr[kMax ? C_WMC2 : C_WMIN2] = 0;
+    J.ctr[C_TOUCHED] = 0;  // (the join side's scan follows saddle_loops in one tick)
   }
   const int ns = J.ctr[kMax ? C_NS2 : C_NS1];
   const int4* oend = kMax ? J.oend2 : J.oend1;
@@ -2658,20 +2763,32 @@ __global__ void __launch_bounds__(256) k_fill_many(const __grid_constant__ FillL
   }
 }
 
-// The counter blocks to the host's (mapped) copy at the end of a tick, then the
-// tick's number, which the host waits for: a copy and a stream synchronisation
-// behind the kernels took about 8 us longer.
-__global__ void __launch_bounds__(256) k_publish(const int* __restrict__ ctr, int n, int* host,
-                                                 unsigned* seq, volatile unsigned* host_seq) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) host[i] = ctr[i];
-  __threadfence_system();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned s = *seq + 1u;
-    *seq = s;
-    __threadfence_system();
-    *host_seq = s;
+// End of a tick, one block: the bookkeeping of the first `slots` jobs' phases
+// (a thread per job), then, with host set, every counter to the host's mapped
+// copy beside the tick's number in the same 8 bytes, so that the host can see
+// for each whether it has come and no fence is needed.  (A copy and a stream
+// synchronisation behind the kernels took about 8 us longer; a flag written
+// behind two system-wide fences about 5 us.)
+template <class T>
+__global__ void __launch_bounds__(256) k_tick_end(Job<T>* jobs, int* ctr, int slots, unsigned* seq,
+                                                  volatile unsigned long long* host) {
+  if (threadIdx.x < slots) {
+    int* c = ctr + threadIdx.x * C_COUNT;
+    c[C_TOUCHED] = 0;
+    if (c[C_DETECTED]) {
+      c[C_DETECTED] = 0;
+      detect_end(jobs[threadIdx.x]);
+    }
+    if (c[C_MFRUN]) {
+      c[C_MFRUN] = 0;
+      mf_end(c);
+    }
   }
+  if (!host) return;
+  const unsigned long long s = (unsigned long long)(*seq + 1u) << 32;
+  __syncthreads();
+  for (int i = threadIdx.x; i < slots * C_COUNT; i += blockDim.x) host[i] = s | (unsigned)ctr[i];
+  if (threadIdx.x == 0) *seq = (unsigned)(s >> 32);
 }
 
 template <class K>
