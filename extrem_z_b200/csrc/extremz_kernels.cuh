@@ -6,6 +6,8 @@
 // operations in the field type T (build with -fmad=false).
 #pragma once
 
+#include <type_traits>
+
 #include "extremz_common.cuh"
 
 namespace extremz {
@@ -267,20 +269,27 @@ __device__ __forceinline__ void mark_tiles(int* tdirty, int* list, int* count, c
 
 // Halo tile: TMA box (one bulk tensor copy, zero fill outside the grid) when
 // the field's row stride allows it, else plain loads with every thread's loads
-// issued before its first shared store.  Outside-grid entries are never read.
+// issued before its first shared store, and zeros outside the grid too.
 // A block that loads several tiles initialises the barrier once (init) and
 // waits on alternating phases (parity = loads issued before this one, mod 2).
+// tile_issue starts the bulk copy; between it and load_tile, which waits for it,
+// the block may do other work.
 template <class T>
-__device__ __forceinline__ bool load_tile(Tile<T>& s, uint64_t* bar, const CUtensorMap* map,
-                                          bool tma, const T* __restrict__ a, const Dims& g, int bx,
-                                          int by, int bz, unsigned parity = 0, bool init = true) {
+__device__ __forceinline__ void tile_issue(Tile<T>& s, uint64_t* bar, const CUtensorMap* map, int bx,
+                                           int by, int bz, bool init) {
+  if (threadIdx.x == 0) {
+    tma_map_acquire(map);
+    if (init) mbar_init(bar, 1);
+    mbar_expect_tx(bar, (unsigned)sizeof(Tile<T>));
+    tma_load_3d(&s.v[0][0][0], map, bx - kXOff, by - 1, bz - 1, bar);
+  }
+}
+
+template <class T>
+__device__ __forceinline__ bool load_tile(Tile<T>& s, uint64_t* bar, bool tma,
+                                          const T* __restrict__ a, const Dims& g, int bx, int by,
+                                          int bz, unsigned parity = 0) {
   if (tma) {
-    if (threadIdx.x == 0) {
-      tma_map_acquire(map);
-      if (init) mbar_init(bar, 1);
-      mbar_expect_tx(bar, (unsigned)sizeof(Tile<T>));
-      tma_load_3d(&s.v[0][0][0], map, bx - kXOff, by - 1, bz - 1, bar);
-    }
     __syncthreads();
     return mbar_wait(bar, parity, 1ll << 26);
   }
@@ -295,12 +304,17 @@ __device__ __forceinline__ bool load_tile(Tile<T>& s, uint64_t* bar, const CUten
     const int lx = i % HX, t = i / HX, ly = t % SY, lz = t / SY;
     const int gx = bx + lx - 1, gy = by + ly - 1, gz = bz + lz - 1;
     const bool ok = i < kTotal && gx >= 0 && gx < g.W && gy >= 0 && gy < g.H && gz >= 0 && gz < g.D;
-    off[k] = ok ? (lz * SY + ly) * SX + lx + kXOff - 1 : -1;
+    off[k] = i < kTotal ? (lz * SY + ly) * SX + lx + kXOff - 1 : -1;
     v[k] = ok ? __ldg(a + gx + (long long)gy * g.W + (long long)gz * g.W * g.H) : T(0);
   }
 #pragma unroll
   for (int k = 0; k < kPer; ++k)
     if (off[k] >= 0) (&s.v[0][0][0])[off[k]] = v[k];
+  constexpr int kPad = SX - HX;  // the tile rows' unused columns
+  for (int i = threadIdx.x; i < kPad * SY * SZ; i += 256) {
+    const int c = i % kPad;
+    (&s.v[0][0][0])[(i / kPad) * SX + (c < kXOff - 1 ? c : HX + c)] = T(0);
+  }
   __syncthreads();
   return true;
 }
@@ -373,9 +387,150 @@ __device__ __forceinline__ void count_cats(int* ctr, int cat) {
   }
 }
 
+// In-tile positions of the path following: p = x + 64 y + 1024 z, with one bit
+// free above each coordinate's range.  A step adds the direction's offset in the
+// same measure (step_of); the result left the tile exactly when one of the free
+// bits is set (a borrow below zero sets the bits above), so no coordinate is
+// compared.
+constexpr int kPosY = 64, kPosZ = 1024, kPosOut = 1 << 5 | 1 << 9 | 1 << 12;
+constexpr int kPosCount = kPosZ * (TZ - 1) + kPosY * (TY - 1) + TX;
+static_assert(TX == 32 && TY == 8 && TZ == 4, "the free bits of the in-tile positions");
+__host__ __device__ constexpr int step_of(int dx, int dy, int dz) {
+  return dx + kPosY * dy + kPosZ * dz;
+}
+// Steps are ordered as the vertex ids they lead to.
+static_assert(step_of(1, -1, 0) < step_of(-1, 0, 0) && step_of(1, 0, -1) < step_of(0, -1, 0),
+              "in-tile steps order as (z, y, x)");
+
+// Running best of (value, id) over star members; st is the step to it.
+template <class T>
+struct Best {
+  T v;
+  int st;
+};
+// Offers a member with a larger id than all before: it replaces the best when it
+// is at least as large (maximum), when it is smaller (minimum), or by force.
+template <bool kMax, class T>
+__device__ __forceinline__ void offer(Best<T>& b, const Best<T>& m, bool ok = true,
+                                      bool force = false) {
+  const bool take = force || (ok && (kMax ? m.v >= b.v : m.v < b.v));
+  b.v = take ? m.v : b.v;
+  b.st = take ? m.st : b.st;
+}
+// Of two bests in no id order, the one that comes first by (value, id).
+template <bool kMax, class T>
+__device__ __forceinline__ Best<T> merge(const Best<T>& a, const Best<T>& m) {
+  const bool take = kMax ? m.v > a.v || (m.v == a.v && m.st > a.st)
+                         : m.v < a.v || (m.v == a.v && m.st < a.st);
+  return Best<T>{take ? m.v : a.v, take ? m.st : a.st};
+}
+
+// Which neighbours of a tile column exist (kEdge tiles; all do elsewhere).
+struct ColumnEdges {
+  bool xm, xp, dn, up;
+  int z0, z1;  // tile planes -1 .. TZ that are in the grid: z0 .. z1
+};
+
+// The seven values of a column's voxel and its in-plane neighbours.
+template <class T>
+struct Plane {
+  T c, xm, xp, up, upm, dn, dnp;
+};
+
+// One side's part of a plane: `lo` the best of the four members that the voxel
+// above sees of this plane, `hi` of the four that the voxel below sees (in-plane
+// steps).  Together they are the voxel's own plane.
+template <bool kMax, bool kEdge, class T>
+__device__ __forceinline__ void plane_best(const Plane<T>& q, const ColumnEdges& e, Best<T>& lo,
+                                           Best<T>& hi) {
+  Best<T> bc{q.c, 0};
+  offer<kMax>(bc, Best<T>{q.xp, step_of(1, 0, 0)}, !kEdge || e.xp);
+  lo = Best<T>{q.dn, step_of(0, -1, 0)};
+  offer<kMax>(lo, Best<T>{q.dnp, step_of(1, -1, 0)}, !kEdge || e.xp);
+  offer<kMax>(lo, bc, true, kEdge && !e.dn);
+  hi = Best<T>{q.xm, step_of(-1, 0, 0)};
+  offer<kMax>(hi, Best<T>{q.c, 0}, true, kEdge && !e.xm);
+  Best<T> aup{q.upm, step_of(-1, 1, 0)};
+  offer<kMax>(aup, Best<T>{q.up, step_of(0, 1, 0)}, true, kEdge && !e.xm);
+  offer<kMax>(hi, aup, !kEdge || e.up);
+}
+
+// One tile column (x, y) upwards: for each of its TZ voxels, kSteps, the step to
+// its steepest-ascent and steepest-descent neighbour (0 at a root), and, kMasks,
+// its lower-star direction mask before the validity mask.  The closed star of v is
+// v + C and v - C for C = {0, 1}^3 in (-x, y, z), so a plane's values serve three
+// voxels of the column: 7 loads and 11 two-way choices a voxel and side, where
+// each voxel by itself takes 15 of both.  The steps want finite values (the caller
+// checks).
+template <class T, bool kEdge, bool kSteps, bool kMasks>
+__device__ __forceinline__ void column_steps(const Tile<T>& s, int tx, int ty, const ColumnEdges& e,
+                                             int* up_st, int* dn_st, int* lm) {
+  const T(*row)[SY][SX] = s.v;
+  const int x = tx + kXOff, y = ty + 1;
+  Best<T> plo[2], part[2];  // the plane below: its lo; the voxel below: its best so far
+  T cprev = T(0);
+#pragma unroll
+  for (int pz = 0; pz < SZ; ++pz) {  // tile plane pz - 1
+    Plane<T> q;
+    q.c = row[pz][y][x];
+    if (pz > 0) {
+      q.xm = row[pz][y][x - 1];
+      q.up = row[pz][y + 1][x];
+      q.upm = row[pz][y + 1][x - 1];
+    } else {
+      q.xm = q.up = q.upm = q.c;
+    }
+    if (pz < SZ - 1) {
+      q.xp = row[pz][y][x + 1];
+      q.dn = row[pz][y - 1][x];
+      q.dnp = row[pz][y - 1][x + 1];
+    } else {
+      q.xp = q.dn = q.dnp = q.c;
+    }
+    if (kMasks) {
+      // A tie goes to the lower side exactly when the neighbour's id is smaller
+      // (odd directions).
+      if (pz >= 2) {
+        int& m = lm[pz - 2];
+        m |= (int)(q.c < cprev) << 4 | (int)(q.xm < cprev) << 10 | (int)(q.up < cprev) << 8 |
+             (int)(q.upm < cprev) << 12;
+      }
+      if (pz >= 1 && pz < SZ - 1) {
+        int& m = lm[pz - 1];
+        m |= (int)(q.xp < q.c) << 0 | (int)(q.xm <= q.c) << 1 | (int)(q.up < q.c) << 2 |
+             (int)(q.dn <= q.c) << 3 | (int)(q.upm < q.c) << 6 | (int)(q.dnp <= q.c) << 7;
+      }
+      if (pz < SZ - 2) {
+        const T cn = row[pz + 1][y][x];
+        lm[pz] = (int)(q.c <= cn) << 5 | (int)(q.xp <= cn) << 11 | (int)(q.dn <= cn) << 9 |
+                 (int)(q.dnp <= cn) << 13;
+      }
+      cprev = q.c;
+    }
+    auto side = [&](auto kmax, int k, int* st) {
+      constexpr bool kMax = decltype(kmax)::value;
+      Best<T> lo, hi;
+      plane_best<kMax, kEdge>(q, e, lo, hi);
+      if (pz >= 2) {  // the voxel below is complete
+        offer<kMax>(part[k], Best<T>{hi.v, hi.st + kPosZ}, !kEdge || pz - 1 <= e.z1);
+        st[pz - 2] = part[k].st;
+      }
+      if (pz >= 1 && pz < SZ - 1) {
+        part[k] = Best<T>{plo[k].v, plo[k].st - kPosZ};
+        offer<kMax>(part[k], merge<kMax>(lo, hi), true, kEdge && pz - 2 < e.z0);
+      }
+      plo[k] = lo;
+    };
+    if constexpr (kSteps) {
+      side(std::true_type{}, 0, up_st);
+      side(std::false_type{}, 1, dn_st);
+    }
+  }
+}
+
 // The first detection of a job: the whole decompressed field.
 template <class T>
-__global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ jobs,
+__global__ void __launch_bounds__(256, 8) k_classify(const Job<T>* __restrict__ jobs,
                                                   const __grid_constant__ Sel sel) {
   __shared__ Tile<T> s;
   __shared__ uint64_t bar;
@@ -383,7 +538,8 @@ __global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ job
   const Job<T>& J = tile_job(jobs, sel, bx, by, bz);
   const Dims g = J.dim;
   // The block decides together: its threads meet at barriers further on.
-  if (!__syncthreads_and(load_tile<T>(s, &bar, &J.map_g, J.tma_g, J.g, g, bx, by, bz))) {
+  if (J.tma_g) tile_issue<T>(s, &bar, &J.map_g, bx, by, bz, true);
+  if (!__syncthreads_and(load_tile<T>(s, &bar, J.tma_g, J.g, g, bx, by, bz))) {
     if (threadIdx.x == 0) atomicOr(J.ctr + C_ERROR, kErrTile);
     return;
   }
@@ -401,6 +557,9 @@ __global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ job
   // A tile off the field's faces has every direction valid at every voxel.
   const bool interior = bx > 0 && by > 0 && bz > 0 && bx + TX < g.W && by + TY < g.H &&
                         bz + TZ < g.D;
+  int mask[TZ];
+  column_steps<T, false, false, true>(s, tx, ty, ColumnEdges{}, nullptr, nullptr, mask);
+#pragma unroll
   for (int tz = 0; tz < TZ; ++tz) {
     const int x = bx + tx, y = by + ty, z = bz + tz;
     const bool in = x < g.W && y < g.H && z < g.D;
@@ -408,9 +567,8 @@ __global__ void __launch_bounds__(256) k_classify(const Job<T>* __restrict__ job
       const int v = x + y * g.W + z * g.W * g.H;
       const int bc = interior ? 0 : boundary_code(x, y, z, g.W, g.H, g.D);
       const int valid = interior ? (1 << kNumDirs) - 1 : valid_mask(bc);
-      int lm, um;
-      tile_masks(s, tx, ty, tz, valid, lm, um);
-      const int t = type_from_masks(lm, um, valid, bc, J.tb);
+      const int lm = mask[tz] & valid;
+      const int t = type_from_masks(lm, valid & ~lm, valid, bc, J.tb);
       const int cat = mismatch_cats(t, J.otype[v], lm, J.olm[v]);
       J.mstat[v] = (uint8_t)cat;
       if (cat) {
@@ -583,9 +741,8 @@ __global__ void __launch_bounds__(256) k_redetect(const Job<T>* __restrict__ job
 // maximum (minimum) of (value, id) over the voxel and its valid neighbours.
 // Ids are scanned in ascending order so that ">=" keeps the larger id on a tie;
 // the descent scans in descending order with "<=".  (Finite inputs: the scans
-// start from -inf / +inf and always meet the centre.)  kAll: every direction
-// valid, no per-direction test.
-template <class T, bool kAll>
+// start from -inf / +inf and always meet the centre.)
+template <class T>
 __device__ __forceinline__ void steepest_dirs(const Tile<T>& s, int tx, int ty, int tz, int valid,
                                               int& hd, int& ld) {
   const T c = s.v[tz + 1][ty + 1][tx + kXOff];
@@ -600,35 +757,47 @@ __device__ __forceinline__ void steepest_dirs(const Tile<T>& s, int tx, int ty, 
   for (int j = 0; j < kNumDirs; ++j) {
     const int d = rank_dir(j);
     if (j == kRankCentre && c >= hv) { hv = c; hd = -1; }
-    if ((kAll || (valid >> d & 1)) && nv[d] >= hv) { hv = nv[d]; hd = d; }
+    if ((valid >> d & 1) && nv[d] >= hv) { hv = nv[d]; hd = d; }
   }
 #pragma unroll
   for (int j = kNumDirs - 1; j >= 0; --j) {
     const int d = rank_dir(j);
-    if ((kAll || (valid >> d & 1)) && nv[d] <= lv) { lv = nv[d]; ld = d; }
+    if ((valid >> d & 1) && nv[d] <= lv) { lv = nv[d]; ld = d; }
     if (j == kRankCentre && c <= lv) { lv = c; ld = -1; }
   }
 }
 
-// Next-step codes of the in-tile path following (besides local indices).
-constexpr int kExit = -1, kRoot = -2;
+// The same steps voxel by voxel through the exact scans of steepest_dirs, for a
+// tile that holds an infinity or a NaN.
+template <class T>
+__device__ __noinline__ void column_steps_any(const Tile<T>& s, int tx, int ty, int bx, int by, int bz,
+                                              const Dims& g, int* up_st, int* dn_st, int* lm) {
+  for (int tz = 0; tz < TZ; ++tz) {
+    const int x = bx + tx, y = by + ty, z = bz + tz;
+    int hd = -1, ld = -1, um;
+    lm[tz] = 0;
+    if (x < g.W && y < g.H && z < g.D) {
+      const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
+      steepest_dirs<T>(s, tx, ty, tz, valid, hd, ld);
+      tile_masks(s, tx, ty, tz, valid, lm[tz], um);
+    }
+    up_st[tz] = hd < 0 ? 0 : step_of(ddx(hd), ddy(hd), ddz(hd));
+    dn_st[tz] = ld < 0 ? 0 : step_of(ddx(ld), ddy(ld), ddz(ld));
+  }
+}
 
-// Follows next-pointers inside the tile from local voxel li to the path's
-// exit (global id of the first outside vertex) or root.
-__device__ __forceinline__ int follow(const int16_t* nxt, const int* exit_gid, int li, int bx,
-                                      int by, int bz, int W, int WH, int* err) {
-  int cur = li, t = nxt[li];
-  for (int step = 0; t >= 0; ++step) {
-    cur = t;
-    t = nxt[cur];
+// Follows the tile's next positions from p, whose own is t, to the path's exit
+// from the tile or its root.
+__device__ __forceinline__ int follow(const int16_t* nxt, int p, int t, int* err) {
+  for (int step = 0; t != p && !(t & kPosOut); ++step) {
+    p = t;
+    t = nxt[p];
     if (step > TX * TY * TZ) {  // a path never revisits a voxel; guard anyway
       atomicOr(err, kErrTile);
       break;
     }
   }
-  if (t == kExit) return exit_gid[cur];
-  const int cx = cur % TX, cy = (cur / TX) % TY, cz = cur / (TX * TY);
-  return (bx + cx) + (by + cy) * W + (bz + cz) * WH;
+  return t;
 }
 
 // Steepest pointers of one tile, compressed to the tile's exits: every voxel's
@@ -636,73 +805,86 @@ __device__ __forceinline__ int follow(const int16_t* nxt, const int* exit_gid, i
 // path's root inside the tile.  kDec = false: f into ds / as (setup), with the
 // original classification (otype, olm) from the same tile load; true: g into
 // pdd / pda.  Returns false when the tile's load did not complete.
+// Bound by the integer pipe (62 % busy: the selects of the two-way choices, then
+// the path loops).  A full pass over the 512^3 float64 benchmark field takes
+// 1.50 ms, with the classification 2.05 ms; with every voxel scanning its own
+// star, and steps checked and indexed by coordinates, 2.08 and 2.69 ms.
 template <class T, bool kDec>
 __device__ __noinline__ bool direction_tile(const Job<T>& J, Tile<T>& s, uint64_t* bar,
-                                               int16_t* hnext, int16_t* lnext, int* hexit,
-                                               int* lexit, int bx, int by, int bz,
-                                               unsigned parity, bool init) {
+                                            int16_t* hnext, int16_t* lnext, int bx, int by, int bz,
+                                            unsigned parity) {
   const Dims g = J.dim;
   const int WH = g.W * g.H;
   const T* a = kDec ? J.g : J.f;
   int* ds = kDec ? J.pdd : J.ds;
   int* as = kDec ? J.pda : J.as;
+  const bool loaded = load_tile<T>(s, bar, kDec ? J.tma_g : J.tma_f, a, g, bx, by, bz, parity);
+  // Whether the tile holds a value that is not finite: v * 0 is then NaN.
+  T zero = T(0);
+  if (loaded)
+    for (int i = threadIdx.x; i < SX * SY * SZ; i += 256) {
+      const T v = (&s.v[0][0][0])[i];
+      zero = sizeof(T) == 8 ? (T)__fma_rn((double)v, 0.0, (double)zero)
+                            : (T)__fmaf_rn((float)v, 0.0f, (float)zero);
+    }
   // The block decides together: its threads meet at a barrier further on.
-  if (!__syncthreads_and(load_tile<T>(s, bar, kDec ? &J.map_g : &J.map_f, kDec ? J.tma_g : J.tma_f,
-                                      a, g, bx, by, bz, parity, init))) {
+  const bool usual = __syncthreads_and(loaded && zero == T(0));
+  if (!usual && !__syncthreads_and(loaded)) {
     if (threadIdx.x == 0) atomicOr(J.ctr + C_ERROR, kErrTile);
     return false;
   }
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+  const int x = bx + tx, y = by + ty;
   // A tile off the field's faces has every direction valid at every voxel.
   const bool interior = bx > 0 && by > 0 && bz > 0 && bx + TX < g.W && by + TY < g.H &&
                         bz + TZ < g.D;
+  int hs[TZ], ls[TZ], lm[TZ];
+  if (!usual) {
+    column_steps_any<T>(s, tx, ty, bx, by, bz, g, hs, ls, lm);
+  } else if (interior) {
+    column_steps<T, false, true, !kDec>(s, tx, ty, ColumnEdges{}, hs, ls, lm);
+  } else {
+    const ColumnEdges e{x > 0, x + 1 < g.W, y > 0, y + 1 < g.H, bz > 0 ? -1 : 0,
+                        min(TZ, g.D - 1 - bz)};
+    column_steps<T, true, true, !kDec>(s, tx, ty, e, hs, ls, lm);
+  }
+  const bool col = x < g.W && y < g.H;
+  const int p0 = tx + kPosY * ty;
+#pragma unroll
   for (int tz = 0; tz < TZ; ++tz) {
-    const int li = (tz * TY + ty) * TX + tx;
-    const int x = bx + tx, y = by + ty, z = bz + tz;
-    int hd = -1, ld = -1;
-    const bool in = x < g.W && y < g.H && z < g.D;
-    if (interior) {
-      steepest_dirs<T, true>(s, tx, ty, tz, (1 << kNumDirs) - 1, hd, ld);
-    } else if (in) {
-      const int bc = boundary_code(x, y, z, g.W, g.H, g.D);
-      if (bc == 0) steepest_dirs<T, true>(s, tx, ty, tz, (1 << kNumDirs) - 1, hd, ld);
-      else steepest_dirs<T, false>(s, tx, ty, tz, valid_mask(bc), hd, ld);
-    }
-    const int v = x + y * g.W + z * WH;
-    if (!kDec && in) {
+    const int p = p0 + kPosZ * tz;
+    hs[tz] += p;
+    ls[tz] += p;
+    hnext[p] = (int16_t)hs[tz];
+    lnext[p] = (int16_t)ls[tz];
+    const int z = bz + tz;
+    if (!kDec && col && z < g.D) {
       // The original field's classification from the same tile
       // (classifyVertex_CUDA, the type = 0 call :5289): type and lower-star
       // direction mask.
+      const int v = x + y * g.W + z * WH;
       const int bc = interior ? 0 : boundary_code(x, y, z, g.W, g.H, g.D);
       const int valid = interior ? (1 << kNumDirs) - 1 : valid_mask(bc);
-      int lm, um;
-      tile_masks(s, tx, ty, tz, valid, lm, um);
-      J.otype[v] = (int8_t)type_from_masks(lm, um, valid, bc, J.tb);
-      J.olm[v] = (uint16_t)lm;
+      const int m = lm[tz] & valid;
+      J.otype[v] = (int8_t)type_from_masks(m, valid & ~m, valid, bc, J.tb);
+      J.olm[v] = (uint16_t)m;
     }
-    // Next step in tile terms: the local index when it stays in the tile,
-    // kExit (the first outside vertex to the exit slot) when it leaves it,
-    // kRoot at a root.
-    auto step = [&](int d, int* exit_gid) {
-      if (d < 0) return kRoot;
-      const int dx = ddx(d), dy = ddy(d), dz = ddz(d);
-      const int nx = tx + dx, ny = ty + dy, nz = tz + dz;
-      if ((unsigned)nx < (unsigned)TX && (unsigned)ny < (unsigned)TY && (unsigned)nz < (unsigned)TZ)
-        return (nz * TY + ny) * TX + nx;
-      *exit_gid = v + dx + dy * g.W + dz * WH;
-      return kExit;
-    };
-    hnext[li] = (int16_t)(in ? step(hd, &hexit[li]) : kRoot);
-    lnext[li] = (int16_t)(in ? step(ld, &lexit[li]) : kRoot);
   }
   __syncthreads();
+  if (!col) return true;
+  // Vertex of an in-tile position, one plane, row and column outside included.
+  const int base = (bx - 1) + (by - 1) * g.W + (bz - 1) * WH;
+  auto vertex = [&](int t) {
+    const int q = t + step_of(1, 1, 1);
+    return base + (q & (kPosY - 1)) + (q >> 6 & 15) * g.W + (q >> 10) * WH;
+  };
+#pragma unroll
   for (int tz = 0; tz < TZ; ++tz) {
-    const int x = bx + tx, y = by + ty, z = bz + tz;
-    if (!(x < g.W && y < g.H && z < g.D)) continue;
-    const int li = (tz * TY + ty) * TX + tx;
-    const int v = x + y * g.W + z * WH;
-    ds[v] = follow(hnext, hexit, li, bx, by, bz, g.W, WH, J.ctr + C_ERROR);
-    as[v] = follow(lnext, lexit, li, bx, by, bz, g.W, WH, J.ctr + C_ERROR);
+    if (bz + tz >= g.D) break;
+    const int p = p0 + kPosZ * tz;
+    const int v = x + y * g.W + (bz + tz) * WH;
+    ds[v] = vertex(follow(hnext, p, hs[tz], J.ctr + C_ERROR));
+    as[v] = vertex(follow(lnext, p, ls[tz], J.ctr + C_ERROR));
   }
   return true;
 }
@@ -713,8 +895,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 6) k_direction(const
                                                    const __grid_constant__ Sel sel) {
   __shared__ Tile<T> s;
   __shared__ uint64_t bar;
-  __shared__ int16_t hnext[TZ * TY * TX], lnext[TZ * TY * TX];
-  __shared__ int hexit[TZ * TY * TX], lexit[TZ * TY * TX];
+  __shared__ int16_t hnext[kPosCount], lnext[kPosCount];
   int bx, by, bz, tile;
   const Job<T>& J = tile_job(jobs, sel, bx, by, bz, &tile);
   if (kDec) {
@@ -722,8 +903,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 6) k_direction(const
     if (mf_skip(J.ctr)) return;  // same inputs as the last manifold round
     if (!J.tdirty[tile]) return;  // tile and halo unchanged: pointers stand
   }
-  if (!direction_tile<T, kDec>(J, s, &bar, hnext, lnext, hexit, lexit, bx, by, bz, 0, true))
-    return;
+  if (kDec ? J.tma_g : J.tma_f)
+    tile_issue<T>(s, &bar, kDec ? &J.map_g : &J.map_f, bx, by, bz, true);
+  if (!direction_tile<T, kDec>(J, s, &bar, hnext, lnext, bx, by, bz, 0)) return;
   if (kDec && threadIdx.x == 0) J.tdirty[tile] = 0;
 }
 
@@ -739,8 +921,7 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
                                                         const __grid_constant__ Sel sel) {
   __shared__ Tile<T> s;
   __shared__ uint64_t bar;
-  __shared__ int16_t hnext[TZ * TY * TX], lnext[TZ * TY * TX];
-  __shared__ int hexit[TZ * TY * TX], lexit[TZ * TY * TX];
+  __shared__ int16_t hnext[kPosCount], lnext[kPosCount];
   unsigned loads = 0;  // TMA loads issued by this block: the barrier's phase
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
@@ -753,21 +934,34 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
     const int bx = (t % ntx) * TX, by = ((t / ntx) % nty) * TY, bz = (t / (ntx * nty)) * TZ;
     __syncthreads();  // every thread is done with the shared tile of the last one
     const bool tma = J.tma_g != 0;
-    if (!direction_tile<T, true>(J, s, &bar, hnext, lnext, hexit, lexit, bx, by, bz, loads & 1u,
-                                 loads == 0))
-      return;
-    loads += tma;
-    if (threadIdx.x == 0) J.tdirty[t] = 0;
+    if (tma) tile_issue<T>(s, &bar, &J.map_g, bx, by, bz, loads == 0);
+    // While the tile is on its way: the current labels of its vertices.
     const int x = bx + (int)threadIdx.x % TX, y = by + (int)threadIdx.x / TX;
     if (x < J.dim.W && y < J.dim.H) {
-      for (int tz = 0; tz < TZ && bz + tz < J.dim.D; ++tz) {
-        const int v = x + y * J.dim.W + (bz + tz) * J.dim.W * J.dim.H;
-        const int r2 = J.dds[v], r1 = J.das[v];
-        // Read first: most roots are marked by many vertices.
-        if (!(J.rtouch2[r2 >> 5] >> (r2 & 31) & 1u)) atomicOr(J.rtouch2 + (r2 >> 5), 1u << (r2 & 31));
-        if (!(J.rtouch1[r1 >> 5] >> (r1 & 31) & 1u)) atomicOr(J.rtouch1 + (r1 >> 5), 1u << (r1 & 31));
+      int r2[TZ], r1[TZ];
+      unsigned w2[TZ], w1[TZ];
+      const int v0 = x + y * J.dim.W + bz * J.dim.W * J.dim.H;
+#pragma unroll
+      for (int tz = 0; tz < TZ; ++tz) {
+        const bool in = bz + tz < J.dim.D;
+        r2[tz] = in ? J.dds[v0 + tz * J.dim.W * J.dim.H] : r2[0];
+        r1[tz] = in ? J.das[v0 + tz * J.dim.W * J.dim.H] : r1[0];
+      }
+      // Read first: most roots are marked by many vertices.
+#pragma unroll
+      for (int tz = 0; tz < TZ; ++tz) {
+        w2[tz] = J.rtouch2[r2[tz] >> 5];
+        w1[tz] = J.rtouch1[r1[tz] >> 5];
+      }
+#pragma unroll
+      for (int tz = 0; tz < TZ; ++tz) {
+        if (!(w2[tz] >> (r2[tz] & 31) & 1u)) atomicOr(J.rtouch2 + (r2[tz] >> 5), 1u << (r2[tz] & 31));
+        if (!(w1[tz] >> (r1[tz] & 31) & 1u)) atomicOr(J.rtouch1 + (r1[tz] >> 5), 1u << (r1[tz] & 31));
       }
     }
+    if (!direction_tile<T, true>(J, s, &bar, hnext, lnext, bx, by, bz, loads & 1u)) return;
+    loads += tma;
+    if (threadIdx.x == 0) J.tdirty[t] = 0;
   }
 }
 
