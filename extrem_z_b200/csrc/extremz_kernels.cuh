@@ -61,7 +61,8 @@ struct Job {
   int* hcnt;          // per saddle-pass chunk: seed bits set in it
   int* cpoff;         // per list (2-saddles, 1-saddles, maxima, minima) and
                       // 1024-id block: offset of the block's first entry
-  int* pdd; int* pda; // decompressed steepest pointers, tile-compressed (k_direction)
+  int* pdd; int* pda; // decompressed steepest pointers, tile-compressed (k_direction): the
+                      // path's root with kRootFlag, or the vertex where it leaves the tile
   int* tdirty;        // per tile: a value in the tile or its halo changed since the tile's
                       // pointers were computed (k_apply lists the tile in cand_next then)
   unsigned* rtouch2; unsigned* rtouch1;  // bitsets: labels (of dds / das) of the vertices of
@@ -386,6 +387,9 @@ __device__ __forceinline__ void count_cats(int* ctr, int cat) {
     if (bs) atomicAdd(ctr + C_ASAD, __popc(bs));
   }
 }
+
+// A tile-compressed pointer that is its path's root.
+constexpr int kRootFlag = (int)0x80000000u;
 
 // In-tile positions of the path following: p = x + 64 y + 1024 z, with one bit
 // free above each coordinate's range.  A step adds the direction's offset in the
@@ -872,11 +876,13 @@ __device__ __noinline__ bool direction_tile(const Job<T>& J, Tile<T>& s, uint64_
   }
   __syncthreads();
   if (!col) return true;
-  // Vertex of an in-tile position, one plane, row and column outside included.
+  // Vertex of an in-tile position, one plane, row and column outside included;
+  // flagged when the path ended inside.
   const int base = (bx - 1) + (by - 1) * g.W + (bz - 1) * WH;
   auto vertex = [&](int t) {
     const int q = t + step_of(1, 1, 1);
-    return base + (q & (kPosY - 1)) + (q >> 6 & 15) * g.W + (q >> 10) * WH;
+    const int v = base + (q & (kPosY - 1)) + (q >> 6 & 15) * g.W + (q >> 10) * WH;
+    return t & kPosOut ? v : v | kRootFlag;
   };
 #pragma unroll
   for (int tz = 0; tz < TZ; ++tz) {
@@ -967,8 +973,12 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
 
 // Global pointer jumping of both label arrays (ComputeDescendingManifold /
 // ComputeAscendingManifold, :1514-1611), the two chains interleaved for
-// memory-level parallelism.  Labels always point further along the path, so
-// concurrent readers of a label being finalised see either value correctly.
+// memory-level parallelism.  A pointer that carries the root flag ends its chain:
+// most paths end in their vertex's own tile and load nothing more (without the
+// flag, every chain loads its root's entry once to see that it is one: the L1
+// was 78 % busy).  Original field, in place: labels always point further along the
+// path, so concurrent readers of a label being finalised see either value
+// correctly, and a final label is recognised at its own, unflagged, entry.
 // Every vertex is resolved (the reference resolves descending labels only next
 // to original 2-saddles, the only places they are read).  Iterations are
 // capped; hitting the cap sets the error word instead of spinning.  On the
@@ -1014,21 +1024,19 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       r2 = oas[v];
       c0 = vchg[v >> 5] >> (v & 31);
     }
-    bool d1 = false, d2 = false;
-    int it = 0;
-    for (; it < cap_j && !(d1 && d2); ++it) {
-      if (!d1) {
-        const int w = a[u1];
-        if (w == u1) d1 = true;
-        else u1 = w;
-      }
-      if (!d2) {
-        const int w = b[u2];
-        if (w == u2) d2 = true;
-        else u2 = w;
-      }
+    int it = 2;  // the limit counts the end of a chain and the look at its root too
+    while (it < cap_j && (u1 >= 0 || u2 >= 0)) {
+      int w1 = u1, w2 = u2;
+      if (u1 >= 0) w1 = a[u1];
+      if (u2 >= 0) w2 = b[u2];
+      // An entry that names itself is a final label (original field).
+      u1 = w1 == u1 ? w1 | kRootFlag : w1;
+      u2 = w2 == u2 ? w2 | kRootFlag : w2;
+      ++it;
     }
-    if (it == cap_j) atomicOr(err, kErrJump);
+    if (u1 >= 0 || u2 >= 0 || cap_j < 2) atomicOr(err, kErrJump);
+    u1 &= ~kRootFlag;
+    u2 &= ~kRootFlag;
     if constexpr (kDec) {
       // For the saddle pass: label-mismatch bits, and whether an input of the
       // rows this vertex feeds changed since the previous computed round (its
@@ -1095,26 +1103,35 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
         const unsigned cw = vchg[v0 >> 5] >> (v0 & 31);
         u1[0] = A.x; u1[1] = A.y; u1[2] = A.z; u1[3] = A.w;
         u2[0] = B.x; u2[1] = B.y; u2[2] = B.z; u2[3] = B.w;
-        // One hop of every unfinished chain per iteration: the eight loads
-        // depend only on their own chain, so they are all in flight at once.
-        bool more = true;
-        int it = 0;
-        for (; it < cap_j && more; ++it) {
+        // One hop of every unfinished chain per iteration: the loads depend only
+        // on their own chain, so they are all in flight at once.
+        for (int it = 1; it < cap_j; ++it) {  // (the limit counts the look at the root too)
+          bool more = false;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) more |= (u1[k] >= 0) | (u2[k] >= 0);
+          if (!more) break;
           int w1[4], w2[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            w1[k] = a[u1[k]];
-            w2[k] = b[u2[k]];
+            w1[k] = u1[k];
+            w2[k] = u2[k];
+            if (u1[k] >= 0) w1[k] = a[u1[k]];
+            if (u2[k] >= 0) w2[k] = b[u2[k]];
           }
-          more = false;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            more |= (w1[k] != u1[k]) | (w2[k] != u2[k]);
             u1[k] = w1[k];
             u2[k] = w2[k];
           }
         }
-        if (it == cap_j && more) atomicOr(err, kErrJump);
+        bool open = false;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          open |= (u1[k] >= 0) | (u2[k] >= 0);
+          u1[k] &= ~kRootFlag;
+          u2[k] &= ~kRootFlag;
+        }
+        if (open) atomicOr(err, kErrJump);
         unsigned dv = 0;
         bool n1 = false, n2 = false;
 #pragma unroll
@@ -1888,6 +1905,37 @@ __device__ __noinline__ int row_entry_k(const Job<T>& J, int s, int k) {
   return -1;
 }
 
+// The directions of saddle s's neighbours on the side in the decompressed field.
+template <class T, bool kSplit>
+__device__ __noinline__ unsigned side_of(const Job<T>& J, int s) {
+  const T* __restrict__ gv = J.g;
+  const T sv = __ldg(gv + s);
+  unsigned side = 0u;
+  const Dims g = J.dim;
+  const int WH = g.W * g.H;
+  int x, y, z;
+  coords(s, g, x, y, z);
+  const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
+  // Values seven at a time (fourteen live values spill at 64 registers).
+#pragma unroll
+  for (int h = 0; h < kNumDirs; h += 7) {
+    T val[7];
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+      const int d = h + q;
+      val[q] = (valid >> d & 1) ? __ldg(gv + s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH) : T(0);
+    }
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+      const int d = h + q;
+      const int r = s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
+      if ((valid >> d & 1) && (kSplit ? above(val[q], r, sv, s) : below(val[q], r, sv, s)))
+        side |= 1u << d;
+    }
+  }
+  return side;
+}
+
 // One saddle of one side: its decompressed row summary (count, first and
 // last entry in row order) into the row slots, and whether some neighbour on
 // the side has a wrong label.
@@ -1914,28 +1962,7 @@ __device__ __forceinline__ bool saddle_row(const Job<T>& J, const int* __restric
   if (known) {
     side = kSplit ? J.smask2[i] : J.olm[s];
   } else {
-    const Dims g = J.dim;
-    const int WH = g.W * g.H;
-    int x, y, z;
-    coords(s, g, x, y, z);
-    const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
-    // Values seven at a time (fourteen live values spill at 64 registers).
-#pragma unroll
-    for (int h = 0; h < kNumDirs; h += 7) {
-      T val[7];
-#pragma unroll
-      for (int q = 0; q < 7; ++q) {
-        const int d = h + q;
-        val[q] = (valid >> d & 1) ? __ldg(gv + s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH) : T(0);
-      }
-#pragma unroll
-      for (int q = 0; q < 7; ++q) {
-        const int d = h + q;
-        const int r = s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
-        if ((valid >> d & 1) && (kSplit ? above(val[q], r, sv, s) : below(val[q], r, sv, s)))
-          side |= 1u << d;
-      }
-    }
+    side = side_of<T, kSplit>(J, s);
   }
   int mb = 0;
   if (!kSplit && !J.join_rows) {
@@ -1993,25 +2020,29 @@ __device__ __forceinline__ bool saddle_row(const Job<T>& J, const int* __restric
 }
 
 // Whether any input of saddle s's rows changed since the previous computed
-// round: the changed-input byte of s or of a neighbour (see k_jump2).
+// round: the changed-input byte of s or of a neighbour (see k_jump2).  A
+// neighbour outside the grid reads as some other vertex, which at worst
+// recomputes a row that has not changed, and saves the coordinates.
 template <class T>
-__device__ __forceinline__ bool saddle_inputs_changed(const Job<T>& J, int s) {
-  const Dims g = J.dim;
-  int x, y, z;
-  coords(s, g, x, y, z);
-  const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
-  // Changed-input bytes hold the low byte of the round stamp that set them.
-  const uint8_t st8 = (uint8_t)mf_stamp(J.ctr);
-  bool d = J.dirtyv[s] == st8;
+__device__ __forceinline__ bool saddle_inputs_changed(const Job<T>& J, const int* __restrict__ off,
+                                                      int s, unsigned st8) {
+  const uint8_t* __restrict__ dirty = J.dirtyv;
+  const int last = J.dim.N - 1;
+  unsigned d[kNumDirs + 1];
+  d[kNumDirs] = __ldg(dirty + s);
 #pragma unroll
-  for (int k = 0; k < kNumDirs; ++k)
-    if (valid >> k & 1) d |= J.dirtyv[s + dir_x(k) + dir_y(k) * g.W + dir_z(k) * g.W * g.H] == st8;
-  return d;
+  for (int k = 0; k < kNumDirs; ++k) d[k] = __ldg(dirty + min(max(s + off[k], 0), last));
+  bool hit = false;
+#pragma unroll
+  for (int k = 0; k <= kNumDirs; ++k) hit |= d[k] == st8;
+  return hit;
 }
 
 // Fused pass over the original saddles after a manifold round, both sides in
 // one grid.  A saddle whose inputs did not change since the previous computed
-// round keeps its row slots and reuses its stored seed bit.  A block takes a chunk of the id space (pass_chunk blocks of 1024
+// round keeps its row slots and reuses its stored seed bit; the others of a later
+// round are gathered in shared memory and computed a full block at a time (they
+// are a tenth or so of the saddles, and nearly every warp holds one).  A block takes a chunk of the id space (pass_chunk blocks of 1024
 // ids) and the entries of both saddle lists in it, so that the two sides read
 // the same neighbourhoods together:
 //  * decompressed row slots.  The reference rewrites row i (findAscPaths /
@@ -2031,9 +2062,11 @@ template <class T>
 __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict__ jobs,
                                                         const __grid_constant__ Sel sel) {
   __shared__ int off[kNumDirs];
+  __shared__ int queue[512], queued;  // changed rows waiting: index << 1 | side
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
   if (mf_skip(J.ctr)) return;
+  if (threadIdx.x == 0) queued = 0;
   fill_offsets(off, J.dim);
   // The bitsets that the round's jump has read, and the flags of the last
   // round's wrong neighbours, start empty again.
@@ -2061,6 +2094,40 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
   // next to the chunk, one id wider on each side.
   const bool by_block = !all_new && (J.dim.N & 3) == 0;
   const long long W = J.dim.W, WH = W * J.dim.H, N = J.dim.N;
+  const unsigned st8 = (unsigned)mf_stamp(J.ctr) & 0xffu;  // changed-input bytes of this round
+  // Seed s into its side's list.  All lanes of a warp call it.
+  auto list = [&](bool split, bool has, int s) {
+    const int slot2 = warp_append(J.ctr + C_CAND, has && split, 0xffffffffu);
+    if (slot2 >= 0) J.cand[slot2] = s;
+    const int slot1 = warp_append(J.ctr + C_CANDJ, has && !split, 0xffffffffu);
+    if (slot1 >= 0) J.cand_j[slot1] = s;
+  };
+  // Row i of a side: slots and seed bit.
+  auto row = [&](bool split, int i, int s) {
+    const bool has = split ? saddle_row<T, true>(J, off, i, s, known)
+                           : saddle_row<T, false>(J, off, i, s, known);
+    (split ? J.has2 : J.has1)[i] = (uint8_t)has;
+    return has;
+  };
+  // The last (up to) 256 of the qn queued rows.  The whole block calls it.
+  int qn = 0;  // the same in every thread; `queued` hands out the places
+  auto drain = [&] {
+    const int left = max(qn - (int)blockDim.x, 0), k = left + (int)threadIdx.x;
+    bool has = false, split = false;
+    int s = 0;
+    if (k < qn) {
+      const int i = queue[k] >> 1;
+      split = queue[k] & 1;
+      s = split ? J.sad2[i] : J.sad1[i];
+      has = row(split, i, s);
+      if (has) atomicAdd(J.hcnt + (s >> 10) / chunk, 1);
+    }
+    list(split, has, s);
+    qn = left;
+    __syncthreads();
+    if (threadIdx.x == 0) queued = left;
+    __syncthreads();
+  };
   for (int c = blk; c < nchunk; c += nblk) {
     const int b0 = c * chunk, b1 = min(b0 + chunk, nb);
     const int a2 = J.cpoff[b0], e2 = b1 < nb ? J.cpoff[b1] : ns2;
@@ -2090,41 +2157,58 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
             s = split ? J.sad2[i] : J.sad1[i];
             has = (split ? J.has2 : J.has1)[i] != 0;
           }
-          const int slot2 = warp_append(J.ctr + C_CAND, has && split, 0xffffffffu);
-          if (slot2 >= 0) J.cand[slot2] = s;
-          const int slot1 = warp_append(J.ctr + C_CANDJ, has && !split, 0xffffffffu);
-          if (slot1 >= 0) J.cand_j[slot1] = s;
+          list(split, has, s);
         }
         continue;
       }
     }
-    int nhas = 0;  // seed bits set in the chunk
+    if (all_new) {
+      int nhas = 0;  // seed bits set in the chunk
+      for (int base = 0; base < n; base += blockDim.x) {  // uniform in the block
+        const int k = base + threadIdx.x;
+        const bool split = k < n2;
+        bool has = false;
+        int s = 0;
+        if (k < n) {
+          const int i = split ? a2 + k : a1 + k - n2;
+          s = split ? J.sad2[i] : J.sad1[i];
+          has = row(split, i, s);
+        }
+        list(split, has, s);
+        nhas += __syncthreads_count(has);
+      }
+      if (threadIdx.x == 0) J.hcnt[c] = nhas;
+      continue;
+    }
+    if (threadIdx.x == 0) J.hcnt[c] = 0;  // counted as the chunk's saddles are done
+    __syncthreads();
     for (int base = 0; base < n; base += blockDim.x) {  // uniform in the block
       const int k = base + threadIdx.x;
       const bool split = k < n2;
-      bool has = false;
-      int s = 0;
+      bool has = false, changed = false;
+      int s = 0, i = 0;
       if (k < n) {
-        const int i = split ? a2 + k : a1 + k - n2;
-        uint8_t* hb = split ? J.has2 : J.has1;
+        i = split ? a2 + k : a1 + k - n2;
         s = split ? J.sad2[i] : J.sad1[i];
-        const uint8_t kept = hb[i];  // loaded with the id: no round trip of its own
-        if (all_new || saddle_inputs_changed(J, s)) {
-          has = split ? saddle_row<T, true>(J, off, i, s, known)
-                      : saddle_row<T, false>(J, off, i, s, known);
-          hb[i] = (uint8_t)has;
-        } else {  // rows and seed bit as computed in an earlier round
-          has = kept != 0;
-        }
+        const uint8_t kept = (split ? J.has2 : J.has1)[i];  // loaded with the id
+        changed = saddle_inputs_changed(J, off, s, st8);
+        has = !changed && kept != 0;
       }
-      const int slot2 = warp_append(J.ctr + C_CAND, has && split, 0xffffffffu);
-      if (slot2 >= 0) J.cand[slot2] = s;
-      const int slot1 = warp_append(J.ctr + C_CANDJ, has && !split, 0xffffffffu);
-      if (slot1 >= 0) J.cand_j[slot1] = s;
-      nhas += __syncthreads_count(has);
+      list(split, has, s);
+      const unsigned m = __ballot_sync(0xffffffffu, changed);
+      const unsigned h = __ballot_sync(0xffffffffu, has);
+      int at = 0;
+      if (lane_id() == 0) {
+        if (m) at = atomicAdd(&queued, __popc(m));
+        if (h) atomicAdd(J.hcnt + c, __popc(h));
+      }
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (changed) queue[at + __popc(m & ((1u << lane_id()) - 1u))] = i << 1 | (int)split;
+      qn += __syncthreads_count(changed);
+      if (qn >= (int)blockDim.x) drain();
     }
-    if (threadIdx.x == 0) J.hcnt[c] = nhas;
   }
+  if (qn > 0) drain();
 }
 
 template <class T, bool kSplit>
