@@ -157,14 +157,15 @@ constexpr long long job_bytes_lists(long long ns2, long long ns1, long long nmax
   return arr_bytes(ns2, 4) + arr_bytes(ns1, 4) + arr_bytes(nmax, 4) + arr_bytes(nmin, 4) + 4096;
 }
 
-// Per tile: change mark.
-constexpr long long job_bytes_tiles(long long nt) { return arr_bytes(nt, 4); }
+// Per tile: change mark, jump stamp and queue entry.
+constexpr long long job_bytes_tiles(long long nt) { return 2 * arr_bytes(nt, 4) + arr_bytes(nt, 8); }
 
 // Worst case (every voxel a critical point of every kind; a voxel's upper and
-// lower neighbours, at most 14, give the row entries of both sides; at most
-// one tile per voxel).
+// lower neighbours, at most 14, give the row entries of both sides; a tile for
+// every four voxels and one more, as a 1 x 1 x n column has).
+static_assert(TZ == 4 && TY >= 4 && TX >= 4, "the worst case's tiles");
 constexpr long long job_bytes_sz(long long n, long long ksz) {
-  return job_bytes_voxels(n, ksz) + job_bytes_tiles(n) +
+  return job_bytes_voxels(n, ksz) + job_bytes_tiles(n / 4 + 1) +
          job_bytes_cps(n, n, n, n, 7 * n, 7 * n, ksz);
 }
 template <class T>
@@ -424,6 +425,8 @@ class BatchEngine {
       J.dirtyv = A.take<uint8_t>(N);
       J.bdirty = A.take<int>(jh.nb);
       J.hcnt = A.take<int>(jh.nb);
+      J.tseen = A.take<int>(jh.ntiles);
+      J.tqueue = A.take<unsigned long long>(jh.ntiles);
       J.tdirty = A.take<int>(jh.ntiles);
       J.g0 = keep_input ? A.take<T>(N) : nullptr;
       J.edited = track_edits ? A.take<unsigned>((N + 31) / 32) : nullptr;
@@ -1302,6 +1305,13 @@ class BatchEngine {
           if (!later.empty()) {
             const Sel lt = tile_span(later);
             launch(K_DIRECTION, k_direction_list<T>, blocks(lt), 256, jobs, lt);
+            std::vector<int> large;
+            for (int i : later)
+              if (slots_[i].J.dim.N >= kTouchMin) large.push_back(i);
+            if (!large.empty()) {
+              const Sel qt = tile_span(large);
+              launch(K_JUMP, k_touched_tiles<T>, blocks(qt), 256, jobs, qt);
+            }
           }
           if (!fresh.empty()) {
             const Sel fs = make_span(fresh);
@@ -1630,6 +1640,8 @@ class BatchEngine {
     // stamps start below its stamp, no root is touched, every value counts as
     // changed for it and none for the wrong-saddle scans and detections.
     fl.add(J.tdirty, jh.ntiles, ~0ull);
+    fl.add(J.tseen, jh.ntiles, 0);
+    fl.add(J.tqueue, jh.ntiles, 0);
     fl.add(J.bdirty, jh.nb, 0);
     fl.add(J.rtouch2, words, 0);
     fl.add(J.rtouch1, words, 0);

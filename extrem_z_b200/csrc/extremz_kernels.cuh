@@ -65,6 +65,8 @@ struct Job {
                       // path's root with kRootFlag, or the vertex where it leaves the tile
   int* tdirty;        // per tile: a value in the tile or its halo changed since the tile's
                       // pointers were computed (k_apply lists the tile in cand_next then)
+  int* tseen;         // per tile: the stamp of the round that last listed it in tqueue
+  unsigned long long* tqueue;  // tiles a light round's jump goes over, stamp << 32 | tile
   unsigned* rtouch2; unsigned* rtouch1;  // bitsets: labels (of dds / das) of the vertices of
                                          // the tiles whose pointers this round recomputes
 
@@ -156,6 +158,9 @@ enum Ctr : int {
   C_AFF,       // extrema queued for the current wrong-saddle update
   C_WLONG,     // of those, the ones with long entry lists (wlong)
   C_DETECTED, C_MFRUN,  // a detection, a manifold round ran in this tick
+  C_NAFF,      // tiles that hold a vertex whose label may change this round (k_touched_tiles)
+  C_QHEAD, C_QDONE,  // of those, taken up and searched
+  C_JDENSE,    // they are not listed: the jump goes over every vertex
   C_COUNT
 };
 
@@ -167,12 +172,19 @@ __device__ __forceinline__ bool mf_skip(const int* ctr) {
   return ctr[C_MFDONE] && !ctr[C_CHANGED];
 }
 __device__ __forceinline__ int mf_stamp(const int* ctr) { return ctr[C_WNSTAMP] + 1; }
+// A light round's jump goes over the tiles that k_touched_tiles finds only in
+// fields of at least this many vertices: a pass over every vertex costs about
+// 2.2 us per million, the search some 35 us whatever the field.
+constexpr int kTouchMin = 1 << 25;
 // Start of a round, in its first kernel (which uses none of these).
-__device__ __forceinline__ void mf_begin(int* ctr) {
+__device__ __forceinline__ void mf_begin(int* ctr, int n) {
   ctr[C_MFRUN] = 1;
   if (mf_skip(ctr)) return;
   ctr[C_NFC] = ctr[C_NFC1] = 0;
   ctr[C_CAND] = ctr[C_CANDJ] = ctr[C_CAND_NEXT] = 0;
+  ctr[C_NAFF] = ctr[C_TLIST];  // the recomputed tiles come first
+  ctr[C_QHEAD] = ctr[C_QDONE] = 0;
+  ctr[C_JDENSE] = n < kTouchMin;
 }
 // End of a round.
 __device__ __forceinline__ void mf_end(int* ctr) {
@@ -905,7 +917,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 6) k_direction(const
   int bx, by, bz, tile;
   const Job<T>& J = tile_job(jobs, sel, bx, by, bz, &tile);
   if (kDec) {
-    if (tile == 0 && threadIdx.x == 0) mf_begin(J.ctr);
+    if (tile == 0 && threadIdx.x == 0) mf_begin(J.ctr, J.dim.N);
     if (mf_skip(J.ctr)) return;  // same inputs as the last manifold round
     if (!J.tdirty[tile]) return;  // tile and halo unchanged: pointers stand
   }
@@ -931,7 +943,7 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
   unsigned loads = 0;  // TMA loads issued by this block: the barrier's phase
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
-  if (blk == 0 && threadIdx.x == 0) mf_begin(J.ctr);
+  if (blk == 0 && threadIdx.x == 0) mf_begin(J.ctr, J.dim.N);
   if (mf_skip(J.ctr)) return;
   const int n = J.ctr[C_TLIST];
   const int ntx = (J.dim.W + TX - 1) / TX, nty = (J.dim.H + TY - 1) / TY;
@@ -967,7 +979,108 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
     }
     if (!direction_tile<T, true>(J, s, &bar, hnext, lnext, bx, by, bz, loads & 1u)) return;
     loads += tma;
-    if (threadIdx.x == 0) J.tdirty[t] = 0;
+    if (threadIdx.x == 0) {
+      J.tdirty[t] = 0;
+      J.tseen[t] = mf_stamp(J.ctr);
+      J.tqueue[k] = (unsigned long long)mf_stamp(J.ctr) << 32 | (unsigned)t;
+    }
+  }
+}
+
+// The tiles that hold a vertex whose label may change this round: one with a
+// touched root's label (rtouch2 / rtouch1, see k_direction_list).  The vertices
+// of one label are connected (each one's path stays in its label), and a touched
+// label has a vertex in a recomputed tile, so they are found outwards from the
+// recomputed tiles, the queue's first entries: when a tile's halo holds a touched
+// label, the halo vertex's tile is next, unless it is stamped already.  A light
+// round (a few dozen changed tiles) of a large field then jumps in some hundred
+// tiles instead of reading every vertex's two labels (8 B a voxel, 0.29 ms at
+// 512^3 for a handful of changes).  With more than a 64th of the tiles
+// recomputed, or a quarter found, the jump goes over every vertex.
+//
+// A block takes the queue's entries by ticket.  It waits for its entry only
+// while another running block still searches (entries done < entries pushed);
+// should that take too long, it asks for the pass over every vertex, which is
+// always right, and everyone stops.
+template <class T>
+__global__ void __launch_bounds__(256) k_touched_tiles(const Job<T>* __restrict__ jobs,
+                                                       const __grid_constant__ Sel sel) {
+  __shared__ int tile;
+  __shared__ unsigned found;
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  int* ctr = J.ctr;
+  if (mf_skip(ctr) || __ldcg(ctr + C_JDENSE)) return;
+  const Dims g = J.dim;
+  const int WH = g.W * g.H;
+  const int ntx = (g.W + TX - 1) / TX, nty = (g.H + TY - 1) / TY, ntz = (g.D + TZ - 1) / TZ;
+  const int nt = ntx * nty * ntz;
+  const unsigned stamp = (unsigned)mf_stamp(ctr);
+  if (ctr[C_TLIST] > nt / 64) {
+    if (threadIdx.x == 0) ctr[C_JDENSE] = 1;
+    return;
+  }
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const int h = atomicAdd(ctr + C_QHEAD, 1);
+      int t = -1;
+      for (int spin = 0;; ++spin) {
+        const int done = __ldcg(ctr + C_QDONE), pushed = __ldcg(ctr + C_NAFF);  // in this order
+        if (__ldcg(ctr + C_JDENSE)) break;
+        if (pushed > h && h < nt) {  // the entry may still be on its way
+          const unsigned long long e = __ldcg(J.tqueue + h);
+          if ((unsigned)(e >> 32) == stamp) {
+            t = (int)(unsigned)e;
+            break;
+          }
+        } else if (done == pushed) {
+          break;
+        }
+        if (spin > (1 << 16)) {
+          ctr[C_JDENSE] = 1;
+          break;
+        }
+        __nanosleep(100);
+      }
+      tile = t;
+      found = 0u;
+    }
+    __syncthreads();
+    const int t = tile;
+    if (t < 0) return;
+    const int bx = (t % ntx) * TX, by = ((t / ntx) % nty) * TY, bz = (t / (ntx * nty)) * TZ;
+    // The halo around the tile, in which each vertex stands for one of the 26
+    // neighbouring tiles.
+    unsigned mine = 0u;
+    for (int i = threadIdx.x; i < (TX + 2) * (TY + 2) * (TZ + 2); i += 256) {
+      const int lx = i % (TX + 2) - 1, r = i / (TX + 2), ly = r % (TY + 2) - 1, lz = r / (TY + 2) - 1;
+      const int nx = lx < 0 ? 0 : lx < TX ? 1 : 2, ny = ly < 0 ? 0 : ly < TY ? 1 : 2,
+                nz = lz < 0 ? 0 : lz < TZ ? 1 : 2;
+      const int which = (nz * 3 + ny) * 3 + nx;
+      const int x = bx + lx, y = by + ly, z = bz + lz;
+      if (which == 13 || (unsigned)x >= (unsigned)g.W || (unsigned)y >= (unsigned)g.H ||
+          (unsigned)z >= (unsigned)g.D)
+        continue;
+      const int v = x + y * g.W + z * WH;
+      if (bit_of(J.rtouch2, J.dds[v]) || bit_of(J.rtouch1, J.das[v])) mine |= 1u << which;
+    }
+    mine = __reduce_or_sync(0xffffffffu, mine);
+    if (lane_id() == 0 && mine) atomicOr(&found, mine);
+    __syncthreads();
+    if (threadIdx.x < 27 && (found >> threadIdx.x & 1u)) {
+      const int q = threadIdx.x;
+      const int u = t + (q % 3 - 1) + (q / 3 % 3 - 1) * ntx + (q / 9 - 1) * ntx * nty;
+      if (atomicExch(J.tseen + u, (int)stamp) != (int)stamp) {
+        const int at = atomicAdd(ctr + C_NAFF, 1);
+        if (at < nt / 4) __stcg(J.tqueue + at, (unsigned long long)stamp << 32 | (unsigned)u);
+        else ctr[C_JDENSE] = 1;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(ctr + C_QDONE, 1);
+    }
   }
 }
 
@@ -1043,15 +1156,17 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       // value, either label, or the value of either label's root).  The
       // change bitset starts full, so the first round marks every vertex.
       const unsigned c1 = vchg[u1 >> 5] >> (u1 & 31), c2 = vchg[u2 >> 5] >> (u2 & 31);
-      dirtyv[v] = ((o1 != u1) | (o2 != u2) | ((c0 | c1 | c2) & 1u)) ? (uint8_t)mf_stamp(J.ctr)
-                                                                    : (uint8_t)0;
+      const bool d = (o1 != u1) | (o2 != u2) | ((c0 | c1 | c2) & 1u);
+      dirtyv[v] = d ? (uint8_t)mf_stamp(J.ctr) : (uint8_t)0;
+      if (d) J.bdirty[v >> 10] = mf_stamp(J.ctr);
       mis[v] = (uint8_t)((u1 != r1) | (u2 != r2) << 1);
     }
     ra[v] = u1;
     rb[v] = u2;
   };
+  int from = 0;  // the vertices that are left to the loop at the end
   if constexpr (kDec) {
-    if ((N & 3) == 0) {
+    {
       // Four consecutive vertices per thread: one 16-byte load per array and
       // one 4-byte store per byte array, a quarter of the memory requests of
       // the vertex-per-thread loop, with eight chains interleaved.  A quad
@@ -1070,6 +1185,38 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       // root, lies in a recomputed tile too).
       const int stamp = mf_stamp(J.ctr);
       const unsigned st8 = (unsigned)stamp & 0xffu;
+      // Four vertices' chains to their ends.
+      auto chase = [&](int* u1, int* u2) {
+        // One hop of every unfinished chain per iteration: the loads depend only
+        // on their own chain, so they are all in flight at once.
+        for (int it = 1; it < cap_j; ++it) {  // (the limit counts the look at the root too)
+          bool more = false;
+  #pragma unroll
+          for (int k = 0; k < 4; ++k) more |= (u1[k] >= 0) | (u2[k] >= 0);
+          if (!more) break;
+          int w1[4], w2[4];
+  #pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            w1[k] = u1[k];
+            w2[k] = u2[k];
+            if (u1[k] >= 0) w1[k] = a[u1[k]];
+            if (u2[k] >= 0) w2[k] = b[u2[k]];
+          }
+  #pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            u1[k] = w1[k];
+            u2[k] = w2[k];
+          }
+        }
+        bool open = false;
+  #pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          open |= (u1[k] >= 0) | (u2[k] >= 0);
+          u1[k] &= ~kRootFlag;
+          u2[k] &= ~kRootFlag;
+        }
+        if (open) atomicOr(err, kErrJump);
+      };
       // Returns the quad's labels through u1 / u2 (the old ones when it is
       // not followed) and the old ones through o1 / o2 (-1 in a first round).
       auto quad = [&](int v0, int* u1, int* u2, int* o1, int* o2) {
@@ -1103,35 +1250,7 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
         const unsigned cw = vchg[v0 >> 5] >> (v0 & 31);
         u1[0] = A.x; u1[1] = A.y; u1[2] = A.z; u1[3] = A.w;
         u2[0] = B.x; u2[1] = B.y; u2[2] = B.z; u2[3] = B.w;
-        // One hop of every unfinished chain per iteration: the loads depend only
-        // on their own chain, so they are all in flight at once.
-        for (int it = 1; it < cap_j; ++it) {  // (the limit counts the look at the root too)
-          bool more = false;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) more |= (u1[k] >= 0) | (u2[k] >= 0);
-          if (!more) break;
-          int w1[4], w2[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            w1[k] = u1[k];
-            w2[k] = u2[k];
-            if (u1[k] >= 0) w1[k] = a[u1[k]];
-            if (u2[k] >= 0) w2[k] = b[u2[k]];
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            u1[k] = w1[k];
-            u2[k] = w2[k];
-          }
-        }
-        bool open = false;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          open |= (u1[k] >= 0) | (u2[k] >= 0);
-          u1[k] &= ~kRootFlag;
-          u2[k] &= ~kRootFlag;
-        }
-        if (open) atomicOr(err, kErrJump);
+        chase(u1, u2);
         unsigned dv = 0;
         bool n1 = false, n2 = false;
 #pragma unroll
@@ -1164,17 +1283,67 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
         if (n2) *reinterpret_cast<int4*>(rb + v0) = make_int4(u2[0], u2[1], u2[2], u2[3]);
         if (dv) J.bdirty[v0 >> 10] = stamp;
       };
+      // A light round: only the tiles listed by k_touched_tiles, a thread per
+      // tile column (its four vertices' chains together).  Vertices without a
+      // touched label keep their labels, as above.
+      if (kLater && !J.ctr[C_JDENSE]) {
+        const Dims g = J.dim;
+        const int WH = g.W * g.H;
+        const int ntx = (g.W + TX - 1) / TX, nty = (g.H + TY - 1) / TY;
+        const int na = J.ctr[C_NAFF];
+        for (int k = blk; k < na; k += nblk) {
+          const int t = (int)(unsigned)J.tqueue[k];
+          const int x = (t % ntx) * TX + (int)threadIdx.x % TX;
+          const int y = ((t / ntx) % nty) * TY + (int)threadIdx.x / TX, z = (t / (ntx * nty)) * TZ;
+          if (x >= g.W || y >= g.H) continue;
+          const int v0 = x + y * g.W + z * WH;
+          int u1[TZ], u2[TZ], o1[TZ], o2[TZ];
+          unsigned in = 0u;
+#pragma unroll
+          for (int q = 0; q < TZ; ++q) {
+            if (z + q < g.D) in |= 1u << q;
+            o1[q] = in >> q & 1u ? ra[v0 + q * WH] : o1[0];
+            o2[q] = in >> q & 1u ? rb[v0 + q * WH] : o2[0];
+          }
+          bool hit = false;
+#pragma unroll
+          for (int q = 0; q < TZ; ++q)
+            hit |= (in >> q & 1u) && (bit_of(J.rtouch2, o1[q]) || bit_of(J.rtouch1, o2[q]));
+          if (!hit) continue;
+#pragma unroll
+          for (int q = 0; q < TZ; ++q) {
+            u1[q] = in >> q & 1u ? a[v0 + q * WH] : kRootFlag;
+            u2[q] = in >> q & 1u ? b[v0 + q * WH] : kRootFlag;
+          }
+          chase(u1, u2);
+#pragma unroll
+          for (int q = 0; q < TZ; ++q) {
+            if (!(in >> q & 1u)) continue;
+            const int v = v0 + q * WH;
+            const bool d = o1[q] != u1[q] || o2[q] != u2[q] || bit_of(vchg, v) ||
+                           bit_of(vchg, u1[q]) || bit_of(vchg, u2[q]);
+            dirtyv[v] = d ? (uint8_t)st8 : (uint8_t)0;
+            if (d) J.bdirty[v >> 10] = stamp;
+            if (o1[q] != u1[q] || o2[q] != u2[q]) {
+              mis[v] = (uint8_t)((u1[q] != ods[v]) | (u2[q] != oas[v]) << 1);
+              ra[v] = u1[q];
+              rb[v] = u2[q];
+            }
+          }
+        }
+        return;
+      }
       const int nq = N >> 2;
       const int qstride = nblk * blockDim.x;
       for (int q = blk * blockDim.x + threadIdx.x; q < nq; q += qstride) {
         int u1[4], u2[4], o1[4], o2[4];
         quad(q << 2, u1, u2, o1, o2);
       }
-      return;
+      from = nq << 2;
     }
   }
   const int stride = nblk * blockDim.x;
-  for (int v = blk * blockDim.x + threadIdx.x; v < N; v += stride) jump_one(v);
+  for (int v = from + blk * blockDim.x + threadIdx.x; v < N; v += stride) jump_one(v);
 }
 
 // ---------------------------------------------------------------------------
@@ -2063,6 +2232,8 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
                                                         const __grid_constant__ Sel sel) {
   __shared__ int off[kNumDirs];
   __shared__ int queue[512], queued;  // changed rows waiting: index << 1 | side
+  __shared__ uint8_t state[256];
+  constexpr uint8_t kChunkClean = 0, kChunkSeeds = 1, kChunkChanged = 2;
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
   if (mf_skip(J.ctr)) return;
@@ -2088,12 +2259,25 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
   // In the first round every changed-input byte is set (the change bitset
   // starts full), so the check is skipped.
   const bool all_new = J.ctr[C_MFDONE] == 0;
-  // Later rounds first ask the jump's per-block flags (written when N is a
-  // multiple of 4) whether any changed-input byte is set where the chunk's
-  // saddles could see one: the 3 x 3 row windows of the planes and rows
-  // next to the chunk, one id wider on each side.
-  const bool by_block = !all_new && (J.dim.N & 3) == 0;
   const long long W = J.dim.W, WH = W * J.dim.H, N = J.dim.N;
+  // Later rounds first ask the jump's per-block flags whether any changed-input
+  // byte is set where a chunk's saddles could see one: the 3 x 3 row windows of
+  // the planes and rows next to the chunk, one id wider on each side.  A thread
+  // asks for one of the block's next 256 chunks, so that a light round passes
+  // over the clean ones without a barrier each.
+  auto sees_change = [&](int c) {
+    const long long first = (long long)c * chunk * kCpBlock;
+    const long long end = min((long long)(c + 1) * chunk, (long long)nb) * kCpBlock;
+    const int stamp = mf_stamp(J.ctr);
+    bool seen = false;
+    for (int t = 0; t < 9; ++t) {
+      const long long shift = (long long)(t / 3 - 1) * WH + (long long)(t % 3 - 1) * W;
+      const long long lo = max(0ll, first + shift - 1), hi = min(N - 1, end + shift);
+      for (long long b = lo >> 10; b <= (hi >> 10) && lo <= hi; ++b)
+        seen |= J.bdirty[b] == stamp;
+    }
+    return seen;
+  };
   const unsigned st8 = (unsigned)mf_stamp(J.ctr) & 0xffu;  // changed-input bytes of this round
   // Seed s into its side's list.  All lanes of a warp call it.
   auto list = [&](bool split, bool has, int s) {
@@ -2128,39 +2312,37 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
     if (threadIdx.x == 0) queued = left;
     __syncthreads();
   };
-  for (int c = blk; c < nchunk; c += nblk) {
+  const int mine = blk < nchunk ? (nchunk - blk + nblk - 1) / nblk : 0;  // chunks of the block
+  for (int kc = 0; kc < mine; ++kc) {
+    if (!all_new && kc % 256 == 0) {  // what the next 256 chunks ask for
+      const int k = kc + (int)threadIdx.x, c = blk + k * nblk;
+      uint8_t st = kChunkClean;
+      if (k < mine) st = sees_change(c) ? kChunkChanged : J.hcnt[c] ? kChunkSeeds : kChunkClean;
+      __syncthreads();
+      state[threadIdx.x] = st;
+      __syncthreads();
+    }
+    const uint8_t st = all_new ? kChunkChanged : state[kc % 256];
+    if (st == kChunkClean) continue;  // rows and seed bits stand, and no seed bit is set
+    const int c = blk + kc * nblk;
     const int b0 = c * chunk, b1 = min(b0 + chunk, nb);
     const int a2 = J.cpoff[b0], e2 = b1 < nb ? J.cpoff[b1] : ns2;
     const int a1 = J.cpoff[nb + b0], e1 = b1 < nb ? J.cpoff[nb + b1] : ns1;
     const int n2 = e2 - a2, n = n2 + (e1 - a1);
-    if (by_block) {
-      int seen = 0;
-      if (threadIdx.x < 9) {
-        const int t = (int)threadIdx.x;  // signed: the offsets below go negative
-        const long long off = (long long)(t / 3 - 1) * WH + (long long)(t % 3 - 1) * W;
-        const long long lo = max(0ll, (long long)b0 * kCpBlock + off - 1);
-        const long long hi = min(N - 1, (long long)b1 * kCpBlock - 1 + off + 1);
-        const int stamp = mf_stamp(J.ctr);
-        for (long long b = lo >> 10; b <= (hi >> 10) && lo <= hi; ++b)
-          seen |= J.bdirty[b] == stamp;
-      }
-      if (!__syncthreads_or(seen)) {  // no saddle here has a changed input
-        // Seed bits as computed in an earlier round; none set: nothing to list.
-        if (J.hcnt[c] == 0) continue;
-        for (int base = 0; base < n; base += blockDim.x) {
-          const int k = base + threadIdx.x;
-          const bool split = k < n2;
-          bool has = false;
-          int s = 0;
-          if (k < n) {
-            const int i = split ? a2 + k : a1 + k - n2;
-            s = split ? J.sad2[i] : J.sad1[i];
-            has = (split ? J.has2 : J.has1)[i] != 0;
-          }
-          list(split, has, s);
+    if (st == kChunkSeeds) {  // seed bits as computed in an earlier round
+      for (int base = 0; base < n; base += blockDim.x) {
+        const int k = base + threadIdx.x;
+        const bool split = k < n2;
+        bool has = false;
+        int s = 0;
+        if (k < n) {
+          const int i = split ? a2 + k : a1 + k - n2;
+          s = split ? J.sad2[i] : J.sad1[i];
+          has = (split ? J.has2 : J.has1)[i] != 0;
         }
-        continue;
+        list(split, has, s);
       }
+      continue;
     }
     if (all_new) {
       int nhas = 0;  // seed bits set in the chunk
@@ -3024,7 +3206,7 @@ __global__ void __launch_bounds__(256) k_join_scan(const Job<T>* __restrict__ jo
 // 16-byte pieces (arrays are padded to 256 bytes) of the 8-byte pattern `value`.
 // One launch in place of some twenty fills and clears, whose issue took the host
 // longer than a small field's setup takes the device.
-constexpr int kMaxFills = 28;
+constexpr int kMaxFills = 32;
 struct FillList {
   int n;
   ulonglong2* at[kMaxFills];
