@@ -135,7 +135,7 @@ constexpr long long job_bytes_cps(long long ns2, long long ns1, long long nmax, 
          + arr_bytes(ns2 * kRowStride, 4) + arr_bytes(ns2 * 2, 4) + arr_bytes(ns2, 1)
          + arr_bytes(ns1 * kRowStride, 4) + arr_bytes(ns1 * 2, 4) + arr_bytes(ns1, 1)
          + 2 * arr_bytes(ns2, 16) + 2 * arr_bytes(ns1, 16)  // compact rows (orm, oend)
-         + arr_bytes(ns2, 1) + arr_bytes(ns1, 1)                    // seed bits
+         + 2 * arr_bytes(ns2, 1) + 2 * arr_bytes(ns1, 1)            // seed bits, wrong-row bits
          + 4 * arr_bytes(nmax, 4) + 4 * arr_bytes(nmin, 4)
          + arr_bytes(nmax > nmin ? nmax : nmin, ksz) + arr_bytes(nmax > nmin ? nmax : nmin, 4)
          + arr_bytes(8, 8)
@@ -585,7 +585,7 @@ class BatchEngine {
     unsigned* table = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(cand) + cand_bytes);
     unsigned* member = table + kMergeWords;
     int* ctot = J.ctr + C_CAND;  // two free counter slots of the finished job
-    launch(K_OTHER, k_pp_merge_table, kMergeWords * 32 / 256, 256, table);
+    launch(K_OTHER, k_pp_merge_table, kMergeWords * 32 / 256, 256, tb_, table);
     launch(K_OTHER, k_pp_cand_count<T>, jh.nb, kCpBlock, J.f, J.dim, (const unsigned*)table, member,
            jh.bcount);
     launch(K_OTHER, k_scan_lists, 2, 1024, jh.bcount, jh.nb, ctot, (int*)nullptr);
@@ -634,7 +634,9 @@ class BatchEngine {
     auto sort = [&](const int* list, int n, bool reverse, bool complement, int* out_li) {
       launch(K_OTHER, k_pp_keys<T>, grid_, 256, J.f, list, n, reverse, complement, kin, vin);
       size_t tb = cub_bytes;
-      if (cub::DeviceRadixSort::SortPairs(cub_tmp, tb, kin, kout, vin, out_li, n, 0, 64, st_) !=
+      // A float's key has 32 bits (complemented, the others are all ones).
+      if (cub::DeviceRadixSort::SortPairs(cub_tmp, tb, kin, kout, vin, out_li, n, 0,
+                                          8 * (int)sizeof(K), st_) !=
           cudaSuccess)
         rc = EXTREMZ_CUDA_ERR;
     };
@@ -660,24 +662,30 @@ class BatchEngine {
       // Saddles descending in the tree's order.
       if (n_s) sort(slist[side], n_s, kmax, kmax, sad_li);
       if (kmax)
-        launch(K_OTHER, k_pp_rows<T, true>, grid_, 256, J.f, J.dim, slist[0], (const int*)sad_li,
-               n_s, (const int*)J.ds, (const int*)J.ext, (const int*)erank, rows, cnt);
+        launch(K_OTHER, k_pp_rows<true>, grid_, 256, (const uint16_t*)J.olm, J.dim, slist[0],
+               (const int*)sad_li, n_s, (const int*)J.ds, (const int*)J.ext, (const int*)erank, rows,
+               cnt);
       else
-        launch(K_OTHER, k_pp_rows<T, false>, grid_, 256, J.f, J.dim, slist[1], (const int*)sad_li,
-               n_s, (const int*)J.as, (const int*)J.ext, (const int*)erank, rows, cnt);
+        launch(K_OTHER, k_pp_rows<false>, grid_, 256, (const uint16_t*)J.olm, J.dim, slist[1],
+               (const int*)sad_li, n_s, (const int*)J.as, (const int*)J.ext, (const int*)erank, rows,
+               cnt);
       launch(K_OTHER, k_fill<int>, grid_, 256, largest, kInf, (long long)n_e);
       launch(K_OTHER, k_fill<int>, grid_, 256, pair, -1, (long long)n_e);
       launch(K_OTHER, k_iota, grid_, 256, ptr, n_e);
-      for (int round = 0; round <= n_e; ++round) {  // every round but the last pairs one
-        EZ_CHECK(cudaMemsetAsync(flag, 0, 4, st_));
+      // Every round but the last pairs one; a round that pairs none changes
+      // nothing, so the host asks only after every fourth.
+      for (int round = 0; round <= n_e; ++round) {
+        if (round % 4 == 0) EZ_CHECK(cudaMemsetAsync(flag, 0, 4, st_));
         if (n_s) launch(K_OTHER, k_pp_largest, grid_, 256, (const int*)rows, (const int*)cnt, n_s,
                         n_e - 1, largest);
         launch(K_OTHER, k_pp_pair, grid_, 256, (const int*)rows, (const int*)cnt, n_e, n_s,
                largest, ptr, pair, lmax, flag);
-        int changed = 0;
-        EZ_CHECK(cudaMemcpyAsync(&changed, flag, 4, cudaMemcpyDeviceToHost, st_));
-        EZ_CHECK(cudaStreamSynchronize(st_));
-        if (!changed) break;
+        if (round % 4 == 3) {
+          int changed = 0;
+          EZ_CHECK(cudaMemcpyAsync(&changed, flag, 4, cudaMemcpyDeviceToHost, st_));
+          EZ_CHECK(cudaStreamSynchronize(st_));
+          if (!changed) break;
+        }
         launch(K_OTHER, k_pp_jump, grid_, 256, ptr, n_e, n_e + 1, flag + 1);
         if (n_s) launch(K_OTHER, k_pp_remap, grid_, 256, rows, cnt, n_s, (const int*)ptr);
       }
@@ -1569,8 +1577,7 @@ class BatchEngine {
     if (!J.minima) return EXTREMZ_OOM;
     launch(K_OTHER, k_cp_write, (jh.nb + kCpWarps - 1) / kCpWarps, 32 * kCpWarps,
            (const int8_t*)J.otype, N, jh.nb, (const int*)jh.bcount,
-           J.sad2, J.sad1, J.maxima, J.minima);
-    launch(K_OTHER, k_ext_index<T>, grid_, 256, J);
+           J.sad2, J.sad1, J.maxima, J.minima, J.ext);
     // The lists and the extremum index are all that an analysis needs.
     if (jh.p.flags & kFlagAnalysis) return EXTREMZ_OK;
     J.smask2 = A.take<uint16_t>(ns2);
@@ -1586,6 +1593,8 @@ class BatchEngine {
     J.ocnt1 = A.take<uint8_t>(ns1);
     J.has2 = A.take<uint8_t>(ns2);
     J.has1 = A.take<uint8_t>(ns1);
+    J.bad2 = A.take<uint8_t>(ns2);
+    J.bad1 = A.take<uint8_t>(ns1);
     J.largest = A.take<int>(nmax);
     J.first1 = A.take<int>(nmax);
     J.flag2 = A.take<int>(nmax);
@@ -1636,6 +1645,8 @@ class BatchEngine {
     // Decompressed row slots start at zero: the reference's rows are fresh
     // cudaMalloc memory read before first written (:5338-5341, :3128-3130).
     fl.add(J.drow2, ns2 * 2ll, 0);
+    fl.add(J.bad2, ns2, 0);
+    if (J.join_rows) fl.add(J.bad1, ns1, 0);
     // Every tile's pointers are computed in the first manifold round, block
     // stamps start below its stamp, no root is touched, every value counts as
     // changed for it and none for the wrong-saddle scans and detections.

@@ -58,6 +58,8 @@ struct Job {
   int* bdirty;        // per 1024-id block: the round stamp when some dirtyv byte in it was
                       // set (when N % 4 == 0)
   uint8_t* has2; uint8_t* has1;  // per saddle row: its wrong-neighbour seed bit
+  uint8_t* bad2; uint8_t* bad1;  // per saddle row: 1 if its first row slot differs from the
+                                 // original row's first entry, 2 if its second from the last
   int* hcnt;          // per saddle-pass chunk: seed bits set in it
   int* cpoff;         // per list (2-saddles, 1-saddles, maxima, minima) and
                       // 1024-id block: offset of the block's first entry
@@ -155,6 +157,7 @@ enum Ctr : int {
   C_WNSMALL,   // this side's candidate list is small: the block completion does it all
   C_TLIST,     // tiles listed for the next manifold round's steepest pointers (k_apply)
   C_WEP2, C_WEP1,  // wrong-saddle scans so far (maxima, minima); the first computes every extremum
+  C_WLIST2, C_WLIST1,  // extrema named by a wrong row in this tick's scan (k_wim_scan)
   C_AFF,       // extrema queued for the current wrong-saddle update
   C_WLONG,     // of those, the ones with long entry lists (wlong)
   C_DETECTED, C_MFRUN,  // a detection, a manifold round ran in this tick
@@ -583,9 +586,11 @@ __global__ void __launch_bounds__(256, 8) k_classify(const Job<T>* __restrict__ 
       const int v = x + y * g.W + z * g.W * g.H;
       const int bc = interior ? 0 : boundary_code(x, y, z, g.W, g.H, g.D);
       const int valid = interior ? (1 << kNumDirs) - 1 : valid_mask(bc);
-      const int lm = mask[tz] & valid;
-      const int t = type_from_masks(lm, valid & ~lm, valid, bc, J.tb);
-      const int cat = mismatch_cats(t, J.otype[v], lm, J.olm[v]);
+      const int lm = mask[tz] & valid, om = J.olm[v];
+      // The type follows from the mask: with the original's mask nothing differs.
+      const int cat = lm == om ? 0
+                               : mismatch_cats(type_from_masks(lm, valid & ~lm, valid, bc, J.tb),
+                                               J.otype[v], lm, om);
       J.mstat[v] = (uint8_t)cat;
       if (cat) {
         s_list[atomicAdd(&s_n, 1)] = v | (cat << kCatShift);
@@ -1405,18 +1410,33 @@ __global__ void __launch_bounds__(32 * kCpWarps) k_cp_count(const int8_t* __rest
   if ((bits[0] | bits[1]) != 0u) {
     int x, y, z;
     coords(v0, g, x, y, z);
-    for (int k = 0; k < 32; ++k) {
-      if (((bits[0] | bits[1]) >> k) & 1u) {
-        const int nvalid = __popc(valid_mask(boundary_code(x, y, z, g.W, g.H, g.D)));
-        const int lower = __popc((unsigned)olm[v0 + k]);
-        if ((bits[0] >> k) & 1u) e2 += nvalid - lower;
-        if ((bits[1] >> k) & 1u) e1 += lower;
+    if (v0 + 32 <= g.N && x > 0 && x + 31 < g.W - 1 && y > 0 && y < g.H - 1 && z > 0 && z < g.D - 1) {
+      // Off the faces every vertex has 14 neighbours; the masks come in together.
+      uint4 q[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = reinterpret_cast<const uint4*>(olm + v0)[k];
+#pragma unroll
+      for (int k = 0; k < 32; ++k) {
+        const uint4& w = q[k >> 3];
+        const unsigned pair = (k & 6) == 0 ? w.x : (k & 6) == 2 ? w.y : (k & 6) == 4 ? w.z : w.w;
+        const int lower = __popc(k & 1 ? pair >> 16 : pair & 0xffffu);
+        e2 += (bits[0] >> k & 1u) ? kNumDirs - lower : 0;
+        e1 += (bits[1] >> k & 1u) ? lower : 0;
       }
-      if (++x == g.W) {
-        x = 0;
-        if (++y == g.H) {
-          y = 0;
-          ++z;
+    } else {
+      for (int k = 0; k < 32; ++k) {
+        if (((bits[0] | bits[1]) >> k) & 1u) {
+          const int nvalid = __popc(valid_mask(boundary_code(x, y, z, g.W, g.H, g.D)));
+          const int lower = __popc((unsigned)olm[v0 + k]);
+          if ((bits[0] >> k) & 1u) e2 += nvalid - lower;
+          if ((bits[1] >> k) & 1u) e1 += lower;
+        }
+        if (++x == g.W) {
+          x = 0;
+          if (++y == g.H) {
+            y = 0;
+            ++z;
+          }
         }
       }
     }
@@ -1431,8 +1451,9 @@ __global__ void __launch_bounds__(32 * kCpWarps) k_cp_count(const int8_t* __rest
 
 // Exclusive scan of gridDim.x lists of nb counts in place (a block per list),
 // list totals to totals[0 .. gridDim.x).  The CP lists use totals = ctr + C_NS2.
-// Each thread takes 32 consecutive counts per pass.  cursor (optional, one
-// list): a second copy of the scanned counts.
+// Each thread takes up to 32 consecutive counts per pass, no more than it takes to
+// cover the list.  cursor (optional, one list): a second copy of the scanned
+// counts.
 __global__ void __launch_bounds__(1024) k_scan_lists(int* __restrict__ bcount, int nb, int* totals,
                                                      int* __restrict__ cursor) {
   constexpr int kPer = 32;
@@ -1442,13 +1463,14 @@ __global__ void __launch_bounds__(1024) k_scan_lists(int* __restrict__ bcount, i
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
   int* c = bcount + (long long)l * nb;
-  for (int base = 0; base < nb; base += 1024 * kPer) {
-    const int i0 = base + (int)threadIdx.x * kPer;
+  const int per = min(kPer, (nb + 1023) / 1024);
+  for (int base = 0; base < nb; base += 1024 * per) {
+    const int i0 = base + (int)threadIdx.x * per;
     int x[kPer];
     int sum = 0;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-      x[k] = i0 + k < nb ? c[i0 + k] : 0;
+      x[k] = k < per && i0 + k < nb ? c[i0 + k] : 0;
       sum += x[k];
     }
     int incl = sum;
@@ -1470,7 +1492,7 @@ __global__ void __launch_bounds__(1024) k_scan_lists(int* __restrict__ bcount, i
     int run = carry + warp_sums[threadIdx.x / 32] + incl - sum;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-      if (i0 + k < nb) {
+      if (k < per && i0 + k < nb) {
         c[i0 + k] = run;
         if (cursor) cursor[i0 + k] = run;
       }
@@ -1537,11 +1559,13 @@ __global__ void __launch_bounds__(1024) k_chunk_scan(int* __restrict__ c, int n,
   }
 }
 
+// The four lists, and ext[v] = the index of a maximum or minimum v in its list
+// (computeMaxIndex / computeMinIndex :1928-1939 share one array).
 __global__ void __launch_bounds__(32 * kCpWarps) k_cp_write(const int8_t* __restrict__ otype,
                                                            int N, int nb,
                                                            const int* __restrict__ boff,
                                                            int* sad2, int* sad1, int* maxima,
-                                                           int* minima) {
+                                                           int* minima, int* __restrict__ ext) {
   const int b = blockIdx.x * kCpWarps + (int)(threadIdx.x >> 5);
   if (b >= nb) return;
   const int v0 = b * kCpBlock + (int)lane_id() * 32;
@@ -1560,20 +1584,9 @@ __global__ void __launch_bounds__(32 * kCpWarps) k_cp_write(const int8_t* __rest
     for (unsigned m = bits[l]; m; m &= m - 1) {
       const int v = v0 + __ffs(m) - 1;
       outs[l][pos] = v;
+      if (l >= 2) ext[v] = pos;
       ++pos;
     }
-  }
-}
-
-// ext[maxima[i]] = i and ext[minima[i]] = i (computeMaxIndex / computeMinIndex
-// :1928-1939 share one array).
-template <class T>
-__global__ void k_ext_index(Job<T> J) {
-  const int nmax = J.ctr[C_NMAX], nmin = J.ctr[C_NMIN];
-  const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nmax + nmin; i += stride) {
-    if (i < nmax) J.ext[J.maxima[i]] = i;
-    else J.ext[J.minima[i - nmax]] = i - nmax;
   }
 }
 
@@ -2173,17 +2186,20 @@ __device__ __forceinline__ bool saddle_row(const Job<T>& J, const int* __restric
     }
   }
   const int oc = (kSplit ? J.ocnt2 : J.ocnt1)[i];
-  if (oc > 0 && cnt > 0) {
-    int* slots = kSplit ? J.drow2 : J.drow1;
+  if (oc > 0) {
+    int* slots = (kSplit ? J.drow2 : J.drow1) + 2ll * i;
     const int k = oc - 1;
-    slots[2ll * i] = fm;
+    int first = fm, kth = lm;
     if (cnt > k) {
-      int kth;
-      if (k == cnt - 1) kth = lm;
-      else if (k == 0) kth = fm;
-      else kth = row_entry_k<T, kSplit>(J, s, k);
-      slots[2ll * i + 1] = kth;
+      if (k != cnt - 1) kth = k == 0 ? fm : row_entry_k<T, kSplit>(J, s, k);
+      *reinterpret_cast<int2*>(slots) = make_int2(fm, kth);
+    } else {  // a shorter row keeps what it does not rewrite
+      if (cnt > 0) slots[0] = fm;
+      else first = slots[0];
+      kth = slots[1];
     }
+    const int2 o = *reinterpret_cast<const int2*>((kSplit ? J.oend2 : J.oend1) + i);
+    (kSplit ? J.bad2 : J.bad1)[i] = (uint8_t)((o.x != first) | (o.y != kth) << 1);
   }
   return (mb >> (kSplit ? 0 : 1)) & 1;
 }
@@ -2754,6 +2770,12 @@ __global__ void __launch_bounds__(256) k_fixpath(const Job<T>* __restrict__ jobs
 // (:3113-3141) and get_wrong_index_min (:3143-3171) with the lowest saddle row
 // winning per extremum, followed by the fixes (:3320-3413).
 // ---------------------------------------------------------------------------
+// The saddle pass has compared each row it computed with the original's (bad2 /
+// bad1), so a scan reads a byte per row and goes on only at the wrong ones, and
+// lists the extrema they name (in mm_next, free between detections: the index
+// times two, plus one for the second kind) for the collecting pass.  Reading
+// every row's ends and slots, then every extremum's two arbitration slots, took
+// 0.16 ms per scan at 512^3, mostly to find nothing.
 template <class T, bool kMax>
 __global__ void __launch_bounds__(256) k_wim_scan(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
   int blk, nblk;
@@ -2765,29 +2787,39 @@ __global__ void __launch_bounds__(256) k_wim_scan(const Job<T>* __restrict__ job
   }
   const int ns = J.ctr[kMax ? C_NS2 : C_NS1];
   const int4* oend = kMax ? J.oend2 : J.oend1;
-  const int* drow = kMax ? J.drow2 : J.drow1;
+  const uint8_t* bad = kMax ? J.bad2 : J.bad1;
   int* first = kMax ? J.first1 : J.first_min1;
   int* flag = kMax ? J.flag2 : J.flag_min2;
+  int* count = J.ctr + (kMax ? C_WLIST2 : C_WLIST1);
   const int stride = nblk * blockDim.x;
-  for (int i = blk * blockDim.x + threadIdx.x; i < ns; i += stride) {
-    const int cnt = (kMax ? J.ocnt2 : J.ocnt1)[i];
-    if (cnt == 0) continue;
-    // Original entries 0 and count - 1 (labels, extremum indices) against the
-    // decompressed row slots: entry 0, entry (count - 1).
-    const int4 o = oend[i];
-    const int2 d = *reinterpret_cast<const int2*>(drow + 2ll * i);
-    if (o.x != d.x) atomicMin(first + o.z, i);
-    if (o.y != d.y) flag[o.w] = 1;
+  for (int q = blk * blockDim.x + threadIdx.x; q < (ns + 15) >> 4; q += stride) {
+    // (The arrays are padded; rows past the last are not looked at.)
+    const uint4 w = reinterpret_cast<const uint4*>(bad)[q];
+    const unsigned word[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      for (unsigned rest = word[j]; rest;) {
+        const int byte = (__ffs((int)rest) - 1) >> 3, i = 16 * q + 4 * j + byte;
+        const unsigned kinds = rest >> (8 * byte) & 3u;
+        rest &= ~(0xffu << (8 * byte));
+        if (i >= ns) break;
+        const int4 o = oend[i];
+        if ((kinds & 1u) && atomicMin(first + o.z, i) == kInf) J.mm_next[atomicAdd(count, 1)] = o.z << 1;
+        if ((kinds & 2u) && atomicExch(flag + o.w, 1) == 0)
+          J.mm_next[atomicAdd(count, 1)] = o.w << 1 | 1;
+      }
+    }
   }
 }
 
-// Collect per extremum, count, propose the fix and reset the arbitration slots.
-// fix = false: detection only (the third block of the outer loop, :5932-5951).
+// Collect per listed extremum, count, propose the fix and reset the arbitration
+// slots.  fix = false: detection only (the third block of the outer loop,
+// :5932-5951).
 template <class T, bool kMax>
 __global__ void __launch_bounds__(256) k_wim_collect(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel, int fix) {
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
-  const int next = J.ctr[kMax ? C_NMAX : C_NMIN];
+  const int n = J.ctr[kMax ? C_WLIST2 : C_WLIST1];
   const int* ext_list = kMax ? J.maxima : J.minima;
   const int* drow = kMax ? J.drow2 : J.drow1;
   int* first = kMax ? J.first1 : J.first_min1;
@@ -2795,13 +2827,15 @@ __global__ void __launch_bounds__(256) k_wim_collect(const Job<T>* __restrict__ 
   int* c1 = J.ctr + (kMax ? C_WMC : C_WMIN);
   int* c2 = J.ctr + (kMax ? C_WMC2 : C_WMIN2);
   const int stride = nblk * blockDim.x;
-  for (int base = blk * blockDim.x; base < next; base += stride) {
-    const int m = base + threadIdx.x;
+  for (int base = blk * blockDim.x; base < n; base += stride) {
+    const int e = base + threadIdx.x;
     bool h1 = false, h2 = false;
-    if (m < next) {
-      const int row = first[m];
-      if (row != kInf) {
-        h1 = true;
+    if (e < n) {
+      const int m = J.mm_next[e] >> 1;
+      h2 = J.mm_next[e] & 1;
+      h1 = !h2;
+      if (h1) {
+        const int row = first[m];
         first[m] = kInf;
         if (fix) {
           // split: lower the false maximum, entry 0 of the winning
@@ -2810,16 +2844,10 @@ __global__ void __launch_bounds__(256) k_wim_collect(const Job<T>* __restrict__ 
           const int target = kMax ? drow[2ll * row] : ext_list[m];
           propose(J, target, step_delta(J, target));
         }
-      }
-      if (flag[m]) {
-        h2 = true;
+      } else {
         flag[m] = 0;
-        if (fix) {
-          if (kMax) {
-            // lower the true maximum (:3346-3364)
-            propose(J, ext_list[m], step_delta(J, ext_list[m]));
-          }
-        }
+        // lower the true maximum (:3346-3364)
+        if (fix && kMax) propose(J, ext_list[m], step_delta(J, ext_list[m]));
       }
     }
     const unsigned mask = 0xffffffffu;
@@ -2833,31 +2861,37 @@ __global__ void __launch_bounds__(256) k_wim_collect(const Job<T>* __restrict__ 
 
 // get_wrong_index_min direction 1 (:3157-3168, fix :3393-3410) keeps the pair of
 // the lowest row per minimum and lowers the row's FALSE last entry, so it needs
-// the winning row: one more scan, arbitrating through ext_id (the setup's
-// array, left at kInf; first_sj keeps the wrong-saddle results between
-// scans).
+// the winning row: one more scan, arbitrating through ext_id (left at kInf;
+// first_sj keeps the wrong-saddle results between scans), then the minima of
+// the second kind in k_wim_scan's list.
 template <class T>
 __global__ void __launch_bounds__(256) k_wim_min2_scan(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
   const int ns = J.ctr[C_NS1];
   const int stride = nblk * blockDim.x;
-  for (int i = blk * blockDim.x + threadIdx.x; i < ns; i += stride) {
-    const int cnt = J.ocnt1[i];
-    if (cnt == 0) continue;
-    const int4 o = J.oend1[i];
-    if (o.y != J.drow1[2ll * i + 1]) atomicMin(J.ext_id + o.w, i);
+  for (int q = blk * blockDim.x + threadIdx.x; q < (ns + 15) >> 4; q += stride) {
+    const uint4 w = reinterpret_cast<const uint4*>(J.bad1)[q];
+    const unsigned word[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      for (unsigned rest = word[j] & 0x02020202u; rest; rest &= rest - 1u) {
+        const int i = 16 * q + 4 * j + ((__ffs((int)rest) - 1) >> 3);
+        if (i < ns) atomicMin(J.ext_id + J.oend1[i].w, i);
+      }
+    }
   }
 }
 template <class T>
 __global__ void __launch_bounds__(256) k_wim_min2_collect(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
-  const int next = J.ctr[C_NMIN];
+  const int n = J.ctr[C_WLIST1];
   const int stride = nblk * blockDim.x;
-  for (int m = blk * blockDim.x + threadIdx.x; m < next; m += stride) {
+  for (int e = blk * blockDim.x + threadIdx.x; e < n; e += stride) {
+    if (!(J.mm_next[e] & 1)) continue;
+    const int m = J.mm_next[e] >> 1;
     const int row = J.ext_id[m];
-    if (row == kInf) continue;
     J.ext_id[m] = kInf;
     const int target = J.drow1[2ll * row + 1];
     propose(J, target, step_delta(J, target));
@@ -3235,6 +3269,7 @@ __global__ void __launch_bounds__(256) k_tick_end(Job<T>* jobs, int* ctr, int sl
   if (threadIdx.x < slots) {
     int* c = ctr + threadIdx.x * C_COUNT;
     c[C_TOUCHED] = 0;
+    c[C_WLIST2] = c[C_WLIST1] = 0;
     if (c[C_DETECTED]) {
       c[C_DETECTED] = 0;
       detect_end(jobs[threadIdx.x]);

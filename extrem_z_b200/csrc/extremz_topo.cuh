@@ -29,47 +29,18 @@ namespace extremz {
 
 constexpr int kPpRow = 16;  // entries per row (<= 14 neighbours)
 
-// Link adjacency of the 14-neighbourhood: two neighbours are joined by a link
-// edge when their offset is itself one of the 14 directions.
-__host__ __device__ constexpr int link_adj(int a) {
-  int m = 0;
-  for (int b = 0; b < kNumDirs; ++b) {
-    if (a == b) continue;
-    const int dx = dir_x(b) - dir_x(a), dy = dir_y(b) - dir_y(a), dz = dir_z(b) - dir_z(a);
-    for (int c = 0; c < kNumDirs; ++c)
-      if (dir_x(c) == dx && dir_y(c) == dy && dir_z(c) == dz) m |= 1 << b;
-  }
-  return m;
-}
-
-// Connected components of a set of link vertices (bit d = direction d).
-__device__ __forceinline__ int link_comps(int nodes) {
-  int comps = 0, left = nodes;
-  while (left) {
-    int comp = left & -left;
-    for (;;) {
-      int grow = comp;
-#pragma unroll
-      for (int d = 0; d < kNumDirs; ++d)
-        if (comp >> d & 1) grow |= link_adj(d) & nodes;
-      if (grow == comp) break;
-      comp = grow;
-    }
-    left &= ~comp;
-    ++comps;
-  }
-  return comps;
-}
-
 // Which of the 2^14 sets of link vertices fall into two or more components, one
-// bit per set (kMergeWords words, 2 KB).  Flooding the link at every voxel took
-// 17 ms per pass of a 160x144x128 field; the sets are few, so each call floods
-// each set once (a few microseconds) and a voxel's test is a bit in shared
-// memory.
+// bit per set (kMergeWords words, 2 KB).  An interior vertex whose upper
+// neighbours are the set is a 2-saddle (or both kinds of saddle) exactly then,
+// so the bits come from the type table's interior entries; the empty and the
+// full set have none and one component.  Flooding the link at every voxel took
+// 17 ms per pass of a 160x144x128 field; a voxel's test is a bit in shared memory.
 constexpr int kMergeWords = (1 << kNumDirs) / 32;
-__global__ void __launch_bounds__(256) k_pp_merge_table(unsigned* __restrict__ table) {
+__global__ void __launch_bounds__(256) k_pp_merge_table(DeviceTables tb, unsigned* __restrict__ table) {
   const int set = blockIdx.x * 256 + threadIdx.x;
-  const unsigned m = __ballot_sync(0xffffffffu, link_comps(set) >= 2);
+  const int t = tb.lut[tb.key_offset[0] + set];
+  const bool merges = set != 0 && set != (1 << kNumDirs) - 1 && (t == 2 || t == 3);
+  const unsigned m = __ballot_sync(0xffffffffu, merges);
   if (lane_id() == 0) table[set >> 5] = m;
 }
 
@@ -165,55 +136,90 @@ __global__ void k_pp_rank(const int* __restrict__ sorted_li, int n, int* __restr
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride) rank[sorted_li[p]] = p;
 }
 
+// Stores the distinct entries of r (kInf = none) ascending, unless there is only
+// one; returns how many.
+__device__ __forceinline__ int pp_store_row(const int* r, int* row) {
+  unsigned keep = 0u;
+#pragma unroll
+  for (int q = 0; q < kPpRow; ++q) {
+    bool again = r[q] == kInf;
+#pragma unroll
+    for (int k = 0; k < q; ++k) again |= r[k] == r[q];
+    if (!again) keep |= 1u << q;
+  }
+  const int n = __popc(keep);
+  if (n < 2) return 0;
+#pragma unroll
+  for (int q = 0; q < kPpRow; ++q) {
+    if (!(keep >> q & 1u)) continue;
+    int at = 0;
+#pragma unroll
+    for (int k = 0; k < kPpRow; ++k) at += (keep >> k & 1u) && r[k] < r[q];
+    row[at] = r[q];
+  }
+  return n;
+}
+
 // Row of each saddle (by sorted position): distinct extremum ranks of the
-// labels of its neighbours on the tree's side, ascending.
-template <class T, bool kMax>
-__global__ void k_pp_rows(const T* __restrict__ a, Dims g, const int* __restrict__ sad,
-                          const int* __restrict__ sorted_li, int ns, const int* __restrict__ lab,
-                          const int* __restrict__ ext, const int* __restrict__ erank,
-                          int* __restrict__ rows, int* __restrict__ cnt) {
+// labels of its neighbours on the tree's side, ascending.  The neighbours are
+// the classification's direction mask; an entry's place is the number of smaller
+// distinct ones, so nothing is sorted in local memory.
+template <bool kMax>
+__global__ void __launch_bounds__(256) k_pp_rows(const uint16_t* __restrict__ olm, Dims g,
+                                                 const int* __restrict__ sad,
+                                                 const int* __restrict__ sorted_li, int ns,
+                                                 const int* __restrict__ lab,
+                                                 const int* __restrict__ ext,
+                                                 const int* __restrict__ erank, int* __restrict__ rows,
+                                                 int* __restrict__ cnt) {
+  __shared__ int off[kNumDirs];
+  fill_offsets(off, g);
+  __syncthreads();
   const int stride = gridDim.x * blockDim.x;
-  const int WH = g.W * g.H;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
     const int s = sad[sorted_li[i]];
-    int x, y, z;
-    coords(s, g, x, y, z);
-    const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
-    const T sv = a[s];
-    int r[kPpRow];
-    int n = 0;
-    for (int d = 0; d < kNumDirs; ++d) {
-      if (!(valid >> d & 1)) continue;
-      const int v = s + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
-      const T vv = a[v];
-      if (!(kMax ? above(vv, v, sv, s) : below(vv, v, sv, s))) continue;
-      const int e = erank[ext[lab[v]]];
-      int j = n;  // insertion, dropping duplicates
-      bool dup = false;
-      for (int q = 0; q < n; ++q) dup |= r[q] == e;
-      if (dup) continue;
-      while (j > 0 && r[j - 1] > e) {
-        r[j] = r[j - 1];
-        --j;
-      }
-      r[j] = e;
-      ++n;
+    unsigned side = olm[s];
+    if (kMax) {
+      int x, y, z;
+      coords(s, g, x, y, z);
+      side = (unsigned)valid_mask(boundary_code(x, y, z, g.W, g.H, g.D)) & ~side;
     }
-    if (n == 1) n = 0;
-    for (int q = 0; q < n; ++q) rows[(long long)i * kPpRow + q] = r[q];
-    cnt[i] = n;
+    int r[kPpRow];
+#pragma unroll
+    for (int h = 0; h < kPpRow; h += 4) {
+#pragma unroll
+      for (int q = h; q < h + 4; ++q) {
+        r[q] = kInf;
+        if (side) r[q] = lab[s + off[__ffs((int)side) - 1]];
+        side &= side - 1u;
+      }
+#pragma unroll
+      for (int q = h; q < h + 4; ++q)
+        if (r[q] != kInf) r[q] = ext[r[q]];
+#pragma unroll
+      for (int q = h; q < h + 4; ++q)
+        if (r[q] != kInf) r[q] = erank[r[q]];
+    }
+    cnt[i] = pp_store_row(r, rows + (long long)i * kPpRow);
   }
 }
 
 // Largest saddle of every extremum but the global one.
-__global__ void k_pp_largest(const int* __restrict__ rows, const int* __restrict__ cnt, int ns,
-                             int glob, int* __restrict__ largest) {
+__global__ void __launch_bounds__(256) k_pp_largest(const int* __restrict__ rows,
+                                                    const int* __restrict__ cnt, int ns, int glob,
+                                                    int* __restrict__ largest) {
   const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride)
-    for (int q = 0; q < cnt[i]; ++q) {
-      const int e = rows[(long long)i * kPpRow + q];
-      if (e != glob) atomicMin(largest + e, i);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
+    const int c = cnt[i];
+    const int* row = rows + (long long)i * kPpRow;
+    for (int h = 0; h < c; h += 4) {
+      const int4 e = *reinterpret_cast<const int4*>(row + h);
+      if (e.x != glob) atomicMin(largest + e.x, i);
+      if (h + 1 < c && e.y != glob) atomicMin(largest + e.y, i);
+      if (h + 2 < c && e.z != glob) atomicMin(largest + e.z, i);
+      if (h + 3 < c && e.w != glob) atomicMin(largest + e.w, i);
     }
+  }
 }
 
 // Pairing of the round; resets largest for the next round.  lmax keeps the
@@ -252,31 +258,48 @@ __global__ void k_pp_jump(int* __restrict__ ptr, int ne, int cap, int* err) {
   }
 }
 
-// Rows rewritten through the pointers, deduplicated, emptied at one entry.
-__global__ void k_pp_remap(int* __restrict__ rows, int* __restrict__ cnt, int ns,
-                           const int* __restrict__ ptr) {
+// Rows rewritten through the pointers, deduplicated, emptied at one entry.  (Rows
+// of up to four entries, nearly all, stay in four registers.)
+__global__ void __launch_bounds__(256) k_pp_remap(int* __restrict__ rows, int* __restrict__ cnt, int ns,
+                                                  const int* __restrict__ ptr) {
   const int stride = gridDim.x * blockDim.x;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
     const int c = cnt[i];
     if (c == 0) continue;
+    int* row = rows + (long long)i * kPpRow;
     int r[kPpRow];
-    int n = 0;
-    for (int q = 0; q < c; ++q) {
-      const int e = ptr[rows[(long long)i * kPpRow + q]];
-      int j = n;
-      bool dup = false;
-      for (int k = 0; k < n; ++k) dup |= r[k] == e;
-      if (dup) continue;
-      while (j > 0 && r[j - 1] > e) {
-        r[j] = r[j - 1];
-        --j;
-      }
-      r[j] = e;
-      ++n;
+#pragma unroll
+    for (int h = 0; h < kPpRow; h += 4) {
+      int4 e = make_int4(kInf, kInf, kInf, kInf);
+      if (h < c) e = *reinterpret_cast<const int4*>(row + h);
+      r[h] = h < c ? ptr[e.x] : kInf;
+      r[h + 1] = h + 1 < c ? ptr[e.y] : kInf;
+      r[h + 2] = h + 2 < c ? ptr[e.z] : kInf;
+      r[h + 3] = h + 3 < c ? ptr[e.w] : kInf;
     }
-    if (n == 1) n = 0;
-    for (int q = 0; q < n; ++q) rows[(long long)i * kPpRow + q] = r[q];
-    cnt[i] = n;
+    if (c <= 4) {
+      int n = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        bool again = r[q] == kInf;
+        int at = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (k < q) again |= r[k] == r[q];
+          // Distinct smaller entries: the first of each value counts.
+          bool first = r[k] < r[q];
+#pragma unroll
+          for (int j = 0; j < k; ++j) first &= r[j] != r[k];
+          at += first;
+        }
+        if (again) continue;
+        row[at] = r[q];
+        ++n;
+      }
+      cnt[i] = n < 2 ? 0 : n;
+    } else {
+      cnt[i] = pp_store_row(r, row);
+    }
   }
 }
 
