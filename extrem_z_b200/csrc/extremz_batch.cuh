@@ -1299,7 +1299,6 @@ class BatchEngine {
           }
         }
         if (!busy.empty()) {
-          const Sel bs = make_span(busy);
           // Steepest pointers: every tile in a job's first round, one block
           // per tile; in later rounds the tiles that changed, as k_apply
           // listed them, taken by a fixed grid (a launch of one block per tile
@@ -1329,7 +1328,20 @@ class BatchEngine {
             const Sel ls = make_span(later);
             launch(K_JUMP, k_jump2<T, true, true>, blocks(ls), 256, jobs, ls);
           }
-          launch(K_ROWS, k_saddle_pass<T>, blocks(bs), 256, jobs, bs);
+          // The first round of a correction runs right after a detection without
+          // mismatch; a census's may not.
+          std::vector<int> first, other;
+          for (int i : busy)
+            (slots_[i].manifold_rounds == 0 && !(slots_[i].p.flags & kFlagCensus) ? first : other)
+                .push_back(i);
+          if (!first.empty()) {
+            const Sel fs = make_span(first);
+            launch(K_ROWS, k_saddle_first<T>, blocks(fs), 256, jobs, fs);
+          }
+          if (!other.empty()) {
+            const Sel os = make_span(other);
+            launch(K_ROWS, k_saddle_pass<T>, blocks(os), 256, jobs, os);
+          }
           // Lockstep jobs: the fourteen steps in one block per job when the
           // job's previous round had short candidate lists (the counts of
           // that round are still in the host copy of its counters), else one
@@ -1654,6 +1666,7 @@ class BatchEngine {
     fl.add(J.tseen, jh.ntiles, 0);
     fl.add(J.tqueue, jh.ntiles, 0);
     fl.add(J.bdirty, jh.nb, 0);
+    fl.add(J.hcnt, jh.nb, 0);
     fl.add(J.rtouch2, words, 0);
     fl.add(J.rtouch1, words, 0);
     fl.add(J.vchg, words, ~0ull);

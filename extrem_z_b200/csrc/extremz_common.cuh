@@ -56,7 +56,9 @@ __host__ __device__ __forceinline__ int valid_mask(int bc);
 struct DeviceTables {
   const int8_t* lut;      // 24 800 entries, the reference's LUT.bin layout
   const int* key_offset;  // 64 entries: boundary code -> LUT offset, -1 unknown key
+  const unsigned* packed; // the interior entries, two bits each (0 for type 5), 16 to a word
 };
+constexpr int kTypeWords = (1 << kNumDirs) / 16;  // 4 KB
 
 // Boundary code of (x, y, z): bit 0 = x-1 invalid, 1 = x+1 invalid, 2 = y-1,
 // 3 = y+1, 4 = z-1, 5 = z+1.

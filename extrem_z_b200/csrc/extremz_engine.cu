@@ -47,8 +47,19 @@ cudaError_t& last_cuda_error() {
 struct DeviceLut {
   int8_t* lut = nullptr;
   int* key_offset = nullptr;
+  unsigned* packed = nullptr;
   bool ready = false;
 };
+
+// The interior entries of the table, two bits each (DeviceTables::packed).
+static std::vector<unsigned> pack_types(const HostTables& t) {
+  std::vector<unsigned> p(kTypeWords, 0u);
+  for (int set = 0; set < (1 << kNumDirs); ++set) {
+    const int type = t.lut[t.key_offset[0] + set];
+    if (type >= 1 && type <= 3) p[set >> 4] |= (unsigned)type << (2 * (set & 15));
+  }
+  return p;
+}
 
 static std::mutex g_lut_mu;
 static DeviceLut g_lut[64];
@@ -69,10 +80,14 @@ static int device_tables(DeviceTables* out) {
     EZ_CHECK(cudaMalloc(&d.key_offset, 64 * sizeof(int)));
     EZ_CHECK(cudaMemcpy(d.lut, host->lut, kLutSize, cudaMemcpyHostToDevice));
     EZ_CHECK(cudaMemcpy(d.key_offset, host->key_offset, 64 * sizeof(int), cudaMemcpyHostToDevice));
+    const std::vector<unsigned> packed = pack_types(*host);
+    EZ_CHECK(cudaMalloc(&d.packed, kTypeWords * sizeof(unsigned)));
+    EZ_CHECK(cudaMemcpy(d.packed, packed.data(), kTypeWords * sizeof(unsigned), cudaMemcpyHostToDevice));
     d.ready = true;
   }
   out->lut = d.lut;
   out->key_offset = d.key_offset;
+  out->packed = d.packed;
   return EXTREMZ_OK;
 }
 
@@ -495,6 +510,7 @@ static_assert(job_bytes_max(kNoAllocMaxVoxels) <= (long long)(kNoAllocScratchByt
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 static __device__ int8_t g_noalloc_lut[kLutSize];
 static __device__ int g_noalloc_key_offset[64];
+static __device__ __align__(16) unsigned g_noalloc_packed[kTypeWords];
 
 struct NoAllocDevice {
   bool ready = false;
@@ -515,14 +531,18 @@ static int noalloc_setup(int dev) {
   void* scratch = nullptr;
   void* lut = nullptr;
   void* keys = nullptr;
+  void* packed = nullptr;
   EZ_CHECK(cudaGetSymbolAddress(&scratch, g_noalloc_scratch));
   EZ_CHECK(cudaGetSymbolAddress(&lut, g_noalloc_lut));
   EZ_CHECK(cudaGetSymbolAddress(&keys, g_noalloc_key_offset));
+  EZ_CHECK(cudaGetSymbolAddress(&packed, g_noalloc_packed));
   const HostTables& t = host_tables();
   EZ_CHECK(cudaMemcpyToSymbol(g_noalloc_lut, t.lut, kLutSize));
   EZ_CHECK(cudaMemcpyToSymbol(g_noalloc_key_offset, t.key_offset, 64 * sizeof(int)));
+  EZ_CHECK(cudaMemcpyToSymbol(g_noalloc_packed, pack_types(t).data(), kTypeWords * sizeof(unsigned)));
   d.tables.lut = static_cast<const int8_t*>(lut);
   d.tables.key_offset = static_cast<const int*>(keys);
+  d.tables.packed = static_cast<const unsigned*>(packed);
   d.engine_store.base = static_cast<char*>(scratch);
   d.engine_store.cap = kNoAllocEngineBytes;
   d.engine_store.fixed = true;

@@ -379,6 +379,16 @@ __device__ __forceinline__ int type_from_masks(int lm, int um, int valid, int bc
   return __ldg(tb.lut + off + idx);
 }
 
+// Type of an interior vertex from its lower mask and the packed table in shared
+// memory.  (From global memory, the 32 lanes' bytes lie in up to 32 lines of the
+// 16 KB table: a third of the original field's direction pass.)
+__device__ __forceinline__ int interior_type(int lm, const unsigned* types) {
+  constexpr int kAll = (1 << kNumDirs) - 1;
+  const int um = kAll & ~lm;
+  const int code = (int)(types[um >> 4] >> (2 * (um & 15)) & 3u);
+  return um == 0 ? 4 : lm == 0 ? 0 : code ? code : 5;
+}
+
 __device__ __forceinline__ int mismatch_cats(int t, int o, int lm, int olm) {
   int cat = 0;
   if (t != o) {
@@ -832,8 +842,8 @@ __device__ __forceinline__ int follow(const int16_t* nxt, int p, int t, int* err
 // star, and steps checked and indexed by coordinates, 2.08 and 2.69 ms.
 template <class T, bool kDec>
 __device__ __noinline__ bool direction_tile(const Job<T>& J, Tile<T>& s, uint64_t* bar,
-                                            int16_t* hnext, int16_t* lnext, int bx, int by, int bz,
-                                            unsigned parity) {
+                                            int16_t* hnext, int16_t* lnext, const unsigned* types,
+                                            int bx, int by, int bz, unsigned parity) {
   const Dims g = J.dim;
   const int WH = g.W * g.H;
   const T* a = kDec ? J.g : J.f;
@@ -887,7 +897,8 @@ __device__ __noinline__ bool direction_tile(const Job<T>& J, Tile<T>& s, uint64_
       const int bc = interior ? 0 : boundary_code(x, y, z, g.W, g.H, g.D);
       const int valid = interior ? (1 << kNumDirs) - 1 : valid_mask(bc);
       const int m = lm[tz] & valid;
-      J.otype[v] = (int8_t)type_from_masks(m, valid & ~m, valid, bc, J.tb);
+      J.otype[v] = (int8_t)(bc == 0 ? interior_type(m, types)
+                                    : type_from_masks(m, valid & ~m, valid, bc, J.tb));
       J.olm[v] = (uint16_t)m;
     }
   }
@@ -928,7 +939,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 6) k_direction(const
   }
   if (kDec ? J.tma_g : J.tma_f)
     tile_issue<T>(s, &bar, kDec ? &J.map_g : &J.map_f, bx, by, bz, true);
-  if (!direction_tile<T, kDec>(J, s, &bar, hnext, lnext, bx, by, bz, 0)) return;
+  // The packed interior types (k_pack_types), while the tile is on its way.
+  __shared__ uint4 types[kDec ? 1 : kTypeWords / 4];
+  if (!kDec) types[threadIdx.x] = reinterpret_cast<const uint4*>(J.tb.packed)[threadIdx.x];
+  if (!direction_tile<T, kDec>(J, s, &bar, hnext, lnext, reinterpret_cast<const unsigned*>(types), bx,
+                               by, bz, 0))
+    return;
   if (kDec && threadIdx.x == 0) J.tdirty[tile] = 0;
 }
 
@@ -982,7 +998,7 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
         if (!(w1[tz] >> (r1[tz] & 31) & 1u)) atomicOr(J.rtouch1 + (r1[tz] >> 5), 1u << (r1[tz] & 31));
       }
     }
-    if (!direction_tile<T, true>(J, s, &bar, hnext, lnext, bx, by, bz, loads & 1u)) return;
+    if (!direction_tile<T, true>(J, s, &bar, hnext, lnext, nullptr, bx, by, bz, loads & 1u)) return;
     loads += tma;
     if (threadIdx.x == 0) {
       J.tdirty[t] = 0;
@@ -1347,6 +1363,37 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       from = nq << 2;
     }
   }
+  if constexpr (!kDec) {
+    // Four consecutive vertices per thread where the labels' arrays (a caller's
+    // own, in extremz_classify) allow 16-byte accesses.
+    if (((reinterpret_cast<uintptr_t>(ra) | reinterpret_cast<uintptr_t>(rb)) & 15) == 0) {
+      const int nq = N >> 2, qstride = nblk * blockDim.x;
+      for (int q = blk * blockDim.x + threadIdx.x; q < nq; q += qstride) {
+        const int4 A = reinterpret_cast<const int4*>(ra)[q], B = reinterpret_cast<const int4*>(rb)[q];
+        int u[8] = {A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w};
+        // As jump_one, for eight chains; the limit counts the end of a chain and
+        // the look at its root too.
+        bool open = true;
+        for (int it = 2;; ++it) {
+          open = false;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) open |= u[k] >= 0;
+          if (!open || it >= cap_j) break;
+          int w[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) w[k] = u[k] >= 0 ? (k < 4 ? a : b)[u[k]] : u[k];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) u[k] = w[k] == u[k] ? w[k] | kRootFlag : w[k];
+        }
+        if (open || cap_j < 2) atomicOr(err, kErrJump);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) u[k] &= ~kRootFlag;
+        reinterpret_cast<int4*>(ra)[q] = make_int4(u[0], u[1], u[2], u[3]);
+        reinterpret_cast<int4*>(rb)[q] = make_int4(u[4], u[5], u[6], u[7]);
+      }
+      from = nq << 2;
+    }
+  }
   const int stride = nblk * blockDim.x;
   for (int v = from + blk * blockDim.x + threadIdx.x; v < N; v += stride) jump_one(v);
 }
@@ -1359,37 +1406,42 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
 constexpr int kCpBlock = 1024;
 static_assert(kCpBlockJ == kCpBlock, "the jump's flags cover the CP-list blocks");
 
-__device__ __forceinline__ int cp_bits(int t) {
-  return ((t == 2 || t == 3) ? 1 : 0) | ((t == 1 || t == 3) ? 2 : 0) | (t == 4 ? 4 : 0) |
-         (t == 0 ? 8 : 0);
-}
-
 // One warp per 1024-id block, each lane 32 consecutive ids: the types come in
 // as two 16-byte loads per lane (one coalesced kilobyte per warp), where one
 // 1024-thread block per 1024 ids spent its time scheduling blocks.
 constexpr int kCpWarps = 8;  // warps (1024-id blocks) per CTA
 
-// The CP-list membership bits of the lane's 32 ids, one word per list.
+// The CP-list membership bits of the lane's 32 ids, one word per list: types 2
+// and 3, 1 and 3, 4, 0 (5 and -1 are in none).  Four types at a time: a type's
+// three low bits, one per byte, decide each list, and a multiplication gathers
+// the four answers.
 __device__ __forceinline__ void cp_lane_bits(const int8_t* __restrict__ otype, int N, int v0,
                                              unsigned bits[4]) {
-  int8_t t[32];
+  unsigned w[8];
   if (v0 + 32 <= N) {
-    const int4 q0 = *reinterpret_cast<const int4*>(otype + v0);
-    const int4 q1 = *reinterpret_cast<const int4*>(otype + v0 + 16);
-    const int w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-    for (int k = 0; k < 32; ++k) t[k] = (int8_t)(w[k >> 2] >> (8 * (k & 3)));
+    const uint4 q0 = *reinterpret_cast<const uint4*>(otype + v0);
+    const uint4 q1 = *reinterpret_cast<const uint4*>(otype + v0 + 16);
+    w[0] = q0.x; w[1] = q0.y; w[2] = q0.z; w[3] = q0.w;
+    w[4] = q1.x; w[5] = q1.y; w[6] = q1.z; w[7] = q1.w;
   } else {
 #pragma unroll
-    for (int k = 0; k < 32; ++k) t[k] = v0 + k < N ? otype[v0 + k] : (int8_t)-1;
+    for (int k = 0; k < 8; ++k) {
+      w[k] = 0u;
+      for (int j = 0; j < 4; ++j) {
+        const int v = v0 + 4 * k + j;
+        w[k] |= (v < N ? (unsigned)(uint8_t)otype[v] : 0xffu) << (8 * j);
+      }
+    }
   }
 #pragma unroll
   for (int l = 0; l < 4; ++l) bits[l] = 0u;
 #pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    const int b = cp_bits(t[k]);
+  for (int k = 0; k < 8; ++k) {
+    const unsigned b0 = w[k], b1 = w[k] >> 1, b2 = w[k] >> 2, one = 0x01010101u;
+    const unsigned in[4] = {b1 & ~b2 & one, b0 & ~b2 & one, b2 & ~b1 & ~b0 & one,
+                            ~(b2 | b1 | b0) & one};
 #pragma unroll
-    for (int l = 0; l < 4; ++l) bits[l] |= (unsigned)((b >> l) & 1) << k;
+    for (int l = 0; l < 4; ++l) bits[l] |= (in[l] * 0x01020408u >> 24 & 15u) << (4 * k);
   }
 }
 
@@ -1411,18 +1463,21 @@ __global__ void __launch_bounds__(32 * kCpWarps) k_cp_count(const int8_t* __rest
     int x, y, z;
     coords(v0, g, x, y, z);
     if (v0 + 32 <= g.N && x > 0 && x + 31 < g.W - 1 && y > 0 && y < g.H - 1 && z > 0 && z < g.D - 1) {
-      // Off the faces every vertex has 14 neighbours; the masks come in together.
-      uint4 q[4];
+      // Off the faces every vertex has 14 neighbours; the masks come in together,
+      // two to a word.
+      int low2 = 0;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) q[k] = reinterpret_cast<const uint4*>(olm + v0)[k];
+      for (int k = 0; k < 4; ++k) {
+        const uint4 q = reinterpret_cast<const uint4*>(olm + v0)[k];
+        const unsigned pair[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        const uint4& w = q[k >> 3];
-        const unsigned pair = (k & 6) == 0 ? w.x : (k & 6) == 2 ? w.y : (k & 6) == 4 ? w.z : w.w;
-        const int lower = __popc(k & 1 ? pair >> 16 : pair & 0xffffu);
-        e2 += (bits[0] >> k & 1u) ? kNumDirs - lower : 0;
-        e1 += (bits[1] >> k & 1u) ? lower : 0;
+        for (int j = 0; j < 4; ++j) {
+          const unsigned p2 = bits[0] >> (8 * k + 2 * j) & 3u, p1 = bits[1] >> (8 * k + 2 * j) & 3u;
+          low2 += __popc(pair[j] & ((p2 & 1u) * 0xffffu | (p2 >> 1) * 0xffff0000u));
+          e1 += __popc(pair[j] & ((p1 & 1u) * 0xffffu | (p1 >> 1) * 0xffff0000u));
+        }
       }
+      e2 = kNumDirs * __popc(bits[0]) - low2;
     } else {
       for (int k = 0; k < 32; ++k) {
         if (((bits[0] | bits[1]) >> k) & 1u) {
@@ -2407,6 +2462,52 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
     }
   }
   if (qn > 0) drain();
+}
+
+// The saddle pass of a correction's first round: every saddle, right after a
+// detection without mismatch, so the direction masks are the original field's
+// (known).  Without the later rounds' checks and queue it holds few registers,
+// and its gathers are bound by latency: 2-saddles (rows) and 1-saddles (seed
+// bits; rows too with join_rows) in two loops.
+template <class T>
+__global__ void __launch_bounds__(256, 5) k_saddle_first(const Job<T>* __restrict__ jobs,
+                                                         const __grid_constant__ Sel sel) {
+  __shared__ int off[kNumDirs];
+  int blk, nblk;
+  const Job<T>& J = span_job(jobs, sel, blk, nblk);
+  if (mf_skip(J.ctr)) return;
+  fill_offsets(off, J.dim);
+  const int stride = nblk * blockDim.x, t0 = blk * blockDim.x + threadIdx.x;
+  const int nw = (J.dim.N + 31) >> 5;
+  for (int w = t0; w < nw; w += stride) {
+    J.vchg[w] = 0u;
+    J.rtouch2[w] = 0u;
+    J.rtouch1[w] = 0u;
+    J.taken[w] = 0u;
+    J.taken1[w] = 0u;
+  }
+  __syncthreads();
+  const int chunk = J.pass_chunk;
+  auto side = [&](auto split) {
+    constexpr bool kSplit = decltype(split)::value;
+    const int ns = J.ctr[kSplit ? C_NS2 : C_NS1];
+    const int* __restrict__ sad = kSplit ? J.sad2 : J.sad1;
+    for (int base = t0 - (int)lane_id(); base < ns; base += stride) {  // uniform per warp
+      const int i = base + (int)lane_id();
+      bool has = false;
+      int s = 0;
+      if (i < ns) {
+        s = sad[i];
+        has = saddle_row<T, kSplit>(J, off, i, s, true);
+        (kSplit ? J.has2 : J.has1)[i] = (uint8_t)has;
+        if (has) atomicAdd(J.hcnt + (s >> 10) / chunk, 1);
+      }
+      const int slot = warp_append(J.ctr + (kSplit ? C_CAND : C_CANDJ), has, 0xffffffffu);
+      if (slot >= 0) (kSplit ? J.cand : J.cand_j)[slot] = s;
+    }
+  };
+  side(std::true_type{});
+  side(std::false_type{});
 }
 
 template <class T, bool kSplit>
