@@ -263,9 +263,10 @@ __device__ __forceinline__ const Job<T>& tile_job(const Job<T>* __restrict__ job
 // Lists the tiles whose halo tile contains vertex (x, y, z), those holding one
 // of its 26 neighbours or itself, unless they are listed already (or not yet
 // computed: every mark is set before a job's first round).  The marks of the (at
-// most eight) tiles are read together.
+// most eight) tiles are read together.  All lanes of a warp call it, those with
+// `any`, to list theirs with one atomic per warp.
 __device__ __forceinline__ void mark_tiles(int* tdirty, int* list, int* count, const Dims& g, int x,
-                                           int y, int z) {
+                                           int y, int z, bool any) {
   const int ntx = (g.W + TX - 1) / TX, nty = (g.H + TY - 1) / TY;
   const int x0 = max(x - 1, 0) / TX, x1 = min(x + 1, g.W - 1) / TX;
   const int y0 = max(y - 1, 0) / TY, y1 = min(y + 1, g.H - 1) / TY;
@@ -274,13 +275,20 @@ __device__ __forceinline__ void mark_tiles(int* tdirty, int* list, int* count, c
   unsigned need = 0u;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    const bool own = (!(k & 1) || x1 != x0) && (!(k & 2) || y1 != y0) && (!(k & 4) || z1 != z0);
+    const bool own = any && (!(k & 1) || x1 != x0) && (!(k & 2) || y1 != y0) && (!(k & 4) || z1 != z0);
     t[k] = ((k & 4 ? z1 : z0) * nty + (k & 2 ? y1 : y0)) * ntx + (k & 1 ? x1 : x0);
     if (own && tdirty[t[k]] == 0) need |= 1u << k;
   }
+  if (!__any_sync(0xffffffffu, need != 0u)) return;
+  unsigned mine = 0u;
 #pragma unroll
   for (int k = 0; k < 8; ++k)
-    if ((need >> k & 1u) && atomicExch(tdirty + t[k], 1) == 0) list[atomicAdd(count, 1)] = t[k];
+    if ((need >> k & 1u) && atomicExch(tdirty + t[k], 1) == 0) mine |= 1u << k;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int slot = warp_append(count, mine >> k & 1u, 0xffffffffu);
+    if (slot >= 0) list[slot] = t[k];
+  }
 }
 
 // Halo tile: TMA box (one bulk tensor copy, zero fill outside the grid) when
@@ -1900,11 +1908,12 @@ __device__ __forceinline__ void propose(const Job<T>& J, int i, T d) {
   }
 }
 
-// Several proposals of one thread: the atomics go out together, then the
-// vertices that left the sentinel are listed.  (One after the other, each waits
-// for the last one's round trip to L2.)
+// Up to kN proposals of every lane of a warp (bits of `which`): the atomics go out
+// together, then the vertices that left the sentinel are listed with one atomic
+// per warp.  (With one per thread, half a million of them queued on the same
+// counter: 235 us for the first proposals of the 256^3 benchmark field.)
 template <class T, int kN>
-__device__ __forceinline__ void propose_all(const Job<T>& J, const int* at, const T* d, unsigned which) {
+__device__ __forceinline__ void propose_warp(const Job<T>& J, const int* at, const T* d, unsigned which) {
   using K = typename KeyOf<T>::K;
   K old[kN];
 #pragma unroll
@@ -1914,8 +1923,16 @@ __device__ __forceinline__ void propose_all(const Job<T>& J, const int* at, cons
 #pragma unroll
   for (int k = 0; k < kN; ++k)
     if ((which >> k & 1u) && old[k] == J.sentinel_key && KeyOf<T>::enc(d[k]) > old[k]) fresh |= 1u << k;
-  if (!fresh) return;
-  int slot = atomicAdd(J.ctr + C_TOUCHED, __popc(fresh));
+  const int n = __popc(fresh);
+  int incl = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane_id() >= (unsigned)o) incl += y;
+  }
+  int slot = 0;
+  if (lane_id() == 31 && incl) slot = atomicAdd(J.ctr + C_TOUCHED, incl);
+  slot = __shfl_sync(0xffffffffu, slot, 31) + incl - n;
 #pragma unroll
   for (int k = 0; k < kN; ++k)
     if (fresh >> k & 1u) J.touched[slot++] = at[k];
@@ -1930,8 +1947,9 @@ __global__ void __launch_bounds__(256) k_propose_cp(const Job<T>* __restrict__ j
   const int stride = nblk * blockDim.x;
   const Dims g = J.dim;
   const int WH = g.W * g.H;
-  for (int e = blk * blockDim.x + threadIdx.x; e < n; e += stride) {
-    const int ent = J.mm[e];
+  for (int base = blk * blockDim.x; base < n; base += stride) {  // uniform per warp
+    const int e = base + threadIdx.x;
+    const int ent = e < n ? J.mm[e] : 0;
     const int v = ent & ((1 << kCatShift) - 1);
     const int cat = (unsigned)ent >> kCatShift;
     int x, y, z;
@@ -1939,7 +1957,7 @@ __global__ void __launch_bounds__(256) k_propose_cp(const Job<T>* __restrict__ j
     // Neighbours in direction order (the reference's scan order), visited
     // through static indices so that the values stay in registers and their
     // loads go out together.
-    const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
+    const int valid = e < n ? valid_mask(boundary_code(x, y, z, g.W, g.H, g.D)) : 0;
     const int ot = J.otype[v];
     const T gv = J.g[v];
     const bool need_g = (cat & kCatSaddle) || ((cat & kCatMax) && ot == 4);
@@ -1947,6 +1965,10 @@ __global__ void __launch_bounds__(256) k_propose_cp(const Job<T>* __restrict__ j
 #pragma unroll
     for (int d = 0; d < kNumDirs; ++d)
       gn[d] = (need_g && (valid >> d & 1)) ? J.g[v + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH] : T(0);
+    // The proposals of c_loop(1), slot 0, and c_loop(0), slot 1.
+    int at[4] = {v, v, v, v};
+    T dl[4];
+    unsigned which = 0u;
     if (cat & kCatMin) {  // c_loop(1) (:2965-3039)
       if (ot != 0) {
         T fn[kNumDirs];
@@ -1961,13 +1983,36 @@ __global__ void __launch_bounds__(256) k_propose_cp(const Job<T>* __restrict__ j
           if ((valid >> d & 1) && below(fn[d], r, sval, S)) { S = r; sval = fn[d]; }
         }
         const T gs = J.g[S];
-        const T d = J.edit_type == 1 ? ((sval - J.bound) + gs) / T(2) - gs : -J.bound / T(J.q);
-        if (!(gv > gs || (gv == gs && v > S))) propose(J, S, d);
+        dl[0] = J.edit_type == 1 ? ((sval - J.bound) + gs) / T(2) - gs : -J.bound / T(J.q);
+        if (!(gv > gs || (gv == gs && v > S))) {
+          at[0] = S;
+          which |= 1u;
+        }
       } else {
-        propose(J, v, step_delta(J, v));
+        dl[0] = step_delta(J, v);
+        which |= 1u;
       }
     }
-    if (cat & kCatSaddle) {  // c_loop(2) -> fix_saddle_local (:2804-2884)
+    if (cat & kCatMax) {  // c_loop(0) (:2890-2963)
+      if (ot != 4) {
+        which |= 2u;
+      } else {
+        T lval = gv;
+#pragma unroll
+        for (int d = 0; d < kNumDirs; ++d) {
+          const int r = v + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
+          if ((valid >> d & 1) && above(gn[d], r, lval, at[1])) { at[1] = r; lval = gn[d]; }
+        }
+        if (at[1] != v) which |= 2u;
+      }
+      if (which & 2u) dl[1] = step_delta(J, at[1]);
+    }
+    propose_warp<T, 2>(J, at, dl, which);
+    // c_loop(2) -> fix_saddle_local (:2804-2884): the original's lower neighbours
+    // that are not lower now, four at a time, and the vertex itself when it has
+    // lower neighbours it should not have.
+    unsigned rest = 0u;
+    if (cat & kCatSaddle) {
       int dm = 0;
 #pragma unroll
       for (int d = 0; d < kNumDirs; ++d) {
@@ -1975,41 +2020,23 @@ __global__ void __launch_bounds__(256) k_propose_cp(const Job<T>* __restrict__ j
         if ((valid >> d & 1) && (gn[d] < gv || (gn[d] == gv && r < v))) dm |= 1 << d;
       }
       const int om = J.olm[v];
-      // The original's lower neighbours that are not lower now, four at a time,
-      // and the vertex itself when it has lower neighbours it should not have.
-      unsigned rest = (unsigned)(valid & om & ~dm) | ((dm & ~om) ? 1u << kNumDirs : 0u);
-      while (rest) {
-        int at[4];
-        T dl[4];
-        unsigned which = 0u;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          at[q] = v;
-          if (rest) {
-            const int d = __ffs((int)rest) - 1;
-            if (d < kNumDirs) at[q] = v + ddx(d) + ddy(d) * g.W + ddz(d) * WH;
-            which |= 1u << q;
-          }
-          rest &= rest - 1u;
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dl[q] = (which >> q & 1u) ? step_delta(J, at[q]) : T(0);
-        propose_all<T, 4>(J, at, dl, which);
-      }
+      rest = (unsigned)(valid & om & ~dm) | ((dm & ~om) ? 1u << kNumDirs : 0u);
     }
-    if (cat & kCatMax) {  // c_loop(0) (:2890-2963)
-      if (ot != 4) {
-        propose(J, v, step_delta(J, v));
-      } else {
-        int L = v;
-        T lval = gv;
+    while (__any_sync(0xffffffffu, rest != 0u)) {
+      which = 0u;
 #pragma unroll
-        for (int d = 0; d < kNumDirs; ++d) {
-          const int r = v + dir_x(d) + dir_y(d) * g.W + dir_z(d) * WH;
-          if ((valid >> d & 1) && above(gn[d], r, lval, L)) { L = r; lval = gn[d]; }
+      for (int q = 0; q < 4; ++q) {
+        at[q] = v;
+        if (rest) {
+          const int d = __ffs((int)rest) - 1;
+          if (d < kNumDirs) at[q] = v + ddx(d) + ddy(d) * g.W + ddz(d) * WH;
+          which |= 1u << q;
         }
-        if (L != v) propose(J, L, step_delta(J, L));
+        rest &= rest - 1u;
       }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) dl[q] = (which >> q & 1u) ? step_delta(J, at[q]) : T(0);
+      propose_warp<T, 4>(J, at, dl, which);
     }
   }
 }
@@ -2027,8 +2054,8 @@ __global__ void __launch_bounds__(256) k_apply(const Job<T>* __restrict__ jobs, 
   const int stride = nblk * blockDim.x;
   for (int base = blk * blockDim.x; base < n; base += stride) {  // uniform per warp
     const int e = base + threadIdx.x;
-    int v = 0;
-    bool fresh = false;  // changed, and not in the dirty list yet
+    int v = 0, x = 0, y = 0, z = 0;
+    bool fresh = false, changed = false;  // changed, and not in the dirty list yet
     if (e < n) {
       v = J.touched[e];
       const T d = KeyOf<T>::dec(J.delta[v]);
@@ -2060,11 +2087,11 @@ __global__ void __launch_bounds__(256) k_apply(const Job<T>* __restrict__ jobs, 
         atomicOr(J.wchg2 + w, bit);
         if (J.join_rows) atomicOr(J.wchg1 + w, bit);
         if (J.edited) atomicOr(J.edited + w, bit);
-        int x, y, z;
         coords(v, J.dim, x, y, z);
-        mark_tiles(J.tdirty, J.cand_next, J.ctr + C_TLIST, J.dim, x, y, z);
+        changed = true;
       }
     }
+    mark_tiles(J.tdirty, J.cand_next, J.ctr + C_TLIST, J.dim, x, y, z, changed);
     const int slot = warp_append(J.ctr + C_DIRTY, fresh, 0xffffffffu);
     if (slot >= 0) dirty[slot] = v;
   }
@@ -2182,13 +2209,13 @@ __device__ __noinline__ unsigned side_of(const Job<T>& J, int s) {
 // lower star matched): the direction mask is read instead of 14 neighbour
 // values.  Two thirds of the rounds, the first one (every saddle) among them,
 // run right after such a detection (with the 1-saddles' shortcut below: 7.0 ->
-// 5.7 ms per 512^3 correction).  The loop goes over the set bits four at a
-// time, so that a group's gathers (labels and mismatch bits; the labels'
+// 5.7 ms per 512^3 correction).  The loop goes over the set bits kWide at
+// a time, so that a group's gathers (labels and mismatch bits; the labels'
 // values) are in flight together.
 //
 // A 1-saddle's slots are read only with join_rows; else only its seed bit is
 // needed: the mismatch bytes of its neighbours.
-template <class T, bool kSplit>
+template <class T, bool kSplit, int kWide = 4>
 __device__ __forceinline__ bool saddle_row(const Job<T>& J, const int* __restrict__ off, int i,
                                            int s, bool known) {
   const T* __restrict__ gv = J.g;
@@ -2205,7 +2232,7 @@ __device__ __forceinline__ bool saddle_row(const Job<T>& J, const int* __restric
   if (!kSplit && !J.join_rows) {
     while (side) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < kWide; ++q) {
         if (side) mb |= __ldg(mis + s + off[__ffs((int)side) - 1]);
         side &= side - 1u;
       }
@@ -2215,10 +2242,10 @@ __device__ __forceinline__ bool saddle_row(const Job<T>& J, const int* __restric
   T fv = T(0), lv = T(0);
   int cnt = 0, fm = -1, lm = -1;
   while (side) {
-    int ml[4];
-    T val[4];
+    int ml[kWide];
+    T val[kWide];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kWide; ++q) {
       ml[q] = -1;
       if (side) {
         const int r = s + off[__ffs((int)side) - 1];
@@ -2228,9 +2255,9 @@ __device__ __forceinline__ bool saddle_row(const Job<T>& J, const int* __restric
       side &= side - 1u;
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) val[q] = ml[q] >= 0 ? __ldg(gv + ml[q]) : T(0);
+    for (int q = 0; q < kWide; ++q) val[q] = ml[q] >= 0 ? __ldg(gv + ml[q]) : T(0);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kWide; ++q) {
       const int m = ml[q];
       const T v = val[q];
       if (m >= 0 && (!kSplit || tabs(T(v - sv)) >= J.thr)) {
@@ -2470,7 +2497,7 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
 // and its gathers are bound by latency: 2-saddles (rows) and 1-saddles (seed
 // bits; rows too with join_rows) in two loops.
 template <class T>
-__global__ void __launch_bounds__(256, 5) k_saddle_first(const Job<T>* __restrict__ jobs,
+__global__ void __launch_bounds__(256, 4) k_saddle_first(const Job<T>* __restrict__ jobs,
                                                          const __grid_constant__ Sel sel) {
   __shared__ int off[kNumDirs];
   int blk, nblk;
@@ -2498,7 +2525,7 @@ __global__ void __launch_bounds__(256, 5) k_saddle_first(const Job<T>* __restric
       int s = 0;
       if (i < ns) {
         s = sad[i];
-        has = saddle_row<T, kSplit>(J, off, i, s, true);
+        has = saddle_row<T, kSplit, 8>(J, off, i, s, true);
         (kSplit ? J.has2 : J.has1)[i] = (uint8_t)has;
         if (has) atomicAdd(J.hcnt + (s >> 10) / chunk, 1);
       }
