@@ -38,7 +38,7 @@ CLASSES = [
 HALOS = ("tma", "plain")
 BLOCKS_PER_SM = (4, 8, 16)
 PASS_CHUNKS = (1, 4, 16)
-DEFAULT = {"halo": "tma", "blocks_per_sm": 8, "pass_chunk": 4}
+DEFAULT = {"halo": "tma", "blocks_per_sm": 4, "pass_chunk": 4}
 
 _cache = None
 

@@ -202,7 +202,7 @@ struct JobHost {
   int32_t* trace = nullptr;
   int trace_cap = 0, trace_len = 0;
   std::vector<int> pending;  // trace phases to emit once the tick's counters are back
-  int blocks_per_sm = 8;      // grid-stride kernels' blocks per SM (tuning knob)
+  int blocks_per_sm = 4;      // grid-stride kernels' blocks per SM (tuning knob)
   long long applied_tick = -1;  // last tick that issued edits for this job
   long long tag = 0;
 
@@ -341,7 +341,7 @@ class BatchEngine {
     J.pass_chunk = p.tune_pass_chunk > 0 ? p.tune_pass_chunk : 4;
     J.wn_lockstep = (p.flags & EXTREMZ_FLAG_WN_ASCENDING) == 0;
     J.join_rows = p.preserve_join || (p.flags & kFlagCensus);
-    jh.blocks_per_sm = p.tune_blocks_per_sm > 0 ? p.tune_blocks_per_sm : 8;
+    jh.blocks_per_sm = p.tune_blocks_per_sm > 0 ? p.tune_blocks_per_sm : 4;
     J.tb = tb_;
     J.ctr = ctr_dev_ + (size_t)slot * C_COUNT;
     const int N = J.dim.N;
@@ -1342,18 +1342,20 @@ class BatchEngine {
             const Sel os = make_span(other);
             launch(K_ROWS, k_saddle_pass<T>, blocks(os), 256, jobs, os);
           }
-          // Lockstep jobs: the fourteen steps in one block per job when the
+          // Lockstep jobs: the fourteen steps in one cluster per job when the
           // job's previous round had short candidate lists (the counts of
-          // that round are still in the host copy of its counters), else one
-          // grid launch per step.  Either is exact for any list length.
+          // that round are still in the host copy of its counters), or before
+          // its first round when it has few saddles, else one grid launch per
+          // step.  Either is exact for any list length.
           std::vector<int> vote, lock_small, lock_large;
           for (int i : busy) {
             if (!slots_[i].J.wn_lockstep) {
               vote.push_back(i);
               continue;
             }
-            const bool small = slots_[i].manifold_rounds > 0 &&
-                               h(i, C_CAND) + h(i, C_CANDJ) <= kWnBlockMax;
+            const bool small = slots_[i].manifold_rounds > 0
+                                   ? h(i, C_CAND) + h(i, C_CANDJ) <= kWnClusterMax
+                                   : h(i, C_NS2) + h(i, C_NS1) <= kWnClusterFirst;
             (small ? lock_small : lock_large).push_back(i);
           }
           if (!vote.empty()) {

@@ -2360,19 +2360,26 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
   const long long W = J.dim.W, WH = W * J.dim.H, N = J.dim.N;
   // Later rounds first ask the jump's per-block flags whether any changed-input
   // byte is set where a chunk's saddles could see one: the 3 x 3 row windows of
-  // the planes and rows next to the chunk, one id wider on each side.  A thread
-  // asks for one of the block's next 256 chunks, so that a light round passes
-  // over the clean ones without a barrier each.
-  auto sees_change = [&](int c) {
+  // the planes and rows next to the chunk, one id wider on each side.  The
+  // block's next 256 chunks are asked for together, a thread per chunk and
+  // window with its flags' loads in flight at once, so that a light round passes
+  // over the clean ones without a barrier each (one thread per chunk took nine
+  // windows' loads in turn, 8 us before a small field's pass began).
+  const int stamp = mf_stamp(J.ctr);
+  auto window_changed = [&](int c, int t) {
     const long long first = (long long)c * chunk * kCpBlock;
     const long long end = min((long long)(c + 1) * chunk, (long long)nb) * kCpBlock;
-    const int stamp = mf_stamp(J.ctr);
+    const long long shift = (long long)(t / 3 - 1) * WH + (long long)(t % 3 - 1) * W;
+    const long long lo = max(0ll, first + shift - 1), hi = min(N - 1, end + shift);
+    if (lo > hi) return false;
+    const int b0 = (int)(lo >> 10), b1 = (int)(hi >> 10);
     bool seen = false;
-    for (int t = 0; t < 9; ++t) {
-      const long long shift = (long long)(t / 3 - 1) * WH + (long long)(t % 3 - 1) * W;
-      const long long lo = max(0ll, first + shift - 1), hi = min(N - 1, end + shift);
-      for (long long b = lo >> 10; b <= (hi >> 10) && lo <= hi; ++b)
-        seen |= J.bdirty[b] == stamp;
+    for (int b = b0; b <= b1; b += 6) {
+      int f[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) f[k] = J.bdirty[min(b + k, b1)];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) seen |= f[k] == stamp;
     }
     return seen;
   };
@@ -2413,11 +2420,13 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
   const int mine = blk < nchunk ? (nchunk - blk + nblk - 1) / nblk : 0;  // chunks of the block
   for (int kc = 0; kc < mine; ++kc) {
     if (!all_new && kc % 256 == 0) {  // what the next 256 chunks ask for
-      const int k = kc + (int)threadIdx.x, c = blk + k * nblk;
-      uint8_t st = kChunkClean;
-      if (k < mine) st = sees_change(c) ? kChunkChanged : J.hcnt[c] ? kChunkSeeds : kChunkClean;
+      const int some = min(256, mine - kc);
       __syncthreads();
-      state[threadIdx.x] = st;
+      if ((int)threadIdx.x < some)
+        state[threadIdx.x] = J.hcnt[blk + (kc + (int)threadIdx.x) * nblk] ? kChunkSeeds : kChunkClean;
+      __syncthreads();
+      for (int p = threadIdx.x; p < 9 * some; p += blockDim.x)
+        if (window_changed(blk + (kc + p / 9) * nblk, p % 9)) state[p / 9] = kChunkChanged;
       __syncthreads();
     }
     const uint8_t st = all_new ? kChunkChanged : state[kc % 256];
@@ -2775,6 +2784,10 @@ __device__ __forceinline__ unsigned wn_mask(const Job<T>& J, bool split, int s) 
 // dependent loads per step took 14-20 us, and a list that outgrew the block
 // (several thousand saddles) 500 us.
 constexpr int kWnCluster = 8, kWnHeld = 2;
+// Lists that go to the cluster: what its threads hold in registers, and, before a
+// job's first round, saddles of which a tenth or so will be candidates (fourteen
+// launches are 35-70 us on a 64^3 field, the cluster's steps about 25).
+constexpr int kWnClusterMax = kWnHeld * kWnCluster * 1024, kWnClusterFirst = 1 << 17;
 template <class T>
 __global__ void __cluster_dims__(kWnCluster, 1, 1) __launch_bounds__(1024)
     k_wn_steps_block(const Job<T>* __restrict__ jobs, const __grid_constant__ Sel sel) {
@@ -3266,24 +3279,24 @@ __global__ void __launch_bounds__(256, 4) k_join_keys(const Job<T>* __restrict__
     int lb[16], mp[16];
     int cnt = 0, m0 = -1, m1 = -1, m2 = -1, m3 = -1;
 #pragma unroll
-    for (int h = 0; h < 16; h += 4) {
+    for (int h = 0; h < 16; h += 8) {
 #pragma unroll
-      for (int q = h; q < h + 4; ++q) lb[q] = mp[q] = -1;
+      for (int q = h; q < h + 8; ++q) lb[q] = mp[q] = -1;
       if (h >= pmax) continue;  // uniform per warp
 #pragma unroll
-      for (int q = h; q < h + 4; ++q) {
+      for (int q = h; q < h + 8; ++q) {
         if (rest) lb[q] = lab[s + off[__ffs((int)rest) - 1]];
         rest &= rest - 1u;
       }
 #pragma unroll
-      for (int q = h; q < h + 4; ++q) {
+      for (int q = h; q < h + 8; ++q) {
         bool fresh = lb[q] >= 0;
 #pragma unroll
         for (int e = 0; e < q; ++e) fresh &= lb[e] != lb[q];
         if (fresh) mp[q] = ext[lb[q]];
       }
 #pragma unroll
-      for (int q = h; q < h + 4; ++q) {
+      for (int q = h; q < h + 8; ++q) {
         if (mp[q] < 0) continue;
         m0 = cnt == 0 ? mp[q] : m0;
         m1 = cnt == 1 ? mp[q] : m1;
@@ -3292,11 +3305,11 @@ __global__ void __launch_bounds__(256, 4) k_join_keys(const Job<T>* __restrict__
         if (cnt >= 4) J.orow1[(long long)i * kRowStride + cnt] = mp[q];
         ++cnt;
       }
-      KK cur[4];
+      KK cur[8];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) cur[q] = mp[h + q] >= 0 ? J.ext_key[mp[h + q]] : KK(0);
+      for (int q = 0; q < 8; ++q) cur[q] = mp[h + q] >= 0 ? J.ext_key[mp[h + q]] : KK(0);
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+      for (int q = 0; q < 8; ++q)
         if (mp[h + q] >= 0 && key < cur[q]) atomicMin(J.ext_key + mp[h + q], key);
     }
     if (act) {

@@ -75,7 +75,7 @@ typedef struct {
                           returns EXTREMZ_DEVICE_TIMEOUT. */
   /* Launch-shape knobs, picked per dtype and size class by the project's
    * autotuner (extrem_z_b200/autotune.py); results do not depend on them.
-   * 0 = defaults (8 and 4). */
+   * 0 = defaults (4 and 4). */
   int tune_blocks_per_sm; /* blocks per SM of the grid-stride kernels, 1..32 */
   int tune_pass_chunk;    /* 1024-id blocks per saddle-pass work item, 1..64 */
   int reserved[2];
