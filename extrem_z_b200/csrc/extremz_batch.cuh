@@ -68,6 +68,19 @@ enum Pc : int {
   PC_COUNT = PC_DONE
 };
 
+// The branch of a phase.  A job that passes through several phases in one tick
+// stays in one branch: setup to detection, r_loops to the manifold round,
+// saddle_loops to the join variants, the third block to its detection.
+constexpr int kBranches = 6;
+constexpr int branch_of(int pc) {
+  return pc <= PC_CL_DETECT                       ? 0
+         : pc == PC_CL_ROUND                      ? 1
+         : pc == PC_RLOOPS || pc == PC_MANIFOLD   ? 2
+         : pc == PC_SLOOPS                        ? 3
+         : pc <= PC_PRE_END || pc == PC_FINAL_JOIN ? 4
+                                                  : 5;
+}
+
 template <class T>
 __global__ void k_checksum(const T* __restrict__ a, int N, unsigned long long* out) {
   unsigned long long acc = 0;
@@ -767,8 +780,10 @@ class BatchEngine {
             EZ_CHECK(cudaStreamWaitEvent(st_, slots_[i].input_ready, 0));
             slots_[i].input_ready = nullptr;
           }
+      branch_ = branch_of(ph);
       rc = run_phase(ph, sel);
     }
+    branch_ = -1;
     // A tick that launched nothing (a manifold round over an unchanged field, a
     // re-read of the counters) leaves the host's copy as it is.
     launched_ = rc == EXTREMZ_OK && launches_ != launches0;
@@ -889,7 +904,16 @@ class BatchEngine {
   // Tick graphs (see tick_issue).
   bool graphs_on_ = true, recording_ = false, capturing_ = false;
   std::string sig_;
-  std::vector<std::function<void(cudaStream_t)>> pending_;
+  // A recorded launch and its branch: the phases of a tick work on different
+  // jobs, so those of different branches run side by side (kBranchOf), each
+  // branch on a stream of its own between a fork and a join; -1 comes after the
+  // join.
+  struct Launch {
+    int branch;
+    std::function<void(cudaStream_t)> go;
+  };
+  std::vector<Launch> pending_;
+  int branch_ = 0;
   // Timed launches of the tick being recorded: class, and the event pair the
   // launch records around itself (filled in just before the launches run).
   std::vector<Rec> pending_timed_;
@@ -909,6 +933,9 @@ class BatchEngine {
   // repeat once or twice, where a capture would not pay for itself.
   static constexpr int kCaptureAt = 3;
   cudaStream_t cap_ = nullptr;  // capture stream
+  cudaStream_t side_[kBranches] = {};
+  cudaEvent_t fork_ = nullptr, join_[kBranches] = {};
+  bool branches_ok_ = false;
   cudaMemPool_t pool_mem_ = nullptr;
   bool ready_ = false, borrowed_ = false, issued_ = false, launched_ = false;
   long long tick_id_ = 0;
@@ -994,20 +1021,21 @@ class BatchEngine {
       sig_append(reinterpret_cast<const void*>(kern));
       sig_append(grid);
       sig_append(block);
+      sig_append(branch_);
       (sig_append(args), ...);
       if (timed) {
         const size_t k = pending_timed_.size();
         pending_timed_.push_back({cls, nullptr, nullptr, false});
-        pending_.push_back([=](cudaStream_t s) {
+        pending_.push_back({branch_, [=](cudaStream_t s) {
           // In a capture the events become event-record nodes of the graph.
           const Rec& r = pending_timed_[k];
           const unsigned fl = capturing_ ? cudaEventRecordExternal : cudaEventRecordDefault;
           if (r.a) cudaEventRecordWithFlags(r.a, s, fl);
           kern<<<grid, block, 0, s>>>(args...);
           if (r.b) cudaEventRecordWithFlags(r.b, s, fl);
-        });
+        }});
       } else {
-        pending_.push_back([=](cudaStream_t s) { kern<<<grid, block, 0, s>>>(args...); });
+        pending_.push_back({branch_, [=](cudaStream_t s) { kern<<<grid, block, 0, s>>>(args...); }});
       }
       ++launches_;
       return;
@@ -1035,9 +1063,55 @@ class BatchEngine {
     }
   }
 
+  // The recorded launches on stream `main`: its branches side by side when there
+  // are several (fork), else in order.
+  void run_pending(cudaStream_t main, bool fork) {
+    int used = 0, first = -1;
+    for (const Launch& l : pending_)
+      if (l.branch >= 0 && !(used >> l.branch & 1)) {
+        used |= 1 << l.branch;
+        if (first < 0) first = l.branch;
+      }
+    cudaStream_t on[kBranches];
+    for (int b = 0; b < kBranches; ++b) on[b] = main;
+    const int rest = used & ~(1 << std::max(first, 0));
+    fork = fork && rest && ensure_branches() && cudaEventRecord(fork_, main) == cudaSuccess;
+    if (fork)
+      for (int b = 0; b < kBranches; ++b)
+        if (rest >> b & 1) {
+          on[b] = side_[b];
+          cudaStreamWaitEvent(side_[b], fork_, 0);
+        }
+    for (const Launch& l : pending_)
+      if (l.branch >= 0) l.go(on[l.branch]);
+    if (fork)
+      for (int b = 0; b < kBranches; ++b)
+        if (rest >> b & 1) {
+          cudaEventRecord(join_[b], side_[b]);
+          cudaStreamWaitEvent(main, join_[b], 0);
+        }
+    for (const Launch& l : pending_)
+      if (l.branch < 0) l.go(main);
+  }
+
+  // The branches' streams (of the engine stream's priority) and events, made
+  // when a tick first has two branches.
+  bool ensure_branches() {
+    if (fork_) return branches_ok_;
+    int prio = 0;
+    branches_ok_ = cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming) == cudaSuccess &&
+                   cudaStreamGetPriority(st_, &prio) == cudaSuccess;
+    for (int b = 0; b < kBranches && branches_ok_; ++b)
+      branches_ok_ =
+          cudaStreamCreateWithPriority(&side_[b], cudaStreamNonBlocking, prio) == cudaSuccess &&
+          cudaEventCreateWithFlags(&join_[b], cudaEventDisableTiming) == cudaSuccess;
+    if (!branches_ok_) cudaGetLastError();
+    return branches_ok_;
+  }
+
   void run_direct(bool timing = true) {
     if (timing) arm_timed();
-    for (auto& go : pending_) go(st_);
+    run_pending(st_, timing && pending_timed_.empty());
     pending_.clear();
     for (const Rec& r : pending_timed_)
       if (r.a) recs_.push_back(r);
@@ -1062,6 +1136,14 @@ class BatchEngine {
     seen_.clear();
     if (cap_) cudaStreamDestroy(cap_);
     cap_ = nullptr;
+    for (int b = 0; b < kBranches; ++b) {
+      if (side_[b]) cudaStreamDestroy(side_[b]);
+      if (join_[b]) cudaEventDestroy(join_[b]);
+      side_[b] = nullptr;
+      join_[b] = nullptr;
+    }
+    if (fork_) cudaEventDestroy(fork_);
+    fork_ = nullptr;
   }
 
   // Launches the recorded tick: replays its graph, captures it on the third
@@ -1126,7 +1208,7 @@ class BatchEngine {
     }
     arm_timed();
     capturing_ = true;
-    for (auto& go : pending_) go(cap_);
+    run_pending(cap_, pending_timed_.empty());
     capturing_ = false;
     const cudaError_t ec = cudaStreamEndCapture(cap_, &g);
     if (ec != cudaSuccess || !g || cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) {
