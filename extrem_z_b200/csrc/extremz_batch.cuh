@@ -128,7 +128,7 @@ constexpr long long job_bytes_voxels(long long n, long long ksz) {
   return arr_bytes(n, 1) + arr_bytes(n, 2)                          // otype, olm
          + 5 * arr_bytes(n, 4)                                      // ds, as, dds, das, ext
          + arr_bytes(n, ksz) + 3 * arr_bytes(n, 4)                  // delta, counter, touched, mm
-         + arr_bytes(n, 4) + arr_bytes(n, 1) + 2 * arr_bytes(n, 4)  // mm_next, mstat, dirty lists
+         + 3 * arr_bytes(n, 4)                                      // mm_next, dirty lists
          + arr_bytes(n, 8)                                          // claim
          + 4 * arr_bytes(n, 4)                                      // cand(_next), flagged(1)
          + arr_bytes(n, 4) + arr_bytes(n, 1)                        // cand_j, mis
@@ -414,7 +414,6 @@ class BatchEngine {
       J.touched = A.take<int>(N);
       J.mm = A.take<int>(N);
       J.mm_next = A.take<int>(N);
-      J.mstat = A.take<uint8_t>(N);
       J.dirty = A.take<int>(N);
       J.dirty1 = A.take<int>(N);
       J.claim = A.take<unsigned long long>(N);

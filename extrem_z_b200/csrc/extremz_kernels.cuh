@@ -40,7 +40,6 @@ struct Job {
   int* touched;       // vertices whose delta left the sentinel in this phase
   int* mm;            // mismatch list: v | cat << 29
   int* mm_next;       // the list being rebuilt by the incremental detection
-  uint8_t* mstat;     // current mismatch categories of every vertex
   int* dirty; int* dirty1;  // vertices whose value changed since the last detection, and since
                             // the one before it (they change roles at each detection)
   unsigned* dbits; unsigned* dbits1;  // their membership bitsets
@@ -421,6 +420,15 @@ __device__ __forceinline__ void count_cats(int* ctr, int cat) {
   }
 }
 
+// Vertex-id offsets of the 14 directions, for loops over the set bits of a
+// direction mask (threads 0..13 fill it; the caller synchronises).
+__device__ __forceinline__ void fill_offsets(int* off, const Dims& g) {
+  if (threadIdx.x < kNumDirs) {
+    const int d = threadIdx.x;
+    off[d] = ddx(d) + ddy(d) * g.W + ddz(d) * g.W * g.H;
+  }
+}
+
 // A tile-compressed pointer that is its path's root.
 constexpr int kRootFlag = (int)0x80000000u;
 
@@ -609,7 +617,6 @@ __global__ void __launch_bounds__(256, 8) k_classify(const Job<T>* __restrict__ 
       const int cat = lm == om ? 0
                                : mismatch_cats(type_from_masks(lm, valid & ~lm, valid, bc, J.tb),
                                                J.otype[v], lm, om);
-      J.mstat[v] = (uint8_t)cat;
       if (cat) {
         s_list[atomicAdd(&s_n, 1)] = v | (cat << kCatShift);
         if (cat & kCatMax) atomicAdd(&s_cat[0], 1);
@@ -644,34 +651,26 @@ __global__ void __launch_bounds__(256, 8) k_classify(const Job<T>* __restrict__ 
 // (detect_end), so a detection is one launch (four with a stamp per vertex, a
 // second kernel for the carried entries and two for the bookkeeping).
 // ---------------------------------------------------------------------------
+// Mismatch categories of vertex v on the decompressed field.
 template <class T>
-__device__ __forceinline__ int global_type(const Job<T>& J, int v, int& lmask) {
+__device__ __forceinline__ int vertex_cats(const Job<T>& J, int v) {
   const Dims g = J.dim;
   int x, y, z;
   coords(v, g, x, y, z);
   const int bc = boundary_code(x, y, z, g.W, g.H, g.D);
+  const int valid = valid_mask(bc);
+  const int om = J.olm[v];
   const T c = J.g[v];
-  int lm = 0, up = 0, k = 0, nl = 0, nu = 0;
+  int lm = 0;
 #pragma unroll
   for (int d = 0; d < kNumDirs; ++d) {
-    if (!dir_valid(d, bc)) continue;
+    if (!(valid >> d & 1)) continue;
     const T nv = J.g[v + dir_x(d) + dir_y(d) * g.W + dir_z(d) * g.W * g.H];
-    const bool before = dir_neighbour_is_before(d);
-    if (nv < c || (nv == c && before)) {
-      lm |= 1 << d;
-      ++nl;
-    } else if (nv > c || (nv == c && !before)) {
-      up |= 1 << k;
-      ++nu;
-    }
-    ++k;
+    if (dir_neighbour_is_before(d) ? nv <= c : nv < c) lm |= 1 << d;
   }
-  lmask = lm;
-  if (nu == 0) return 4;
-  if (nl == 0) return 0;
-  const int off = J.tb.key_offset[bc];
-  if (off < 0) return -1;
-  return __ldg(J.tb.lut + off + up);
+  // The type follows from the mask: with the original's mask nothing differs.
+  return lm == om ? 0
+                  : mismatch_cats(type_from_masks(lm, valid & ~lm, valid, bc, J.tb), J.otype[v], lm, om);
 }
 
 __device__ __forceinline__ bool bit_of(const unsigned* bits, int v) {
@@ -695,6 +694,9 @@ __device__ __forceinline__ void detect_end(Job<T>& J) {
   c[C_DEPOCH] += 1;
 }
 
+// Changed vertices (one in this many) from which k_redetect goes by the bitset.
+constexpr int kRedetectMany = 64;
+
 template <class T>
 __global__ void __launch_bounds__(256) k_redetect(const Job<T>* __restrict__ jobs,
                                                   const __grid_constant__ Sel sel) {
@@ -705,7 +707,43 @@ __global__ void __launch_bounds__(256) k_redetect(const Job<T>* __restrict__ job
   const int* __restrict__ dirty = odd ? J.dirty1 : J.dirty;
   const unsigned* __restrict__ bits = odd ? J.dbits1 : J.dbits;
   const int n = J.ctr[C_DIRTY], nmm = J.ctr[C_MM];
-  const long long nd = (long long)n * (kNumDirs + 1), total = nd + nmm;
+  // Many changed vertices: their dilated bitset, a word (32 vertices) per lane,
+  // then word by word a vertex per lane, instead of fifteen candidates per changed
+  // vertex and a search for each one's owner.  Across the ends of rows the
+  // dilation is too wide, which evaluates a vertex that need not be; the carried
+  // entries are tested against the same set.  (By the list, the first detection
+  // after the first edits took 0.16 ms at 256^3.)
+  const bool many = n > g.N / kRedetectMany;
+  __shared__ int off[kNumDirs];
+  fill_offsets(off, g);
+  __syncthreads();
+  const int nw = (g.N + 31) >> 5;
+  if (many) {
+    for (int w0 = (blk * 8 + (int)(threadIdx.x >> 5)) * 32; w0 < nw; w0 += nblk * 256) {
+      const int w = w0 + (int)lane_id();
+      unsigned near = 0u;
+      if (w < nw) {
+        near = bits[w];
+#pragma unroll
+        for (int k = 0; k < kNumDirs; ++k) {
+          const int at = 32 * w + off[k], i = at >> 5;
+          const unsigned lo = (unsigned)i < (unsigned)nw ? bits[i] : 0u;
+          const unsigned hi = (unsigned)(i + 1) < (unsigned)nw ? bits[i + 1] : 0u;
+          near |= __funnelshift_r(lo, hi, at & 31);
+        }
+      }
+      for (int j = 0; j < 32; ++j) {
+        const unsigned word = __shfl_sync(0xffffffffu, near, j);
+        if (!word) continue;
+        const int v = 32 * (w0 + j) + (int)lane_id();
+        const int cat = (word >> lane_id() & 1u) && v < g.N ? vertex_cats(J, v) : 0;
+        const int slot = warp_append(J.ctr + C_MM_NEXT, cat != 0, 0xffffffffu);
+        if (slot >= 0) J.mm_next[slot] = v | (cat << kCatShift);
+        count_cats(J.ctr, cat);
+      }
+    }
+  }
+  const long long nd = many ? 0 : (long long)n * (kNumDirs + 1), total = nd + nmm;
   const long long stride = (long long)nblk * blockDim.x;
   for (long long base = blk * (long long)blockDim.x; base < total; base += stride) {
     const long long e = base + threadIdx.x;
@@ -733,23 +771,26 @@ __global__ void __launch_bounds__(256) k_redetect(const Job<T>* __restrict__ job
           if (earlier) v = -1;
         }
       }
-      if (v >= 0) {
-        int lm;
-        const int t = global_type(J, v, lm);
-        cat = mismatch_cats(t, J.otype[v], lm, J.olm[v]);
-        J.mstat[v] = (uint8_t)cat;
-      }
+      if (v >= 0) cat = vertex_cats(J, v);
     } else if (e < total) {
       const int ent = J.mm[e - nd];
       v = ent & ((1 << kCatShift) - 1);
-      int x, y, z;
-      coords(v, g, x, y, z);
-      const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
       bool near = bit_of(bits, v);
+      if (many) {
 #pragma unroll
-      for (int k = 0; k < kNumDirs; ++k)
-        if (valid >> k & 1)
-          near |= bit_of(bits, v + dir_x(k) + dir_y(k) * g.W + dir_z(k) * g.W * g.H);
+        for (int k = 0; k < kNumDirs; ++k) {
+          const int u = v + off[k];
+          near |= (unsigned)u < (unsigned)(32 * nw) && bit_of(bits, u);
+        }
+      } else {
+        int x, y, z;
+        coords(v, g, x, y, z);
+        const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
+#pragma unroll
+        for (int k = 0; k < kNumDirs; ++k)
+          if (valid >> k & 1)
+            near |= bit_of(bits, v + dir_x(k) + dir_y(k) * g.W + dir_z(k) * g.W * g.H);
+      }
       if (!near) cat = (unsigned)ent >> kCatShift;
     }
     const int slot = warp_append(J.ctr + C_MM_NEXT, cat != 0, 0xffffffffu);
@@ -1659,15 +1700,6 @@ __global__ void __launch_bounds__(32 * kCpWarps) k_cp_write(const int8_t* __rest
 // and the count are written, so entries past a shorter row keep their last
 // value, as in the reference.
 // ---------------------------------------------------------------------------
-// Vertex-id offsets of the 14 directions, for loops over the set bits of a
-// direction mask (threads 0..13 fill it; the caller synchronises).
-__device__ __forceinline__ void fill_offsets(int* off, const Dims& g) {
-  if (threadIdx.x < kNumDirs) {
-    const int d = threadIdx.x;
-    off[d] = ddx(d) + ddy(d) * g.W + ddz(d) * g.W * g.H;
-  }
-}
-
 // The rows of one side of the original field.  A saddle's neighbours on the
 // side are the set bits of the direction mask that the classification left
 // (upper neighbours of a 2-saddle, lower ones of a 1-saddle): 4.3 of 14 on
