@@ -1675,21 +1675,25 @@ __global__ void __launch_bounds__(32 * kCpWarps) k_cp_write(const int8_t* __rest
   const int v0 = b * kCpBlock + (int)lane_id() * 32;
   unsigned bits[4];
   cp_lane_bits(otype, N, v0, bits);
+  // Word by word, a vertex per lane: a list's entries of 32 ids are consecutive,
+  // so the stores are coalesced (a lane writing its own 32 ids' entries spread
+  // every store over 32 places: 0.40 ms at 512^3, now 0.34).
   int* outs[4] = {sad2, sad1, maxima, minima};
+  int pos[4];
 #pragma unroll
-  for (int l = 0; l < 4; ++l) {
-    const int c = __popc(bits[l]);
-    int incl = c;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane_id() >= (unsigned)o) incl += y;
-    }
-    int pos = boff[l * nb + b] + incl - c;
-    for (unsigned m = bits[l]; m; m &= m - 1) {
-      const int v = v0 + __ffs(m) - 1;
-      outs[l][pos] = v;
-      if (l >= 2) ext[v] = pos;
-      ++pos;
+  for (int l = 0; l < 4; ++l) pos[l] = boff[l * nb + b];
+  const unsigned lt = (1u << lane_id()) - 1u;
+  for (int j = 0; j < 32; ++j) {
+    const int v = b * kCpBlock + 32 * j + (int)lane_id();
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const unsigned word = __shfl_sync(0xffffffffu, bits[l], j);
+      if (word >> lane_id() & 1u) {
+        const int at = pos[l] + __popc(word & lt);
+        outs[l][at] = v;
+        if (l >= 2) ext[v] = at;
+      }
+      pos[l] += __popc(word);
     }
   }
 }
