@@ -135,7 +135,7 @@ constexpr long long job_bytes_voxels(long long n, long long ksz) {
          + 2 * arr_bytes(n, 4)                                      // pdd, pda
          + arr_bytes((n + 31) / 32, 4) + arr_bytes(n, 1)            // change bitset, dirtyv
          + 8 * arr_bytes((n + 31) / 32, 4)  // wrong-saddle change, touched roots, dirty, taken
-         + 2 * arr_bytes((n + kCpBlock - 1) / kCpBlock, 4)  // dirtyv stamp, seed count per block
+         + 2 * arr_bytes((n + kCpBlock - 1) / kCpBlock, 4)  // bdirty, seed count per block
          + arr_bytes(6 * ((n + kCpBlock - 1) / kCpBlock), 4)        // CP block counts
          + arr_bytes(6 * ((n + kCpBlock - 1) / kCpBlock / 1024 + 1), 4)  // and their chunk sums
          + 4096;
@@ -186,6 +186,24 @@ constexpr long long job_bytes(long long n) {
   return job_bytes_sz(n, sizeof(typename KeyOf<T>::K));
 }
 constexpr long long job_bytes_max(long long n) { return job_bytes_sz(n, 8); }
+
+// What a field of n voxels is charged against a server's budget and reported as
+// its footprint: a published number, so it does not follow every change of the
+// workspace.  It stands for the arrays below (count x bytes each) and must cover
+// the worst case; the 64 KiB are for alignment, which only fields of some thousand
+// voxels notice.
+constexpr long long job_charge(long long n) {
+  const long long words = (n + 31) / 32, blocks = (n + kCpBlock - 1) / kCpBlock;
+  return 9 * arr_bytes(n, 1) + arr_bytes(n, 2) + 38 * arr_bytes(n, 4) + 5 * arr_bytes(n, 8) +
+         4 * arr_bytes(n, 16) + 2 * arr_bytes(7 * n, 4) + 2 * arr_bytes(n * kRowStride, 4) +
+         2 * arr_bytes(n + 1, 4) + 5 * arr_bytes(words, 4) + 2 * arr_bytes(blocks, 4) +
+         arr_bytes(6 * blocks, 4) + arr_bytes(6 * (blocks / 1024 + 1), 4) +
+         arr_bytes(n / 1024 + 2, 4) + arr_bytes(8, 8) + 2 * 4096;
+}
+static_assert(job_charge(1) + (64 << 10) >= job_bytes_max(1) &&
+                  job_charge(1 << 12) >= job_bytes_max(1 << 12) &&
+                  job_charge(1ll << 28) >= job_bytes_max(1ll << 28),
+              "a field's charge covers its worst case");
 
 // One job's host-side state.
 template <class T>

@@ -55,7 +55,7 @@ struct Job {
   uint8_t* dirtyv;    // per vertex: the round stamp's low byte when an input of its saddle
                       // rows changed in that round
   int* bdirty;        // per 1024-id block: the round stamp when some dirtyv byte in it was
-                      // set (when N % 4 == 0)
+                      // set
   uint8_t* has2; uint8_t* has1;  // per saddle row: its wrong-neighbour seed bit
   uint8_t* bad2; uint8_t* bad1;  // per saddle row: 1 if its first row slot differs from the
                                  // original row's first entry, 2 if its second from the last
