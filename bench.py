@@ -84,10 +84,10 @@ DOMINANT = ("direction_first", "jump_first")
 LATER = ("direction", "jump")
 DOMINANT_KERNEL = ("first manifold round of the decompressed field (k_direction + k_jump2, "
                    "every tile and vertex)")
-# The next kernel by device time (the saddle pass after each manifold round),
+# The next kernels by device time (the saddle passes after each manifold round),
 # timed beside the dominant ones in a few extra steps.
 RUNNER_UP = "rows"
-RUNNER_UP_KERNEL = "k_saddle_pass"
+RUNNER_UP_KERNEL = "k_saddle_first, k_saddle_pass"
 
 
 def round_bytes(n: int, s: int) -> int:

@@ -754,8 +754,8 @@ class BatchEngine {
     return tick_complete();
   }
 
-  // First half of a tick: the launches and the asynchronous copy of the
-  // counter blocks.  Engines on different streams issue, then complete, so
+  // First half of a tick: the launches, the last of which publishes the counters
+  // the host branches on.  Engines on different streams issue, then complete, so
   // their ticks overlap on the device.
   int tick_issue() {
     issued_ = false;
