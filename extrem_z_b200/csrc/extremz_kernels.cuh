@@ -1289,7 +1289,11 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       };
       // Returns the quad's labels through u1 / u2 (the old ones when it is
       // not followed) and the old ones through o1 / o2 (-1 in a first round).
-      auto quad = [&](int v0, const int4& O1, const int4& O2, int* u1, int* u2, int* o1, int* o2) {
+      auto quad = [&](int v0, int* u1, int* u2, int* o1, int* o2) {
+        // A job's first round writes every label (its change bitset starts
+        // full, and the stored labels may be another job's): no old labels.
+        const int4 O1 = kLater ? *reinterpret_cast<const int4*>(ra + v0) : make_int4(-1, -1, -1, -1);
+        const int4 O2 = kLater ? *reinterpret_cast<const int4*>(rb + v0) : make_int4(-1, -1, -1, -1);
         o1[0] = O1.x; o1[1] = O1.y; o1[2] = O1.z; o1[3] = O1.w;
         o2[0] = O2.x; o2[1] = O2.y; o2[2] = O2.z; o2[3] = O2.w;
         if constexpr (kLater) {
@@ -1401,26 +1405,9 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       }
       const int nq = N >> 2;
       const int qstride = nblk * blockDim.x;
-      // A job's first round writes every label (its change bitset starts full, and
-      // the stored labels may be another job's): no old labels.  In a later one the
-      // next quad's are on their way while this one's roots are looked up: most
-      // quads end there (later rounds at 256^3, f64: 734 -> 676 us together).
-      int q = blk * blockDim.x + threadIdx.x;
-      int4 O1 = make_int4(-1, -1, -1, -1), O2 = O1;
-      if (kLater && q < nq) {
-        O1 = reinterpret_cast<const int4*>(ra)[q];
-        O2 = reinterpret_cast<const int4*>(rb)[q];
-      }
-      for (; q < nq; q += qstride) {
+      for (int q = blk * blockDim.x + threadIdx.x; q < nq; q += qstride) {
         int u1[4], u2[4], o1[4], o2[4];
-        int4 P1 = O1, P2 = O2;
-        if (kLater && q + qstride < nq) {
-          P1 = reinterpret_cast<const int4*>(ra)[q + qstride];
-          P2 = reinterpret_cast<const int4*>(rb)[q + qstride];
-        }
-        quad(q << 2, O1, O2, u1, u2, o1, o2);
-        O1 = P1;
-        O2 = P2;
+        quad(q << 2, u1, u2, o1, o2);
       }
       from = nq << 2;
     }
