@@ -52,8 +52,8 @@ struct Job {
   uint8_t* mis;       // per vertex: 1 if dds != ds, 2 if das != as
   unsigned* vchg;     // bitset: vertices whose value changed since the last computed round
   unsigned* edited;   // bitset: vertices whose value changed in this correction (or null)
-  uint8_t* dirtyv;    // per vertex: the round stamp's low byte when an input of its saddle
-                      // rows changed in that round
+  uint8_t* dirtyv;    // per vertex: the round's byte (mf_byte) when an input of its saddle
+                      // rows changed in that round, else 0 or an earlier round's
   int* bdirty;        // per 1024-id block: the round stamp when some dirtyv byte in it was
                       // set
   uint8_t* has2; uint8_t* has1;  // per saddle row: its wrong-neighbour seed bit
@@ -174,6 +174,10 @@ __device__ __forceinline__ bool mf_skip(const int* ctr) {
   return ctr[C_MFDONE] && !ctr[C_CHANGED];
 }
 __device__ __forceinline__ int mf_stamp(const int* ctr) { return ctr[C_WNSTAMP] + 1; }
+// A round's stamp as a byte (dirtyv), never the zero of an unchanged vertex: with
+// the stamp's low byte, every 256th round's changes read as no change and their
+// blocks were not flagged.
+__device__ __forceinline__ unsigned mf_byte(int stamp) { return 1u + (unsigned)stamp % 255u; }
 // A light round's jump goes over the tiles that k_touched_tiles finds only in
 // fields of at least this many vertices: a pass over every vertex costs about
 // 2.2 us per million, the search some 35 us whatever the field.
@@ -1227,7 +1231,7 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       // change bitset starts full, so the first round marks every vertex.
       const unsigned c1 = vchg[u1 >> 5] >> (u1 & 31), c2 = vchg[u2 >> 5] >> (u2 & 31);
       const bool d = (o1 != u1) | (o2 != u2) | ((c0 | c1 | c2) & 1u);
-      dirtyv[v] = d ? (uint8_t)mf_stamp(J.ctr) : (uint8_t)0;
+      dirtyv[v] = d ? (uint8_t)mf_byte(mf_stamp(J.ctr)) : (uint8_t)0;
       if (d) J.bdirty[v >> 10] = mf_stamp(J.ctr);
       mis[v] = (uint8_t)((u1 != r1) | (u2 != r2) << 1);
     }
@@ -1243,8 +1247,9 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       // with a changed-input byte stamps its 1024-id block (bdirty, read by
       // the saddle pass; its address is read where it is used: kept in a
       // register for the whole loop it costs spills).  Changed-input bytes
-      // are round stamps (low byte): a quad that is not followed leaves its
-      // bytes, which then read as unchanged.
+      // are the round's (mf_byte): a quad that is not followed leaves its
+      // bytes, which then read as unchanged (or, when they are 255 rounds old,
+      // as changed, which recomputes rows that have not changed).
       //
       // kLater: a vertex's label on a side can change only when its path
       // crosses a tile whose pointers this round recomputed, and every vertex
@@ -1254,7 +1259,7 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       // mismatch bits and has no changed input (a changed value, own or of a
       // root, lies in a recomputed tile too).
       const int stamp = mf_stamp(J.ctr);
-      const unsigned st8 = (unsigned)stamp & 0xffu;
+      const unsigned st8 = mf_byte(stamp);
       // Four vertices' chains to their ends.
       auto chase = [&](int* u1, int* u2) {
         // One hop of every unfinished chain per iteration: the loads depend only
@@ -2419,7 +2424,7 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
     }
     return seen;
   };
-  const unsigned st8 = (unsigned)mf_stamp(J.ctr) & 0xffu;  // changed-input bytes of this round
+  const unsigned st8 = mf_byte(mf_stamp(J.ctr));  // changed-input bytes of this round
   // Seed s into its side's list.  All lanes of a warp call it.
   auto list = [&](bool split, bool has, int s) {
     const int slot2 = warp_append(J.ctr + C_CAND, has && split, 0xffffffffu);
