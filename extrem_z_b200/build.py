@@ -19,7 +19,7 @@ COMPAT_SOURCES = [os.path.join(PKG, "compat", "extrem_api.cpp"),
 
 SOURCES = ["extremz_engine.cu"]
 HEADERS = ["extremz_common.cuh", "extremz_kernels.cuh", "extremz_batch.cuh", "extremz_encode.cuh",
-           "extremz_topo.cuh", "extremz_lut.h"]
+           "extremz_topo.cuh", "extremz_lut.h", "extremz_queue.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

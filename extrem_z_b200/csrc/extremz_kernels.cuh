@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "extremz_common.cuh"
+#include "extremz_queue.h"
 
 namespace extremz {
 
@@ -1072,10 +1073,45 @@ __global__ void __launch_bounds__(256, 4) k_direction_list(const Job<T>* __restr
 // 512^3 for a handful of changes).  With more than a 64th of the tiles
 // recomputed, or a quarter found, the jump goes over every vertex.
 //
-// A block takes the queue's entries by ticket.  It waits for its entry only
-// while another running block still searches (entries done < entries pushed);
+// A block takes the queue's entries by ticket (queue_take).  It waits for its entry
+// only while another running block still searches (entries done < entries pushed);
 // should that take too long, it asks for the pass over every vertex, which is
 // always right, and everyone stops.
+__device__ __forceinline__ int load_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int load_relaxed(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+struct TileQueue {
+  int* ctr;
+  unsigned long long* at;
+  __device__ int ticket() const { return atomicAdd(ctr + C_QHEAD, 1); }
+  __device__ int place() const { return atomicAdd(ctr + C_NAFF, 1); }
+  // Called by one thread, behind a barrier with those that pushed.
+  __device__ void finished() const {
+    __threadfence();
+    atomicAdd(ctr + C_QDONE, 1);
+  }
+  __device__ int done() const { return load_acquire(ctr + C_QDONE); }
+  __device__ int pushed() const { return load_relaxed(ctr + C_NAFF); }
+  __device__ bool dense() const { return load_relaxed(ctr + C_JDENSE) != 0; }
+  __device__ void ask_dense() const { atomicExch(ctr + C_JDENSE, 1); }
+  __device__ unsigned long long entry(int i) const {
+    unsigned long long e;
+    asm volatile("ld.relaxed.gpu.b64 %0, [%1];" : "=l"(e) : "l"(at + i) : "memory");
+    return e;
+  }
+  __device__ void store(int i, unsigned long long e) const {
+    asm volatile("st.relaxed.gpu.b64 [%0], %1;" ::"l"(at + i), "l"(e) : "memory");
+  }
+  __device__ void pause() const { __nanosleep(100); }
+};
+constexpr int kQueueWait = 1 << 16;  // looks at the queue, at least 100 ns apart
 template <class T>
 __global__ void __launch_bounds__(256) k_touched_tiles(const Job<T>* __restrict__ jobs,
                                                        const __grid_constant__ Sel sel) {
@@ -1094,29 +1130,10 @@ __global__ void __launch_bounds__(256) k_touched_tiles(const Job<T>* __restrict_
     if (threadIdx.x == 0) ctr[C_JDENSE] = 1;
     return;
   }
+  TileQueue queue{ctr, J.tqueue};
   for (;;) {
     if (threadIdx.x == 0) {
-      const int h = atomicAdd(ctr + C_QHEAD, 1);
-      int t = -1;
-      for (int spin = 0;; ++spin) {
-        const int done = __ldcg(ctr + C_QDONE), pushed = __ldcg(ctr + C_NAFF);  // in this order
-        if (__ldcg(ctr + C_JDENSE)) break;
-        if (pushed > h && h < nt) {  // the entry may still be on its way
-          const unsigned long long e = __ldcg(J.tqueue + h);
-          if ((unsigned)(e >> 32) == stamp) {
-            t = (int)(unsigned)e;
-            break;
-          }
-        } else if (done == pushed) {
-          break;
-        }
-        if (spin > (1 << 16)) {
-          ctr[C_JDENSE] = 1;
-          break;
-        }
-        __nanosleep(100);
-      }
-      tile = t;
+      tile = queue_take(queue, stamp, nt, kQueueWait);
       found = 0u;
     }
     __syncthreads();
@@ -1144,17 +1161,10 @@ __global__ void __launch_bounds__(256) k_touched_tiles(const Job<T>* __restrict_
     if (threadIdx.x < 27 && (found >> threadIdx.x & 1u)) {
       const int q = threadIdx.x;
       const int u = t + (q % 3 - 1) + (q / 3 % 3 - 1) * ntx + (q / 9 - 1) * ntx * nty;
-      if (atomicExch(J.tseen + u, (int)stamp) != (int)stamp) {
-        const int at = atomicAdd(ctr + C_NAFF, 1);
-        if (at < nt / 4) __stcg(J.tqueue + at, (unsigned long long)stamp << 32 | (unsigned)u);
-        else ctr[C_JDENSE] = 1;
-      }
+      if (atomicExch(J.tseen + u, (int)stamp) != (int)stamp) queue_push(queue, stamp, u, nt / 4);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      atomicAdd(ctr + C_QDONE, 1);
-    }
+    if (threadIdx.x == 0) queue.finished();
   }
 }
 
