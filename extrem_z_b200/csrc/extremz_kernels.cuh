@@ -1120,7 +1120,11 @@ __global__ void __launch_bounds__(256) k_touched_tiles(const Job<T>* __restrict_
   int blk, nblk;
   const Job<T>& J = span_job(jobs, sel, blk, nblk);
   int* ctr = J.ctr;
-  if (mf_skip(ctr) || __ldcg(ctr + C_JDENSE)) return;
+  // A block's threads leave together: on values that nothing writes during this
+  // launch, or on the tile that the first thread took.  C_JDENSE, which other blocks
+  // set meanwhile, is looked at by that thread alone (a block of which only some
+  // threads saw it set would go on without the one that writes `tile`).
+  if (mf_skip(ctr)) return;
   const Dims g = J.dim;
   const int WH = g.W * g.H;
   const int ntx = (g.W + TX - 1) / TX, nty = (g.H + TY - 1) / TY, ntz = (g.D + TZ - 1) / TZ;
@@ -1130,7 +1134,7 @@ __global__ void __launch_bounds__(256) k_touched_tiles(const Job<T>* __restrict_
     if (threadIdx.x == 0) ctr[C_JDENSE] = 1;
     return;
   }
-  TileQueue queue{ctr, J.tqueue};
+  TileQueue queue{ctr, J.tqueue};  // (its first look finds C_JDENSE set from the start too)
   for (;;) {
     if (threadIdx.x == 0) {
       tile = queue_take(queue, stamp, nt, kQueueWait);
