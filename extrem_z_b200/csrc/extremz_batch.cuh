@@ -263,6 +263,7 @@ class BatchEngine {
   ~BatchEngine() { release_all(); }
 
   int init(const DeviceTables* preset_tables, Arena* fixed_storage) {
+    wait_known_ = false;
     if (ready_) return EXTREMZ_OK;
     int dev = 0;
     EZ_CHECK(cudaGetDevice(&dev));
@@ -861,9 +862,21 @@ class BatchEngine {
 
   // Takes over the published counters as they arrive.  The stream is asked now
   // and then: an error ends the wait, and once all its work is done they are
-  // there.
+  // there.  A process that asked for blocking or yielding waits gets them: there
+  // the counters are read once the stream is done.
   int await_published() {
     bool all_done = false;
+    if (!wait_known_) {  // asked at the first wait of a call, while the device works
+      unsigned flags = 0;
+      if (cudaGetDeviceFlags(&flags) != cudaSuccess) cudaGetLastError();
+      flags &= cudaDeviceScheduleMask;
+      spin_ = flags != cudaDeviceScheduleBlockingSync && flags != cudaDeviceScheduleYield;
+      wait_known_ = true;
+    }
+    if (!spin_) {
+      EZ_CHECK(cudaStreamSynchronize(st_));
+      all_done = true;
+    }
     for (int i = 0, spins = 0; i < pub_n_;) {
       const unsigned long long p = pub_host_[i];
       if ((unsigned)(p >> 32) == seq_next_) {
@@ -970,6 +983,7 @@ class BatchEngine {
   unsigned* seq_dev_ = nullptr;
   unsigned seq_next_ = 0;
   bool seq_known_ = true;
+  bool wait_known_ = false, spin_ = true;  // wait for the published counters by reading them
   int pub_n_ = 0;           // counters published by this tick; 0: copied
   int static_ctr_host_[C_COUNT * kMaxSel];
   std::vector<JobHost<T>> slots_;
