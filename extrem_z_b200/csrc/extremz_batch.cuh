@@ -693,11 +693,13 @@ class BatchEngine {
       // Saddles descending in the tree's order.
       if (n_s) sort(slist[side], n_s, kmax, kmax, sad_li);
       if (kmax)
-        launch(K_OTHER, k_pp_rows<true>, grid_, 256, (const uint16_t*)J.olm, J.dim, slist[0],
+        launch(K_OTHER, k_pp_rows<T, true>, grid_, 256, J.f, (const uint16_t*)J.olm,
+               (const int*)J.ctr, J.dim, slist[0],
                (const int*)sad_li, n_s, (const int*)J.ds, (const int*)J.ext, (const int*)erank, rows,
                cnt);
       else
-        launch(K_OTHER, k_pp_rows<false>, grid_, 256, (const uint16_t*)J.olm, J.dim, slist[1],
+        launch(K_OTHER, k_pp_rows<T, false>, grid_, 256, J.f, (const uint16_t*)J.olm,
+               (const int*)J.ctr, J.dim, slist[1],
                (const int*)sad_li, n_s, (const int*)J.as, (const int*)J.ext, (const int*)erank, rows,
                cnt);
       launch(K_OTHER, k_fill<int>, grid_, 256, largest, kInf, (long long)n_e);
@@ -1445,7 +1447,9 @@ class BatchEngine {
           // mismatch; a census's may not.
           std::vector<int> first, other;
           for (int i : busy)
-            (slots_[i].manifold_rounds == 0 && !(slots_[i].p.flags & kFlagCensus) ? first : other)
+            (slots_[i].manifold_rounds == 0 && !(slots_[i].p.flags & kFlagCensus) && !h(i, C_NAN)
+                 ? first
+                 : other)
                 .push_back(i);
           if (!first.empty()) {
             const Sel fs = make_span(first);
@@ -1702,6 +1706,8 @@ class BatchEngine {
     J.maxima = A.take<int>(nmax);
     J.minima = A.take<int>(nmin);
     if (!J.minima) return EXTREMZ_OOM;
+    // Without NaNs every path ends at an extremum, so only their entries are read.
+    if (h(slot, C_NAN)) launch(K_OTHER, k_fill<int>, grid_, 256, J.ext, 0, (long long)N);
     launch(K_OTHER, k_cp_write, (jh.nb + kCpWarps - 1) / kCpWarps, 32 * kCpWarps,
            (const int8_t*)J.otype, N, jh.nb, (const int*)jh.bcount,
            J.sad2, J.sad1, J.maxima, J.minima, J.ext);

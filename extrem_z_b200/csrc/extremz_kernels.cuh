@@ -140,6 +140,7 @@ enum Ctr : int {
   C_MM = 0, C_CMAX, C_CMIN, C_CSAD, C_TOUCHED, C_NFC, C_NFC1, C_CAND, C_CAND_NEXT,
   C_WMC, C_WMC2, C_WSC, C_WMIN, C_WMIN2, C_WSCJ, C_NS2, C_NS1, C_NMAX, C_NMIN,
   C_E2, C_E1,  // row entries of the 2-saddles' / 1-saddles' original rows (upper bound)
+  C_NAN,       // the original field holds a NaN
   C_ERROR,
   C_CHANGED,   // some value changed since the last computed manifold round began
   C_DIRTY, C_MM_NEXT, C_CANDJ,
@@ -432,6 +433,19 @@ __device__ __forceinline__ void fill_offsets(int* off, const Dims& g) {
     const int d = threadIdx.x;
     off[d] = ddx(d) + ddy(d) * g.W + ddz(d) * g.W * g.H;
   }
+}
+
+// The upper neighbours of a vertex are the valid ones that are not lower, except a
+// NaN, which is neither (only fields with C_NAN look): side without its NaNs.
+template <class T>
+__device__ __forceinline__ unsigned drop_nans(const T* __restrict__ a, const int* off, int s,
+                                              unsigned side) {
+  for (unsigned rest = side; rest; rest &= rest - 1u) {
+    const int d = __ffs((int)rest) - 1;
+    const T v = a[s + off[d]];
+    if (v != v) side &= ~(1u << d);
+  }
+  return side;
 }
 
 // A tile-compressed pointer that is its path's root.
@@ -853,10 +867,12 @@ __device__ __forceinline__ void steepest_dirs(const Tile<T>& s, int tx, int ty, 
 }
 
 // The same steps voxel by voxel through the exact scans of steepest_dirs, for a
-// tile that holds an infinity or a NaN.
+// tile that holds an infinity or a NaN.  nan: set when a voxel of the column is one
+// (or null).
 template <class T>
 __device__ __noinline__ void column_steps_any(const Tile<T>& s, int tx, int ty, int bx, int by, int bz,
-                                              const Dims& g, int* up_st, int* dn_st, int* lm) {
+                                              const Dims& g, int* up_st, int* dn_st, int* lm,
+                                              int* nan) {
   for (int tz = 0; tz < TZ; ++tz) {
     const int x = bx + tx, y = by + ty, z = bz + tz;
     int hd = -1, ld = -1, um;
@@ -865,6 +881,8 @@ __device__ __noinline__ void column_steps_any(const Tile<T>& s, int tx, int ty, 
       const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
       steepest_dirs<T>(s, tx, ty, tz, valid, hd, ld);
       tile_masks(s, tx, ty, tz, valid, lm[tz], um);
+      const T c = s.v[tz + 1][ty + 1][tx + kXOff];
+      if (nan && c != c) *nan = 1;
     }
     up_st[tz] = hd < 0 ? 0 : step_of(ddx(hd), ddy(hd), ddz(hd));
     dn_st[tz] = ld < 0 ? 0 : step_of(ddx(ld), ddy(ld), ddz(ld));
@@ -925,7 +943,7 @@ __device__ __noinline__ bool direction_tile(const Job<T>& J, Tile<T>& s, uint64_
                         bz + TZ < g.D;
   int hs[TZ], ls[TZ], lm[TZ];
   if (!usual) {
-    column_steps_any<T>(s, tx, ty, bx, by, bz, g, hs, ls, lm);
+    column_steps_any<T>(s, tx, ty, bx, by, bz, g, hs, ls, lm, kDec ? nullptr : J.ctr + C_NAN);
   } else if (interior) {
     column_steps<T, false, true, !kDec>(s, tx, ty, ColumnEdges{}, hs, ls, lm);
   } else {
@@ -1754,6 +1772,9 @@ __global__ void __launch_bounds__(256, 4) k_rows(Job<T> J) {
       int x, y, z;
       coords(s, g, x, y, z);
       side = (unsigned)valid_mask(boundary_code(x, y, z, g.W, g.H, g.D)) & ~side;
+      // Next to a NaN a path may end at a vertex that is no maximum, whose index
+      // in ext is 0 then: in a field without maxima no row names one.
+      if (J.ctr[C_NAN]) side = J.ctr[C_NMAX] ? drop_nans(a, off, s, side) : 0u;
       J.smask2[i] = (uint16_t)side;
     }
     const int pmax = (int)__reduce_max_sync(0xffffffffu, __popc(side));
@@ -2403,8 +2424,9 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
     J.taken1[w] = 0u;
   }
   __syncthreads();
-  // No mismatch at the last detection and no value changed since.
-  const bool known = J.ctr[C_MM] == 0 && J.ctr[C_DIRTY] == 0;
+  // No mismatch at the last detection and no value changed since (and no NaN, whose
+  // neighbours' sides the masks do not tell).
+  const bool known = J.ctr[C_MM] == 0 && J.ctr[C_DIRTY] == 0 && J.ctr[C_NAN] == 0;
   const int ns2 = J.ctr[C_NS2], ns1 = J.ctr[C_NS1];
   const int nb = (J.dim.N + kCpBlock - 1) / kCpBlock;
   const int chunk = J.pass_chunk;
@@ -2557,7 +2579,7 @@ __global__ void __launch_bounds__(256, 4) k_saddle_pass(const Job<T>* __restrict
 
 // The saddle pass of a correction's first round: every saddle, right after a
 // detection without mismatch, so the direction masks are the original field's
-// (known).  Without the later rounds' checks and queue it holds few registers,
+// (known; a field with a NaN takes k_saddle_pass).  Without the later rounds' checks and queue it holds few registers,
 // and its gathers are bound by latency: 2-saddles (rows) and 1-saddles (seed
 // bits; rows too with join_rows) in two loops.
 template <class T>

@@ -164,8 +164,10 @@ __device__ __forceinline__ int pp_store_row(const int* r, int* row) {
 // labels of its neighbours on the tree's side, ascending.  The neighbours are
 // the classification's direction mask; an entry's place is the number of smaller
 // distinct ones, so nothing is sorted in local memory.
-template <bool kMax>
-__global__ void __launch_bounds__(256) k_pp_rows(const uint16_t* __restrict__ olm, Dims g,
+template <class T, bool kMax>
+__global__ void __launch_bounds__(256) k_pp_rows(const T* __restrict__ a,
+                                                 const uint16_t* __restrict__ olm,
+                                                 const int* __restrict__ ctr, Dims g,
                                                  const int* __restrict__ sad,
                                                  const int* __restrict__ sorted_li, int ns,
                                                  const int* __restrict__ lab,
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(256) k_pp_rows(const uint16_t* __restrict__ ol
       int x, y, z;
       coords(s, g, x, y, z);
       side = (unsigned)valid_mask(boundary_code(x, y, z, g.W, g.H, g.D)) & ~side;
+      if (ctr[C_NAN]) side = drop_nans(a, off, s, side);
     }
     int r[kPpRow];
 #pragma unroll
