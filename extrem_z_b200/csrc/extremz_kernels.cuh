@@ -867,12 +867,10 @@ __device__ __forceinline__ void steepest_dirs(const Tile<T>& s, int tx, int ty, 
 }
 
 // The same steps voxel by voxel through the exact scans of steepest_dirs, for a
-// tile that holds an infinity or a NaN.  nan: set when a voxel of the column is one
-// (or null).
+// tile that holds an infinity or a NaN.
 template <class T>
 __device__ __noinline__ void column_steps_any(const Tile<T>& s, int tx, int ty, int bx, int by, int bz,
-                                              const Dims& g, int* up_st, int* dn_st, int* lm,
-                                              int* nan) {
+                                              const Dims& g, int* up_st, int* dn_st, int* lm) {
   for (int tz = 0; tz < TZ; ++tz) {
     const int x = bx + tx, y = by + ty, z = bz + tz;
     int hd = -1, ld = -1, um;
@@ -881,8 +879,6 @@ __device__ __noinline__ void column_steps_any(const Tile<T>& s, int tx, int ty, 
       const int valid = valid_mask(boundary_code(x, y, z, g.W, g.H, g.D));
       steepest_dirs<T>(s, tx, ty, tz, valid, hd, ld);
       tile_masks(s, tx, ty, tz, valid, lm[tz], um);
-      const T c = s.v[tz + 1][ty + 1][tx + kXOff];
-      if (nan && c != c) *nan = 1;
     }
     up_st[tz] = hd < 0 ? 0 : step_of(ddx(hd), ddy(hd), ddz(hd));
     dn_st[tz] = ld < 0 ? 0 : step_of(ddx(ld), ddy(ld), ddz(ld));
@@ -936,6 +932,9 @@ __device__ __noinline__ bool direction_tile(const Job<T>& J, Tile<T>& s, uint64_
     if (threadIdx.x == 0) atomicOr(J.ctr + C_ERROR, kErrTile);
     return false;
   }
+  if (!kDec && !usual)
+    for (int i = threadIdx.x; i < SX * SY * SZ; i += 256)
+      if (isnan((&s.v[0][0][0])[i])) J.ctr[C_NAN] = 1;
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const int x = bx + tx, y = by + ty;
   // A tile off the field's faces has every direction valid at every voxel.
@@ -943,7 +942,7 @@ __device__ __noinline__ bool direction_tile(const Job<T>& J, Tile<T>& s, uint64_
                         bz + TZ < g.D;
   int hs[TZ], ls[TZ], lm[TZ];
   if (!usual) {
-    column_steps_any<T>(s, tx, ty, bx, by, bz, g, hs, ls, lm, kDec ? nullptr : J.ctr + C_NAN);
+    column_steps_any<T>(s, tx, ty, bx, by, bz, g, hs, ls, lm);
   } else if (interior) {
     column_steps<T, false, true, !kDec>(s, tx, ty, ColumnEdges{}, hs, ls, lm);
   } else {
