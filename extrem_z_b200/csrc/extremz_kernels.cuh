@@ -450,6 +450,11 @@ __device__ __forceinline__ unsigned drop_nans(const T* __restrict__ a, const int
 
 // A tile-compressed pointer that is its path's root.
 constexpr int kRootFlag = (int)0x80000000u;
+// At the jump's limit: the end u of a chain that names itself is a root after all
+// (the look at a root is not a hop of its own in the limit's count).
+__device__ __forceinline__ int root_at_limit(const int* a, int u) {
+  return u >= 0 && (a[u] & ~kRootFlag) == u ? u | kRootFlag : u;
+}
 
 // In-tile positions of the path following: p = x + 64 y + 1024 z, with one bit
 // free above each coordinate's range.  A step adds the direction's offset in the
@@ -1252,6 +1257,10 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
       u2 = w2 == u2 ? w2 | kRootFlag : w2;
       ++it;
     }
+    if (u1 >= 0 || u2 >= 0) {
+      u1 = root_at_limit(a, u1);
+      u2 = root_at_limit(b, u2);
+    }
     if (u1 >= 0 || u2 >= 0 || cap_j < 2) atomicOr(err, kErrJump);
     u1 &= ~kRootFlag;
     u2 &= ~kRootFlag;
@@ -1316,8 +1325,14 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
         }
         bool open = false;
   #pragma unroll
+        for (int k = 0; k < 4; ++k) open |= (u1[k] >= 0) | (u2[k] >= 0);
+        if (open) {
+          open = false;
+          for (int k = 0; k < 8; ++k)
+            open |= root_at_limit(k < 4 ? a : b, k < 4 ? u1[k] : u2[k - 4]) >= 0;
+        }
+  #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          open |= (u1[k] >= 0) | (u2[k] >= 0);
           u1[k] &= ~kRootFlag;
           u2[k] &= ~kRootFlag;
         }
@@ -1469,6 +1484,11 @@ __global__ void __launch_bounds__(256, 4) k_jump2(const Job<T>* __restrict__ job
           for (int k = 0; k < 8; ++k) w[k] = u[k] >= 0 ? (k < 4 ? a : b)[u[k]] : u[k];
 #pragma unroll
           for (int k = 0; k < 8; ++k) u[k] = w[k] == u[k] ? w[k] | kRootFlag : w[k];
+        }
+        if (open) {
+          open = false;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) open |= root_at_limit(k < 4 ? a : b, u[k]) >= 0;
         }
         if (open || cap_j < 2) atomicOr(err, kErrJump);
 #pragma unroll
