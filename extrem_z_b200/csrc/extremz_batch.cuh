@@ -1810,7 +1810,8 @@ class BatchEngine {
     // scratch (ext_key) and the fill cursors (aff), so they go one after the
     // other.  Rows name only extrema, so a side with rows has extrema.  Without
     // join_rows the minima's side waits for the final join pass (k_join_*).
-    launch(K_SETUP, k_rows<T, true>, grid_, 256, J);
+    if (h(slot, C_NAN)) launch(K_SETUP, k_rows<T, true, true>, grid_, 256, J);
+    else launch(K_SETUP, k_rows<T, true>, grid_, 256, J);
     if (nmax) {
       EZ_RUN(scan_counts(J.moff2, nmax, 1, J.moff2 + nmax, chunk, J.aff));
       launch(K_OTHER, k_extreme_saddle<T, true>, grid_, 256, J);

@@ -890,6 +890,13 @@ __device__ __noinline__ void column_steps_any(const Tile<T>& s, int tx, int ty, 
   }
 }
 
+// Sets *nan when the tile holds a NaN.
+template <class T>
+__device__ __noinline__ void note_nans(const Tile<T>& s, int* nan) {
+  for (int i = threadIdx.x; i < SX * SY * SZ; i += 256)
+    if (isnan((&s.v[0][0][0])[i])) *nan = 1;
+}
+
 // Follows the tile's next positions from p, whose own is t, to the path's exit
 // from the tile or its root.
 __device__ __forceinline__ int follow(const int16_t* nxt, int p, int t, int* err) {
@@ -937,9 +944,7 @@ __device__ __noinline__ bool direction_tile(const Job<T>& J, Tile<T>& s, uint64_
     if (threadIdx.x == 0) atomicOr(J.ctr + C_ERROR, kErrTile);
     return false;
   }
-  if (!kDec && !usual)
-    for (int i = threadIdx.x; i < SX * SY * SZ; i += 256)
-      if (isnan((&s.v[0][0][0])[i])) J.ctr[C_NAN] = 1;
+  if (!kDec && !usual) note_nans(s, J.ctr + C_NAN);
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const int x = bx + tx, y = by + ty;
   // A tile off the field's faces has every direction valid at every voxel.
@@ -1769,7 +1774,9 @@ __global__ void __launch_bounds__(32 * kCpWarps) k_cp_write(const int8_t* __rest
 // issue of the per-entry work: 1.58 ms for the 22 M 2-saddles of the 512^3
 // benchmark field, 2.38 ms when it went over all 14 directions and compared
 // their values.
-template <class T, bool kAsc>
+// kNan: the field holds a NaN (a variant of its own: the look for one in every field
+// cost 4 %).
+template <class T, bool kAsc, bool kNan = false>
 __global__ void __launch_bounds__(256, 4) k_rows(Job<T> J) {
   __shared__ int off[kNumDirs];
   fill_offsets(off, J.dim);
@@ -1793,7 +1800,7 @@ __global__ void __launch_bounds__(256, 4) k_rows(Job<T> J) {
       side = (unsigned)valid_mask(boundary_code(x, y, z, g.W, g.H, g.D)) & ~side;
       // Next to a NaN a path may end at a vertex that is no maximum, whose index
       // in ext is 0 then: in a field without maxima no row names one.
-      if (J.ctr[C_NAN]) side = J.ctr[C_NMAX] ? drop_nans(a, off, s, side) : 0u;
+      if (kNan) side = J.ctr[C_NMAX] ? drop_nans(a, off, s, side) : 0u;
       J.smask2[i] = (uint16_t)side;
     }
     const int pmax = (int)__reduce_max_sync(0xffffffffu, __popc(side));
