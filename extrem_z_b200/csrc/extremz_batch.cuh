@@ -9,8 +9,9 @@
 // per kernel serves all jobs in that phase (kernels take the device array of
 // job descriptors and a selection), and a job moves on through phases whose
 // successor does not depend on a counter within the same tick.  At the end of
-// a tick the counter blocks of all jobs come back in one copy and every job
-// that stopped at a branch takes it, with the reference's rules.
+// a tick its last kernel publishes the counter blocks of all jobs to the host
+// (k_tick_end; a copy brings them where it cannot) and every job that stopped at a
+// branch takes it, with the reference's rules.
 //
 // The branches read exactly the counters the reference reads at the same
 // points, so a job's sequence of kernel launches, and its result, do not
@@ -749,9 +750,9 @@ class BatchEngine {
     for (auto& j : slots_) free_job(j);
   }
 
-  // One tick: every phase any job is in, in program order; then one copy of
-  // all counter blocks and the branches.  Returns a status (the jobs keep
-  // their own statuses).
+  // One tick: every phase any job is in, in program order; then all counter
+  // blocks and the branches.  Returns a status (the jobs keep their own
+  // statuses).
   int tick() {
     EZ_RUN(tick_issue());
     return tick_complete();
@@ -774,7 +775,9 @@ class BatchEngine {
     // one CUDA graph: recorded, captured the third time its signature is
     // seen, replayed from then on.  Ticks that allocate (setup) launch
     // directly.  Timed launches (EXTREMZ_FLAG_PROFILE) keep their events
-    // inside the graph, so profiling does not change how a tick launches.
+    // inside the graph; a tick with timed launches runs its branches one after the
+    // other, and a profiled correction's counters come by a copy, so that the times
+    // by class are not those of overlapped ticks.
     bool graph = graphs_on_;
     for (const auto& j : slots_)
       if (j.used && !j.waiting && j.pc == PC_SETUP_B) graph = false;
@@ -937,7 +940,7 @@ class BatchEngine {
   bool graphs_on_ = true, recording_ = false, capturing_ = false;
   std::string sig_;
   // A recorded launch and its branch: the phases of a tick work on different
-  // jobs, so those of different branches run side by side (kBranchOf), each
+  // jobs, so those of different branches run side by side (branch_of), each
   // branch on a stream of its own between a fork and a join; -1 comes after the
   // join.
   struct Launch {

@@ -182,7 +182,12 @@ __device__ __forceinline__ int mf_stamp(const int* ctr) { return ctr[C_WNSTAMP] 
 __device__ __forceinline__ unsigned mf_byte(int stamp) { return 1u + (unsigned)stamp % 255u; }
 // A light round's jump goes over the tiles that k_touched_tiles finds only in
 // fields of at least this many vertices: a pass over every vertex costs about
-// 2.2 us per million, the search some 35 us whatever the field.
+// 2.2 us per million, the search 50-100 us whatever the field.  Corrections of noisy
+// fields (512 Gaussians per 256^3 and noise, bound 1e-5) without the search and with
+// it: 3.90 and 4.04 ms at 272^3, 4.74 and 4.75 at 300^3, 6.66 and 6.58 at 340^3, 10.55
+// and 10.35 at 400^3, 21.3 and 20.1 at 512^3.  A smooth field, whose few labels lie in
+// more than a quarter of the tiles, pays the search for nothing (4.77 and 5.15 ms at
+// 400^3).
 constexpr int kTouchMin = 1 << 25;
 // Start of a round, in its first kernel (which uses none of these).
 __device__ __forceinline__ void mf_begin(int* ctr, int n) {
@@ -1020,7 +1025,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 6) k_direction(const
   }
   if (kDec ? J.tma_g : J.tma_f)
     tile_issue<T>(s, &bar, kDec ? &J.map_g : &J.map_f, bx, by, bz, true);
-  // The packed interior types (k_pack_types), while the tile is on its way.
+  // The packed interior types (pack_types, on the host), while the tile is on its way.
   __shared__ uint4 types[kDec ? 1 : kTypeWords / 4];
   if (!kDec) types[threadIdx.x] = reinterpret_cast<const uint4*>(J.tb.packed)[threadIdx.x];
   if (!direction_tile<T, kDec>(J, s, &bar, hnext, lnext, reinterpret_cast<const unsigned*>(types), bx,
@@ -1771,7 +1776,7 @@ __global__ void __launch_bounds__(32 * kCpWarps) k_cp_write(const int8_t* __rest
 // average and 8.2 in the fullest lane of a warp, so the passes below go over
 // set bits in groups of four, up to the warp's fullest lane, and no neighbour
 // value is read or compared.  Bound by the label and value gathers and by the
-// issue of the per-entry work: 1.58 ms for the 22 M 2-saddles of the 512^3
+// issue of the per-entry work: 1.34 ms for the 22 M 2-saddles of the 512^3
 // benchmark field, 2.38 ms when it went over all 14 directions and compared
 // their values.
 // kNan: the field holds a NaN (a variant of its own: the look for one in every field
@@ -2310,8 +2315,9 @@ __device__ __noinline__ unsigned side_of(const Job<T>& J, int s) {
 // saddle's neighbours on the side are the original field's (its type and
 // lower star matched): the direction mask is read instead of 14 neighbour
 // values.  Two thirds of the rounds, the first one (every saddle) among them,
-// run right after such a detection (with the 1-saddles' shortcut below: 7.0 ->
-// 5.7 ms per 512^3 correction).  The loop goes over the set bits kWide at
+// run right after such a detection (with the 1-saddles' shortcut below, the saddle
+// passes of a 512^3 correction went from 7.0 to 5.7 ms; with a kernel of its own for
+// the first round and packed queues for the later ones they take 3.1).  The loop goes over the set bits kWide at
 // a time, so that a group's gathers (labels and mismatch bits; the labels'
 // values) are in flight together.
 //

@@ -28,6 +28,8 @@ EXTREMZ_HD int queue_take(Q& q, unsigned stamp, int cap, int limit) {
   const int h = q.ticket();
   for (int spin = 0; spin <= limit; ++spin) {
     if (q.dense()) return -1;
+    // (A block sees an entry counted before it takes it, so that what it releases
+    // with finished() counts the entry: its stamp alone would not do.)
     if (q.pushed() > h && h < cap) {  // the entry may still be on its way
       const unsigned long long e = q.entry(h);
       if ((unsigned)(e >> 32) == stamp) return (int)(unsigned)e;
@@ -36,8 +38,7 @@ EXTREMZ_HD int queue_take(Q& q, unsigned stamp, int cap, int limit) {
       // acquire order, so that `pushed` counts all that the finished blocks pushed.
       // An older `pushed` could equal a newer `done` while entries are open; the
       // block would leave with the ticket of one, and the last block to push would
-      // wait for that one up to the limit.  (Only here: on every look at the queue
-      // the acquire cost the search 12 % at 512^3.)
+      // wait for that one up to the limit.
       const int done = q.done();
       if (done == q.pushed()) return -1;
     }

@@ -14,6 +14,8 @@
  *     s_loops, saddle_loops).
  * Buffers are caller-owned plain pointers; no C++ or torch types cross this
  * boundary.  Every entry point returns a status code instead of exiting.
+ * Field values may be infinite.  A NaN compares as nothing: it is on neither side
+ * of a saddle, and results next to one are otherwise unspecified.
  */
 #ifndef EXTREMZ_H
 #define EXTREMZ_H
@@ -252,7 +254,10 @@ extremz_status extremz_correct_encode(extremz_ctx* ctx, const void* d_orig, void
  * steepest-ascent (d_ds, the maximum a vertex ascends to) and steepest-descent
  * (d_as, the minimum) paths of every vertex, into caller device buffers of
  * width*height*depth entries (any of the three may be NULL).  Ties are broken
- * by vertex id.  Synchronises the stream.
+ * by vertex id.  Synchronises the stream.  The results are computed in the
+ * caller's buffers where that is possible, so a call that fails on the device
+ * (EXTREMZ_DEVICE_TIMEOUT, EXTREMZ_CUDA_ERR) leaves them unspecified: labels may
+ * be unfinished, negative ones among them.
  * Replaces: classifyVertex_CUDA (src/ExtreM_cuda.cu:3720-3911) and
  * ComputeDirection + ComputeDescendingManifold / ComputeAscendingManifold
  * (:1464-1611), which the host API exposes as classifyAllVertices and
